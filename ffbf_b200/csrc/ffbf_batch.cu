@@ -76,7 +76,7 @@ ffbf_status build_plan(const std::vector<PlanJob>& jobs, int num_sms, ScanPlan& 
         uint64_t covered = 0;
         if (use_fast(c, a.n)) {
             TRY(prepare_fast(c));
-            const ffbf::FastConfig cfg = c->cfg;
+            const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, a.n, num_sms, true);
             const int threads = ffbf::config_threads(cfg);
             // in a batch other jobs fill the GPU, so rows per stream follow this job's size alone
             const uint32_t rows = cfg.rows ? cfg.rows : ffbf::fast_rows(a.n, cfg, num_sms, true);
@@ -417,12 +417,10 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
     uint32_t* saved = nullptr;
     TRY(dalloc_t(c, &saved, c->filter_bytes / 4));
     CUDA_TRY(c, cudaMemcpyAsync(saved, c->d_ff, c->filter_bytes, cudaMemcpyDeviceToDevice, c->st));
-    // shared-memory mode at three CTA sizes with candidates queued per byte (512 also with per-stage
-    // barriers) and at two with candidates deferred to the end of each block, dense mode at three (its probe
-    // order follows the filter's fills; 192 runs two CTAs per SM, and probe order 2 runs 192 as 384)
-    const ffbf::FastConfig cands[] = {{512, 0, 0, 0}, {512, 3, 0, 0}, {384, 0, 0, 0}, {256, 0, 0, 0},
-                                      {256, 2, 0, 0}, {192, 2, 0, 0}, {384, 1, 0, 0}, {192, 1, 0, 0},
-                                      {256, 1, 0, 0}};
+    // shared-memory mode at four CTA sizes (smaller ones have larger tables), dense mode at three (its probe
+    // order follows the filter's fills; 192 runs two CTAs per SM, and probe orders 2 and 3 run 192 as 384)
+    const ffbf::FastConfig cands[] = {{512, 3, 0, 0}, {384, 0, 0, 0}, {256, 0, 0, 0}, {192, 2, 0, 0},
+                                      {384, 1, 0, 0}, {192, 1, 0, 0}, {256, 1, 0, 0}};
     ffbf::FastConfig best = c->cfg;
     double best_score = 1e300;
     cudaEvent_t e0, e1;
@@ -448,9 +446,10 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
         if (s != FFBF_OK) break;
         double score = ms;
         if (per_sm) {
-            const int t = ffbf::config_threads(cand);
+            const ffbf::FastConfig run = ffbf::launch_config(cand, sample_len, c->num_sms, false);
+            const int t = ffbf::config_threads(run);
             const uint64_t bytes = sample_len / ffbf::kScanTile * ffbf::kScanTile;
-            const uint64_t streams = bytes / ((uint64_t)ffbf::fast_rows(sample_len, cand, c->num_sms, false) * 128);
+            const uint64_t streams = bytes / ((uint64_t)ffbf::fast_rows(sample_len, run, c->num_sms, false) * 128);
             const uint64_t items = (streams + t - 1) / t;
             score = ms * (double)std::min<uint64_t>(items, (uint64_t)c->num_sms);
         }

@@ -174,24 +174,21 @@ void reset_scan(ffbf_ctx* c) {
 
 const uint64_t kInitialHitsCap = 1u << 16;
 
-// Builds the stage-1 table for a CTA size and layout (the sparse mode's, or the dense mode's prefilter, which
-// has the room the dense kernel leaves) unless the table on the device already is that one.
-ffbf_status ensure_stage1(ffbf_ctx* c, int threads, bool dense, bool force) {
-    if (!force && c->d_stage1 && c->stage1_threads == threads && c->stage1_dense == dense) return FFBF_OK;
-    const uint32_t nw = ffbf::stage1_words_for(c->g, threads, dense);
+// Builds the stage-1 table for a CTA size unless the table on the device already is that one.
+ffbf_status ensure_stage1(ffbf_ctx* c, int threads, bool force) {
+    if (!force && c->d_stage1 && c->stage1_threads == threads) return FFBF_OK;
+    const uint32_t nw = ffbf::stage1_words_for(c->g, threads);
     if (c->d_stage1 && c->stage1_words != nw) dfree(c, c->d_stage1);
     if (!c->d_stage1) TRY(dalloc_t(c, &c->d_stage1, nw));
     c->stage1_words = nw;
     c->stage1_threads = threads;
-    c->stage1_dense = dense;
-    CUDA_TRY(c, ffbf::build_stage1(c->d_main, c->g, threads, dense, c->d_stage1, c->st));
+    CUDA_TRY(c, ffbf::build_stage1(c->d_main, c->g, threads, c->d_stage1, c->st));
     return FFBF_OK;
 }
 
 // Makes the tuned scan ready for this context's filter: the stage-1 table the configured kernel reads and,
-// unless the autotuner or the environment fixed them, the probe mode (from the sparse table's fill: the
-// shared-memory stage only pays while it rejects most windows) and the dense mode's probe order (from the
-// fills of the filter's regions).
+// unless the autotuner or the environment fixed them, the probe mode and the dense mode's probe order (from the
+// fills of the stage-1 table and of the filter's regions).
 ffbf_status prepare_fast(ffbf_ctx* c) {
     if (!c->d_popc) TRY(dalloc_t(c, &c->d_popc, 3));
     if (!c->h_job) {
@@ -204,9 +201,7 @@ ffbf_status prepare_fast(ffbf_ctx* c) {
     if (!c->d_job) TRY(dalloc_t(c, &c->d_job, 1));
     if (c->borrowed) return FFBF_OK;  // the filter's owner built the table and chose the configuration
     if (c->stage1_dirty || !c->d_stage1) {
-        // measured on the sparse table of the configured CTA size (512 while the mode is open)
-        const int tm = c->cfg.mode != 1 ? ffbf::config_threads(c->cfg) : 512;
-        TRY(ensure_stage1(c, tm, false, true));
+        TRY(ensure_stage1(c, 512, true));  // measured on the 512-thread table
         CUDA_TRY(c, ffbf::popcount_words(c->d_stage1, c->stage1_words, c->d_popc, c->st));
         const uint32_t cw = c->g.cache_bits / 32, ew = (uint32_t)(((uint64_t)c->g.ext_mask + 1) / 32);
         CUDA_TRY(c, ffbf::popcount_words(c->d_main, cw, c->d_popc + 1, c->st));
@@ -215,28 +210,26 @@ ffbf_status prepare_fast(ffbf_ctx* c) {
         CUDA_TRY(c, cudaMemcpyAsync(ones, c->d_popc, sizeof ones, cudaMemcpyDeviceToHost, c->st));
         TRY(sync(c));
         c->stage1_fill = (double)ones[0] / (32.0 * c->stage1_words);
-        c->probe_order = ffbf::dense_probe_order(c->g, (double)ones[1] / (32.0 * cw), (double)ones[2] / (32.0 * ew));
+        const ffbf::ScanChoice best = ffbf::choose_scan(c->g, c->stage1_fill, (double)ones[1] / (32.0 * cw),
+                                                        (double)ones[2] / (32.0 * ew));
+        c->probe_order = best.order;
         if (!c->cfg_tuned) {
-            // the shared-memory stage passes about fill^2 of the windows (fill with S = 1); below 1 % the
-            // warps rarely queue candidates and run apart through per-stage barriers (mode 3)
-            const double pass = c->g.s > 1 ? c->stage1_fill * c->stage1_fill : c->stage1_fill;
-            c->cfg.mode = c->force_mode >= 0 ? c->force_mode : c->stage1_fill > 0.3 ? 1 : pass < 0.01 ? 3 : 0;
+            c->cfg.mode = c->force_mode >= 0 ? c->force_mode : best.mode;
             // default CTA sizes (measured best on the 10k- and 1M-pattern workloads): 512 threads for the
-            // shared-memory stage, 2 x 192 per SM for dense filters
-            // (dense: two 192-thread CTAs per SM; probe order 2 needs the 384-thread CTA's room for its table)
+            // shared-memory stage (768 for large texts), 2 x 192 per SM for dense filters, 384 with their prefilter
             c->cfg.threads = c->threads_env ? c->threads_env : c->cfg.mode == 1 ? 192 : c->cfg.mode == 2 ? 256 : 512;
         }
         c->stage1_dirty = false;
     }
     if (c->force_mode >= 0) c->cfg.mode = c->force_mode;
-    // the dense mode pipelines two probes of distinct index functions: with K = 1 only the sparse mode applies
+    // the dense mode probes distinct index functions: with K = 1 only the sparse mode applies
     if (c->g.k < 2 && c->cfg.mode == 1) c->cfg.mode = 0;
-    // the dense mode's probe order is the filter's, unless the environment fixes it
+    // the dense mode's probe order is the filter's, unless the environment fixes it (orders 1 and 3 need f2 and f3)
     c->cfg.order = c->force_order >= 0 ? c->force_order : c->probe_order;
-    if (c->g.k < 4 && c->cfg.order == 1) c->cfg.order = 0;  // order 1 probes f2 and f3 first
+    if (c->g.k < 4 && c->cfg.order == 1) c->cfg.order = 0;
+    if (c->g.k >= 4 && c->cfg.order == 2) c->cfg.order = 3;
     // the table the configured kernel reads (a dense kernel without prefilter reads none)
-    if (c->cfg.mode != 1) TRY(ensure_stage1(c, ffbf::config_threads(c->cfg), false, false));
-    else if (c->cfg.order == 2) TRY(ensure_stage1(c, ffbf::config_threads(c->cfg), true, false));
+    if (c->cfg.mode != 1 || c->cfg.order >= 2) TRY(ensure_stage1(c, ffbf::config_threads(c->cfg), false));
     return FFBF_OK;
 }
 
@@ -449,7 +442,6 @@ void attach_filters(ffbf_ctx* slot, const ffbf_ctx* owner) {
     slot->d_ff = owner->d_ff;
     slot->d_stage1 = owner->d_stage1;
     slot->stage1_threads = owner->stage1_threads;
-    slot->stage1_dense = owner->stage1_dense;
     slot->stage1_words = owner->stage1_words;
     slot->stage1_fill = owner->stage1_fill;
     slot->stage1_dirty = false;
@@ -801,12 +793,13 @@ ffbf_status scan_host_pipelined(ffbf_ctx* c, const uint8_t* text, size_t len) {
     TRY(prepare_fast(c));
     c->scan_path = 1;
     const ffbf::ScanArgs a = make_scan_args(c);
-    const int threads = ffbf::config_threads(c->cfg);
     const uint64_t chunk = pipe_chunk(len);
-    const uint32_t rows = c->cfg.rows ? c->cfg.rows : ffbf::fast_rows(chunk, c->cfg, c->num_sms, false);
+    const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, chunk, c->num_sms, false);
+    const int threads = ffbf::config_threads(cfg);
+    const uint32_t rows = cfg.rows ? cfg.rows : ffbf::fast_rows(chunk, cfg, c->num_sms, false);
     ffbf::FastJob job;
     cudaError_t e;
-    const uint64_t covered = ffbf::fill_fast_job(a, c->d_stage1, c->cfg, rows, &job, &e);
+    const uint64_t covered = ffbf::fill_fast_job(a, c->d_stage1, cfg, rows, &job, &e);
     if (e != cudaSuccess) return fail(c, FFBF_ECUDA, "tensor map encoding failed");
     const uint64_t item_bytes = (uint64_t)threads * rows * 128;
     const uint32_t per_chunk = (uint32_t)std::max<uint64_t>(1, chunk / item_bytes);
@@ -854,7 +847,7 @@ ffbf_status scan_host_pipelined(ffbf_ctx* c, const uint8_t* text, size_t len) {
         CUDA_TRY(c, cudaEventRecord(c->pipe_events[i], c->st_copy));
         CUDA_TRY(c, cudaStreamWaitEvent(c->st, c->pipe_events[i], 0));
         CUDA_TRY(c, cudaMemsetAsync(c->d_counters + ffbf::CNT_QUEUE, 0, sizeof(uint32_t), c->st));
-        CUDA_TRY(c, ffbf::launch_fast_jobs(c->g.len, c->cfg, c->d_jobs + i, 1, count, job.stage1_nwords,
+        CUDA_TRY(c, ffbf::launch_fast_jobs(c->g.len, cfg, c->d_jobs + i, 1, count, job.stage1_nwords,
                                            c->d_counters + ffbf::CNT_ERROR, c->num_sms, c->st));
     }
     if (copied < len) {
@@ -1286,7 +1279,7 @@ ffbf_status ffbf_get_scan_config(const ffbf_ctx* c, int* threads, int* mode) {
 
 ffbf_status ffbf_get_probe_order(const ffbf_ctx* c, int* order) {
     if (!c || !order) return FFBF_EINVAL;
-    *order = c->cfg.order;
+    *order = c->cfg.order == 3 ? 2 : c->cfg.order;
     return FFBF_OK;
 }
 

@@ -1,30 +1,39 @@
 // ffbf_scan_fast.cu -- the tuned sm_100a scan of processFile (src/rabin-karp/ffbf.cpp:310-392).
 //
 // Work decomposition. The text is cut into streams of SLEN = rows * 128 bytes. A CTA of THREADS threads
-// owns THREADS consecutive streams (a "supertile") at a time, one stream per thread, and walks them row by
-// row. Each thread rolls the hash over its stream without restarting, so the LEN-byte warm-up is paid once
+// owns THREADS consecutive streams (a "supertile") at a time, one stream per thread, and walks them in parts of 64
+// bytes. Each thread rolls the hash over its stream without restarting, so the LEN-byte warm-up is paid once
 // per stream (from a 32-byte halo) instead of once per tile.
 //
-// Staging. Row r of the CTA's streams is loaded by TMA as 3-D boxes {128 bytes, 1 row, <=256 streams}
-// (cp.async.bulk.tensor, 128B swizzle, one CTA per load) into a double-buffered shared-memory stage completed on
-// an mbarrier. The 128B swizzle puts chunk c of thread t's row at chunk c ^ (t & 7), so the 16-byte reads
-// of a quarter-warp hit eight different bank groups.
+// Staging. Part p of the CTA's streams is loaded by TMA as 3-D boxes {64 bytes, 1 row, <=256 streams}
+// (cp.async.bulk.tensor, 64B swizzle, one CTA per load) into one of two shared-memory stages. A "full" mbarrier
+// completes when the load lands, an "empty" one when every warp has left the stage, so warps run up to a stage
+// apart. The swizzle XORs a 16-byte chunk's index with bits of its thread's number, so the 16-byte reads of a
+// quarter-warp hit eight different bank groups.
 //
 // Hash. h <- rol64(h,1) ^ S[in] ^ rol64(S[out], LEN) (hash_rot_sbox_pre_2.h:42-51 with the ring folded into
 // the outgoing byte, still in registers), on two 32-bit halves. S sits in shared memory as 16 interleaved
-// copies of 8-byte entries, so the 16 lanes of each half-warp read disjoint banks whatever their bytes. Bytes
-// with the high bit set index entries that hold S[0] (ffbf.cpp:127-130).
+// copies of 8-byte entries, so the 16 lanes of each half-warp read disjoint banks whatever their bytes, and a byte's
+// entry address is one byte-wise dot product (dp4a) of the text word, off the ALU pipe that the rest of the hash
+// fills. Bytes with the high bit set hash as byte 0 (ffbf.cpp:127-130).
 //
-// Probes. Stage 1 tests the first index function, h1 & (C-1), against a shared-memory table: the cache
-// region itself when it fits, else its OR-summary (bit j = OR of cache bits [j<<sh, (j+1)<<sh)), which only
-// rejects windows the full test rejects. A window that passes (and holds no '\n') is appended to its warp's
-// candidate queue in shared memory; full queues and row ends are flushed by the whole warp, each lane taking
-// queued candidates and running the full K-bit test on the global filter in the reference order
-// (checkInFilter, ffbf.cpp:214-239). The queue keeps the per-byte path free of branches that wait on L2.
+// Probes. Sparse filters test the first two index functions against a shared-memory table: the cache region itself
+// when it fits, else its fold (bit j = OR of the cache bits i with i mod T == j), which only rejects windows the full
+// test rejects. Dense filters probe the global filter, in L2, through register rings. Surviving windows are
+// queued by position per warp; a full queue, or the stream's end, is flushed by the whole warp, each lane hashing
+// its queued windows again and running the full K-bit test on the global filter in the reference order (checkInFilter,
+// ffbf.cpp:214-239).
 //
-// Validity. A window is tested only when its LEN bytes hold no '\n' (processFile resets the hash at '\n').
-// The last '\n' is tracked per thread; each stream's first and last '\n' feed the per-16 KiB-tile newline
-// summaries the line resolver reads.
+// Validity. A window is tested only when its LEN bytes hold no '\n' (processFile resets the hash at '\n'), from a
+// newline mask per 32-byte block. Each stream's first and last '\n' feed the per-16 KiB-tile newline summaries the
+// line resolver reads.
+//
+// What bounds it. Sparse: the shared-memory pipe (9 wavefronts per warp and byte: 4 for the two S-box entries, 3.5
+// for the first table probe's random words, the rest for the predicated second probe and the text) and the ALU pipe,
+// at 24 warps per SM. Dense: the L1TEX unit, which looks up one random sector per clock and SM (words, 1M patterns: 0.93
+// of that). On one B200, before -> now, GB/s of text: 10k patterns, 4 GiB 662 -> 931; LEN 24, 8k patterns in 2^20 + 2^24
+// bits, 2 GiB 487 -> 879 and 40k in 2^22 + 2^26 299 -> 623; 150k in 2^23 + 2^27, 256 MiB 295 -> 511; words, 1M
+// patterns 311 -> 354; 4M 16-byte signatures 245 -> 271.
 //
 // Every mbarrier wait is bounded; on timeout the CTA records an error flag and stops.
 #include <cuda.h>
@@ -45,7 +54,6 @@ namespace {
 constexpr int kRowBytes = 128;
 constexpr int kTabBytes = 256 * 16 * 8;  // 16 copies of the 256-entry S-box
 constexpr int kQueueCap = 64;            // candidates per warp queue
-constexpr int kQueueBytes = kQueueCap * 16;
 constexpr uint32_t kWaitLimit = 1u << 24;
 constexpr size_t kSmemLimit = 232448;    // opt-in shared memory per block on sm_100
 
@@ -121,6 +129,21 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     return v;
 }
 
+// The same load for memory that changes between reads.
+__device__ __forceinline__ uint32_t lds32_volatile(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+// The same load where `pred` holds; 0 elsewhere.
+__device__ __forceinline__ uint32_t lds32_if(uint32_t addr, bool pred) {
+    uint32_t v;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.u32 %0, 0;\n\t@q ld.shared.u32 %0, [%1];\n\t}"
+        : "=r"(v)
+        : "r"(addr), "r"((uint32_t)pred));
+    return v;
+}
+
 // Global load of one filter word when `pred` holds (0 otherwise); read-only path.
 __device__ __forceinline__ uint32_t ldg_if(const uint32_t* p, bool pred) {
     uint32_t v;
@@ -130,22 +153,16 @@ __device__ __forceinline__ uint32_t ldg_if(const uint32_t* p, bool pred) {
     return v;
 }
 
-// byte i (0..3) of w, zero-extended
-__device__ __forceinline__ uint32_t byte_at(uint32_t w, int i) { return __byte_perm(w, 0u, 0x4440u + (uint32_t)i); }
+// base + 128 * byte i (0..3) of w: the address of a byte's S-box entry in one byte-wise dot product, which runs
+// beside the ALU pipe that bounds the hash
+__device__ __forceinline__ uint32_t entry_addr(uint32_t w, int i, uint32_t base) {
+    return __dp4a(w, 128u << (8 * i), base);
+}
 
-// rol64 of (hi:lo) by N, 0 < N < 64, on 32-bit halves
-template <int N>
-__device__ __forceinline__ void rol_pair(uint32_t lo, uint32_t hi, uint32_t& rlo, uint32_t& rhi) {
-    if constexpr (N == 32) {
-        rlo = hi;
-        rhi = lo;
-    } else if constexpr (N < 32) {
-        rlo = __funnelshift_l(hi, lo, N);
-        rhi = __funnelshift_l(lo, hi, N);
-    } else {
-        rlo = __funnelshift_l(lo, hi, N - 32);
-        rhi = __funnelshift_l(hi, lo, N - 32);
-    }
+// Zeroes the bytes of w that have their high bit set: they hash as byte 0 (ffbf.cpp:127-130).
+__device__ __forceinline__ uint32_t clear_high_bytes(uint32_t w) {
+    const uint32_t hb = w & 0x80808080u;
+    return w & ~((hb >> 7) * 255u);
 }
 
 // rol32 by a compile-time amount (0: identity)
@@ -165,83 +182,57 @@ __device__ __forceinline__ bool full_check_from(const Geom& g, const uint32_t* _
     return true;
 }
 
-// The whole warp drains its candidate queue: lane i takes entries i, i+32, ... (PER_LANE at most). An entry
-// is {position | lane << 8, h1, h2, first}: probes before `first` are known to be set. Every lane issues the
-// probe `first` of all its entries before testing any, so its L2 round trips overlap; survivors finish the
-// test one by one.
-template <int PER_LANE>
-__device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int qn, uint64_t warp_row_pos0,
-                                         uint64_t row_stride, int lane) {
+// The whole warp drains its candidate queue: lane i takes entries i, i + 32, ... (PER_LANE at most). An entry is a
+// window's end, {position in the stream | lane << 16}. Each lane reads its windows' bytes back from the text (still in
+// L2), hashes them and runs the full K-bit test: few windows get here, so this costs less than carrying every
+// window's hash to its test in the byte loop. All of a lane's loads of one kind are issued before any is used.
+template <int L, int PER_LANE>
+__device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int qn, uint64_t warp_pos0, uint64_t stride,
+                                         int lane, uint32_t lane_tab) {
     // the job's fields are read here rather than passed: the caller's loop keeps only its hot values live
     const Geom g = J->g;
     const uint32_t* __restrict__ main_words = J->main_words;
-    uint32_t* ff_words = J->ff_words;
-    HitRec* hits = J->hits;
-    const uint32_t hits_cap = J->hits_cap;
-    uint32_t* counters = J->counters;
-    uint4 e[PER_LANE];
+    const uint8_t* __restrict__ text = J->text;
+    constexpr int kWords = (L + 3) / 4;
+    uint64_t start[PER_LANE], h[PER_LANE];
     uint32_t v[PER_LANE], bi[PER_LANE];
 #pragma unroll
     for (int t = 0; t < PER_LANE; t++) {
         const int i = lane + 32 * t;
-        e[t] = make_uint4(0, 0, 0, 0);
-        v[t] = 0xffffffffu;
-        bi[t] = 0;
-        if (i < qn) {
-            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(e[t].x), "=r"(e[t].y), "=r"(e[t].z), "=r"(e[t].w)
-                         : "r"(qaddr + 16u * (uint32_t)i));
-            if (e[t].w < g.k) {
-                const uint64_t h = ((uint64_t)e[t].z << 32) | e[t].y;
-                bi[t] = bit_index<1>(g, h, e[t].w);
-                v[t] = __ldg(main_words + (bi[t] >> 5));
-            }
+        v[t] = bi[t] = 0;
+        if (i >= qn) continue;
+        const uint32_t e = lds32_volatile(qaddr + 4u * (uint32_t)i);
+        start[t] = warp_pos0 + (e >> 16) * stride + (e & 0xFFFFu) + 1 - L;
+        // the aligned words that hold the window's bytes, and no others
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(text + (start[t] & ~3ull));
+        const uint32_t off = (uint32_t)start[t] & 3u;
+        uint32_t w[kWords + 1];
+#pragma unroll
+        for (int q = 0; q <= kWords; q++) w[q] = 4u * q < off + L ? __ldg(src + q) : 0u;
+        uint32_t hl = 0, hh = 0;
+#pragma unroll
+        for (int j = 0; j < L; j++) {
+            const uint32_t c = clear_high_bytes(__funnelshift_r(w[j / 4], w[j / 4 + 1], 8 * off));
+            const uint2 sv = lds64(entry_addr(c, j & 3, lane_tab));
+            const uint32_t nl = __funnelshift_l(hh, hl, 1) ^ sv.x, nh = __funnelshift_l(hl, hh, 1) ^ sv.y;
+            hl = nl;
+            hh = nh;
         }
+        h[t] = ((uint64_t)hh << 32) | hl;
+        bi[t] = bit_index<1>(g, h[t], 0);
+        v[t] = __ldg(main_words + (bi[t] >> 5));
     }
 #pragma unroll
     for (int t = 0; t < PER_LANE; t++) {
-        const int i = lane + 32 * t;
-        if (i >= qn) continue;
-        const uint64_t h = ((uint64_t)e[t].z << 32) | e[t].y;
         if (!((v[t] >> (bi[t] & 31)) & 1u)) continue;
-        if (!full_check_from(g, main_words, h, e[t].w + 1)) continue;
-        // p = window end + 128 relative to the owner's current row (the dense rings carry the previous row's
-        // last windows into the next row)
-        const uint32_t owner = e[t].x >> 8, p = e[t].x & 0xFFu;
-        if (owner >= 32) {
-            atomicOr(counters + CNT_ERROR, 0x400u);
-            continue;
-        }
-        const uint64_t start = warp_row_pos0 + owner * row_stride + p + 1 - g.len - kRowBytes;
-        set_all<2>(g, ff_words, h);
-        const uint32_t slot = atomicAdd(counters + CNT_HITS, 1u);
-        if (slot < hits_cap) hits[slot] = HitRec{start, h};
+        if (!full_check_from(g, main_words, h[t], 1)) continue;
+        set_all<2>(g, J->ff_words, h[t]);
+        const uint32_t slot = atomicAdd(J->counters + CNT_HITS, 1u);
+        if (slot < J->hits_cap) J->hits[slot] = HitRec{start[t], h[t]};
     }
     __syncwarp();
 }
 
-// Work items. Job j owns items [item_begin_j, item_begin_{j+1}), one per supertile of THREADS streams; CTA b
-// takes items b, b + gridDim.x, ... Each item is one TMA load of the streams' halo rows followed by `rows`
-// row loads. Thread 0 issues load k+1 while the CTA consumes load k and records in meta[] which job, item
-// and row each buffer holds.
-//
-// MODE 0 (sparse filters): stage 1 in shared memory, candidates queued per byte.
-// MODE 1 (dense filters, where a shared-memory table would pass most windows): the exact probes of the
-// first two index functions are global loads issued per valid window and consumed kRing bytes later from
-// register rings, so L2 latency overlaps the hashing of the next windows; only windows whose two probed bits
-// are set go to the queue.
-// MODE 2: MODE 1 with the pipelined probes on index functions f2 = rot16(h1) and f3 = rot16(h2) (the
-// external region for S <= 2, usually much sparser than the cache region, so fewer windows need a second
-// probe); queued windows then run the whole K-bit test.
-// MODE 3: MODE 1 with a shared-memory prefilter: the f0 load is issued only for windows whose bit in the
-// folded cache region (the stage-1 table, sized for the room this kernel leaves) is set, so filters whose
-// fold still rejects many windows issue that many fewer L2 probes.
-// MODE 4 (sparse filters, deferred): MODE 0's two shared-memory probes, but the byte loop only shifts each
-// window's pass bit into a 32-bit register mask; it carries no newline test and no warp vote, so a 32-byte
-// block is one branch-free stretch of code. After the block, the block's newline mask (SWAR) gives each
-// window's validity, and only when a lane of the warp holds a valid passing window is the hash of its 8-byte
-// segment recomputed from a checkpoint, this time queueing the candidates as MODE 0 does. It pays where the
-// stage-1 table rejects nearly every window (a large table: fewer threads per CTA).
 template <int N>
 __device__ __forceinline__ void shl64_or(uint32_t& lo, uint32_t& hi) {
     // (hi:lo) |= (hi:lo) << N, 0 < N < 32
@@ -282,103 +273,131 @@ __device__ __forceinline__ uint32_t window_has_newline(uint32_t prev, uint32_t c
     return rhi;
 }
 
-// Newline mask of 4 text bytes: bit k set when byte k of w is '\n' (exact per byte).
-__device__ __forceinline__ uint32_t newline_bits4(uint32_t w) {
-    const uint32_t t = w ^ 0x0A0A0A0Au;
-    const uint32_t zb = ~(((t & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | t) & 0x80808080u;
-    return (zb * 0x00204081u) >> 28;  // bits 7, 15, 23, 31 -> 28..31, without carries
-}
-
+// Newline mask of a block's 32 bytes: bit i set when byte i is '\n' (exact). Each word's zero-byte mask keeps
+// its high bits (0x80 per '\n'); byte-wise dot products with weights 1, 2, 4, 8 (and 16, 32, 64, 128 for the
+// next word) gather two words' eight bits into bits 7..14 without shifts.
 __device__ __forceinline__ uint32_t newline_mask32(const uint32_t (&w)[8]) {
-    uint32_t m = 0;
+    uint32_t f[4];
 #pragma unroll
-    for (int q = 0; q < 8; q++) m |= newline_bits4(w[q]) << (4 * q);
-    return m;
+    for (int q = 0; q < 8; q++) {
+        const uint32_t z = ((w[q] ^ 0x0A0A0A0Au) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu;
+        const uint32_t zb = ~(z | w[q]) & 0x80808080u;
+        f[q >> 1] = __dp4a(zb, (q & 1) ? 0x80402010u : 0x08040201u, (q & 1) ? f[q >> 1] : 0u);
+    }
+    return ((f[0] + (f[1] << 8)) >> 7) | ((f[2] + (f[3] << 8)) << 9);
 }
 
-// CTAs per SM: the dense modes at 192 threads run two CTAs per SM (12 warps, as one 384-thread CTA, but two
-// independent pipelines and barriers of 6 warps each); every other configuration runs one.
-__host__ __device__ constexpr int ctas_per_sm(int threads, int mode) { return threads == 192 && mode >= 1 && mode <= 3 ? 2 : 1; }
-// MODE 5 is MODE 0 whose warps meet through per-stage barriers instead of a block barrier per stage
-__host__ __device__ constexpr bool sparse_mode(int mode) { return mode == 0 || mode == 5; }
+// Kernel modes.
+// MODE 0 (sparse filters): both first index functions are tested against a shared-memory table, the cache region
+// itself when it fits, else its fold, which only rejects windows the full test rejects.
+// MODE 1 (dense filters, where a shared-memory table would pass most windows): the exact probes of the first two
+// index functions are global loads, the first issued per valid window, the second for the windows that pass it;
+// both are consumed kRing bytes later from register rings, so L2 latency overlaps the hashing of the next windows.
+// MODE 2: MODE 1 with the pipelined probes on index functions f2 = rot16(h1) and f3 = rot16(h2) (the
+// external region for S <= 2, usually much sparser than the cache region, so fewer windows need a second probe).
+// MODE 3: a window's f0 and f1 are tested against the shared-memory table as in MODE 0, and for the windows that
+// pass, one exact probe of f0 is pipelined as in MODE 1; MODE 4 pipelines f2 instead. They suit filters whose table
+// passes too many windows for MODE 0's queue (above about 2 %) but still rejects most.
+//
+// In every mode the byte loop over a 32-byte block is one branch-free stretch: a window's verdict is shifted into a
+// 32-bit register mask, and only after the block do the lanes with surviving windows queue their positions. Against
+// a warp vote and a queue append per byte this took the sparse scan of a 4 GiB text from 662 to 749 GB/s.
+__host__ __device__ constexpr bool sparse_mode(int mode) { return mode == 0; }
 
+// CTAs per SM: dense modes 1 and 2 at 192 threads run two CTAs per SM (12 warps, as one 384-thread CTA, but two
+// independent pipelines); every other configuration runs one.
+__host__ __device__ constexpr int ctas_per_sm(int threads, int mode) {
+    return threads == 192 && (mode == 1 || mode == 2) ? 2 : 1;
+}
+// Bytes of each stream that a stage holds. Half a row leaves shared memory for a stage-1 table of twice the size
+// (prefiltered dense scan of 150k patterns: 343 -> 406 GB/s) and more often lets a warp leave a stage (dense scan of
+// 1M patterns: 343 -> 353 GB/s).
+constexpr int kPart = 64;
+constexpr int kParts = kRowBytes / kPart;
+// Streams per TMA box (<= 256), a divisor of the CTA's threads.
+__host__ __device__ constexpr int box_streams_for(int threads) {
+    return threads <= 256 ? threads : threads <= 512 ? threads / 2 : threads % 3 == 0 ? threads / 3 : threads / 4;
+}
+
+// Work items. Job j owns items [item_begin_j, item_begin_{j+1}), one per supertile of THREADS streams; CTA b starts
+// with item b and takes the next ones from the work queue. Each item is one TMA load of the last part of the
+// streams before (the halo) followed by the loads of its streams' parts. Thread 0 issues load k+1 while the CTA
+// consumes load k and records in meta[] which job, item and part each stage holds.
 template <int L, int THREADS, int MODE>
 __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fast(const FastJob* __restrict__ jobs, uint32_t n_jobs,
                                                           uint32_t n_items, uint32_t max_s1_words,
                                                           uint32_t* __restrict__ ctl) {
     // ctl[0]: error flags; ctl[1]: the work queue, the count of items handed out past the first wave
     uint32_t* const error_flag = ctl;
-    constexpr int kStageBytes = THREADS * kRowBytes;
-    constexpr int kQCap = (sparse_mode(MODE) || MODE == 4) ? kQueueCap : 2 * kQueueCap;
-    constexpr int kQBytes = kQCap * 16;
-    // dense mode: ring depth per stage (divides 32); 384-thread CTAs trade depth for warps (more L2 probes
+    constexpr int kStageBytes = THREADS * kPart;
+    // dense modes: ring depth per probe (divides 32); 384-thread CTAs trade depth for warps (more L2 probes
     // in flight per SM within the register file)
     constexpr int kRing = THREADS >= 384 || ctas_per_sm(THREADS, MODE) == 2 ? 4 : 8;
-    constexpr int kBox = THREADS > 256 ? THREADS / 2 : THREADS;  // streams per TMA box (<= 256)
-    constexpr bool kTable = sparse_mode(MODE) || MODE == 3 || MODE == 4;  // reads the stage-1 table
+    constexpr int kBox = box_streams_for(THREADS);
     constexpr bool kSparse = sparse_mode(MODE);
+    constexpr bool kPre = MODE == 3 || MODE == 4;  // dense with the shared-memory prefilter and one pipelined probe
+    constexpr int kLag = kPre ? kRing : 2 * kRing;  // bytes from a window's first probe to its verdict
+    constexpr bool kTable = kSparse || kPre;  // reads the stage-1 table
+    // S-box layout: 16 bank-private copies of S[0..127] and of rol64(S[0..127], LEN), so the byte that leaves the
+    // window needs no rotation; a block's high bytes are cleared beforehand (they hash as byte 0). With LEN = 32
+    // the rotation only swaps the halves, and the table holds all 256 bytes once.
+    constexpr bool kTwoTables = L != 32;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
-    // layout: [stage 0][stage 1][S tables][mbarriers, meta (128 B)][warp queues][stage-1 table]
+    // layout: [stage 0][stage 1][S tables][mbarriers, meta, a word of ones (128 B)][warp queues][stage-1 table]
     const uint32_t stage0 = base;
     const uint32_t tab = base + 2 * kStageBytes;
-    const uint32_t bar0 = tab + kTabBytes, bar1 = bar0 + 8;
-    // Stage k & 1's "full" barrier completes when load k lands. With kStageBarriers (MODE 5) its "empty"
-    // barrier completes when every warp is done reading it, load k + 2 reuses the stage only after that, and
-    // warps otherwise run apart by up to a stage. It pays where few windows pass the shared-memory stage
-    // (plain workload: 596 -> 630 GB/s); where many do, warps that wait for the stage of a warp busy with
-    // its queue cost more than a block barrier (a 2^22-bit batched class: 370 -> 306), and in the dense
-    // modes too (325 -> 308). The other modes keep one block barrier per stage.
-    constexpr bool kStageBarriers = MODE == 5;
-    auto ebar = [&](uint32_t k) { return bar0 + 48u + 8u * (k & 1u); };
-    int* meta = reinterpret_cast<int*>(smem + 2 * kStageBytes + kTabBytes + 16);  // [buf][4]: job, item, row, valid
-    const uint32_t queues = bar0 + 128;
-    const uint32_t s1 = queues + (THREADS / 32) * kQBytes;
+    const uint32_t bar0 = tab + kTabBytes;
+    // Stage k & 1's "full" barrier completes when load k lands, its "empty" barrier when every warp is done reading
+    // it; load k + 2 reuses the stage only after that, and warps otherwise run apart by up to a stage.
+    auto fbar = [&](uint32_t k) { return bar0 + 8u * (k & 1u); };
+    auto ebar = [&](uint32_t k) { return bar0 + 16u + 8u * (k & 1u); };
+    int* meta = reinterpret_cast<int*>(smem + 2 * kStageBytes + kTabBytes + 32);  // [stage][4]: job, item, part, valid
+    const uint32_t ones = bar0 + 64u;
+    const uint32_t queues = bar0 + 128u;
+    const uint32_t s1 = queues + (THREADS / 32) * 4u * kQueueCap;
     uint32_t* s1p = reinterpret_cast<uint32_t*>(smem + (s1 - base));
-    // Per-CTA state kept in shared memory rather than registers, which the dense mode's rings need:
-    // the load sequencer (thread 0 only), each warp's first text position of its current row, each
-    // thread's first and last '\n' so far in its stream.
+    // the load sequencer's state (thread 0 only) and each warp's first text position
     __shared__ int s_abort;
     __shared__ uint32_t s_ni, s_nj;
     __shared__ int s_nr;
     __shared__ uint64_t s_wpos[THREADS / 32];
-    __shared__ long long s_fnl[THREADS], s_lnl[THREADS];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     {
         uint64_t* tp = reinterpret_cast<uint64_t*>(smem + 2 * kStageBytes);
         for (int i = tid; i < 256 * 16; i += THREADS) {
             const int c = i >> 4;
-            tp[i] = c_sbox[(c & 0x80) ? 0 : c];
+            if constexpr (kTwoTables) tp[i] = c < 128 ? c_sbox[c] : rol64(c_sbox[c - 128], L);
+            else tp[i] = c_sbox[(c & 0x80) ? 0 : c];
         }
     }
-    // load sequencer, run by thread 0: the next load is row nr (-1: halo) of item ni, which belongs to job nj.
+    // Load sequencer, run by thread 0: the next load is part nr (-1: halo) of item ni, which belongs to job nj.
     // Load k waits (bounded) until every warp has released load k - 2's stage; with no item left it completes
     // the stage's full barrier without a load and marks the end in meta. Returns false when the wait gave up.
     auto issue = [&](uint32_t k) -> bool {
-        if constexpr (kStageBarriers) {
-            if (k >= 2 && !mbar_wait_bounded(ebar(k), ((k - 2) >> 1) & 1u)) {
-                atomicOr(error_flag, 4u);
-                return false;
-            }
+        if (k >= 2 && !mbar_wait_bounded(ebar(k), ((k - 2) >> 1) & 1u)) {
+            atomicOr(error_flag, 4u);
+            return false;
         }
         int* m = meta + 4 * (k & 1);
         uint32_t ni = s_ni, nj = s_nj;
         int nr = s_nr;
         if (ni >= n_items) {
             m[3] = 0;
-            if constexpr (kStageBarriers) mbar_arrive((k & 1) ? bar1 : bar0);
+            mbar_arrive(fbar(k));
             return true;
         }
         while (nj + 1 < n_jobs && __ldg(&jobs[nj + 1].item_begin) <= ni) nj++;
         const FastJob* J = jobs + nj;
         const uint32_t R = __ldg(&J->rows);
         const uint32_t st = ni - __ldg(&J->item_begin);
-        const int y = nr < 0 ? (int)R - 1 : nr;
+        const int y = nr < 0 ? (int)R - 1 : nr / kParts;
+        const int x = nr < 0 ? kRowBytes - kPart : nr % kParts * kPart;
         const int z = (int)(st * THREADS) + (nr < 0 ? -1 : 0);
-        const uint32_t bar = (k & 1) ? bar1 : bar0;
+        const uint32_t bar = fbar(k);
         const uint32_t dst = stage0 + (k & 1) * kStageBytes;
         m[0] = (int)nj;
         m[1] = (int)st;
@@ -388,12 +407,12 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         if (__ldg(&J->text_evict_first)) {
             const uint64_t pol = l2_evict_first_policy();
             for (int b = 0; b < THREADS / kBox; b++)
-                tma_load_3d_hint(dst + b * kBox * kRowBytes, &J->tmap, 0, y, z + b * kBox, bar, pol);
+                tma_load_3d_hint(dst + b * kBox * kPart, &J->tmap, x, y, z + b * kBox, bar, pol);
         } else {
             for (int b = 0; b < THREADS / kBox; b++)
-                tma_load_3d(dst + b * kBox * kRowBytes, &J->tmap, 0, y, z + b * kBox, bar);
+                tma_load_3d(dst + b * kBox * kPart, &J->tmap, x, y, z + b * kBox, bar);
         }
-        if (++nr == (int)R) {
+        if (++nr == (int)R * kParts) {
             nr = -1;
             ni = gridDim.x + atomicAdd(ctl + 1, 1u);  // next item from the queue
         }
@@ -407,13 +426,11 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         s_ni = blockIdx.x;
         s_nj = 0;
         s_nr = -1;
-        mbar_init(bar0, 1);
-        mbar_init(bar1, 1);
-        if constexpr (kStageBarriers) {
-            mbar_init(ebar(0), THREADS / 32);
-            mbar_init(ebar(1), THREADS / 32);
+        for (uint32_t b = 0; b < 2; b++) {
+            mbar_init(fbar(b), 1);
+            mbar_init(ebar(b), THREADS / 32);
         }
-        *reinterpret_cast<uint32_t*>(smem + (bar0 - base) + 64) = 0xFFFFFFFFu;  // the S = 1 second-probe word
+        *reinterpret_cast<uint32_t*>(smem + (ones - base)) = 0xFFFFFFFFu;  // the S = 1 second-probe word
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // publication gate: a bounded poll, and no load in flight if it gives up
         bool open = true;
@@ -433,147 +450,120 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
             issue(0);
         } else {
             meta[3] = 0;
-            if constexpr (kStageBarriers) mbar_arrive(bar0);
+            mbar_arrive(fbar(0));
         }
     }
     __syncthreads();
 
     const uint32_t lane_tab = tab + (uint32_t)(lane & 15) * 8u;  // entry c of this lane's copy: + c * 128
-    const uint32_t qaddr = queues + (uint32_t)warp * kQBytes;
+    const uint32_t lane_out = kTwoTables ? lane_tab + 128u * 128u : lane_tab;
+    // S-box entry of byte i of the 64-byte span (p, c): as it enters the window, and rotated by LEN as it leaves
+    auto sbox_in = [&](const uint32_t (&c)[8], int i) { return lds64(entry_addr(c[i >> 2], i & 3, lane_tab)); };
+    auto sbox_out = [&](const uint32_t (&p)[8], const uint32_t (&c)[8], int i) {
+        const uint2 o = lds64(i >= L ? entry_addr(c[(i - L) >> 2], (i - L) & 3, lane_out)
+                                     : entry_addr(p[(i - L + 32) >> 2], (i - L + 32) & 3, lane_out));
+        return kTwoTables ? o : make_uint2(o.y, o.x);
+    };
+    // Zeroes the block's high bytes where the table does not map them (rare in text: one test per block).
+    auto map_high_bytes = [&](uint32_t (&w)[8]) {
+        if constexpr (kTwoTables) {
+            if (((w[0] | w[1] | w[2]) | (w[3] | w[4] | w[5]) | (w[6] | w[7])) & 0x80808080u) {
+#pragma unroll
+                for (int q = 0; q < 8; q++) w[q] = clear_high_bytes(w[q]);
+            }
+        }
+    };
+    const uint32_t qaddr = queues + (uint32_t)warp * 4u * kQueueCap;
     const unsigned lt_mask = (1u << lane) - 1u;
 
     // the current job's parameters (reloaded when the job changes)
     int cur_job = -1;
-    uint32_t R = 0, s1_bmask = 0, s1_first = 0, spt_log2 = 0;
-    uint32_t a_mask = 0, a_add = 0, b_mask = 0, b_add = 0;  // dense mode: regions of the two pipelined probes
-    bool two = false;
-    auto job_desc = [&]() { return jobs + cur_job; };
-    // The filter pointer is held in a register: the loop's global stores would otherwise make the compiler
-    // reload it from the descriptor before every probe. Fields used once per row or per queue flush are
-    // read from the descriptor where they are used, so they hold no registers across the byte loop.
-    const uint32_t* main_words = nullptr;
+    uint32_t R = 0, s1_bmask = 0;
+    uint32_t a_mask = 0, b_mask = 0;  // dense modes: the regions of the two pipelined probes
+    const uint32_t *a_words = nullptr, *b_words = nullptr;
+    uint32_t s2 = s1, s2_bmask = 0;  // sparse mode: the second probe's table (the stage-1 table, or with S = 1 a word of ones)
     bool s1_fits = true;
+    auto job_desc = [&]() { return jobs + cur_job; };
 
     int qn = 0;  // warp-uniform queue fill
-    // Appends the lanes with `pass` to the warp queue; flushes when fewer than 32 slots remain.
-    auto enqueue = [&](bool pass, uint32_t pos, uint32_t ql, uint32_t qh, uint32_t first) {
-        const unsigned m = __ballot_sync(0xffffffffu, pass);
-        if (m) {
-            if (pass) {
-                // qn <= kQCap - 32 holds on entry (the queue flushes above that), so slot < kQCap
-                const uint32_t slot = (uint32_t)qn + __popc(m & lt_mask);
-                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(qaddr + 16u * slot),
-                             "r"(pos | ((uint32_t)lane << 8)), "r"(ql), "r"(qh), "r"(first)
+    auto flush = [&]() {
+        __syncwarp();
+        flush_queue<L, kQueueCap / 32>(job_desc(), qaddr, qn, s_wpos[warp], (uint64_t)R * kRowBytes, lane, lane_tab);
+        qn = 0;
+    };
+    // Queues the windows whose bits are set in each lane's mask; bit i is the window ending at pos + i in the lane's
+    // stream. Every round takes one window of each lane that has any.
+    auto enqueue = [&](uint32_t cand, uint32_t pos) {
+        while (__any_sync(0xffffffffu, cand != 0u)) {
+            const unsigned m = __ballot_sync(0xffffffffu, cand != 0u);
+            if (cand) {
+                // qn <= kQueueCap - 32 holds on entry (the queue flushes above that)
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(qaddr + 4u * (uint32_t)(qn + __popc(m & lt_mask))),
+                             "r"((pos + (uint32_t)__ffs(cand) - 1u) | ((uint32_t)lane << 16))
                              : "memory");
+                cand &= cand - 1;
             }
             qn += __popc(m);
-            if (qn > kQCap - 32) {
-                __syncwarp();
-                flush_queue<kQCap / 32>(job_desc(), qaddr, qn, s_wpos[warp], (uint64_t)R * kRowBytes, lane);
-                qn = 0;
-            }
+            if (qn > kQueueCap - 32) flush();
         }
     };
-    // dense-mode rings. Stage A: the first probe's word (0 when the window was not valid, so its test fails),
-    // h1, h2. Stage B: the second probe's word (0 when stage A failed), h1, h2.
-    constexpr int kR = (MODE == 1 || MODE == 2 || MODE == 3) ? kRing : 1;
-    // dense mode: rotation of h1/h2 giving the pipelined probes' index functions, and the first probe a
-    // queued window still needs in the reference order (MODE 1 knows f0 and f1; MODE 2 retests all)
-    constexpr int kRot = MODE == 2 ? 16 : 0;
-    constexpr uint32_t kFirstB = MODE == 2 ? 0u : 2u, kFirstA = MODE == 2 ? 0u : 1u;
-    uint32_t ring_v[kR], ring_l[kR], ring_h[kR], ring2_v[kR], ring2_l[kR], ring2_h[kR];
+    // dense-mode rings. Stage A: the first probe's word (0 when the window was not valid, so its test fails) and the
+    // window's two index functions. Stage B: the second probe's word (0 when stage A failed) and its index function.
+    constexpr int kR = kSparse ? 1 : kRing;
+    constexpr int kRot = MODE == 2 || MODE == 4 ? 16 : 0;  // rotation of h1/h2 giving the pipelined probes' index functions
+    uint32_t ring_v[kR], ring_a[kR], ring_b[kR], ring2_v[kR], ring2_b[kR];
 #pragma unroll
-    for (int q = 0; q < kR; q++) ring_v[q] = ring_l[q] = ring_h[q] = ring2_v[q] = ring2_l[q] = ring2_h[q] = 0;
+    for (int q = 0; q < kR; q++) ring_v[q] = ring_a[q] = ring_b[q] = ring2_v[q] = ring2_b[q] = 0;
 
     uint32_t hl = 0, hh = 0;
-    int lnp = -1000;  // last '\n' relative to the current row start
     uint32_t prev[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    // MODE 4: newline mask of the previous block (bit 31 forced at the text's start, where nothing precedes
-    // offset 0). MODE 0 and 4: the second probe's table (the stage-1 table, or with S = 1 a word of ones)
+    // newline mask of the previous block (bit 31 forced at the text's start, where nothing precedes offset 0)
     uint32_t nl_prev = 0;
-    uint32_t s2 = s1, s2_bmask = 0;
+    uint32_t first_nl = ~0u, last_nl = ~0u;  // first and last '\n' of the stream so far
 
     for (uint32_t k = 0;; k++) {
-        const uint32_t bar = (k & 1) ? bar1 : bar0;
-        const uint32_t parity = (k >> 1) & 1u;
-        int job, r;
-        uint32_t st;
-        if constexpr (kStageBarriers) {
-            // Warps meet only through the stages' barriers: a warp may start stage k + 1 while others still
-            // read stage k, and thread 0 refills a stage once every warp has released it.
+        {
             uint32_t it = 0;
-            while (!mbar_try_wait(bar, parity)) {
+            while (!mbar_try_wait(fbar(k), (k >> 1) & 1u)) {
                 if (++it >= kWaitLimit) {
                     atomicOr(error_flag, 4u);
                     s_abort = 1;
                     break;
                 }
-            }
-            if (s_abort) {
-                // Give a load still in flight a bounded chance to land before the shared memory goes away.
-                if (tid == 0 && meta[4 * (k & 1) + 3])
-                    for (uint32_t j = 0; j < kWaitLimit && !mbar_try_wait(bar, parity); j++) {
-                    }
-                break;
-            }
-            // the stage's meta is written before its full barrier completes, so it is read after the wait
-            const int* m = meta + 4 * (k & 1);
-            if (!m[3]) break;
-            job = m[0];
-            st = (uint32_t)m[1];
-            r = m[2];
-            if (tid == 0 && !issue(k + 1)) s_abort = 1;
-        } else {
-            // meta of stage k was written before the previous stage's block barrier
-            const int* m = meta + 4 * (k & 1);
-            if (!m[3]) break;
-            job = m[0];
-            st = (uint32_t)m[1];
-            r = m[2];
-            if (tid == 0) issue(k + 1);
-            uint32_t it = 0;
-            while (!mbar_try_wait(bar, parity)) {
-                if (++it >= kWaitLimit) {
-                    atomicOr(error_flag, 4u);
-                    s_abort = 1;
-                    break;
-                }
-            }
-            if (s_abort) {
-                // Give the load issued for k + 1 a bounded chance to land before the shared memory goes away.
-                if (tid == 0 && meta[4 * ((k + 1) & 1) + 3]) {
-                    const uint32_t nb = ((k + 1) & 1) ? bar1 : bar0;
-                    for (uint32_t j = 0; j < kWaitLimit && !mbar_try_wait(nb, ((k + 1) >> 1) & 1u); j++) {
-                    }
-                }
-                break;
             }
         }
+        if (s_abort) {
+            // Give a load still in flight a bounded chance to land before the shared memory goes away.
+            if (tid == 0 && meta[4 * (k & 1) + 3])
+                for (uint32_t j = 0; j < kWaitLimit && !mbar_try_wait(fbar(k), (k >> 1) & 1u); j++) {
+                }
+            break;
+        }
+        // the stage's meta is written before its full barrier completes, so it is read after the wait
+        const int* m = meta + 4 * (k & 1);
+        if (!m[3]) break;
+        const int job = m[0], r = m[2];
+        const uint32_t st = (uint32_t)m[1];
+        if (tid == 0 && !issue(k + 1)) s_abort = 1;
         if (job != cur_job) {
             cur_job = job;
             const FastJob* J = job_desc();
             const Geom g = J->g;
             R = J->rows;
-            spt_log2 = J->streams_per_tile_log2;
-            main_words = J->main_words;
             s1_fits = !kTable || J->stage1_nwords <= max_s1_words;
-            const uint32_t cmask = g.cache_mask;
-            two = g.s > 1;
             // stage-1 table of T = C >> shift bits, folded modulo T: the byte offset of bit (h & (T-1))'s
             // word is (h >> 3) & s1_bmask
-            s1_bmask = (((cmask >> J->stage1_shift) >> 3) & ~3u);
+            s1_bmask = (((g.cache_mask >> J->stage1_shift) >> 3) & ~3u);
             a_mask = J->a_mask;
-            a_add = J->a_add;
+            a_words = J->main_words + J->a_add / 32;
             b_mask = J->b_mask;
-            b_add = J->b_add;
-            // sparse mode: the stage-1 probes are exact when the table is the cache region itself
-            s1_first = J->stage1_shift == 0 ? (two ? 2u : 1u) : 0u;
-            s2 = two ? s1 : bar0 + 64;
-            s2_bmask = two ? s1_bmask : 0u;
+            b_words = J->main_words + J->b_add / 32;
+            s2 = g.s > 1 ? s1 : ones;
+            s2_bmask = g.s > 1 ? s1_bmask : 0u;
             if constexpr (kTable) {
                 // every warp is done with the previous job's table before it is overwritten (all warps change
                 // job at the same stage)
-                if constexpr (kStageBarriers) __syncthreads();
+                __syncthreads();
                 const uint32_t nw = s1_fits ? J->stage1_nwords : 0u;
                 const uint32_t* src = J->stage1_words;
                 for (uint32_t i = tid; i < nw; i += THREADS) s1p[i] = src[i];
@@ -582,65 +572,41 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         }
 
         // self-checks: a bad descriptor or sequencing records a code and skips the work
-        if ((uint32_t)job >= n_jobs || st >= job_desc()->n_supertiles || r < -1 || r >= (int)R || !s1_fits) {
+        if ((uint32_t)job >= n_jobs || st >= job_desc()->n_supertiles || r < -1 || r >= (int)R * kParts || !s1_fits) {
             if (tid == 0) atomicOr(error_flag, 0x100u);
-            if constexpr (kStageBarriers) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(ebar(k));
-            } else {
-                __syncthreads();
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ebar(k));
             continue;
         }
         const uint64_t z = (uint64_t)st * THREADS + tid;
         const bool active = z < job_desc()->n_streams;
-        const uint8_t* row = smem + (k & 1) * kStageBytes + tid * kRowBytes;
-        const int sw = tid & 7;
+        const uint8_t* row = smem + (k & 1) * kStageBytes + tid * kPart;
+        const int sw = (tid >> 1) & 3;  // the 64-byte swizzle XORs a 16-byte chunk's index with its address bits 7 and 8
 
         if (r < 0) {
-            // halo: the last 32 bytes before the stream (chunks 6 and 7 of the previous stream's last row)
-            const uint4 c6 = *reinterpret_cast<const uint4*>(row + ((6 ^ sw) << 4));
-            const uint4 c7 = *reinterpret_cast<const uint4*>(row + ((7 ^ sw) << 4));
+            // halo: the last 32 bytes before the stream
+            const uint4 c6 = *reinterpret_cast<const uint4*>(row + (((kPart / 16 - 2) ^ sw) << 4));
+            const uint4 c7 = *reinterpret_cast<const uint4*>(row + (((kPart / 16 - 1) ^ sw) << 4));
             prev[0] = c6.x; prev[1] = c6.y; prev[2] = c6.z; prev[3] = c6.w;
             prev[4] = c7.x; prev[5] = c7.y; prev[6] = c7.z; prev[7] = c7.w;
+            map_high_bytes(prev);
             hl = 0;
             hh = 0;
-            lnp = -1000;
+            // the hash of the halo's last LEN bytes, from a zero state: nothing leaves the window
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-                const uint32_t c = byte_at(prev[j >> 2], j & 3);
-                const uint2 sv = lds64(lane_tab + c * 128u);
-                uint32_t nl = __funnelshift_l(hh, hl, 1), nh = __funnelshift_l(hl, hh, 1);
-                nl ^= sv.x;
-                nh ^= sv.y;
-                if (j >= L) {
-                    const uint32_t co = byte_at(prev[(j - L) >> 2], (j - L) & 3);
-                    const uint2 o = lds64(lane_tab + co * 128u);
-                    uint32_t rl, rh;
-                    rol_pair<L>(o.x, o.y, rl, rh);
-                    nl ^= rl;
-                    nh ^= rh;
-                }
+            for (int j = 32 - L; j < 32; j++) {
+                const uint2 sv = sbox_in(prev, j);
+                const uint32_t nl = __funnelshift_l(hh, hl, 1) ^ sv.x, nh = __funnelshift_l(hl, hh, 1) ^ sv.y;
                 hl = nl;
                 hh = nh;
-                if (c == 0x0Au) lnp = j - 32;
             }
-            if (z == 0) lnp = -1;  // text start: nothing before offset 0
-            if constexpr (MODE == 4) nl_prev = newline_mask32(prev) | (z == 0 ? 0x80000000u : 0u);
-            s_fnl[tid] = LLONG_MAX;
-            s_lnl[tid] = -1;
+            nl_prev = newline_mask32(prev) | (z == 0 ? 0x80000000u : 0u);  // text start: nothing before offset 0
+            first_nl = last_nl = ~0u;
+            if (lane == 0) s_wpos[warp] = ((uint64_t)st * THREADS + (uint64_t)warp * 32) * R * kRowBytes;
         } else {
-            // A stream past the job's end reads zero-filled rows (no '\n'): a last newline far ahead keeps all
-            // its windows invalid, so the byte loop needs no separate `active` test.
-            if (!active) lnp = 1 << 29;
-            const int lnp_in = lnp;
-            qn = 0;
-            if (lane == 0)
-                s_wpos[warp] = ((uint64_t)st * THREADS + (uint64_t)warp * 32) * R * kRowBytes + (uint64_t)r * kRowBytes;
-            const bool need_first = s_fnl[tid] == LLONG_MAX;
-            int row_first = -1;  // first '\n' of this row, found once per stream
+            const uint32_t pos0 = (uint32_t)r * kPart;  // this part's first byte in the stream
 #pragma unroll 1
-            for (int b = 0; b < kRowBytes / 32; b++) {
+            for (int b = 0; b < kPart / 32; b++) {
                 uint32_t cur[8];
                 {
                     const uint4 v0 = *reinterpret_cast<const uint4*>(row + (((2 * b) ^ sw) << 4));
@@ -648,199 +614,84 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                     cur[0] = v0.x; cur[1] = v0.y; cur[2] = v0.z; cur[3] = v0.w;
                     cur[4] = v1.x; cur[5] = v1.y; cur[6] = v1.z; cur[7] = v1.w;
                 }
-                const int lnp_blk = lnp;
-                if constexpr (MODE == 4) {
-                    // pass bits of the block's windows (bit j: the window ending at byte j passed both table
-                    // probes), and the hash before each 8-byte segment
-                    uint32_t pass = 0, ckl[4], ckh[4];
+                map_high_bytes(cur);
+                const uint32_t nlm = newline_mask32(cur);
+                // valid windows hold no '\n' (processFile resets the hash there); a stream past the job's end,
+                // which reads zero-filled rows, has none
+                const uint32_t valid = active ? ~window_has_newline<L>(nl_prev, nlm) : 0u;
+                uint32_t pass = 0;
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        if ((j & 7) == 0) {
-                            ckl[j >> 3] = hl;
-                            ckh[j >> 3] = hh;
-                        }
-                        const uint32_t c = byte_at(cur[j >> 2], j & 3);
-                        uint32_t co;
-                        if (j >= L) co = byte_at(cur[(j - L) >> 2], (j - L) & 3);
-                        else co = byte_at(prev[(j - L + 32) >> 2], (j - L + 32) & 3);
-                        const uint2 sv = lds64(lane_tab + c * 128u);
-                        const uint2 o = lds64(lane_tab + co * 128u);
-                        uint32_t rl, rh;
-                        rol_pair<L>(o.x, o.y, rl, rh);
-                        const uint32_t nl = __funnelshift_l(hh, hl, 1), nh = __funnelshift_l(hl, hh, 1);
-                        hl = nl ^ sv.x ^ rl;
-                        hh = nh ^ sv.y ^ rh;
-                        const uint32_t w0 = lds32(s1 + ((hl >> 3) & s1_bmask));
-                        const uint32_t w1 = lds32(s2 + ((hh >> 3) & s2_bmask));
-                        const uint32_t t = __funnelshift_r(w0, w0, hl) & __funnelshift_r(w1, w1, hh);
-                        pass = __funnelshift_r(pass, t, 1);  // t's bit 0 enters at bit 31
-                    }
-                    const uint32_t nlm = newline_mask32(cur);
-                    if (__any_sync(0xffffffffu, pass != 0u)) {
-                        // valid windows hold no '\n' (processFile resets the hash there); a stream past the
-                        // job's end has none
-                        const uint32_t cand = active ? pass & ~window_has_newline<L>(nl_prev, nlm) : 0u;
-#pragma unroll
-                        for (int sg = 0; sg < 4; sg++) {
-                            if (__any_sync(0xffffffffu, ((cand >> (8 * sg)) & 0xFFu) != 0u)) {
-                                uint32_t ql = ckl[sg], qh = ckh[sg];
-#pragma unroll
-                                for (int jj = 0; jj < 8; jj++) {
-                                    const int j = 8 * sg + jj;
-                                    const uint32_t c = byte_at(cur[j >> 2], j & 3);
-                                    uint32_t co;
-                                    if (j >= L) co = byte_at(cur[(j - L) >> 2], (j - L) & 3);
-                                    else co = byte_at(prev[(j - L + 32) >> 2], (j - L + 32) & 3);
-                                    const uint2 sv = lds64(lane_tab + c * 128u);
-                                    const uint2 o = lds64(lane_tab + co * 128u);
-                                    uint32_t rl, rh;
-                                    rol_pair<L>(o.x, o.y, rl, rh);
-                                    const uint32_t nl = __funnelshift_l(qh, ql, 1), nh = __funnelshift_l(ql, qh, 1);
-                                    ql = nl ^ sv.x ^ rl;
-                                    qh = nh ^ sv.y ^ rh;
-                                    enqueue(((cand >> j) & 1u) != 0u, (uint32_t)(kRowBytes + 32 * b + j), ql, qh,
-                                            s1_first);
-                                }
-                            }
-                        }
-                    }
-                    nl_prev = nlm;
-                    if (nlm) {
-                        lnp = 31 - __clz(nlm);
-                        if (row_first < 0 && need_first) row_first = 32 * b + __ffs(nlm) - 1;
-                    }
-                } else {
-                    // MODE 0 tests each window one byte late: the table words of byte j are loaded, then byte
-                    // j - 1's (loaded a byte earlier) are tested and queued, so the shared-memory latency of a
-                    // byte's probes overlaps the next byte's hash instead of stalling before its warp vote
-                    uint32_t pw0 = 0, pw1 = 0, pl = 0, ph = 0;
-                    bool pv = false;
-                    // S-box entries of byte j's incoming and outgoing bytes; MODE 0 loads them a byte ahead
-                    auto sbox_in = [&](int j) { return lds64(lane_tab + byte_at(cur[j >> 2], j & 3) * 128u); };
-                    auto sbox_out = [&](int j) {
-                        const uint32_t co = j >= L ? byte_at(cur[(j - L) >> 2], (j - L) & 3)
-                                                   : byte_at(prev[(j - L + 32) >> 2], (j - L + 32) & 3);
-                        return lds64(lane_tab + co * 128u);
-                    };
-                    uint2 nsv = make_uint2(0, 0), no = make_uint2(0, 0);
+                for (int j = 0; j < 32; j++) {
+                    const uint2 sv = sbox_in(cur, j), o = sbox_out(prev, cur, j);
+                    const uint32_t nl = __funnelshift_l(hh, hl, 1), nh = __funnelshift_l(hl, hh, 1);
+                    hl = nl ^ sv.x ^ o.x;
+                    hh = nh ^ sv.y ^ o.y;
                     if constexpr (kSparse) {
-                        nsv = sbox_in(0);
-                        no = sbox_out(0);
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const uint32_t c = byte_at(cur[j >> 2], j & 3);
-                        uint2 sv, o;
-                        if constexpr (kSparse) {
-                            sv = nsv;
-                            o = no;
-                            if (j + 1 < 32) {
-                                nsv = sbox_in(j + 1);
-                                no = sbox_out(j + 1);
-                            }
+                        // the second probe is loaded only where the first passes: its random words would cost the
+                        // shared-memory pipe, which bounds this loop, another 3.5 wavefronts per warp
+                        const uint32_t w0 = lds32(s1 + ((hl >> 3) & s1_bmask));
+                        const uint32_t w1 =
+                            lds32_if(s2 + ((hh >> 3) & s2_bmask), (__funnelshift_r(w0, w0, hl) & 1u) != 0);
+                        pass = __funnelshift_r(pass, __funnelshift_r(w1, w1, hh), 1);  // the bit enters at bit 31
+                    } else {
+                        const int slot = j % kRing;
+                        // The window that entered stage A kLag bytes ago leaves its last stage (a probe's bit sits
+                        // at f & 31 in its word: region offsets are multiples of 32).
+                        if constexpr (kPre) {
+                            pass = __funnelshift_r(pass, __funnelshift_r(ring_v[slot], ring_v[slot], ring_a[slot]), 1);
                         } else {
-                            sv = sbox_in(j);
-                            o = sbox_out(j);
-                        }
-                        uint32_t rl, rh;
-                        rol_pair<L>(o.x, o.y, rl, rh);
-                        const uint32_t nl = __funnelshift_l(hh, hl, 1), nh = __funnelshift_l(hl, hh, 1);
-                        hl = nl ^ sv.x ^ rl;
-                        hh = nh ^ sv.y ^ rh;
-                        if (c == 0x0Au) lnp = j;
-                        if constexpr (kSparse) {
-                            // with S = 1 the second probe reads a word of ones
-                            const uint32_t w0 = lds32(s1 + ((hl >> 3) & s1_bmask));
-                            const uint32_t w1 = lds32(s2 + ((hh >> 3) & s2_bmask));
-                            const bool valid = j - lnp >= L;
-                            if (j > 0) {
-                                const uint32_t t = __funnelshift_r(pw0, pw0, pl) & __funnelshift_r(pw1, pw1, ph);
-                                enqueue(pv && (t & 1u) != 0, (uint32_t)(kRowBytes + 32 * b + j - 1), pl, ph, s1_first);
-                            }
-                            pw0 = w0;
-                            pw1 = w1;
-                            pl = hl;
-                            ph = hh;
-                            pv = valid;
-                        } else {
-                            const int slot = j % kRing;
-                            // stage B: the window that entered stage A 2*kRing bytes ago (a probe's bit sits at
-                            // f & 31 in its word: region offsets are multiples of 32)
-                            const uint32_t fb_old = rot_const<kRot>(ring2_h[slot]);
-                            const bool pass2 = (__funnelshift_r(ring2_v[slot], ring2_v[slot], fb_old) & 1u) != 0;
-                            enqueue(pass2, (uint32_t)(kRowBytes + 32 * b + j - 2 * kRing), ring2_l[slot], ring2_h[slot],
-                                    kFirstB);
+                            pass = __funnelshift_r(pass, __funnelshift_r(ring2_v[slot], ring2_v[slot], ring2_b[slot]),
+                                                   1);
                             // stage A: the window issued kRing bytes ago; its word has arrived by now
-                            const uint32_t fa_old = rot_const<kRot>(ring_l[slot]);
-                            const bool pass1 = (__funnelshift_r(ring_v[slot], ring_v[slot], fa_old) & 1u) != 0;
-                            ring2_l[slot] = ring_l[slot];
-                            ring2_h[slot] = ring_h[slot];
-                            const uint32_t fb = rot_const<kRot>(ring_h[slot]);
-                            ring2_v[slot] = ldg_if(main_words + (((fb & b_mask) + b_add) >> 5), pass1);
-                            bool issue = j - lnp >= L;
-                            if constexpr (MODE == 3) {
-                                // the folded table's bit: clear means the cache bit of f0 is clear too
-                                const uint32_t w = lds32(s1 + ((hl >> 3) & s1_bmask));
-                                issue = issue && (__funnelshift_r(w, w, hl) & 1u) != 0;
-                            }
-                            ring_l[slot] = hl;
-                            ring_h[slot] = hh;
-                            const uint32_t fa = rot_const<kRot>(hl);
-                            if constexpr (MODE != 2)  // f0 is in the cache region (S >= 1): no offset
-                                ring_v[slot] = ldg_if(main_words + ((fa & a_mask) >> 5), issue);
-                            else
-                                ring_v[slot] = ldg_if(main_words + (((fa & a_mask) + a_add) >> 5), issue);
+                            const bool pass1 = (__funnelshift_r(ring_v[slot], ring_v[slot], ring_a[slot]) & 1u) != 0;
+                            ring2_b[slot] = ring_b[slot];
+                            ring2_v[slot] = ldg_if(b_words + ((ring_b[slot] & b_mask) >> 5), pass1);
                         }
-                    }
-                    if constexpr (kSparse) {  // the block's last window
-                        const uint32_t t = __funnelshift_r(pw0, pw0, pl) & __funnelshift_r(pw1, pw1, ph);
-                        enqueue(pv && (t & 1u) != 0, (uint32_t)(kRowBytes + 32 * b + 31), pl, ph, s1_first);
+                        bool issue = (valid & (1u << j)) != 0;
+                        if constexpr (kPre) {
+                            // the table's bits: a clear one means the cache bit of f0 or f1 is clear too
+                            const uint32_t w0 = lds32(s1 + ((hl >> 3) & s1_bmask));
+                            const uint32_t w1 =
+                                lds32_if(s2 + ((hh >> 3) & s2_bmask), (__funnelshift_r(w0, w0, hl) & 1u) != 0);
+                            issue = issue && (__funnelshift_r(w1, w1, hh) & 1u) != 0;
+                        }
+                        ring_a[slot] = rot_const<kRot>(hl);
+                        ring_b[slot] = rot_const<kRot>(hh);
+                        ring_v[slot] = ldg_if(a_words + ((ring_a[slot] & a_mask) >> 5), issue);
                     }
                 }
-                if (MODE != 4 && lnp != lnp_blk && row_first < 0 && need_first) {
-                    for (int q = 0; q < 8 && row_first < 0; q++) {
-                        const uint32_t t = cur[q] ^ 0x0A0A0A0Au;
-                        const uint32_t zb = ~(((t & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | t) & 0x80808080u;
-                        if (zb) row_first = 32 * b + 4 * q + (__ffs(zb) - 1) / 8;
-                    }
+                if constexpr (kSparse) enqueue(pass & valid, pos0 + (uint32_t)(32 * b));
+                else enqueue(pass, pos0 + (uint32_t)(32 * b - kLag));
+                if (nlm) {
+                    last_nl = pos0 + (uint32_t)(32 * b + 31 - __clz(nlm));
+                    if (first_nl == ~0u) first_nl = pos0 + (uint32_t)(32 * b + __ffs(nlm) - 1);
                 }
-                lnp -= 32;
+                nl_prev = nlm;
 #pragma unroll
                 for (int q = 0; q < 8; q++) prev[q] = cur[q];
             }
-            if constexpr (MODE == 1 || MODE == 2 || MODE == 3) {
-                // The rings carry over into the stream's next row (whose bytes follow this row's); at the
-                // stream's end they drain: stage-B slot q holds the window ending at 128 - 2*kRing + q,
-                // stage-A slot q the one at 128 - kRing + q; stage-A survivors go to the queue with only
-                // their first probe known.
-                if ((uint32_t)r == R - 1) {
+            if (r == (int)R * kParts - 1) {
+                if constexpr (!kSparse) {
+                    // The rings carry over between a stream's parts and drain at its end: the last stage's slot q
+                    // holds the window kLag - q bytes before the end; with two stages, stage A's survivors are queued
+                    // with only their first probe known.
+                    uint32_t rest = 0;
 #pragma unroll
                     for (int q = 0; q < kRing; q++) {
-                        const uint32_t fb = rot_const<kRot>(ring2_h[q]);
-                        const bool pass2 = (__funnelshift_r(ring2_v[q], ring2_v[q], fb) & 1u) != 0;
-                        enqueue(pass2, (uint32_t)(2 * kRowBytes - 2 * kRing + q), ring2_l[q], ring2_h[q], kFirstB);
-                        const uint32_t fa = rot_const<kRot>(ring_l[q]);
-                        const bool pass1 = (__funnelshift_r(ring_v[q], ring_v[q], fa) & 1u) != 0;
-                        enqueue(pass1, (uint32_t)(2 * kRowBytes - kRing + q), ring_l[q], ring_h[q], kFirstA);
+                        const uint32_t a = (__funnelshift_r(ring_v[q], ring_v[q], ring_a[q]) & 1u) << q;
+                        rest |= kPre ? a : (a << kRing) | (__funnelshift_r(ring2_v[q], ring2_v[q], ring2_b[q]) & 1u) << q;
                         ring_v[q] = 0;
                         ring2_v[q] = 0;
                     }
+                    enqueue(rest, pos0 + (uint32_t)(kPart - kLag));
                 }
-            }
-            if (qn) {
-                __syncwarp();
-                flush_queue<kQCap / 32>(job_desc(), qaddr, qn, s_wpos[warp], (uint64_t)R * kRowBytes, lane);
-                qn = 0;
-            }
-            // lnp is now relative to the next row's start; lnp + 128 is its position in this row
-            if (active && lnp + kRowBytes != lnp_in) {
-                const long long row_pos = (long long)(z * R + (uint32_t)r) * kRowBytes;
-                if (need_first) s_fnl[tid] = row_pos + row_first;
-                s_lnl[tid] = row_pos + lnp + kRowBytes;
-            }
-            if ((uint32_t)r == R - 1) {
+                if (qn) flush();  // the queue keeps its candidates across the stream's parts, not across streams
                 // per-16 KiB-tile newline summary: reduce over the lanes whose streams share the tile
-                long long f = active ? s_fnl[tid] : LLONG_MAX, l = active ? s_lnl[tid] : -1;
+                const FastJob* J = job_desc();
+                const uint64_t pos = z * R * kRowBytes;
+                long long f = active && first_nl != ~0u ? (long long)(pos + first_nl) : LLONG_MAX;
+                long long l = active && last_nl != ~0u ? (long long)(pos + last_nl) : -1;
+                const uint32_t spt_log2 = J->streams_per_tile_log2;
                 const int G = 1 << spt_log2;
                 for (int o = 1; o < G; o <<= 1) {
                     f = min(f, __shfl_xor_sync(0xffffffffu, f, o));
@@ -848,7 +699,6 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                 }
                 if (active && (lane & (G - 1)) == 0) {
                     const uint64_t tile = z >> spt_log2;
-                    const FastJob* J = job_desc();
                     if (tile < J->n_tiles) {
                         J->tile_first_nl[tile] = f;
                         J->tile_last_nl[tile] = l;
@@ -858,13 +708,9 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                 }
             }
         }
-        if constexpr (kStageBarriers) {
-            // this warp is done reading the stage
-            __syncwarp();
-            if (lane == 0) mbar_arrive(ebar(k));
-        } else {
-            __syncthreads();
-        }
+        // this warp is done reading the stage
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ebar(k));
     }
 }
 
@@ -880,20 +726,18 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
     return fn;
 }
 
-// static shared memory of k_scan_fast<., THREADS, .> (sequencer, row positions, per-thread newline state)
-constexpr size_t static_smem(int threads) { return 16 * (size_t)threads + 8 * (size_t)(threads / 32) + 64; }
+// static shared memory of k_scan_fast<., THREADS, .> (sequencer, warp positions)
+constexpr size_t static_smem(int threads) { return 8 * (size_t)(threads / 32) + 64; }
 
-template <int THREADS, int MODE>
-constexpr size_t fixed_smem() {
-    return 1024 + 2 * (size_t)THREADS * kRowBytes + kTabBytes + 128 +
-           (THREADS / 32) * (size_t)(sparse_mode(MODE) || MODE == 4 ? kQueueBytes : 2 * kQueueBytes);
+constexpr size_t fixed_smem(int threads) {
+    return 1024 + 2 * (size_t)threads * kPart + kTabBytes + 128 + (threads / 32) * 4 * (size_t)kQueueCap;
 }
 
 template <int L, int THREADS, int MODE>
 cudaError_t launch_cfg(const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items, uint32_t max_s1_words,
                        uint32_t* d_ctl, int num_sms, cudaStream_t st) {
     const size_t smem =
-        fixed_smem<THREADS, MODE>() + (sparse_mode(MODE) || MODE == 3 || MODE == 4 ? 4 * (size_t)max_s1_words : 0);
+        fixed_smem(THREADS) + (sparse_mode(MODE) || MODE >= 3 ? 4 * (size_t)max_s1_words : 0);
     cudaError_t e =
         cudaFuncSetAttribute(k_scan_fast<L, THREADS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -905,46 +749,32 @@ cudaError_t launch_cfg(const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items,
     return cudaGetLastError();
 }
 
+// The kernel of a configuration: its CTA size is config_threads(cfg), the size its descriptors' TMA boxes and work
+// items were made for.
 template <int L>
 cudaError_t launch_len(const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items,
                        uint32_t max_s1_words, uint32_t* d_ctl, int num_sms, cudaStream_t st) {
-    if (cfg.mode == 1) {  // dense: 384 threads (ring depth 4), 256 (depth 8) or 2 x 192 (depth 4); 512 would spill
-        if (cfg.threads == 192 && cfg.order != 2)
-            return cfg.order == 1 ? launch_cfg<L, 192, 2>(d_jobs, n_jobs, n_items, 0, d_ctl, num_sms, st)
-                                  : launch_cfg<L, 192, 1>(d_jobs, n_jobs, n_items, 0, d_ctl, num_sms, st);
-        if (cfg.order == 1)
-            return cfg.threads == 256 ? launch_cfg<L, 256, 2>(d_jobs, n_jobs, n_items, 0, d_ctl, num_sms, st)
-                                      : launch_cfg<L, 384, 2>(d_jobs, n_jobs, n_items, 0, d_ctl, num_sms, st);
-        if (cfg.order == 2)
-            return cfg.threads == 256
-                       ? launch_cfg<L, 256, 3>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st)
-                       : launch_cfg<L, 384, 3>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-        return cfg.threads == 256 ? launch_cfg<L, 256, 1>(d_jobs, n_jobs, n_items, 0, d_ctl, num_sms, st)
-                                  : launch_cfg<L, 384, 1>(d_jobs, n_jobs, n_items, 0, d_ctl, num_sms, st);
-    }
-    if (cfg.mode == 3)  // sparse with per-stage barriers: 512 threads
-        return launch_cfg<L, 512, 5>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-    if (cfg.mode == 2) {  // sparse, deferred candidates: 192, 256 or 384 threads (larger stage-1 tables)
-        switch (cfg.threads) {
-            case 192: return launch_cfg<L, 192, 4>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-            case 384: return launch_cfg<L, 384, 4>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-            default: return launch_cfg<L, 256, 4>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-        }
-    }
-    switch (cfg.threads) {
-        case 256: return launch_cfg<L, 256, 0>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-        case 384: return launch_cfg<L, 384, 0>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-        default: return launch_cfg<L, 512, 0>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-    }
-}
-
-size_t fixed_smem_for(int threads, bool dense) {
-    if (dense) return threads == 256 ? fixed_smem<256, 1>() : threads == 192 ? fixed_smem<192, 1>() : fixed_smem<384, 1>();
-    switch (threads) {
-        case 192: return fixed_smem<192, 0>();
-        case 256: return fixed_smem<256, 0>();
-        case 384: return fixed_smem<384, 0>();
-        default: return fixed_smem<512, 0>();
+    const int mode = cfg.mode != 1 ? 0 : 1 + cfg.order;  // kernel mode: 0 sparse, 1..4 dense in probe order 0..3
+    switch (16 * config_threads(cfg) + mode) {
+#define FFBF_CASE(T, M) \
+    case 16 * T + M: return launch_cfg<L, T, M>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st)
+        FFBF_CASE(192, 0);
+        FFBF_CASE(256, 0);
+        FFBF_CASE(384, 0);
+        FFBF_CASE(512, 0);
+        FFBF_CASE(768, 0);
+        FFBF_CASE(192, 1);
+        FFBF_CASE(256, 1);
+        FFBF_CASE(384, 1);
+        FFBF_CASE(192, 2);
+        FFBF_CASE(256, 2);
+        FFBF_CASE(384, 2);
+        FFBF_CASE(256, 3);
+        FFBF_CASE(384, 3);
+        FFBF_CASE(256, 4);
+        FFBF_CASE(384, 4);
+#undef FFBF_CASE
+        default: return cudaErrorInvalidValue;
     }
 }
 
@@ -961,52 +791,89 @@ bool fast_scan_supported(const Geom& g, uint64_t n) {
 }
 
 // Largest power-of-two stage-1 table (in bits, <= C) that fits beside the fixed shared-memory layout.
-uint32_t stage1_shift_for(const Geom& g, int threads, bool dense) {
-    const size_t room = kSmemLimit - fixed_smem_for(threads, dense) - static_smem(threads) - 64;
+uint32_t stage1_shift_for(const Geom& g, int threads) {
+    const size_t room = kSmemLimit - fixed_smem(threads) - static_smem(threads) - 64;
     uint32_t sh = 0;
     while (((uint64_t)g.cache_bits >> sh) / 8 > room) sh++;
     return sh;
 }
+// the 512-thread kernel's table also fits the 768-thread one, which large texts use (launch_threads)
+static_assert(kSmemLimit - fixed_smem(512) - static_smem(512) - 64 < 131072, "512 threads: a 2^19-bit table");
+static_assert(kSmemLimit - fixed_smem(768) - static_smem(768) - 64 >= 65536, "768 threads: a 2^19-bit table");
 
-uint32_t stage1_words_for(const Geom& g, int threads, bool dense) {
-    return (uint32_t)(((uint64_t)g.cache_bits >> stage1_shift_for(g, threads, dense)) / 32);
+uint32_t stage1_words_for(const Geom& g, int threads) {
+    return (uint32_t)(((uint64_t)g.cache_bits >> stage1_shift_for(g, threads)) / 32);
 }
 
-int dense_probe_order(const Geom& g, double cache_fill, double ext_fill) {
-    // Cost of a plan per valid window, in L2 probes: the first probe always, the second when the first
-    // passes, and a queued window's full test (about three probes' worth of issue and flush work) when both
-    // pass. A probe of a region that the L1 left beside the shared memory can largely hold (about 64 KiB)
-    // mostly hits there.
+ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, double ext_fill) {
+    // Costs per window in units of one L2 probe per window (3.1 ps on the whole GPU: 148 SMs, each looking up one
+    // random sector per clock). Measured against the model: words, 1M patterns, order 1: 354 GB/s; 150k printable
+    // patterns in 2^23 + 2^27 bits, order 3: 511 GB/s (order 1: 323); 40k in 2^22 + 2^26, mode 3: 622, order 3: 630;
+    // 8k in 2^20 + 2^24, mode 3: 879, order 3: 638.
+    // Orders 0 and 1: the first probe always, the second when the first passes, and a queued window's full test
+    // (about three probes' worth of issue and flush work) when both pass. A probe of a region that the L1 left
+    // beside the shared memory can largely hold (about 64 KiB) mostly hits there.
     const double c_bytes = g.cache_bits / 8.0, e_bytes = (g.ext_mask + 1.0) / 8.0;
     auto fill = [&](uint32_t i) { return i < g.s ? cache_fill : ext_fill; };
     auto miss = [&](uint32_t i) { return 1.0 - std::min(1.0, 65536.0 / (i < g.s ? c_bytes : e_bytes)); };
     auto cost = [&](uint32_t a, uint32_t b) {
-        return miss(a) + fill(a) * miss(b) + 3.0 * fill(a) * fill(b);
+        return std::max(0.45, miss(a) + fill(a) * miss(b) + 3.0 * fill(a) * fill(b));
     };
-    int best = 0;
+    ScanChoice best{1, 0};
     double best_cost = cost(0, 1);
     if (g.k >= 4 && cost(2, 3) < best_cost) {
-        best = 1;
+        best.order = 1;
         best_cost = cost(2, 3);
     }
-    // Order 2: f0's load only where the folded cache region (the table the 384-thread dense kernel has room
-    // for) has its bit set, at about 0.15 probes' worth of shared-memory work per window. A table bit ORs
-    // C/T cache bits, so it is set with probability 1 - (1 - fill)^(C/T).
-    const double folds = (double)(1u << stage1_shift_for(g, 384, true));
-    const double fold_fill = 1.0 - std::pow(1.0 - cache_fill, folds);
-    const double c2 = 0.15 + fold_fill * miss(0) + fill(0) * miss(1) + 3.0 * fill(0) * fill(1);
-    if (c2 < best_cost) best = 2;
+    // Orders 2 and 3: both table bits, then one L2 probe for the windows that pass. A bit of the prefiltered dense
+    // kernel's table ORs C/T cache bits, so it is set with probability 1 - (1 - fill)^(C/T).
+    auto both = [&](double f) { return g.s > 1 ? f * f : f; };
+    const double pre_fill = 1.0 - std::pow(1.0 - cache_fill, (double)(1u << stage1_shift_for(g, 384)));
+    const double pre = 0.48 + 1.45 * both(pre_fill);
+    if (pre < best_cost) {
+        best.order = g.k >= 4 ? 3 : 2;
+        best_cost = pre;
+    }
+    // Sparse: both table bits; a window that passes costs its lane's queue append and its share of a flush.
+    if (g.k < 2 || 0.345 + 7.35 * both(table_fill) <= best_cost) best.mode = 3;
     return best;
 }
 
 int config_threads(const FastConfig& cfg) {
-    if (cfg.mode == 1) return cfg.threads == 256 ? 256 : cfg.threads == 192 && cfg.order != 2 ? 192 : 384;
+    if (cfg.mode == 1) return cfg.threads == 256 ? 256 : cfg.threads == 192 && cfg.order < 2 ? 192 : 384;
     if (cfg.mode == 2) return cfg.threads == 192 || cfg.threads == 384 ? cfg.threads : 256;
-    if (cfg.mode == 3) return 512;
+    if (cfg.mode == 3) return cfg.threads == 768 ? 768 : 512;
     return cfg.threads == 384 || cfg.threads == 512 ? cfg.threads : 256;
 }
 
 int fast_ctas_per_sm(const FastConfig& cfg) { return cfg.mode == 1 && config_threads(cfg) == 192 ? 2 : 1; }
+
+namespace {
+
+// What the busiest CTA slot of a scan alone on the GPU takes, in quarter rows: waves of equal items, each its rows
+// and its halo, whose up to 32 hashed bytes are a quarter of a row's work (measured: 256 MiB of the plain workload, 2
+// waves of 16 rows against 7 of 4, took 571 against 528 us).
+uint64_t wave_cost(uint64_t n, int threads, uint64_t slots, uint32_t rows) {
+    const uint64_t items = (n / kScanTile * kScanTile / ((uint64_t)rows * kRowBytes) + threads - 1) / threads;
+    return (items + slots - 1) / slots * (4 * rows + 1);
+}
+
+}  // namespace
+
+FastConfig launch_config(const FastConfig& cfg, uint64_t n, int num_sms, bool batch) {
+    // Mode 3 runs 768 threads where 24 warps per SM, which hide more of the hash's and the tables' latency than 16
+    // (plain 4 GiB: 911 -> 931 GB/s; LEN 24, 40k patterns in 2^22 + 2^26 bits: 560 -> 623, so about 1.07), finish
+    // before 16 warps with smaller items would (plain 64 MiB: 144 us with 512 threads, 164 with 768). In a batch
+    // other jobs fill the GPU, so the job only has to have four items of its own.
+    FastConfig c = cfg;
+    if (c.mode != 3) return c;
+    FastConfig wide = cfg;
+    wide.threads = 768;
+    if (batch) return n >= 4ull * 4 * kRowBytes * 768 ? wide : c;
+    const uint64_t cost = wave_cost(n, 512, num_sms, fast_rows(n, c, num_sms, false)) * 512 * 107;
+    const uint64_t wide_cost = wave_cost(n, 768, num_sms, fast_rows(n, wide, num_sms, false)) * 768 * 100;
+    return wide_cost < cost ? wide : c;
+}
 
 uint32_t fast_rows(uint64_t n, const FastConfig& cfg, int num_sms, bool batch) {
     const int threads = config_threads(cfg);
@@ -1017,21 +884,11 @@ uint32_t fast_rows(uint64_t n, const FastConfig& cfg, int num_sms, bool batch) {
         while (rows > 4 && tiles_bytes < 4ull * rows * kRowBytes * threads) rows >>= 1;
         return rows;
     }
-    // alone: the scan lasts as many waves of equal items as the busiest CTA takes, and an item costs its
-    // rows plus its halo, whose 32 hashed bytes are a quarter of a row's work (measured: 256 MiB of the
-    // plain workload, 2 waves of 16 rows against 7 of 4, took 571 against 528 us). The row count with the
-    // least work per CTA wins; ties go to the longer items.
+    // alone: the row count with the least work per CTA slot; ties go to the longer items
     const uint64_t slots = (uint64_t)num_sms * (uint64_t)fast_ctas_per_sm(cfg);
     uint32_t best = 16;
-    uint64_t best_cost = ~0ull;
-    for (uint32_t rows = 16; rows >= 4; rows >>= 1) {
-        const uint64_t items = (tiles_bytes / ((uint64_t)rows * kRowBytes) + threads - 1) / threads;
-        const uint64_t cost = (items + slots - 1) / slots * (4 * rows + 1);  // in quarter rows
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = rows;
-        }
-    }
+    for (uint32_t rows = 8; rows >= 4; rows >>= 1)
+        if (wave_cost(n, threads, slots, rows) < wave_cost(n, threads, slots, best)) best = rows;
     return best;
 }
 
@@ -1052,18 +909,19 @@ uint64_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const Fa
     job->g = a.g;
     job->main_words = a.main_words;
     job->ff_words = a.ff_words;
+    job->text = a.text;
     job->stage1_words = stage1_words;
     // the table the kernel reads: the sparse mode's, or the dense mode's prefilter (order 2)
-    const bool reads_table = cfg.mode != 1 || cfg.order == 2;
-    job->stage1_shift = reads_table ? stage1_shift_for(a.g, threads, cfg.mode == 1) : 0;
+    const bool reads_table = cfg.mode != 1 || cfg.order >= 2;
+    job->stage1_shift = reads_table ? stage1_shift_for(a.g, threads == 768 ? 512 : threads) : 0;
     job->stage1_nwords = reads_table ? (uint32_t)(((uint64_t)a.g.cache_bits >> job->stage1_shift) / 32) : 0;
     {
         // dense mode: regions of the pipelined probes, index functions f0/f1 (order 0) or f2/f3 (order 1,
         // which only K >= 4 filters set)
         if (cfg.mode < 0 || cfg.mode > 3 ||
-            (cfg.mode == 1 && (a.g.k < 2 || (cfg.order == 1 && a.g.k < 4) || cfg.order < 0 || cfg.order > 2)))
+            (cfg.mode == 1 && (a.g.k < 2 || ((cfg.order & 1) && a.g.k < 4) || cfg.order < 0 || cfg.order > 3)))
             *err = cudaErrorInvalidValue;
-        const uint32_t fa = cfg.order == 1 ? 2u : 0u, fb = fa + 1;
+        const uint32_t fa = (cfg.order & 1) ? 2u : 0u, fb = fa + 1;
         job->a_mask = fa < a.g.s ? a.g.cache_mask : a.g.ext_mask;
         job->a_add = fa < a.g.s ? 0u : a.g.cache_bits;
         job->b_mask = fb < a.g.s ? a.g.cache_mask : a.g.ext_mask;
@@ -1082,13 +940,13 @@ uint64_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const Fa
     }();
     job->text_evict_first = evict_first ? 1u : 0u;
     if (n_streams > 0) {
-        const uint32_t box_streams = threads > 256 ? (uint32_t)threads / 2 : (uint32_t)threads;
+        const uint32_t box_streams = (uint32_t)box_streams_for(threads);
         cuuint64_t dims[3] = {(cuuint64_t)kRowBytes, (cuuint64_t)rows, (cuuint64_t)n_streams};
         cuuint64_t strides[2] = {(cuuint64_t)kRowBytes, (cuuint64_t)slen};
-        cuuint32_t box[3] = {(cuuint32_t)kRowBytes, 1u, box_streams};
+        cuuint32_t box[3] = {(cuuint32_t)kPart, 1u, box_streams};
         cuuint32_t estr[3] = {1u, 1u, 1u};
         CUresult cr = encoder()(&job->tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void*)a.text, dims, strides, box, estr,
-                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) *err = cudaErrorInvalidValue;
     }
@@ -1120,9 +978,9 @@ cudaError_t scan_tail(const ScanArgs& a, uint64_t covered, cudaStream_t st) {
     return scan_generic(t, grid, st);
 }
 
-cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, int num_sms,
+cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& base, int num_sms,
                       FastJob* h_job, FastJob* d_job, cudaStream_t st) {
-    const int threads = config_threads(cfg);
+    const FastConfig cfg = launch_config(base, a.n, num_sms, false);
     const uint32_t rows = cfg.rows ? cfg.rows : fast_rows(a.n, cfg, num_sms, false);
     cudaError_t e;
     const uint64_t covered = fill_fast_job(a, stage1_words, cfg, rows, h_job, &e);
@@ -1149,9 +1007,8 @@ __global__ void k_stage1_fold(const uint32_t* main_words, uint32_t sh, uint32_t*
     out[w] = v;
 }
 
-cudaError_t build_stage1(const uint32_t* main_words, const Geom& g, int threads, bool dense, uint32_t* out,
-                         cudaStream_t st) {
-    const uint32_t sh = stage1_shift_for(g, threads, dense);
+cudaError_t build_stage1(const uint32_t* main_words, const Geom& g, int threads, uint32_t* out, cudaStream_t st) {
+    const uint32_t sh = stage1_shift_for(g, threads);
     const uint32_t nwords = (uint32_t)(((uint64_t)g.cache_bits >> sh) / 32);
     if (sh == 0) return cudaMemcpyAsync(out, main_words, 4ull * nwords, cudaMemcpyDeviceToDevice, st);
     k_stage1_fold<<<(nwords + 255) / 256, 256, 0, st>>>(main_words, sh, out, nwords);

@@ -18,6 +18,7 @@ struct alignas(64) FastJob {
     Geom g;
     const uint32_t* main_words;
     uint32_t* ff_words;
+    const uint8_t* text;     // the text's first byte (the sparse modes read candidate windows back)
     const uint32_t* stage1_words;  // sparse mode: cache region copy or its fold (global), copied into smem
     uint32_t stage1_nwords;
     uint32_t stage1_shift;         // the table holds C >> shift bits (0: exact copy of the cache region)
@@ -39,12 +40,13 @@ struct alignas(64) FastJob {
     const uint32_t* ready;
 };
 
-// How a job is scanned: CTA size (256/384/512), probe mode (0: sparse, shared-memory stage 1; 1: dense,
-// pipelined L2 probes), rows per stream (0: chosen from the text size), and in the dense mode the probe order
-// (0: the pipelined probes are index functions f0 = h1 and f1 = h2; 1: f2 = rot16(h1) and f3 = rot16(h2),
-// the better pair when their region is sparser; 2: f0 and f1, with f0's load issued only when a folded copy
-// of the cache region in shared memory has its bit set). The order only changes which bits are tested
-// first: a window hits iff all K bits are set, in any order.
+// How a job is scanned: CTA size, probe mode, rows per stream (0: chosen from the text size), and in the dense mode
+// the probe order. Modes 0, 2 and 3 are the sparse kernel (shared-memory stage 1) at 256/384/512, 192/256/384 and 512
+// threads, the last grown to 768 for large texts (launch_config); mode 1 is the dense one (pipelined L2 probes). Orders:
+// 0: the pipelined probes are index functions f0 = h1 and f1 = h2; 1: f2 = rot16(h1) and f3 = rot16(h2), the better
+// pair when their region is sparser; 2 and 3: f0 and f1 are tested against the stage-1 table first, and f0 (order 2)
+// or f2 (order 3) is then probed for the windows that pass. The order only changes which bits are tested first: a
+// window hits iff all K bits are set, in any order.
 struct FastConfig {
     int threads;
     int mode;
@@ -52,23 +54,27 @@ struct FastConfig {
     int order;
 };
 
-// Probe order for the dense mode from the fills (fraction of set bits) of the cache and external regions:
-// the plan with the fewest expected L2 probes per window. Order 1 needs f2 and f3 among the K index
-// functions (K >= 4).
-int dense_probe_order(const Geom& g, double cache_fill, double ext_fill);
+// Mode (1 or 3) and dense probe order with the least expected time per window, from the fills (fraction of set bits)
+// of the 512-thread kernel's stage-1 table, of the cache region and of the external region. Orders 1 and 3 need f2
+// and f3 among the K index functions (K >= 4).
+struct ScanChoice {
+    int mode, order;
+};
+ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, double ext_fill);
 
 // True when the tuned kernel handles this geometry and text size; otherwise the generic scan runs.
 bool fast_scan_supported(const Geom& g, uint64_t n);
 
 int config_threads(const FastConfig& cfg);
 
+// The configuration a text of n bytes is launched with, alone on the GPU or in a batch (see mode 3 above).
+FastConfig launch_config(const FastConfig& cfg, uint64_t n, int num_sms, bool batch);
+
 // Stage-1 table for a CTA size: a copy of the cache region when it fits in the shared memory the kernel
-// leaves over (the sparse kernel's, or with `dense` the dense kernel's, whose table prefilters f0 in probe
-// order 2), otherwise its fold to C >> shift bits.
-uint32_t stage1_shift_for(const Geom& g, int threads, bool dense = false);
-uint32_t stage1_words_for(const Geom& g, int threads, bool dense = false);
-cudaError_t build_stage1(const uint32_t* main_words, const Geom& g, int threads, bool dense, uint32_t* out,
-                         cudaStream_t st);
+// leaves over, otherwise its fold to C >> shift bits.
+uint32_t stage1_shift_for(const Geom& g, int threads);
+uint32_t stage1_words_for(const Geom& g, int threads);
+cudaError_t build_stage1(const uint32_t* main_words, const Geom& g, int threads, uint32_t* out, cudaStream_t st);
 
 // CTAs of the tuned kernel resident per SM for a configuration (two for the 192-thread dense kernel).
 int fast_ctas_per_sm(const FastConfig& cfg);

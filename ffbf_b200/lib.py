@@ -370,15 +370,14 @@ class Filter:
         self._check(self._lib.ffbf_debug_scan_unpublished(self._h, ctypes.c_void_p(dev_ptr), n, spins))
 
     def config(self):
-        """(threads, mode) of the tuned scan for this filter (mode 0: shared-memory stage, 1: L2 probes, 2:
-        shared-memory stage with candidates deferred to the end of each 32-byte block, 3: mode 0 with
-        per-stage barriers instead of a block barrier per stage)."""
+        """(threads, mode) of the tuned scan for this filter (mode 1: L2 probes; 0, 2, 3: shared-memory stage,
+        which differ in the CTA sizes they take)."""
         t, m = ctypes.c_int(), ctypes.c_int()
         self._check(self._lib.ffbf_get_scan_config(self._h, ctypes.byref(t), ctypes.byref(m)))
         return t.value, m.value
 
     def probe_order(self):
-        """The dense mode's probe plan (0: f0/f1; 1: f2/f3; 2: f0/f1 behind a shared-memory prefilter)."""
+        """The dense mode's probe plan (0: f0/f1; 1: f2/f3; 2: one probe behind a shared-memory prefilter)."""
         o = ctypes.c_int()
         self._check(self._lib.ffbf_get_probe_order(self._h, ctypes.byref(o)))
         return o.value

@@ -265,16 +265,15 @@ ffbf_status ffbf_autotune(ffbf_ctx* ctx, const uint8_t* d_text, size_t sample_le
  * FFBF_ETIMEOUT and the context stays usable. Nothing is scanned and no result is kept. */
 ffbf_status ffbf_debug_scan_unpublished(ffbf_ctx* ctx, const uint8_t* d_text, size_t len, uint32_t spins);
 
-/* The tuned scan's current configuration for this context (CTA threads; mode 0 shared-memory stage 1 with
- * candidates queued per byte, 1 pipelined L2 probes, 2 shared-memory stage 1 with candidates deferred to the
- * end of each 32-byte block, 3 mode 0 at 512 threads whose warps meet through per-stage barriers), as the
- * autotuner or the filter's fill chose it. Before the first scan or tuning
+/* The tuned scan's current configuration for this context (CTA threads; mode 1 pipelined L2 probes, modes 0, 2 and 3
+ * shared-memory stage 1, which differ in the CTA sizes they take: 256/384/512, 192/256/384 and 512; a mode 3 scan
+ * of a large text runs CTAs of 768), as the autotuner or the filter's fill chose it. Before the first scan or tuning
  * it reports the defaults. */
 ffbf_status ffbf_get_scan_config(const ffbf_ctx* ctx, int* threads, int* mode);
 
 /* The dense mode's probe plan for this context's filter: 0 pipelines the loads of index functions f0 = h1
- * and f1 = h2, 1 those of f2 = rot16(h1) and f3 = rot16(h2) (K >= 4), 2 those of f0 and f1 with f0's load
- * skipped where a folded copy of the cache region in shared memory has its bit clear. Chosen from the
+ * and f1 = h2, 1 those of f2 = rot16(h1) and f3 = rot16(h2) (K >= 4), 2 tests f0 and f1 against a copy or fold of the
+ * cache region in shared memory and pipelines one load for the windows that pass. Chosen from the
  * fills of the filter's regions when the filter is prepared for a scan (FFBF_SCAN_ORDER=0|1|2 fixes it);
  * a window hits iff all K bits are set, so the plan changes the work, never the result. */
 ffbf_status ffbf_get_probe_order(const ffbf_ctx* ctx, int* order);
