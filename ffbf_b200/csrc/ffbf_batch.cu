@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <map>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -50,6 +51,14 @@ struct ffbf_batch {
     uint64_t graph_kernels = 0;  // kernel nodes of the graph
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    // every job's results, collected by one launch after the graph (ffbf_batch_wait)
+    std::shared_ptr<PinnedBlock> results;
+    std::vector<std::pair<size_t, uint32_t>> result_at;  // per job: offset in the block, capacity
+    ffbf::CollectJob* d_collect = nullptr;
+    uint2* d_collect_items = nullptr;
+    uint32_t n_collect_items = 0;
+    bool uncollected = false;  // launched since the last collection
+    uint32_t* h_ctl = nullptr;  // pinned copy of the control words, at the block's end
     // branch streams and events used while capturing the graph's parallel branches
     std::vector<cudaStream_t> branches;
     std::vector<cudaEvent_t> events;
@@ -180,6 +189,10 @@ void batch_release(ffbf_batch* b) {
     for (void* p : b->allocs) cudaFree(p);
     b->allocs.clear();
     b->d_error = nullptr;
+    b->results.reset();
+    b->result_at.clear();
+    b->n_collect_items = 0;
+    b->uncollected = false;
     b->prepared = false;
     b->keys.clear();
     cudaGetLastError();
@@ -278,6 +291,38 @@ ffbf_status ffbf_batch_prepare(ffbf_batch* b) {
         cudaGetLastError();
         return bfail(b, FFBF_ECUDA, "batch table upload failed");
     }
+    // the jobs' results: room for one hit window per 8 KiB of text, at least 512; a job with more takes the plain collect
+    {
+        std::vector<ffbf::CollectJob> cj;
+        std::vector<uint2> items;
+        size_t bytes = 0;
+        for (const auto& j : b->jobs) {
+            const uint32_t cap = (uint32_t)std::min<uint64_t>(ffbf::kSmallResults, std::max<uint64_t>(512, j.len / 8192));
+            b->result_at.push_back({bytes, cap});
+            bytes += 64 + 3 * 8 * (size_t)cap;
+        }
+        auto block = std::make_shared<PinnedBlock>();
+        if (cudaMallocHost(&block->p, bytes + 16 * b->n_ctl) != cudaSuccess) {
+            cudaGetLastError();
+            block->p = nullptr;
+            return bfail(b, FFBF_ENOMEM_HOST, "pinned batch results");
+        }
+        b->results = block;
+        b->h_ctl = reinterpret_cast<uint32_t*>(block->p + bytes);
+        for (size_t i = 0; i < b->jobs.size(); i++) {
+            const auto [at, cap] = b->result_at[i];
+            cj.push_back(collect_job(plan.args[i], b->jobs[i].c->d_hitlines, block->p + at, cap, ffbf::kCollectBatch));
+            for (uint32_t k = 0; k < ffbf::collect_ctas(cj.back()); k++) items.push_back(make_uint2((uint32_t)i, k));
+        }
+        b->n_collect_items = (uint32_t)items.size();
+        TRY(balloc(b, &b->d_collect, cj.size() + 1));
+        TRY(balloc(b, &b->d_collect_items, items.size() + 1));
+        if (!up(b->d_collect, cj.data(), cj.size() * sizeof(ffbf::CollectJob)) ||
+            !up(b->d_collect_items, items.data(), items.size() * sizeof(uint2))) {
+            cudaGetLastError();
+            return bfail(b, FFBF_ECUDA, "batch table upload failed");
+        }
+    }
     // one graph: zero the jobs' counters, one tuned launch per group, one generic launch for all tail tiles
     if (cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         return bfail(b, FFBF_ECUDA, "stream capture failed to start");
@@ -331,23 +376,35 @@ ffbf_status ffbf_batch_launch(ffbf_batch* b) {
         return bfail(b, FFBF_ECUDA, "graph launch failed");
     }
     ffbf::note_launches(b->graph_kernels);
+    b->uncollected = true;
     return FFBF_OK;
 }
 
 ffbf_status ffbf_batch_wait(ffbf_batch* b) {
     if (!b) return FFBF_EINVAL;
     cudaError_t e = cudaSetDevice(b->device);
+    // every job's results by one launch, and the control words, behind the graph: one wait for all of them
+    const bool collect = b->results && b->uncollected;
+    if (e == cudaSuccess && collect)
+        e = ffbf::collect_hits_multi(b->d_collect, b->d_collect_items, b->n_collect_items, b->st);
+    if (e == cudaSuccess && b->results)
+        e = cudaMemcpyAsync(b->h_ctl, b->d_error, 16 * b->n_ctl, cudaMemcpyDeviceToHost, b->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return bfail(b, FFBF_ECUDA, std::string("batch execution failed: ") + cudaGetErrorString(e));
     }
     uint32_t flag = 0;
-    if (b->d_error) {
-        std::vector<uint32_t> ctl(4 * b->n_ctl);
-        if (cudaMemcpy(ctl.data(), b->d_error, 16 * b->n_ctl, cudaMemcpyDeviceToHost) != cudaSuccess)
-            return bfail(b, FFBF_ECUDA, "error flag read failed");
-        for (uint32_t i = 0; i < b->n_ctl; i++) flag |= ctl[4 * i];
+    if (b->results) {
+        for (uint32_t i = 0; i < b->n_ctl; i++) flag |= b->h_ctl[4 * i];
+        b->uncollected = false;
+        for (size_t i = 0; i < b->jobs.size() && collect && !flag; i++) {
+            ffbf_ctx* c = b->jobs[i].c;
+            if (!c->scan_pending) continue;  // collected already
+            c->ready_block = b->results;
+            c->ready = b->results->p + b->result_at[i].first;
+            c->ready_cap = b->result_at[i].second;
+        }
     }
     if (flag) {
         char buf[96];

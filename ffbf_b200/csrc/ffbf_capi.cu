@@ -20,6 +20,7 @@
 #include "ffbf_kernels.cuh"
 #include "ffbf_scan_fast.cuh"
 
+#include "ffbf_collect.cuh"
 #include "ffbf_ctx.cuh"
 #include "ffbf_order.cuh"
 
@@ -76,6 +77,23 @@ ffbf_status ensure_order(ffbf_ctx* c, size_t bytes) {
     TRY(dalloc_t(c, &c->d_order, bytes));
     c->order_bytes = bytes;
     return FFBF_OK;
+}
+
+// The pinned buffer of the single-launch results.
+ffbf_status ensure_results(ffbf_ctx* c) {
+    if (c->h_res) return FFBF_OK;
+    if (cudaMallocHost(&c->h_res, ffbf::kResultBytes) != cudaSuccess) {
+        cudaGetLastError();
+        c->h_res = nullptr;
+        return fail(c, FFBF_ENOMEM_HOST, "pinned result buffer");
+    }
+    return FFBF_OK;
+}
+
+ffbf::ResultHead* result_head(ffbf_ctx* c) { return reinterpret_cast<ffbf::ResultHead*>(c->h_res); }
+
+uint64_t* result_array(ffbf_ctx* c, int i) {
+    return reinterpret_cast<uint64_t*>(c->h_res + 64) + (size_t)i * ffbf::kSmallResults;
 }
 
 ffbf_status enter(ffbf_ctx* c) {
@@ -164,6 +182,8 @@ void order_hits(const HitRec* hr, const HitLine* hl, uint32_t nh, std::vector<ui
 void reset_scan(ffbf_ctx* c) {
     c->have_scan = false;
     c->scan_pending = false;
+    c->ready = nullptr;
+    c->ready_block.reset();
     c->have_prune = false;
     c->r_hits.clear();
     c->r_ls.clear();
@@ -250,6 +270,13 @@ ffbf::ScanArgs make_scan_args(ffbf_ctx* c) {
     a.tile_begin = 0;
     a.cache_in_smem = c->g.cache_bits <= ffbf::kSmemCacheMaxBits;
     return a;
+}
+
+ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta) {
+    uint64_t* arrays = reinterpret_cast<uint64_t*>(res + 64);
+    return ffbf::CollectJob{a.text, a.n, a.g.len, a.hits_cap, a.hits, lines, a.counters, a.tile_first_nl, a.tile_last_nl,
+                            a.ntiles, reinterpret_cast<ffbf::ResultHead*>(res), arrays, arrays + cap,
+                            arrays + 2 * (size_t)cap, cap, per_cta};
 }
 
 bool use_fast(const ffbf_ctx* c, uint64_t n) { return ffbf::fast_scan_supported(c->g, n) && !c->force_generic; }
@@ -462,6 +489,7 @@ void ffbf_destroy(ffbf_ctx* c) {
     for (auto& kv : c->allocs) cudaFree(kv.first);
     c->allocs.clear();
     if (c->h_counters) cudaFreeHost(c->h_counters);
+    if (c->h_res) cudaFreeHost(c->h_res);
     if (c->h_job) cudaFreeHost(c->h_job);
     if (c->h_jobs) cudaFreeHost(c->h_jobs);
     for (auto ev : c->pipe_events) cudaEventDestroy(ev);
@@ -678,6 +706,34 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
     NvtxRange nvtx_("ffbf_scan_collect");
     TRY(enter(c));
     if (!c->scan_pending && !c->have_scan) return fail(c, FFBF_ESTATE, "no scan to collect");
+    const uint64_t ntiles = (c->text_len + ffbf::kScanTile - 1) / ffbf::kScanTile;
+    if (c->scan_pending && !c->host_order && !c->keep_records) {
+        // one launch finishes a result of up to kSmallResults windows, unless the scan's batch has done it already;
+        // the general path below takes the others
+        const uint8_t* res = c->ready;
+        uint32_t cap = c->ready_cap;
+        if (!res) {
+            TRY(ensure_results(c));
+            res = c->h_res;
+            cap = ffbf::kSmallResults;
+            CUDA_TRY(c, ffbf::collect_hits(collect_job(make_scan_args(c), c->d_hitlines, c->h_res, cap,
+                                                          ffbf::kCollectAlone),
+                                              c->st));
+            TRY(sync(c));
+        }
+        const ffbf::ResultHead* head = reinterpret_cast<const ffbf::ResultHead*>(res);
+        if (head->done) {
+            const uint64_t* a = reinterpret_cast<const uint64_t*>(res + 64);
+            c->nhits = (uint32_t)head->n;
+            c->r_hits.assign(a, a + head->n);
+            c->r_ls.assign(a + cap, a + cap + head->n_lines);
+            c->r_le.assign(a + 2 * (size_t)cap, a + 2 * (size_t)cap + head->n_lines);
+            c->ready = nullptr;
+            c->ready_block.reset();
+            c->scan_pending = false;
+            c->have_scan = true;
+        }
+    }
     if (c->scan_pending) {
         CUDA_TRY(c, cudaMemcpyAsync(c->h_counters, c->d_counters, ffbf::CNT_WORDS * 4, cudaMemcpyDeviceToHost, c->st));
         TRY(sync(c));
@@ -699,7 +755,6 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
             nh = c->h_counters[ffbf::CNT_HITS];
         }
         c->nhits = nh;
-        const uint64_t ntiles = (c->text_len + ffbf::kScanTile - 1) / ffbf::kScanTile;
         CUDA_TRY(c, ffbf::resolve_lines(c->d_text, c->text_len, c->g.len, c->d_hits, nh, c->d_tiles,
                                         c->d_tiles + c->tiles_cap, c->d_tiles + 2 * c->tiles_cap,
                                         c->d_tiles + 3 * c->tiles_cap, ntiles, c->d_hitlines, c->st,
@@ -1022,37 +1077,47 @@ ffbf_status ffbf_prune(ffbf_ctx* c, ffbf_prune_result* out) {
     if (!c->have_patterns) return fail(c, FFBF_ESTATE, "ffbf_prune needs ffbf_set_patterns first");
     if (c->scan_pending) TRY(ffbf_scan_collect(c, nullptr));
     const uint64_t n = c->npat;
-    const uint64_t nb = ffbf::compact_blocks(n);
-    TRY(ensure_tmp(c, nb + 1));
-    // the flags and id buffers are kept between calls: a cudaFree would wait for the whole device
-    if (c->pflags_cap < n + 1) {
-        dfree(c, c->d_pflags);
-        c->pflags_cap = 0;
-        TRY(dalloc_t(c, &c->d_pflags, n + 1));
-        c->pflags_cap = n + 1;
-    }
-    uint8_t* d_flags = c->d_pflags;
-    ffbf_status s = FFBF_OK;
     uint64_t cnt = 0;
-    if (ffbf::prune_flags(c->d_pstart, c->d_pend, c->d_phash, n, c->g, c->d_ff, d_flags, c->st) != cudaSuccess ||
-        ffbf::count_flags(d_flags, n, c->d_tmp, c->st) != cudaSuccess ||
-        cudaMemcpyAsync(&cnt, c->d_tmp + nb, 8, cudaMemcpyDeviceToHost, c->st) != cudaSuccess ||
-        cudaStreamSynchronize(c->st) != cudaSuccess)
-        s = fail(c, FFBF_ECUDA, "prune failed: %s", cudaGetErrorString(cudaGetLastError()));
-    if (s == FFBF_OK && c->ids_cap < cnt + 1) {
-        dfree(c, c->d_ids);
-        c->ids_cap = 0;
-        s = dalloc_t(c, &c->d_ids, cnt + 1);
-        if (s == FFBF_OK) c->ids_cap = cnt + 1;
+    if (n) {
+        TRY(ensure_results(c));
+        TRY(ensure_tmp(c, ffbf::prune_blocks(n)));
+        uint32_t* counts = reinterpret_cast<uint32_t*>(c->d_tmp);
+        // the bit and id buffers are kept between calls: a cudaFree would wait for the whole device
+        const uint64_t words = (n + 31) / 32;
+        if (c->pbits_cap < words) {
+            dfree(c, c->d_pbits);
+            c->pbits_cap = 0;
+            TRY(dalloc_t(c, &c->d_pbits, words));
+            c->pbits_cap = words;
+        }
+        auto ids_room = [&](uint64_t want) -> ffbf_status {
+            dfree(c, c->d_ids);
+            c->ids_cap = 0;
+            TRY(dalloc_t(c, &c->d_ids, want));
+            c->ids_cap = want;
+            return FFBF_OK;
+        };
+        if (!c->d_ids && ids_room(std::min<uint64_t>(n, ffbf::kSmallIds)) != FFBF_OK) c->err.clear();
+        CUDA_TRY(c, ffbf::prune_count(c->d_pstart, c->d_pend, c->d_phash, n, c->g, c->d_ff, c->d_pbits, counts, c->st));
+        CUDA_TRY(c, ffbf::prune_emit(c->d_pbits, counts, n, c->d_ids, c->ids_cap, result_head(c), result_array(c, 0),
+                                     c->st));
+        TRY(sync(c));
+        cnt = result_head(c)->n;
+        if (c->ids_cap < cnt) {
+            TRY(ids_room(cnt));
+            CUDA_TRY(c, ffbf::prune_emit(c->d_pbits, counts, n, c->d_ids, c->ids_cap, result_head(c),
+                                         result_array(c, 0), c->st));
+        }
+        if (cnt <= ffbf::kSmallIds) {
+            c->r_ids.assign(result_array(c, 0), result_array(c, 0) + cnt);
+        } else {
+            c->r_ids.resize(cnt);
+            CUDA_TRY(c, cudaMemcpyAsync(c->r_ids.data(), c->d_ids, cnt * 8, cudaMemcpyDeviceToHost, c->st));
+            TRY(sync(c));
+        }
+    } else {
+        c->r_ids.clear();
     }
-    if (s == FFBF_OK) {
-        c->r_ids.resize(cnt);
-        if (ffbf::emit_flags(d_flags, n, c->d_ids, c->d_tmp, c->st) != cudaSuccess ||
-            (cnt && cudaMemcpyAsync(c->r_ids.data(), c->d_ids, cnt * 8, cudaMemcpyDeviceToHost, c->st) != cudaSuccess) ||
-            cudaStreamSynchronize(c->st) != cudaSuccess)
-            s = fail(c, FFBF_ECUDA, "prune compaction failed: %s", cudaGetErrorString(cudaGetLastError()));
-    }
-    if (s != FFBF_OK) return s;
     c->nids = cnt;
     c->have_prune = true;
     if (out) {
@@ -1099,7 +1164,8 @@ ffbf_status ffbf_format_pruned(ffbf_ctx* c, size_t chunk, uint8_t** out, size_t*
 namespace {
 
 // Verifies nh hit records already in c->d_hits against a device text, appending (offset + base, pattern)
-// pairs. The match buffers grow and the pass reruns when they overflow.
+// pairs. The match buffers grow and the pass reruns when they overflow. The counters are zero but for the table
+// build's error flags, which come back with the first pass.
 ffbf_status verify_pass(ffbf_ctx* c, uint32_t nh, const uint8_t* d_text, uint64_t text_len, uint64_t tsize,
                         uint64_t base, std::vector<uint64_t>& off_out, std::vector<uint32_t>& pid_out) {
     if (c->match_cap < std::max<uint32_t>(1024, nh)) {
@@ -1112,14 +1178,17 @@ ffbf_status verify_pass(ffbf_ctx* c, uint32_t nh, const uint8_t* d_text, uint64_
         c->match_cap = cap;
     }
     for (int attempt = 0; attempt < 2; attempt++) {
+        CUDA_TRY(c, ffbf::verify_collect(ffbf::VerifyJob{c->d_hits, nh, c->match_cap, d_text, text_len, c->d_keys,
+                                                         c->d_vals, tsize - 1, c->d_pat, c->d_pstart, c->d_pend,
+                                                         c->d_moff, c->d_mpid, c->d_counters, result_head(c),
+                                                         result_array(c, 0), result_array(c, 1)},
+                                         c->st));
         CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * 4, c->st));
-        CUDA_TRY(c, ffbf::verify_hits(c->d_hits, nh, d_text, text_len, c->d_keys, c->d_vals, tsize - 1, c->d_pat,
-                                      c->d_pstart, c->d_pend, c->d_moff, c->d_mpid, c->match_cap, c->d_counters, c->st));
-        CUDA_TRY(c, cudaMemcpyAsync(c->h_counters, c->d_counters, ffbf::CNT_WORDS * 4, cudaMemcpyDeviceToHost, c->st));
         TRY(sync(c));
-        uint32_t nm = c->h_counters[ffbf::CNT_MATCHES];
+        if (result_head(c)->error) return fail(c, FFBF_ECUDA, "verification table overflow");
+        const uint64_t nm = result_head(c)->n;
         if (nm <= c->match_cap) break;
-        uint64_t cap = (uint64_t)nm + nm / 4 + 1024;
+        uint64_t cap = nm + nm / 4 + 1024;
         if (cap > 0xffffffffull) return fail(c, FFBF_EINVAL, "more than 2^32 matches");
         dfree(c, c->d_moff);
         dfree(c, c->d_mpid);
@@ -1128,7 +1197,12 @@ ffbf_status verify_pass(ffbf_ctx* c, uint32_t nh, const uint8_t* d_text, uint64_
         TRY(dalloc_t(c, &c->d_mpid, cap));
         c->match_cap = (uint32_t)cap;
     }
-    const uint32_t nm = c->h_counters[ffbf::CNT_MATCHES];
+    const uint32_t nm = (uint32_t)result_head(c)->n;
+    if (result_head(c)->done && !c->host_order) {
+        for (uint32_t i = 0; i < nm; i++) off_out.push_back(result_array(c, 0)[i] + base);
+        for (uint32_t i = 0; i < nm; i++) pid_out.push_back((uint32_t)result_array(c, 1)[i]);
+        return FFBF_OK;
+    }
     // (offset, pattern id) order on the device, or on the host as the hits' order is (see ffbf_scan_collect)
     const int kb = ffbf::key_bits_for(text_len);
     const size_t scratch = ffbf::order_matches_scratch(nm, kb);
@@ -1179,9 +1253,7 @@ ffbf_status ffbf_verify(ffbf_ctx* c, ffbf_matches* out) {
     CUDA_TRY(c, cudaMemsetAsync(c->d_vals, 0xff, tsize * 4, c->st));
     CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * 4, c->st));
     CUDA_TRY(c, ffbf::table_build(c->d_ids, c->nids, c->d_phash, c->d_keys, c->d_vals, tsize - 1, c->d_counters, c->st));
-    CUDA_TRY(c, cudaMemcpyAsync(c->h_counters, c->d_counters, ffbf::CNT_WORDS * 4, cudaMemcpyDeviceToHost, c->st));
-    TRY(sync(c));
-    if (c->h_counters[ffbf::CNT_ERROR]) return fail(c, FFBF_ECUDA, "verification table overflow");
+    TRY(ensure_results(c));
     std::vector<uint64_t> off;
     std::vector<uint32_t> pid;
     if (!c->segmented) {

@@ -1,0 +1,384 @@
+// ffbf_collect.cu -- single-launch collection of scan results, matches and pruned ids (see ffbf_collect.cuh).
+//
+// A call on an ordinary text spends its time between kernels: the general path (tile scan, line resolution, radix
+// sorts, selection, copies) is about fifteen launches and three waits for the device, 130 us for 500 hit windows.
+// Here the records are finished by one launch that reads their number from the device: its CTAs share the
+// windows, and the last CTA to finish sorts them in its shared memory and writes the result to pinned host memory. The
+// sort is a bucket sort over the text's span, about two buckets per record, each then sorted by one thread (records of
+// one bucket are few unless a text is very uneven, which takes a bitonic network instead: for 8000 windows about 120 us
+// against 10). What bounds it is latency: the dependent loads of a line search, then four passes over the records.
+// 500 windows of a 64 MiB text: 132 -> 28 us a call, 8000 of 1 GiB: 276 -> 45.
+#include <climits>
+
+#include "ffbf_collect.cuh"
+#include "ffbf_text.cuh"
+
+namespace ffbf {
+
+namespace {
+
+constexpr int kThreads = 1024;
+constexpr uint64_t kWalkTiles = 64;              // tile summaries a line's end is searched in
+// bitonic keys: the offset above the record's index
+constexpr int kIndexBits = 14;
+static_assert(kSmallResults == 1u << kIndexBits, "an index fits beside an offset below 2^50");
+
+// Exclusive sum of v over the CTA; *total is the whole sum.
+__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_warp, uint32_t* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = v;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t w = lane < (int)(blockDim.x >> 5) ? s_warp[lane] : 0u;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, w, d);
+            if (lane >= d) w += y;
+        }
+        s_warp[lane] = w;
+    }
+    __syncthreads();
+    *total = s_warp[31];
+    return x - v + (warp ? s_warp[warp - 1] : 0u);
+}
+
+// True in the last of the launch's (or the job's) `ctas` CTAs to get here, which then sees the others' writes.
+__device__ __forceinline__ bool last_cta(uint32_t* ticket, uint32_t ctas, uint32_t* s_flag) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) *s_flag = atomicAdd(ticket, 1u) == ctas - 1;
+    __syncthreads();
+    __threadfence();
+    return *s_flag != 0;
+}
+
+__device__ __forceinline__ uint32_t pow2_at_least(uint32_t n) { return n < 2 ? 1u : 1u << (32 - __clz(n - 1)); }
+
+// Sorts s_key[0, n) ascending (n <= kSmallResults), where offset(q) is record q's offset, below 2^50, and its key is the
+// offset above q's 14 bits; less orders two keys. s_bucket holds kBuckets words. All of the CTA's threads call it.
+constexpr uint32_t kBuckets = 2 * kSmallResults;
+constexpr uint32_t kMaxBucket = 24;  // records one thread sorts by insertion
+
+template <class Offset, class Less>
+__device__ void sort_records(uint32_t n, uint64_t span, uint64_t* s_key, uint16_t* s_bucket, uint32_t* s_warp,
+                             Offset offset, Less less) {
+    // buckets of 2^shift offsets, more of them than records and a multiple of the threads
+    const uint32_t nb = max(2 * pow2_at_least(n), (uint32_t)kThreads);
+    uint32_t shift = 0;
+    while ((span >> shift) >= nb) shift++;
+    uint32_t* s_pair = reinterpret_cast<uint32_t*>(s_bucket);  // two 16-bit counts per word
+    for (uint32_t b = threadIdx.x; b < nb / 2; b += kThreads) s_pair[b] = 0;
+    __syncthreads();
+    uint32_t most = 0;
+    for (uint32_t q = threadIdx.x; q < n; q += kThreads) {
+        const uint32_t b = (uint32_t)(offset(q) >> shift);
+        const uint32_t old = atomicAdd(&s_pair[b >> 1], (b & 1) ? 0x10000u : 1u);
+        most = max(most, ((b & 1) ? old >> 16 : old & 0xffffu) + 1);
+    }
+    most = (uint32_t)__syncthreads_or((int)(most > kMaxBucket));
+    if (most) {
+        // uneven: a bitonic network over the next power of two
+        const uint32_t n2 = pow2_at_least(n);
+        for (uint32_t q = threadIdx.x; q < n2; q += kThreads) s_key[q] = q < n ? offset(q) << kIndexBits | q : ~0ull;
+        for (uint32_t k = 2; k <= n2; k <<= 1) {
+            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                __syncthreads();
+                for (uint32_t t = threadIdx.x; t < n2 / 2; t += kThreads) {
+                    const uint32_t lo = 2 * t - (t & (j - 1)), hi = lo + j;  // bit j of lo is clear
+                    const uint64_t x = s_key[lo], y = s_key[hi];
+                    if (less(y, x) == ((lo & k) == 0)) {
+                        s_key[lo] = y;
+                        s_key[hi] = x;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        return;
+    }
+    // each thread's consecutive buckets: counts to starts
+    const uint32_t per = nb / kThreads, b0 = threadIdx.x * per;
+    uint32_t mine = 0;
+    for (uint32_t b = b0; b < b0 + per; b++) mine += s_bucket[b];
+    uint32_t total;
+    uint32_t at = block_sum(mine, s_warp, &total);
+    for (uint32_t b = b0; b < b0 + per; b++) {
+        const uint32_t c = s_bucket[b];
+        s_bucket[b] = (uint16_t)at;
+        at += c;
+    }
+    __syncthreads();
+    // a bucket's word counts up to the next bucket's start while its records are placed
+    for (uint32_t q = threadIdx.x; q < n; q += kThreads) {
+        const uint64_t o = offset(q);
+        const uint32_t b = (uint32_t)(o >> shift);
+        const uint32_t old = atomicAdd(&s_pair[b >> 1], (b & 1) ? 0x10000u : 1u);
+        s_key[(b & 1) ? old >> 16 : old & 0xffffu] = o << kIndexBits | q;
+    }
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < nb; b += kThreads) {
+        const uint32_t lo = b ? s_bucket[b - 1] : 0u, hi = s_bucket[b];
+        for (uint32_t x = lo + 1; x < hi; x++) {
+            const uint64_t v = s_key[x];
+            uint32_t y = x;
+            for (; y > lo && less(v, s_key[y - 1]); y--) s_key[y] = s_key[y - 1];
+            s_key[y] = v;
+        }
+    }
+    __syncthreads();
+}
+
+// The ends of the line of the window at w, searched by eight lanes of a warp: lanes 0-3 go back from the byte before
+// the window, 64 bytes a step, and return the line's start; lanes 4-7 go forward from the byte behind it and return its
+// end. -1 when the tile of that first byte holds no '\n' on that side. One thread per window took 16-byte steps, each a
+// memory latency, and its warp as long as its longest line.
+__device__ __forceinline__ long long line_end_of_window(const CollectJob& a, uint64_t w, bool active) {
+    const bool back = (threadIdx.x & 4) == 0;
+    const long long n = (long long)a.n;
+    const long long pos = back ? (long long)w - 1 : (long long)(w + a.len);
+    const long long tile = pos / kScanTile * kScanTile;
+    const long long stop = back ? tile : min(n, tile + kScanTile);
+    long long res = -1, c = (pos & ~63LL) + 16 * (threadIdx.x & 3);
+    bool busy = active;
+    if (back ? pos < 0 : pos >= n) {  // the text's first and last byte end a line
+        res = back ? 0 : n;
+        busy = false;
+    }
+    while (__any_sync(0xffffffffu, busy)) {
+        long long at = back ? -1 : LLONG_MAX;
+        if (busy && c < n) {
+            const uint4 v = chunk16(a.text, c, n);
+            const uint32_t m8 = __dp4a(nl_bytes(v.y), 0x80402010u, __dp4a(nl_bytes(v.x), 0x08040201u, 0u)) >> 7;
+            const uint32_t m16 = __dp4a(nl_bytes(v.w), 0x80402010u, __dp4a(nl_bytes(v.z), 0x08040201u, 0u)) << 1;
+            uint32_t m = m8 | m16;
+            // bytes on the searched side of pos, and before `stop` going forward
+            if (back) m &= pos - c >= 15 ? 0xffffu : pos < c ? 0u : (2u << (pos - c)) - 1u;
+            else m &= (pos <= c ? 0xffffu : pos - c >= 16 ? 0u : 0xffffu << (pos - c)) &
+                      (stop - c >= 16 ? 0xffffu : stop <= c ? 0u : (1u << (stop - c)) - 1u);
+            if (m) at = c + (back ? 31 - __clz(m) : __ffs(m) - 1);
+        }
+        for (int d = 1; d < 4; d <<= 1) {
+            const long long o = __shfl_xor_sync(0xffffffffu, at, d);
+            at = back ? max(at, o) : min(at, o);
+        }
+        if (busy) {
+            if (back ? at >= 0 : at != LLONG_MAX) {
+                res = back ? at + 1 : at;
+                busy = false;
+            } else {
+                c += back ? -64 : 64;
+                busy = back ? (c & ~63LL) >= stop : (c & ~63LL) < stop;
+            }
+        }
+    }
+    // a last line without '\n' ends with the text
+    return !back && res < 0 && stop == n ? n : res;
+}
+
+__device__ void collect_one(const CollectJob& a, uint32_t cta) {
+    extern __shared__ uint64_t s_key[];
+    __shared__ uint32_t s_warp[32], s_flag;
+    const uint32_t nh = a.counters[CNT_HITS];
+    if (nh > a.cap || nh > a.hits_cap) {  // the general path takes over
+        if (cta == 0 && threadIdx.x == 0) {
+            a.head->n = nh;
+            a.head->done = 0;
+        }
+        return;
+    }
+    const uint32_t ctas = nh ? (nh + a.per_cta - 1) / a.per_cta : 1u;
+    if (cta >= ctas) return;
+    const uint32_t end = min(nh, (cta + 1) * a.per_cta);
+    // eight lanes per window; every lane of a warp takes part in every round
+    for (uint32_t i0 = cta * a.per_cta; i0 < end; i0 += kThreads / 8) {
+        const uint32_t i = i0 + threadIdx.x / 8;
+        const uint64_t w = i < end ? a.hits[i].off : 0u;
+        const long long found = line_end_of_window(a, w, i < end);
+        const long long sp = __shfl_sync(0xffffffffu, found, threadIdx.x & 24);
+        const long long ep = __shfl_sync(0xffffffffu, found, (threadIdx.x & 24) + 4);
+        if (i < end && (threadIdx.x & 7) == 0) {
+            long long s = sp, e = ep;
+            if (s < 0) {
+                long long t = (long long)((w - 1) / kScanTile) - 1;
+                for (uint64_t k = 0; k < kWalkTiles && s < 0 && t >= 0; k++, t--) {
+                    const long long l = a.tile_last_nl[t];
+                    if (l >= 0) s = l + 1;
+                }
+                if (t < 0 && s < 0) s = 0;
+            }
+            if (e < 0) {
+                uint64_t t = (w + a.len) / kScanTile + 1;
+                for (uint64_t k = 0; k < kWalkTiles && e < 0 && t < a.ntiles; k++, t++) {
+                    const long long f = a.tile_first_nl[t];
+                    if (f != LLONG_MAX) e = f;
+                }
+                if (t >= a.ntiles && e < 0) e = (long long)a.n;
+            }
+            a.lines[i] = HitLine{(uint64_t)s, (uint64_t)e};  // ~0: not found in the tiles walked
+        }
+    }
+    if (!last_cta(a.counters + CNT_MATCHES, ctas, &s_flag)) return;
+    if (threadIdx.x == 0) a.counters[CNT_MATCHES] = 0;
+    uint32_t open = 0;
+    for (uint32_t q = threadIdx.x; q < nh; q += kThreads)
+        open |= __ldcg(&a.lines[q].start) == ~0ull || __ldcg(&a.lines[q].end) == ~0ull;
+    open = (uint32_t)__syncthreads_or((int)open);
+    sort_records(
+        nh, a.n, s_key, reinterpret_cast<uint16_t*>(s_key + kSmallResults), s_warp,
+        [&](uint32_t q) { return a.hits[q].off; }, [](uint64_t x, uint64_t y) { return x < y; });
+    // lines are disjoint and windows sorted by start, so equal lines are adjacent
+    uint32_t n_lines = 0;
+    for (uint32_t q0 = 0; q0 < nh; q0 += kThreads) {
+        const uint32_t q = q0 + threadIdx.x;
+        uint32_t flag = 0;
+        uint64_t ls = 0, le = 0;
+        if (q < nh) {
+            const uint32_t idx = (uint32_t)s_key[q] & (kSmallResults - 1);
+            ls = __ldcg(&a.lines[idx].start);
+            le = __ldcg(&a.lines[idx].end);
+            flag = q == 0 || __ldcg(&a.lines[(uint32_t)s_key[q - 1] & (kSmallResults - 1)].start) != ls;
+            a.off[q] = s_key[q] >> kIndexBits;
+        }
+        uint32_t total;
+        const uint32_t at = n_lines + block_sum(flag, s_warp, &total);
+        if (flag) {
+            a.line_start[at] = ls;
+            a.line_end[at] = le;
+        }
+        n_lines += total;
+    }
+    if (threadIdx.x == 0) {
+        a.head->n = nh;
+        a.head->n_lines = n_lines;
+        a.head->done = open ? 0 : 1;
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_collect(CollectJob a) { collect_one(a, blockIdx.x); }
+
+__global__ void __launch_bounds__(kThreads) k_collect_multi(const CollectJob* jobs, const uint2* items) {
+    collect_one(jobs[items[blockIdx.x].x], items[blockIdx.x].y);
+}
+
+// One bit and one ballot per pattern (filterPhrases, ffbf.cpp:394-485, as k_prune), counts per block.
+__global__ void __launch_bounds__(kPruneBlock) k_prune_count(const uint64_t* start, const uint64_t* end,
+                                                             const uint64_t* hash, uint64_t npat, Geom g,
+                                                             const uint32_t* ff, uint32_t* bits, uint32_t* counts) {
+    const uint64_t i = blockIdx.x * (uint64_t)kPruneBlock + threadIdx.x;
+    const bool keep = i < npat && end[i] - start[i] >= g.len && check_all<2>(g, ff, hash[i]);
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if ((threadIdx.x & 31) == 0 && i < npat) bits[i >> 5] = m;
+    const int n = __syncthreads_count(keep);
+    if (threadIdx.x == 0) counts[blockIdx.x] = (uint32_t)n;
+}
+
+// Block b writes its patterns' ids behind those of the blocks before it, whose counts it sums (a few coalesced loads
+// per thread, in place of a scan launch).
+__global__ void __launch_bounds__(kPruneBlock) k_prune_emit(const uint32_t* bits, const uint32_t* counts,
+                                                            uint64_t npat, uint64_t* ids, uint64_t ids_cap,
+                                                            ResultHead* head, uint64_t* host_ids) {
+    __shared__ uint32_t s_warp[32];
+    uint32_t before = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kPruneBlock) before += counts[b];
+    uint32_t base, total;
+    block_sum(before, s_warp, &base);
+    const uint64_t i = blockIdx.x * (uint64_t)kPruneBlock + threadIdx.x;
+    const uint32_t keep = i < npat ? bits[i >> 5] >> (threadIdx.x & 31) & 1u : 0u;
+    const uint64_t at = base + block_sum(keep, s_warp, &total);
+    if (keep) {
+        if (at < ids_cap) ids[at] = i;
+        if (at < kSmallIds) host_ids[at] = i;
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) head->n = (unsigned long long)base + total;
+}
+
+// k_verify, and the last CTA orders the matches (offset, then pattern id) when shared memory holds them.
+__global__ void __launch_bounds__(kThreads) k_verify_collect(VerifyJob a) {
+    extern __shared__ uint64_t s_key[];
+    __shared__ uint32_t s_warp[32];
+    __shared__ uint32_t s_flag;
+    // neighbouring windows go to different CTAs: a few hundred windows then wait on as many SMs' memory pipes
+    for (uint64_t j = blockIdx.x + (uint64_t)gridDim.x * threadIdx.x; j < a.nhits; j += (uint64_t)gridDim.x * kThreads)
+        verify_window(a.hits[j], a.text, a.n, a.keys, a.vals, a.mask, a.pat, a.pstart, a.pend, a.m_off, a.m_pid,
+                      a.match_cap, a.counters);
+    if (!last_cta(a.counters + CNT_QUEUE, gridDim.x, &s_flag)) return;
+    const uint32_t nm = __ldcg(a.counters + CNT_MATCHES);
+    const bool small = nm <= kSmallResults && nm <= a.match_cap;
+    if (small) {
+        auto pid = [&](uint64_t key) { return __ldcg(a.m_pid + ((uint32_t)key & (kSmallResults - 1))); };
+        sort_records(
+            nm, a.n, s_key, reinterpret_cast<uint16_t*>(s_key + kSmallResults), s_warp,
+            [&](uint32_t q) { return __ldcg(a.m_off + q); },
+            [&](uint64_t x, uint64_t y) {
+                const uint64_t ox = x >> kIndexBits, oy = y >> kIndexBits;
+                // a network pads with ~0, above every record
+                return ox != oy ? ox < oy : x != ~0ull && pid(x) < pid(y);
+            });
+        for (uint32_t q = threadIdx.x; q < nm; q += kThreads) {
+            a.out_off[q] = s_key[q] >> kIndexBits;
+            a.out_pid[q] = pid(s_key[q]);
+        }
+    }
+    if (threadIdx.x == 0) {
+        a.head->n = nm;
+        a.head->error = a.counters[CNT_ERROR];
+        a.head->done = small;
+    }
+}
+
+constexpr size_t kSmem = (8 + 2 * (kBuckets / kSmallResults)) * (size_t)kSmallResults;  // keys, 16-bit bucket counts
+
+}  // namespace
+
+uint32_t collect_ctas(const CollectJob& job) { return (job.cap + job.per_cta - 1) / job.per_cta; }
+
+cudaError_t collect_hits(const CollectJob& job, cudaStream_t st) {
+    cudaError_t e = cudaFuncSetAttribute(k_collect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e != cudaSuccess) return e;
+    k_collect<<<collect_ctas(job), kThreads, kSmem, st>>>(job);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t collect_hits_multi(const CollectJob* d_jobs, const uint2* d_items, uint32_t n_items, cudaStream_t st) {
+    if (!n_items) return cudaSuccess;
+    cudaError_t e =
+        cudaFuncSetAttribute(k_collect_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e != cudaSuccess) return e;
+    k_collect_multi<<<n_items, kThreads, kSmem, st>>>(d_jobs, d_items);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t prune_count(const uint64_t* d_start, const uint64_t* d_end, const uint64_t* d_hash, uint64_t npat,
+                        const Geom& g, const uint32_t* d_ff, uint32_t* d_bits, uint32_t* d_counts, cudaStream_t st) {
+    k_prune_count<<<(unsigned)prune_blocks(npat), kPruneBlock, 0, st>>>(d_start, d_end, d_hash, npat, g, d_ff, d_bits,
+                                                                      d_counts);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t prune_emit(const uint32_t* d_bits, const uint32_t* d_counts, uint64_t npat, uint64_t* d_ids,
+                       uint64_t ids_cap, ResultHead* head, uint64_t* host_ids, cudaStream_t st) {
+    k_prune_emit<<<(unsigned)prune_blocks(npat), kPruneBlock, 0, st>>>(d_bits, d_counts, npat, d_ids, ids_cap, head,
+                                                                     host_ids);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t verify_collect(const VerifyJob& job, cudaStream_t st) {
+    cudaError_t e =
+        cudaFuncSetAttribute(k_verify_collect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e != cudaSuccess) return e;
+    const uint32_t ctas = job.nhits / 32 + 1;
+    k_verify_collect<<<ctas > 148 ? 148 : ctas, kThreads, kSmem, st>>>(job);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+}  // namespace ffbf

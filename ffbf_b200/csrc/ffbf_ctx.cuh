@@ -6,12 +6,14 @@
 
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <string>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
 
 #include "../../include/ffbf.h"
+#include "ffbf_collect.cuh"
 #include "ffbf_kernels.cuh"
 #include "ffbf_scan_fast.cuh"
 
@@ -21,6 +23,14 @@ struct NvtxRange {
     ~NvtxRange() { nvtxRangePop(); }
     NvtxRange(const NvtxRange&) = delete;
     NvtxRange& operator=(const NvtxRange&) = delete;
+};
+
+// Pinned host memory, shared by a batch and the contexts whose results it holds.
+struct PinnedBlock {
+    uint8_t* p = nullptr;
+    ~PinnedBlock() {
+        if (p) cudaFreeHost(p);
+    }
 };
 
 struct ffbf_ctx {
@@ -114,14 +124,21 @@ struct ffbf_ctx {
     uint32_t match_cap = 0;
     std::vector<uint64_t> r_moff, r_mpid;
 
+    // pinned results of the single-launch paths: a ResultHead, then up to three arrays of kSmallResults words
+    uint8_t* h_res = nullptr;
+    // the pending scan's results where a batch has collected them already (head, then three arrays of ready_cap words)
+    std::shared_ptr<PinnedBlock> ready_block;
+    const uint8_t* ready = nullptr;
+    uint32_t ready_cap = 0;
+
     // scratch for ordered compaction / codec
     uint64_t* d_tmp = nullptr;
     size_t tmp_words = 0;
-    // scratch of the result ordering (sorts and selections), and the prune's per-pattern flags
+    // scratch of the result ordering (sorts and selections), and the prune's bit per pattern
     uint8_t* d_order = nullptr;
     size_t order_bytes = 0;
-    uint8_t* d_pflags = nullptr;
-    uint64_t pflags_cap = 0, ids_cap = 0;
+    uint32_t* d_pbits = nullptr;
+    uint64_t pbits_cap = 0, ids_cap = 0;
     bool host_order = false;  // FFBF_HOST_ORDER: order results on the host (a check of the device ordering)
     uint8_t* d_small = nullptr;  // test_line input
     size_t small_cap = 0;
@@ -181,6 +198,8 @@ void order_hits(const HitRec* hr, const HitLine* hl, uint32_t nh, std::vector<ui
 // Stage-1 table and probe mode of the tuned scan for the context's filter (no-op for borrowed filters).
 ffbf_status prepare_fast(ffbf_ctx* c);
 ffbf::ScanArgs make_scan_args(ffbf_ctx* c);
+// The single-launch collection of a scan's hits into a pinned buffer of a head and three arrays of cap words.
+ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta);
 bool use_fast(const ffbf_ctx* c, uint64_t n);
 ffbf_status launch_scan(ffbf_ctx* c);  // counters reset + scan of c->d_text on the context's stream
 // Sizes the scan buffers for a device text of len bytes and resets the results, without launching.

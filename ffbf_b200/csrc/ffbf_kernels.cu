@@ -6,6 +6,7 @@
 #include <climits>
 
 #include "ffbf_kernels.cuh"
+#include "ffbf_text.cuh"
 
 namespace ffbf {
 
@@ -55,11 +56,6 @@ struct BytePred {
     uint8_t b;
     __device__ bool operator()(uint64_t i) const { return p[i] == b; }
 };
-struct FlagPred {
-    const uint8_t* p;
-    __device__ bool operator()(uint64_t i) const { return p[i] != 0; }
-};
-
 template <class Pred>
 __global__ void __launch_bounds__(kCompThreads) k_count(Pred pred, uint64_t n, uint64_t* counts) {
     __shared__ uint64_t sh[kCompThreads / 32];
@@ -134,13 +130,6 @@ cudaError_t emit_bytes(const uint8_t* d_buf, uint64_t n, uint8_t byte, uint64_t*
                        cudaStream_t st) {
     return compact_emit(BytePred{d_buf, byte}, n, d_pos, d_tmp, st);
 }
-cudaError_t count_flags(const uint8_t* d_flags, uint64_t n, uint64_t* d_tmp, cudaStream_t st) {
-    return compact_count(FlagPred{d_flags}, n, d_tmp, st);
-}
-cudaError_t emit_flags(const uint8_t* d_flags, uint64_t n, uint64_t* d_out, const uint64_t* d_tmp, cudaStream_t st) {
-    return compact_emit(FlagPred{d_flags}, n, d_out, d_tmp, st);
-}
-
 // Line table of a pattern file from its newline positions: line i ends at nl[i] (or at n for a final
 // line without '\n') and starts one past the previous line's end.
 __global__ void k_lines(const uint64_t* nl, uint64_t m, uint64_t n, int tail, uint64_t* start, uint64_t* end) {
@@ -521,82 +510,17 @@ __global__ void __launch_bounds__(1024) k_tile_scan2(const long long* first, con
     }
 }
 
-// Byte masks of '\n' in a 32-bit word (0x80 in each byte that is '\n'; no false positives).
-__device__ __forceinline__ uint32_t nl_bytes(uint32_t w) {
-    const uint32_t t = w ^ 0x0A0A0A0Au;
-    return ~(((t & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | t) & 0x80808080u;
-}
-
-// The aligned 16 bytes of `text` at c (c a multiple of 16, c < n). The last, partial chunk of a text whose
-// length is not a multiple of 16 is read byte by byte, zero-filled past n, so nothing beyond the text is read.
-__device__ __forceinline__ uint4 chunk16(const uint8_t* text, long long c, long long n) {
-    if (c + 16 <= n) return __ldg(reinterpret_cast<const uint4*>(text + c));
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
-    for (int i = 0; i < 16 && c + i < n; i++) w[i >> 2] |= (uint32_t)__ldg(text + c + i) << (8 * (i & 3));
-    return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
-// Last '\n' in [lo, p] (lo <= p < n), or -1: aligned 16-byte chunks from p down to lo.
-__device__ __forceinline__ long long last_nl_back(const uint8_t* text, long long n, long long lo, long long p) {
-    while (p >= lo) {
-        const long long c = p & ~15LL;
-        const uint4 v = chunk16(text, c, n);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        // bytes of the chunk at offsets max(lo - c, 0) .. p - c
-        const int hi = (int)(p - c), low = (int)max(lo - c, 0LL);
-        for (int q = hi >> 2; q >= (low >> 2); q--) {
-            uint32_t m = nl_bytes(w[q]);
-            // keep byte positions 4q + b with low <= 4q + b <= hi
-            const int b_hi = min(hi - 4 * q, 3), b_lo = max(low - 4 * q, 0);
-            m &= (0xFFFFFFFFu >> (8 * (3 - b_hi))) & (0xFFFFFFFFu << (8 * b_lo));
-            if (m) return c + 4 * q + (31 - __clz(m)) / 8;
-        }
-        p = c - 1;
-    }
-    return -1;
-}
-
-// First '\n' in [q, hi) (q < hi <= n), or -1: aligned 16-byte chunks from q up to hi.
-__device__ __forceinline__ long long first_nl_fwd(const uint8_t* text, long long n, long long q, long long hi) {
-    while (q < hi) {
-        const long long c = q & ~15LL;
-        const uint4 v = chunk16(text, c, n);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        const int low = (int)(q - c), top = (int)min(hi - c, 16LL) - 1;  // offsets low .. top
-        for (int k = low >> 2; k <= (top >> 2); k++) {
-            uint32_t m = nl_bytes(w[k]);
-            const int b_lo = max(low - 4 * k, 0), b_hi = min(top - 4 * k, 3);
-            m &= (0xFFFFFFFFu << (8 * b_lo)) & (0xFFFFFFFFu >> (8 * (3 - b_hi)));
-            if (m) return c + 4 * k + (__ffs(m) - 1) / 8;
-        }
-        q = c + 16;
-    }
-    return -1;
-}
-
 __global__ void k_resolve(const uint8_t* text, uint64_t n, uint32_t len, const HitRec* hits, uint32_t nhits,
                           const long long* prev_nl, const long long* next_nl, HitLine* out) {
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nhits) return;
     const uint64_t w = hits[j].off;
-    // line start: the last '\n' before the window in its tile, else the tile summaries' prefix
-    uint64_t s = 0;
-    if (w > 0) {
-        const uint64_t tb = (w - 1) / kScanTile;
-        const long long p = last_nl_back(text, (long long)n, (long long)(tb * kScanTile), (long long)w - 1);
-        s = p >= 0 ? (uint64_t)p + 1 : (uint64_t)(prev_nl[tb] + 1);
-    }
-    // line end: the first '\n' after the window in its tile, else the suffix summary, else the text's end
-    uint64_t e = n;
-    const uint64_t q = w + len;
-    if (q < n) {
-        const uint64_t te = q / kScanTile;
-        const uint64_t hi = min(n, (te + 1) * (uint64_t)kScanTile);
-        const long long f = first_nl_fwd(text, (long long)n, (long long)q, (long long)hi);
-        if (f >= 0) e = (uint64_t)f;
-        else e = next_nl[te] == LLONG_MAX ? n : (uint64_t)next_nl[te];
-    }
-    out[j] = HitLine{s, e};
+    // the line's ends within the tiles of the window's neighbours, else from the tile summaries
+    const long long p = line_start_in_tile(text, n, w);
+    const long long e = line_end_in_tile(text, n, w + len);
+    out[j] = HitLine{p >= 0 ? (uint64_t)p : (uint64_t)(prev_nl[(w - 1) / kScanTile] + 1),
+                     e >= 0 ? (uint64_t)e
+                            : next_nl[(w + len) / kScanTile] == LLONG_MAX ? n : (uint64_t)next_nl[(w + len) / kScanTile]};
 }
 
 cudaError_t resolve_lines(const uint8_t* text, uint64_t n, uint32_t len, const HitRec* hits, uint32_t nhits,
@@ -619,35 +543,9 @@ cudaError_t resolve_lines(const uint8_t* text, uint64_t n, uint32_t len, const H
 }
 
 // ------------------------------------------------------------------------------------------------
-// Feed-forward prune (filterPhrases, ffbf.cpp:394-485): a line survives when it is >= LEN bytes and its
-// prefix window's K feed-forward bits (getHashValue_2 order) are set.
-__global__ void k_prune(const uint64_t* start, const uint64_t* end, const uint64_t* hash, uint64_t npat, Geom g,
-                        const uint32_t* ff, uint8_t* flags) {
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= npat) return;
-    flags[i] = (end[i] - start[i] >= g.len) && check_all<2>(g, ff, hash[i]);
-}
-
-cudaError_t prune_flags(const uint64_t* d_start, const uint64_t* d_end, const uint64_t* d_hash, uint64_t npat,
-                        const Geom& g, const uint32_t* d_ff, uint8_t* d_flags, cudaStream_t st) {
-    if (!npat) return cudaSuccess;
-    k_prune<<<(unsigned)((npat + 255) / 256), 256, 0, st>>>(d_start, d_end, d_hash, npat, g, d_ff, d_flags);
-    note_launches(1);
-    return cudaGetLastError();
-}
-
-// ------------------------------------------------------------------------------------------------
 // Exact verification. Open-addressing multimap keyed by the pruned patterns' 64-bit prefix hash; every
 // pattern gets its own slot (several patterns may share a prefix). Slots are claimed with atomicCAS on
 // the value array (empty = 0xffffffff); lookups run in a later kernel.
-__device__ __forceinline__ uint64_t mix64(uint64_t x) {
-    x ^= x >> 33;
-    x *= 0xff51afd7ed558ccdull;
-    x ^= x >> 33;
-    x *= 0xc4ceb9fe1a85ec53ull;
-    return x ^ (x >> 33);
-}
-
 __global__ void k_table_build(const uint64_t* ids, uint64_t nids, const uint64_t* hash, uint64_t* keys,
                               uint32_t* vals, uint64_t mask, uint32_t* counters) {
     uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -671,80 +569,6 @@ cudaError_t table_build(const uint64_t* d_ids, uint64_t nids, const uint64_t* d_
     if (!nids) return cudaSuccess;
     k_table_build<<<(unsigned)((nids + 255) / 256), 256, 0, st>>>(d_ids, nids, d_hash, d_keys, d_vals, mask,
                                                                     d_counters);
-    note_launches(1);
-    return cudaGetLastError();
-}
-
-// One thread per hit window: look its hash up, byte-compare every candidate pattern at the window start.
-// The 16 bytes at p (any alignment), of which the first `need` (1..16) are used, read as aligned 16-byte
-// loads: the chunk holding p, and the next one only when the bytes reach into it. An aligned chunk that holds a
-// needed byte never crosses a page, so no load leaves the buffer's pages.
-__device__ __forceinline__ uint4 load16_unaligned(const uint8_t* p, uint32_t need) {
-    const uintptr_t a = (uintptr_t)p;
-    const uint4* base = reinterpret_cast<const uint4*>(a & ~(uintptr_t)15);
-    const uint32_t off = (uint32_t)(a & 15);
-    const uint4 x0 = __ldg(base);
-    const uint4 x1 = off + need > 16 ? __ldg(base + 1) : make_uint4(0, 0, 0, 0);
-    const uint32_t ws = off >> 2, bs = (off & 3) * 8;
-    // words ws .. ws + 4 of x0:x1, selected without a runtime-indexed array
-    uint32_t w0, w1, w2, w3, w4;
-    if (ws == 0) { w0 = x0.x; w1 = x0.y; w2 = x0.z; w3 = x0.w; w4 = x1.x; }
-    else if (ws == 1) { w0 = x0.y; w1 = x0.z; w2 = x0.w; w3 = x1.x; w4 = x1.y; }
-    else if (ws == 2) { w0 = x0.z; w1 = x0.w; w2 = x1.x; w3 = x1.y; w4 = x1.z; }
-    else { w0 = x0.w; w1 = x1.x; w2 = x1.y; w3 = x1.z; w4 = x1.w; }
-    return make_uint4(__funnelshift_r(w0, w1, bs), __funnelshift_r(w1, w2, bs), __funnelshift_r(w2, w3, bs),
-                      __funnelshift_r(w3, w4, bs));
-}
-
-// mask of the bytes of 32-bit word i that fall within the first `need` bytes of a 16-byte block
-__device__ __forceinline__ uint32_t word_mask(uint32_t need, uint32_t i) {
-    const uint32_t v = need > 4 * i ? min(need - 4 * i, 4u) : 0u;
-    return v >= 4 ? 0xffffffffu : (1u << (8 * v)) - 1u;
-}
-
-__global__ void k_verify(const HitRec* hits, uint32_t nhits, const uint8_t* text, uint64_t n, const uint64_t* keys,
-                         const uint32_t* vals, uint64_t mask, const uint8_t* pat, const uint64_t* pstart,
-                         const uint64_t* pend, uint64_t* m_off, uint32_t* m_pid, uint32_t cap, uint32_t* counters) {
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nhits) return;
-    const uint64_t w = hits[j].off, h = hits[j].h;
-    uint64_t slot = mix64(h) & mask;
-    for (uint64_t probe = 0; probe <= mask; probe++) {
-        uint32_t id = vals[slot];
-        if (id == 0xffffffffu) break;
-        if (keys[slot] == h) {
-            uint64_t ps = pstart[id], pl = pend[id] - ps;
-            if (w + pl <= n) {
-                const uint8_t* t = text + w;
-                const uint8_t* q = pat + ps;
-                // byte compare, 16 bytes per step from aligned 16-byte loads of both sides
-                bool same = true;
-                for (uint64_t k = 0; k < pl && same; k += 16) {
-                    const uint32_t need = pl - k < 16 ? (uint32_t)(pl - k) : 16u;
-                    const uint4 x = load16_unaligned(t + k, need), y = load16_unaligned(q + k, need);
-                    same = (((x.x ^ y.x) & word_mask(need, 0)) | ((x.y ^ y.y) & word_mask(need, 1)) |
-                            ((x.z ^ y.z) & word_mask(need, 2)) | ((x.w ^ y.w) & word_mask(need, 3))) == 0;
-                }
-                if (same) {
-                    uint32_t o = atomicAdd(counters + CNT_MATCHES, 1u);
-                    if (o < cap) {
-                        m_off[o] = w;
-                        m_pid[o] = id;
-                    }
-                }
-            }
-        }
-        slot = (slot + 1) & mask;
-    }
-}
-
-cudaError_t verify_hits(const HitRec* hits, uint32_t nhits, const uint8_t* text, uint64_t n, const uint64_t* d_keys,
-                        const uint32_t* d_vals, uint64_t mask, const uint8_t* d_pat, const uint64_t* d_start,
-                        const uint64_t* d_end, uint64_t* d_match_off, uint32_t* d_match_pid, uint32_t match_cap,
-                        uint32_t* d_counters, cudaStream_t st) {
-    if (!nhits) return cudaSuccess;
-    k_verify<<<(nhits + 255) / 256, 256, 0, st>>>(hits, nhits, text, n, d_keys, d_vals, mask, d_pat, d_start, d_end,
-                                                   d_match_off, d_match_pid, match_cap, d_counters);
     note_launches(1);
     return cudaGetLastError();
 }

@@ -60,8 +60,6 @@ uint64_t compact_blocks(uint64_t n);
 cudaError_t count_bytes(const uint8_t* d_buf, uint64_t n, uint8_t byte, uint64_t* d_tmp, cudaStream_t st);
 cudaError_t emit_bytes(const uint8_t* d_buf, uint64_t n, uint8_t byte, uint64_t* d_pos, const uint64_t* d_tmp,
                        cudaStream_t st);
-cudaError_t count_flags(const uint8_t* d_flags, uint64_t n, uint64_t* d_tmp, cudaStream_t st);
-cudaError_t emit_flags(const uint8_t* d_flags, uint64_t n, uint64_t* d_out, const uint64_t* d_tmp, cudaStream_t st);
 cudaError_t lines_from_newlines(const uint64_t* d_nl, uint64_t m, uint64_t n, int tail, uint64_t* d_start,
                                 uint64_t* d_end, cudaStream_t st);
 cudaError_t hash_patterns(const uint8_t* d_file, const uint64_t* d_start, const uint64_t* d_end, uint64_t npat,
@@ -84,16 +82,8 @@ cudaError_t resolve_lines(const uint8_t* text, uint64_t n, uint32_t len, const H
                           long long* next_nl, uint64_t ntiles, HitLine* out, cudaStream_t st,
                           long long* agg = nullptr);
 
-cudaError_t prune_flags(const uint64_t* d_start, const uint64_t* d_end, const uint64_t* d_hash, uint64_t npat,
-                        const Geom& g, const uint32_t* d_ff, uint8_t* d_flags, cudaStream_t st);
-
 cudaError_t table_build(const uint64_t* d_ids, uint64_t nids, const uint64_t* d_hash, uint64_t* d_keys,
                         uint32_t* d_vals, uint64_t mask, uint32_t* d_counters, cudaStream_t st);
-cudaError_t verify_hits(const HitRec* hits, uint32_t nhits, const uint8_t* text, uint64_t n, const uint64_t* d_keys,
-                        const uint32_t* d_vals, uint64_t mask, const uint8_t* d_pat, const uint64_t* d_start,
-                        const uint64_t* d_end, uint64_t* d_match_off, uint32_t* d_match_pid, uint32_t match_cap,
-                        uint32_t* d_counters, cudaStream_t st);
-
 // Filter cache file codec (delta-coded uint32 set-bit indices).
 cudaError_t filter_decode(const uint32_t* d_deltas, uint64_t nd, uint32_t nbits, uint32_t* d_idx, uint64_t* d_tmp,
                           uint32_t* d_counters, cudaStream_t st);

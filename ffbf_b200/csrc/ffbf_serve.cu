@@ -13,10 +13,10 @@
 //   4. when the previous launch sequence has finished, launches every ready request as one plan
 //      (build_plan/launch_plan: one tuned launch per (LEN, configuration) group, one generic launch for
 //      ragged ends) on the scan stream;
-//   5. for each request of a finished batch (whose hit counts came back with the batch), enqueues line
-//      resolution and the copy of its hits on the slot's own stream, overlapping the next batch's scan;
-//      a request whose copy has landed is ordered on the host and its slot and arena range are freed.
-//      A request with more hits than its slot's buffer takes the plain collect (regrow and rescan).
+//   5. finishes each request of a finished batch: one launch behind the batch's scan has put its ordered hits and
+//      lines into the slot's pinned buffer. A request with more hits than that buffer holds has its lines resolved
+//      and its hits copied on the slot's own stream, overlapping the next batch's scan, and is ordered on the host;
+//      one with more hits than its slot's device buffer takes the plain collect (regrow and rescan).
 // A slot is a context with its own scan buffers whose filters are attached from the request's set.
 #include <cuda_runtime.h>
 
@@ -64,7 +64,6 @@ constexpr uint64_t kSegmentBytes = 1ull << 30;    // arena growth step (a larger
 constexpr uint64_t kHbmReserve = 1ull << 30;      // device memory the arena leaves free for others
 constexpr double kGrowRetrySeconds = 1e-3;        // pause between growth attempts that found too little memory
 constexpr double kShrinkIdleSeconds = 0.25;       // idle time after which grown segments are given back
-constexpr uint32_t kPreallocHits = 16384;          // hit records each slot's pinned result copy starts with
 
 }  // namespace
 
@@ -108,8 +107,14 @@ struct ffbf_server {
     uint32_t* h_ctl = nullptr;  // error flags read back after each batch
     uint32_t* d_cnt = nullptr;  // every job's counters, gathered after each batch
     uint32_t* h_cnt = nullptr;
+    ffbf::CollectJob* d_collect = nullptr;  // the batch's result collection, and its items {job, CTA}
+    ffbf::CollectJob* h_collect = nullptr;
+    uint2* d_collect_items = nullptr;
+    uint2* h_collect_items = nullptr;
     struct SlotHost {
-        HitRec* hr = nullptr;  // pinned copies of the slot's hit records and lines
+        uint8_t* res = nullptr;  // pinned: the collected results (a head and three arrays)
+        uint32_t res_cap = 0;    // their capacity in the running batch
+        HitRec* hr = nullptr;    // pinned copies of the slot's hit records and lines, for larger results
         HitLine* hl = nullptr;
         uint32_t cap = 0;
         cudaEvent_t done = nullptr;
@@ -410,8 +415,20 @@ void launch_ready(ffbf_server* s) {
     up(s->d_args, s->h_args, plan.args.size() * sizeof(ffbf::ScanArgs));
     up(s->d_tail, s->h_tail, plan.tail.size() * sizeof(uint2));
     up(s->d_counters, s->h_counters, (n + n_ctl) * sizeof(uint32_t*));
+    // results: room for one hit window per 2 KiB of text, at least 512
+    uint32_t n_items = 0;
+    for (uint32_t i = 0; i < n; i++) {
+        auto& h = s->slot_host[batch[i]->slot];
+        h.res_cap = (uint32_t)std::min<uint64_t>(ffbf::kSmallResults, std::max<uint64_t>(512, jobs[i].len / 2048));
+        reinterpret_cast<ffbf::ResultHead*>(h.res)->done = 0;
+        s->h_collect[i] = collect_job(plan.args[i], jobs[i].c->d_hitlines, h.res, h.res_cap, ffbf::kCollectBatch);
+        for (uint32_t k = 0; k < ffbf::collect_ctas(s->h_collect[i]); k++) s->h_collect_items[n_items++] = make_uint2(i, k);
+    }
+    up(s->d_collect, s->h_collect, n * sizeof(ffbf::CollectJob));
+    up(s->d_collect_items, s->h_collect_items, n_items * sizeof(uint2));
     const double t = s->now();
     if (e == cudaSuccess) e = launch_plan(plan, d, s->num_sms, s->st_scan);
+    if (e == cudaSuccess) e = ffbf::collect_hits_multi(s->d_collect, s->d_collect_items, n_items, s->st_scan);
     if (e == cudaSuccess) e = ffbf::gather_counters(s->d_counters, n, s->d_cnt, s->st_scan);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(s->h_cnt, s->d_cnt, 4 * ffbf::CNT_WORDS * n, cudaMemcpyDeviceToHost, s->st_scan);
@@ -565,6 +582,17 @@ void worker_loop(ffbf_server* s) {
                         finish(s, r, st);
                         continue;
                     }
+                    auto& h = s->slot_host[r->slot];
+                    const auto* head = reinterpret_cast<const ffbf::ResultHead*>(h.res);
+                    if (head->done) {
+                        const uint64_t* a = reinterpret_cast<const uint64_t*>(h.res + 64);
+                        const size_t cap = h.res_cap;
+                        r->hits.assign(a, a + head->n);
+                        r->ls.assign(a + cap, a + cap + head->n_lines);
+                        r->le.assign(a + 2 * cap, a + 2 * cap + head->n_lines);
+                        finish(s, r, FFBF_OK);
+                        continue;
+                    }
                     if (r->nh > s->slots[r->slot]->hits_cap) {
                         s->slow.push_back(r);
                         continue;
@@ -616,6 +644,7 @@ void server_free(ffbf_server* s) {
     for (auto* c : s->slots) ffbf_destroy(c);
     for (auto ev : s->copy_done) cudaEventDestroy(ev);
     for (auto& h : s->slot_host) {
+        if (h.res) cudaFreeHost(h.res);
         if (h.hr) cudaFreeHost(h.hr);
         if (h.hl) cudaFreeHost(h.hl);
         if (h.done) cudaEventDestroy(h.done);
@@ -624,10 +653,10 @@ void server_free(ffbf_server* s) {
     for (auto& g : s->segs) cudaFree(g.base);
     s->segs.clear();
     for (void* p : {(void*)s->d_fast, (void*)s->d_args, (void*)s->d_counters, (void*)s->d_ctl,
-                    (void*)s->d_tail, (void*)s->d_cnt})
+                    (void*)s->d_tail, (void*)s->d_cnt, (void*)s->d_collect, (void*)s->d_collect_items})
         if (p) cudaFree(p);
     for (void* p : {(void*)s->h_fast, (void*)s->h_args, (void*)s->h_counters, (void*)s->h_tail, (void*)s->h_ctl,
-                    (void*)s->h_cnt})
+                    (void*)s->h_cnt, (void*)s->h_collect, (void*)s->h_collect_items})
         if (p) cudaFreeHost(p);
     if (s->st_scan) cudaStreamDestroy(s->st_scan);
     if (s->st_copy) cudaStreamDestroy(s->st_copy);
@@ -694,6 +723,7 @@ ffbf_status ffbf_server_create(int device, uint64_t arena_bytes, uint32_t slots,
         s->arena_held = first;
     }
     const size_t n_counters = slots + kMaxCtl;
+    const size_t items_per_slot = ffbf::kSmallResults / ffbf::kCollectBatch;
     if (cudaMalloc(&s->d_fast, slots * sizeof(ffbf::FastJob)) != cudaSuccess ||
         cudaMalloc(&s->d_args, slots * sizeof(ffbf::ScanArgs)) != cudaSuccess ||
         cudaMalloc(&s->d_counters, n_counters * sizeof(uint32_t*)) != cudaSuccess ||
@@ -702,13 +732,17 @@ ffbf_status ffbf_server_create(int device, uint64_t arena_bytes, uint32_t slots,
         cudaMallocHost(&s->h_args, slots * sizeof(ffbf::ScanArgs)) != cudaSuccess ||
         cudaMallocHost(&s->h_counters, n_counters * sizeof(uint32_t*)) != cudaSuccess ||
         cudaMallocHost(&s->h_ctl, 16 * kMaxCtl) != cudaSuccess ||
+        cudaMalloc(&s->d_collect, slots * sizeof(ffbf::CollectJob)) != cudaSuccess ||
+        cudaMallocHost(&s->h_collect, slots * sizeof(ffbf::CollectJob)) != cudaSuccess ||
+        cudaMalloc(&s->d_collect_items, slots * items_per_slot * sizeof(uint2)) != cudaSuccess ||
+        cudaMallocHost(&s->h_collect_items, slots * items_per_slot * sizeof(uint2)) != cudaSuccess ||
         cudaMalloc(&s->d_cnt, 4 * ffbf::CNT_WORDS * (size_t)slots) != cudaSuccess ||
         cudaMallocHost(&s->h_cnt, 4 * ffbf::CNT_WORDS * (size_t)slots) != cudaSuccess || !ensure_tail(s, 4096)) {
         cudaGetLastError();
         return bail(FFBF_ENOMEM_DEVICE);
     }
     // Slots get their scan buffers up front, sized for requests of up to kPreallocText bytes (tile
-    // summaries, 64k hit records, pinned copies for 16k hits), so that serving rarely allocates: an
+    // summaries, 64k hit records, pinned results of 16k hits), so that serving rarely allocates: an
     // allocation inside the loop would synchronise the device and stall every request in flight.
     const uint64_t prealloc_len = kPreallocText;
     for (uint32_t i = 0; i < slots; i++) {
@@ -729,12 +763,10 @@ ffbf_status ffbf_server_create(int device, uint64_t arena_bytes, uint32_t slots,
         s->slot_host.emplace_back();
         auto& h = s->slot_host.back();
         if (cudaEventCreateWithFlags(&h.done, cudaEventDisableTiming) != cudaSuccess ||
-            cudaMallocHost(&h.hr, kPreallocHits * sizeof(HitRec)) != cudaSuccess ||
-            cudaMallocHost(&h.hl, kPreallocHits * sizeof(HitLine)) != cudaSuccess) {
+            cudaMallocHost(&h.res, ffbf::kResultBytes) != cudaSuccess) {
             cudaGetLastError();
             return bail(FFBF_ENOMEM_HOST);
         }
-        h.cap = kPreallocHits;
         s->free_slots.push_back((int)(slots - 1 - i));
     }
     s->stats.arena_bytes = s->arena_held;
