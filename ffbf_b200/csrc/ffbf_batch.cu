@@ -80,34 +80,32 @@ ffbf_status build_plan(const std::vector<PlanJob>& jobs, int num_sms, ScanPlan& 
         *bad = i;
         TRY(enter(c));
         TRY(setup_scan_state(c, jobs[i].text, jobs[i].len));
-        const ffbf::ScanArgs a = make_scan_args(c);
-        plan.args.push_back(a);
-        uint64_t covered = 0;
-        if (use_fast(c, a.n)) {
+        if (use_fast(c, c->text_len)) {
             TRY(prepare_fast(c));
-            const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, a.n, num_sms, true);
+            // in a batch other jobs fill the GPU, so CTA size and rows per stream follow this job's size alone
+            const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->text_len, num_sms, true);
+            c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
+            const ffbf::ScanArgs a = make_scan_args(c);
+            plan.args.push_back(a);
             const int threads = ffbf::config_threads(cfg);
-            // in a batch other jobs fill the GPU, so rows per stream follow this job's size alone
-            const uint32_t rows = cfg.rows ? cfg.rows : ffbf::fast_rows(a.n, cfg, num_sms, true);
             ffbf::FastJob fj;
-            cudaError_t e;
-            covered = ffbf::fill_fast_job(a, c->d_stage1, cfg, rows, &fj, &e);
-            if (e != cudaSuccess) return fail(c, FFBF_ECUDA, "tensor map encoding failed");
-            if (fj.n_supertiles) {
-                Group* gp = nullptr;
-                for (auto& g : groups)
-                    if (g.len == c->g.len && g.cfg.mode == cfg.mode && ffbf::config_threads(g.cfg) == threads &&
-                        (cfg.mode != 1 || g.cfg.order == cfg.order))
-                        gp = &g;
-                if (!gp) {
-                    groups.push_back(Group{c->g.len, cfg, {}});
-                    gp = &groups.back();
-                }
-                gp->jobs.push_back({covered, fj});
+            if (ffbf::fill_fast_job(a, c->d_stage1, cfg, &fj) != cudaSuccess)
+                return fail(c, FFBF_ECUDA, "tensor map encoding failed");
+            Group* gp = nullptr;
+            for (auto& g : groups)
+                if (g.len == c->g.len && (g.cfg.mode == 1) == (cfg.mode == 1) &&
+                    ffbf::config_threads(g.cfg) == ffbf::config_threads(cfg) &&
+                    (cfg.mode != 1 || g.cfg.order == cfg.order))
+                    gp = &g;
+            if (!gp) {
+                groups.push_back(Group{c->g.len, cfg, {}});
+                gp = &groups.back();
             }
+            gp->jobs.push_back({a.n, fj});
+        } else {
+            plan.args.push_back(make_scan_args(c));
+            for (uint64_t t = 0; t < scan_tiles(c); t++) plan.tail.push_back(make_uint2((uint32_t)i, (uint32_t)t));
         }
-        for (uint64_t t = covered / ffbf::kScanTile; t < a.ntiles; t++)
-            plan.tail.push_back(make_uint2((uint32_t)i, (uint32_t)t));
         CUDA_TRY(c, cudaStreamSynchronize(c->st));  // stage-1 tables built on the context's stream
         c->scan_pending = true;
     }
@@ -505,8 +503,7 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
         if (per_sm) {
             const ffbf::FastConfig run = ffbf::launch_config(cand, sample_len, c->num_sms, false);
             const int t = ffbf::config_threads(run);
-            const uint64_t bytes = sample_len / ffbf::kScanTile * ffbf::kScanTile;
-            const uint64_t streams = bytes / ((uint64_t)ffbf::fast_rows(sample_len, run, c->num_sms, false) * 128);
+            const uint64_t streams = sample_len / ((uint64_t)run.rows * 128);
             const uint64_t items = (streams + t - 1) / t;
             score = ms * (double)std::min<uint64_t>(items, (uint64_t)c->num_sms);
         }

@@ -236,12 +236,13 @@ ffbf_status prepare_fast(ffbf_ctx* c) {
         if (!c->cfg_tuned) {
             c->cfg.mode = c->force_mode >= 0 ? c->force_mode : best.mode;
             // default CTA sizes (measured best on the 10k- and 1M-pattern workloads): 512 threads for the
-            // shared-memory stage (768 for large texts), 2 x 192 per SM for dense filters, 384 with their prefilter
+            // shared-memory stage (launch_config fits it to each text), 2 x 192 per SM for dense filters, 384 with their prefilter
             c->cfg.threads = c->threads_env ? c->threads_env : c->cfg.mode == 1 ? 192 : c->cfg.mode == 2 ? 256 : 512;
         }
         c->stage1_dirty = false;
     }
     if (c->force_mode >= 0) c->cfg.mode = c->force_mode;
+    if (c->cfg.mode == 3) c->cfg.threads = 512;  // launch_config picks the size for each text
     // the dense mode probes distinct index functions: with K = 1 only the sparse mode applies
     if (c->g.k < 2 && c->cfg.mode == 1) c->cfg.mode = 0;
     // the dense mode's probe order is the filter's, unless the environment fixes it (orders 1 and 3 need f2 and f3)
@@ -249,7 +250,7 @@ ffbf_status prepare_fast(ffbf_ctx* c) {
     if (c->g.k < 4 && c->cfg.order == 1) c->cfg.order = 0;
     if (c->g.k >= 4 && c->cfg.order == 2) c->cfg.order = 3;
     // the table the configured kernel reads (a dense kernel without prefilter reads none)
-    if (c->cfg.mode != 1 || c->cfg.order >= 2) TRY(ensure_stage1(c, ffbf::config_threads(c->cfg), false));
+    if (c->cfg.mode != 1 || c->cfg.order >= 2) TRY(ensure_stage1(c, ffbf::table_threads(c->cfg), false));
     return FFBF_OK;
 }
 
@@ -266,7 +267,8 @@ ffbf::ScanArgs make_scan_args(ffbf_ctx* c) {
     a.counters = c->d_counters;
     a.tile_first_nl = c->d_tiles;
     a.tile_last_nl = c->d_tiles + c->tiles_cap;
-    a.ntiles = (c->text_len + ffbf::kScanTile - 1) / ffbf::kScanTile;
+    a.tile_bytes = c->tile_bytes;
+    a.ntiles = scan_tiles(c);
     a.tile_begin = 0;
     a.cache_in_smem = c->g.cache_bits <= ffbf::kSmemCacheMaxBits;
     return a;
@@ -275,7 +277,7 @@ ffbf::ScanArgs make_scan_args(ffbf_ctx* c) {
 ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta) {
     uint64_t* arrays = reinterpret_cast<uint64_t*>(res + 64);
     return ffbf::CollectJob{a.text, a.n, a.g.len, a.hits_cap, a.hits, lines, a.counters, a.tile_first_nl, a.tile_last_nl,
-                            a.ntiles, reinterpret_cast<ffbf::ResultHead*>(res), arrays, arrays + cap,
+                            a.tile_bytes, a.ntiles, reinterpret_cast<ffbf::ResultHead*>(res), arrays, arrays + cap,
                             arrays + 2 * (size_t)cap, cap, per_cta};
 }
 
@@ -285,13 +287,16 @@ ffbf_status launch_scan(ffbf_ctx* c) {
     const uint64_t n = c->text_len;
     CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * sizeof(uint32_t), c->st));
     if (n == 0) return FFBF_OK;
-    ffbf::ScanArgs a = make_scan_args(c);
     if (use_fast(c, n)) {
         c->scan_path = 1;
         TRY(prepare_fast(c));
-        CUDA_TRY(c, ffbf::scan_fast(a, c->d_stage1, c->cfg, c->num_sms, c->h_job, c->d_job, c->st));
+        const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, n, c->num_sms, false);
+        c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
+        CUDA_TRY(c, ffbf::scan_fast(make_scan_args(c), c->d_stage1, cfg, c->num_sms, c->h_job, c->d_job, c->st));
     } else {
         c->scan_path = 0;
+        c->tile_bytes = ffbf::kScanTile;
+        const ffbf::ScanArgs a = make_scan_args(c);
         int grid = ffbf::scan_generic_grid(c->g, a.cache_in_smem, a.ntiles);
         if (grid <= 0) return fail(c, FFBF_ECUDA, "scan kernel cannot be launched (occupancy query failed)");
         CUDA_TRY(c, ffbf::scan_generic(a, grid, c->st));
@@ -309,7 +314,7 @@ ffbf_status setup_scan_state(ffbf_ctx* c, const uint8_t* d_text, size_t len) {
         c->segs.clear();
         c->seg_hr.clear();
     }
-    const uint64_t ntiles = (len + ffbf::kScanTile - 1) / ffbf::kScanTile;
+    const uint64_t ntiles = tiles_for(len);
     if (c->tiles_cap < ntiles) {
         dfree(c, c->d_tiles);
         c->tiles_cap = 0;
@@ -324,7 +329,14 @@ ffbf_status setup_scan_state(ffbf_ctx* c, const uint8_t* d_text, size_t len) {
     }
     c->d_text = d_text;
     c->text_len = len;
+    c->tile_bytes = ffbf::kScanTile;
     return FFBF_OK;
+}
+
+uint64_t tiles_for(uint64_t len) {
+    // tiles are 16 KiB or more, but 4 KiB where a small text's scan may use streams of less than four rows
+    const uint64_t tile = len < ffbf::kShortRowsText ? 4096 : ffbf::kScanTile;
+    return (len + tile - 1) / tile;
 }
 
 }  // namespace ffbf_host
@@ -706,7 +718,6 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
     NvtxRange nvtx_("ffbf_scan_collect");
     TRY(enter(c));
     if (!c->scan_pending && !c->have_scan) return fail(c, FFBF_ESTATE, "no scan to collect");
-    const uint64_t ntiles = (c->text_len + ffbf::kScanTile - 1) / ffbf::kScanTile;
     if (c->scan_pending && !c->host_order && !c->keep_records) {
         // one launch finishes a result of up to kSmallResults windows, unless the scan's batch has done it already;
         // the general path below takes the others
@@ -757,8 +768,8 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
         c->nhits = nh;
         CUDA_TRY(c, ffbf::resolve_lines(c->d_text, c->text_len, c->g.len, c->d_hits, nh, c->d_tiles,
                                         c->d_tiles + c->tiles_cap, c->d_tiles + 2 * c->tiles_cap,
-                                        c->d_tiles + 3 * c->tiles_cap, ntiles, c->d_hitlines, c->st,
-                                        c->d_tiles + 4 * c->tiles_cap));
+                                        c->d_tiles + 3 * c->tiles_cap, c->tile_bytes, scan_tiles(c), c->d_hitlines,
+                                        c->st, c->d_tiles + 4 * c->tiles_cap));
         // Text order on the device: sorted window starts, then the distinct lines of the sorted windows. When
         // the device has no room for the sort's scratch (about 60 bytes per hit window), or FFBF_HOST_ORDER is
         // set, the records are ordered on the host instead; the results are the same.
@@ -847,20 +858,17 @@ ffbf_status scan_host_pipelined(ffbf_ctx* c, const uint8_t* text, size_t len) {
     CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * sizeof(uint32_t), c->st));
     TRY(prepare_fast(c));
     c->scan_path = 1;
-    const ffbf::ScanArgs a = make_scan_args(c);
     const uint64_t chunk = pipe_chunk(len);
-    const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, chunk, c->num_sms, false);
-    const int threads = ffbf::config_threads(cfg);
-    const uint32_t rows = cfg.rows ? cfg.rows : ffbf::fast_rows(chunk, cfg, c->num_sms, false);
+    ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, chunk, c->num_sms, false);
+    if (len >= ffbf::kShortRowsText && cfg.rows < 4) cfg.rows = 4;
+    c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
     ffbf::FastJob job;
-    cudaError_t e;
-    const uint64_t covered = ffbf::fill_fast_job(a, c->d_stage1, cfg, rows, &job, &e);
-    if (e != cudaSuccess) return fail(c, FFBF_ECUDA, "tensor map encoding failed");
-    const uint64_t item_bytes = (uint64_t)threads * rows * 128;
+    CUDA_TRY(c, ffbf::fill_fast_job(make_scan_args(c), c->d_stage1, cfg, &job));
+    const uint64_t item_bytes = (uint64_t)ffbf::config_threads(cfg) * cfg.rows * 128;
     const uint32_t per_chunk = (uint32_t)std::max<uint64_t>(1, chunk / item_bytes);
     const uint32_t n_chunks = (job.n_supertiles + per_chunk - 1) / per_chunk;
     if (!c->st_copy) CUDA_TRY(c, cudaStreamCreateWithFlags(&c->st_copy, cudaStreamNonBlocking));
-    while (c->pipe_events.size() < (size_t)n_chunks + 2) {
+    while (c->pipe_events.size() < (size_t)n_chunks + 1) {
         cudaEvent_t ev;
         CUDA_TRY(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         c->pipe_events.push_back(ev);
@@ -887,31 +895,23 @@ ffbf_status scan_host_pipelined(ffbf_ctx* c, const uint8_t* text, size_t len) {
     CUDA_TRY(c, cudaMemcpyAsync(c->d_jobs, c->h_jobs, n_chunks * sizeof(ffbf::FastJob), cudaMemcpyHostToDevice,
                                 c->st));
     // the copies overwrite the text buffer: start them after what the context's stream already holds
-    CUDA_TRY(c, cudaEventRecord(c->pipe_events[n_chunks + 1], c->st));
-    CUDA_TRY(c, cudaStreamWaitEvent(c->st_copy, c->pipe_events[n_chunks + 1], 0));
+    CUDA_TRY(c, cudaEventRecord(c->pipe_events[n_chunks], c->st));
+    CUDA_TRY(c, cudaStreamWaitEvent(c->st_copy, c->pipe_events[n_chunks], 0));
     uint64_t copied = 0;
     for (uint32_t i = 0; i < n_chunks; i++) {
         const uint32_t first = i * per_chunk;
         const uint32_t count = std::min(per_chunk, job.n_supertiles - first);
-        const uint64_t end = std::min<uint64_t>(len, (uint64_t)(first + count) * item_bytes);
-        if (end > copied) {
-            CUDA_TRY(c, cudaMemcpyAsync(c->d_text_own + copied, text + copied, end - copied, cudaMemcpyHostToDevice,
-                                        c->st_copy));
-            copied = end;
-        }
+        // the last item's launch also scans the bytes after the last whole stream
+        const uint64_t end = i + 1 == n_chunks ? len : std::min<uint64_t>(len, (uint64_t)(first + count) * item_bytes);
+        CUDA_TRY(c, cudaMemcpyAsync(c->d_text_own + copied, text + copied, end - copied, cudaMemcpyHostToDevice,
+                                    c->st_copy));
+        copied = end;
         CUDA_TRY(c, cudaEventRecord(c->pipe_events[i], c->st_copy));
         CUDA_TRY(c, cudaStreamWaitEvent(c->st, c->pipe_events[i], 0));
         CUDA_TRY(c, cudaMemsetAsync(c->d_counters + ffbf::CNT_QUEUE, 0, sizeof(uint32_t), c->st));
         CUDA_TRY(c, ffbf::launch_fast_jobs(c->g.len, cfg, c->d_jobs + i, 1, count, job.stage1_nwords,
                                            c->d_counters + ffbf::CNT_ERROR, c->num_sms, c->st));
     }
-    if (copied < len) {
-        CUDA_TRY(c, cudaMemcpyAsync(c->d_text_own + copied, text + copied, len - copied, cudaMemcpyHostToDevice,
-                                    c->st_copy));
-    }
-    CUDA_TRY(c, cudaEventRecord(c->pipe_events[n_chunks], c->st_copy));
-    CUDA_TRY(c, cudaStreamWaitEvent(c->st, c->pipe_events[n_chunks], 0));
-    CUDA_TRY(c, ffbf::scan_tail(a, covered, c->st));
     return FFBF_OK;
 }
 
@@ -944,7 +944,7 @@ ffbf_status scan_one(ffbf_ctx* c, const uint8_t* text, size_t len, ffbf_scan_res
 // Device bytes a scan of `len` text bytes needs beyond what the context holds: the text buffer, the tile
 // summaries and, the first time, the hit buffers.
 uint64_t scan_need(const ffbf_ctx* c, uint64_t len) {
-    const uint64_t ntiles = (len + ffbf::kScanTile - 1) / ffbf::kScanTile;
+    const uint64_t ntiles = tiles_for(len);
     uint64_t need = len + 64 + 8 * (4 * ntiles + 2 * ffbf::tile_agg_words(ntiles));
     if (!c->d_hits) need += 2 * kInitialHitsCap * 16;
     return need;
@@ -1323,16 +1323,13 @@ ffbf_status ffbf_debug_scan_unpublished(ffbf_ctx* c, const uint8_t* d_text, size
     CUDA_TRY(c, cudaMemsetAsync(c->d_gate, 0, sizeof(uint32_t), c->st));  // never published
     CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * sizeof(uint32_t), c->st));
     TRY(prepare_fast(c));
-    const ffbf::ScanArgs a = make_scan_args(c);
-    const int threads = ffbf::config_threads(c->cfg);
-    const uint32_t rows = c->cfg.rows ? c->cfg.rows : ffbf::fast_rows(len, c->cfg, c->num_sms, false);
-    cudaError_t e;
-    ffbf::fill_fast_job(a, c->d_stage1, c->cfg, rows, c->h_job, &e);
-    if (e != cudaSuccess) return fail(c, FFBF_ECUDA, "tensor map encoding failed");
+    const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, len, c->num_sms, false);
+    c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
+    CUDA_TRY(c, ffbf::fill_fast_job(make_scan_args(c), c->d_stage1, cfg, c->h_job));
     c->h_job->ready = c->d_gate;
     c->h_job->ready_spins = spins;
     CUDA_TRY(c, cudaMemcpyAsync(c->d_job, c->h_job, sizeof(ffbf::FastJob), cudaMemcpyHostToDevice, c->st));
-    CUDA_TRY(c, ffbf::launch_fast_jobs(c->g.len, c->cfg, c->d_job, 1, c->h_job->n_supertiles, c->h_job->stage1_nwords,
+    CUDA_TRY(c, ffbf::launch_fast_jobs(c->g.len, cfg, c->d_job, 1, c->h_job->n_supertiles, c->h_job->stage1_nwords,
                                        c->d_counters + ffbf::CNT_ERROR, c->num_sms, c->st));
     CUDA_TRY(c, cudaMemcpyAsync(c->h_counters, c->d_counters, ffbf::CNT_WORDS * 4, cudaMemcpyDeviceToHost, c->st));
     TRY(sync(c));

@@ -141,8 +141,8 @@ __device__ __forceinline__ long long line_end_of_window(const CollectJob& a, uin
     const bool back = (threadIdx.x & 4) == 0;
     const long long n = (long long)a.n;
     const long long pos = back ? (long long)w - 1 : (long long)(w + a.len);
-    const long long tile = pos / kScanTile * kScanTile;
-    const long long stop = back ? tile : min(n, tile + kScanTile);
+    const long long tile = pos / a.tile_bytes * a.tile_bytes;
+    const long long stop = back ? tile : min(n, tile + a.tile_bytes);
     long long res = -1, c = (pos & ~63LL) + 16 * (threadIdx.x & 3);
     bool busy = active;
     if (back ? pos < 0 : pos >= n) {  // the text's first and last byte end a line
@@ -204,7 +204,7 @@ __device__ void collect_one(const CollectJob& a, uint32_t cta) {
         if (i < end && (threadIdx.x & 7) == 0) {
             long long s = sp, e = ep;
             if (s < 0) {
-                long long t = (long long)((w - 1) / kScanTile) - 1;
+                long long t = (long long)((w - 1) / a.tile_bytes) - 1;
                 for (uint64_t k = 0; k < kWalkTiles && s < 0 && t >= 0; k++, t--) {
                     const long long l = a.tile_last_nl[t];
                     if (l >= 0) s = l + 1;
@@ -212,7 +212,7 @@ __device__ void collect_one(const CollectJob& a, uint32_t cta) {
                 if (t < 0 && s < 0) s = 0;
             }
             if (e < 0) {
-                uint64_t t = (w + a.len) / kScanTile + 1;
+                uint64_t t = (w + a.len) / a.tile_bytes + 1;
                 for (uint64_t k = 0; k < kWalkTiles && e < 0 && t < a.ntiles; k++, t++) {
                     const long long f = a.tile_first_nl[t];
                     if (f != LLONG_MAX) e = f;

@@ -26,6 +26,7 @@ struct CollectJob {
     uint32_t* counters;  // CNT_HITS in; CNT_MATCHES counts finished CTAs (zero before and after)
     const long long* tile_first_nl;
     const long long* tile_last_nl;
+    uint32_t tile_bytes;
     uint64_t ntiles;
     ResultHead* head;  // pinned
     uint64_t* off;     // pinned: cap window starts, then line starts, then line ends

@@ -71,6 +71,7 @@ struct ffbf_ctx {
     uint32_t nhits = 0;
     long long* d_tiles = nullptr;  // 4 arrays of tiles_cap (first, last, prev, next), then block aggregates
     uint64_t tiles_cap = 0;
+    uint32_t tile_bytes = ffbf::kScanTile;  // bytes per tile of the last scan's summaries
     int scan_path = 0;             // 0 = generic, 1 = fast
     uint32_t* d_stage1 = nullptr;  // stage-1 table of the tuned scan (cache copy or its fold)
     bool stage1_dirty = true;
@@ -202,6 +203,9 @@ ffbf::ScanArgs make_scan_args(ffbf_ctx* c);
 ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta);
 bool use_fast(const ffbf_ctx* c, uint64_t n);
 ffbf_status launch_scan(ffbf_ctx* c);  // counters reset + scan of c->d_text on the context's stream
+// Tile summaries a scan of len bytes may need, and those of the context's current scan.
+uint64_t tiles_for(uint64_t len);
+inline uint64_t scan_tiles(const ffbf_ctx* c) { return (c->text_len + c->tile_bytes - 1) / c->tile_bytes; }
 // Sizes the scan buffers for a device text of len bytes and resets the results, without launching.
 ffbf_status setup_scan_state(ffbf_ctx* c, const uint8_t* d_text, size_t len);
 
@@ -211,8 +215,8 @@ ffbf_status create_scan_slot(int device, ffbf_ctx** out);
 void attach_filters(ffbf_ctx* slot, const ffbf_ctx* owner);
 
 // A scan of many (context, device text) jobs in a few launches: the tuned kernel's descriptors grouped by
-// (LEN, configuration), one launch per group with its jobs largest first, and the generic kernel over every
-// job's tiles that the tuned kernel does not cover (ragged ends, short texts, other geometries).
+// (LEN, configuration), one launch per group with its jobs largest first, and the generic kernel over the tiles of
+// the jobs that the tuned kernel does not take (short texts, other geometries).
 struct PlanLaunch {
     uint32_t len;
     ffbf::FastConfig cfg;

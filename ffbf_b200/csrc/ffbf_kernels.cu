@@ -511,21 +511,22 @@ __global__ void __launch_bounds__(1024) k_tile_scan2(const long long* first, con
 }
 
 __global__ void k_resolve(const uint8_t* text, uint64_t n, uint32_t len, const HitRec* hits, uint32_t nhits,
-                          const long long* prev_nl, const long long* next_nl, HitLine* out) {
+                          const long long* prev_nl, const long long* next_nl, uint32_t tile_bytes, HitLine* out) {
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nhits) return;
     const uint64_t w = hits[j].off;
     // the line's ends within the tiles of the window's neighbours, else from the tile summaries
-    const long long p = line_start_in_tile(text, n, w);
-    const long long e = line_end_in_tile(text, n, w + len);
-    out[j] = HitLine{p >= 0 ? (uint64_t)p : (uint64_t)(prev_nl[(w - 1) / kScanTile] + 1),
-                     e >= 0 ? (uint64_t)e
-                            : next_nl[(w + len) / kScanTile] == LLONG_MAX ? n : (uint64_t)next_nl[(w + len) / kScanTile]};
+    long long p = line_start_in_tile(text, n, w, tile_bytes);
+    long long e = line_end_in_tile(text, n, w + len, tile_bytes);
+    if (p < 0) p = prev_nl[(w - 1) / tile_bytes] + 1;
+    if (e < 0) e = next_nl[(w + len) / tile_bytes] == LLONG_MAX ? (long long)n : next_nl[(w + len) / tile_bytes];
+    out[j] = HitLine{(uint64_t)p, (uint64_t)e};
 }
 
 cudaError_t resolve_lines(const uint8_t* text, uint64_t n, uint32_t len, const HitRec* hits, uint32_t nhits,
                           const long long* tile_first, const long long* tile_last, long long* prev_nl,
-                          long long* next_nl, uint64_t ntiles, HitLine* out, cudaStream_t st, long long* agg) {
+                          long long* next_nl, uint32_t tile_bytes, uint64_t ntiles, HitLine* out, cudaStream_t st,
+                          long long* agg) {
     if (ntiles && agg) {
         const uint32_t nb = (uint32_t)((ntiles + kTileAggBlock - 1) / kTileAggBlock);
         k_tile_agg<<<nb, 1024, 0, st>>>(tile_first, tile_last, ntiles, agg, agg + nb);
@@ -536,7 +537,7 @@ cudaError_t resolve_lines(const uint8_t* text, uint64_t n, uint32_t len, const H
         note_launches(1);
     }
     if (nhits) {
-        k_resolve<<<(nhits + 255) / 256, 256, 0, st>>>(text, n, len, hits, nhits, prev_nl, next_nl, out);
+        k_resolve<<<(nhits + 255) / 256, 256, 0, st>>>(text, n, len, hits, nhits, prev_nl, next_nl, tile_bytes, out);
         note_launches(1);
     }
     return cudaGetLastError();

@@ -47,8 +47,10 @@ struct ScanArgs {
     HitRec* hits;
     uint32_t hits_cap;
     uint32_t* counters;
-    long long* tile_first_nl;  // per tile: first '\n' position in the tile, or LLONG_MAX
-    long long* tile_last_nl;   // per tile: last '\n' position in the tile, or -1
+    // newline summaries: per tile of tile_bytes, its first '\n' position or LLONG_MAX, and its last or -1
+    long long* tile_first_nl;
+    long long* tile_last_nl;
+    uint32_t tile_bytes;  // kScanTile for the generic scan
     uint64_t ntiles;
     uint64_t tile_begin;  // first tile this launch handles (tiles before it belong to another kernel)
     int cache_in_smem;
@@ -79,7 +81,7 @@ constexpr uint32_t kTileAggBlock = 4096;  // tiles per block of the two-pass til
 inline uint64_t tile_agg_words(uint64_t ntiles) { return ntiles / kTileAggBlock + 1; }
 cudaError_t resolve_lines(const uint8_t* text, uint64_t n, uint32_t len, const HitRec* hits, uint32_t nhits,
                           const long long* tile_first, const long long* tile_last, long long* prev_nl,
-                          long long* next_nl, uint64_t ntiles, HitLine* out, cudaStream_t st,
+                          long long* next_nl, uint32_t tile_bytes, uint64_t ntiles, HitLine* out, cudaStream_t st,
                           long long* agg = nullptr);
 
 cudaError_t table_build(const uint64_t* d_ids, uint64_t nids, const uint64_t* d_hash, uint64_t* d_keys,

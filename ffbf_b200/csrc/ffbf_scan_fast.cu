@@ -22,18 +22,18 @@
 // test rejects. Dense filters probe the global filter, in L2, through register rings. Surviving windows are
 // queued by position per warp; a full queue, or the stream's end, is flushed by the whole warp, each lane hashing
 // its queued windows again and running the full K-bit test on the global filter in the reference order (checkInFilter,
-// ffbf.cpp:214-239).
+// ffbf.cpp:214-239). The bytes after the last whole stream are scanned by the CTA of the last work item.
 //
 // Validity. A window is tested only when its LEN bytes hold no '\n' (processFile resets the hash at '\n'), from a
-// newline mask per 32-byte block. Each stream's first and last '\n' feed the per-16 KiB-tile newline summaries the
-// line resolver reads.
+// newline mask per 32-byte block. Each stream's first and last '\n' feed the newline summaries, per tile of 16
+// KiB or a little more, that the line resolver reads.
 //
 // What bounds it. Sparse: the shared-memory pipe (9 wavefronts per warp and byte: 4 for the two S-box entries, 3.5
 // for the first table probe's random words, the rest for the predicated second probe and the text) and the ALU pipe,
-// at 24 warps per SM. Dense: the L1TEX unit, which looks up one random sector per clock and SM (words, 1M patterns: 0.93
-// of that). On one B200, before -> now, GB/s of text: 10k patterns, 4 GiB 662 -> 931; LEN 24, 8k patterns in 2^20 + 2^24
-// bits, 2 GiB 487 -> 879 and 40k in 2^22 + 2^26 299 -> 623; 150k in 2^23 + 2^27, 256 MiB 295 -> 511; words, 1M
-// patterns 311 -> 354; 4M 16-byte signatures 245 -> 271.
+// at 16 to 20 warps per SM. Dense: the L1TEX unit, which looks up one random sector per clock and SM (words, 1M patterns: 0.93
+// of that). On one B200, before -> now, GB/s of text: 10k patterns, 4 GiB 662 -> 890, 64 MiB 443 -> 618, 8 MiB 69 -> 215; LEN
+// 24, 8k patterns in 2^20 + 2^24 bits, 2 GiB 487 -> 855 and 40k in 2^22 + 2^26 299 -> 647; 150k in 2^23 + 2^27, 256 MiB
+// 295 -> 511; words, 1M patterns 311 -> 354; 4M 16-byte signatures 245 -> 272.
 //
 // Every mbarrier wait is bounded; on timeout the CTA records an error flag and stops.
 #include <cuda.h>
@@ -46,6 +46,7 @@
 #include <cstring>
 
 #include "ffbf_scan_fast.cuh"
+#include "ffbf_text.cuh"
 
 namespace ffbf {
 
@@ -110,6 +111,13 @@ __device__ __forceinline__ void tma_load_3d_hint(uint32_t dst, const CUtensorMap
         : "memory");
 }
 
+// An untiled copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) completed on an mbarrier.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
@@ -121,6 +129,13 @@ __device__ __forceinline__ uint64_t l2_evict_first_policy() {
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     uint2 v;
     asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
+}
+// The same at a constant distance, which the load's own offset takes.
+template <int OFFSET>
+__device__ __forceinline__ uint2 lds64_at(uint32_t addr) {
+    uint2 v;
+    asm("ld.shared.v2.u32 {%0, %1}, [%2+%3];" : "=r"(v.x), "=r"(v.y) : "r"(addr), "n"(OFFSET));
     return v;
 }
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
@@ -182,10 +197,45 @@ __device__ __forceinline__ bool full_check_from(const Geom& g, const uint32_t* _
     return true;
 }
 
+// The hash of the window of L bytes at `start`, its bytes read from the text's aligned words that hold them and no
+// others. *newline tells whether one of them is '\n'.
+template <int L>
+__device__ __forceinline__ uint64_t text_window_hash(const uint8_t* __restrict__ text, uint64_t start, uint32_t lane_tab,
+                                                     bool* newline) {
+    constexpr int kWords = (L + 3) / 4;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(text + (start & ~3ull));
+    const uint32_t off = (uint32_t)start & 3u;
+    uint32_t w[kWords + 1];
+#pragma unroll
+    for (int q = 0; q <= kWords; q++) w[q] = 4u * q < off + L ? __ldg(src + q) : 0u;
+    uint32_t hl = 0, hh = 0, found = 0;
+#pragma unroll
+    for (int q = 0; q < kWords; q++) {
+        const uint32_t v = __funnelshift_r(w[q], w[q + 1], 8 * off);
+        const uint32_t c = clear_high_bytes(v);
+        found |= nl_bytes(v) & (4 * q + 4 <= L ? 0xffffffffu : 0xffffffffu >> (8 * (4 * q + 4 - L)));
+#pragma unroll
+        for (int j = 0; j < 4 && 4 * q + j < L; j++) {
+            const uint2 sv = lds64(entry_addr(c, j, lane_tab));
+            const uint32_t nl = __funnelshift_l(hh, hl, 1) ^ sv.x, nh = __funnelshift_l(hl, hh, 1) ^ sv.y;
+            hl = nl;
+            hh = nh;
+        }
+    }
+    *newline = found != 0;
+    return ((uint64_t)hh << 32) | hl;
+}
+
+__device__ __forceinline__ void record_hit(const FastJob* J, const Geom& g, uint64_t start, uint64_t h) {
+    set_all<2>(g, J->ff_words, h);
+    const uint32_t slot = atomicAdd(J->counters + CNT_HITS, 1u);
+    if (slot < J->hits_cap) J->hits[slot] = HitRec{start, h};
+}
+
 // The whole warp drains its candidate queue: lane i takes entries i, i + 32, ... (PER_LANE at most). An entry is a
 // window's end, {position in the stream | lane << 16}. Each lane reads its windows' bytes back from the text (still in
 // L2), hashes them and runs the full K-bit test: few windows get here, so this costs less than carrying every
-// window's hash to its test in the byte loop. All of a lane's loads of one kind are issued before any is used.
+// window's hash to its test in the byte loop. All of a lane's first probes are issued before any is used.
 template <int L, int PER_LANE>
 __device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int qn, uint64_t warp_pos0, uint64_t stride,
                                          int lane, uint32_t lane_tab) {
@@ -193,7 +243,6 @@ __device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int q
     const Geom g = J->g;
     const uint32_t* __restrict__ main_words = J->main_words;
     const uint8_t* __restrict__ text = J->text;
-    constexpr int kWords = (L + 3) / 4;
     uint64_t start[PER_LANE], h[PER_LANE];
     uint32_t v[PER_LANE], bi[PER_LANE];
 #pragma unroll
@@ -203,34 +252,145 @@ __device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int q
         if (i >= qn) continue;
         const uint32_t e = lds32_volatile(qaddr + 4u * (uint32_t)i);
         start[t] = warp_pos0 + (e >> 16) * stride + (e & 0xFFFFu) + 1 - L;
-        // the aligned words that hold the window's bytes, and no others
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(text + (start[t] & ~3ull));
-        const uint32_t off = (uint32_t)start[t] & 3u;
-        uint32_t w[kWords + 1];
-#pragma unroll
-        for (int q = 0; q <= kWords; q++) w[q] = 4u * q < off + L ? __ldg(src + q) : 0u;
-        uint32_t hl = 0, hh = 0;
-#pragma unroll
-        for (int j = 0; j < L; j++) {
-            const uint32_t c = clear_high_bytes(__funnelshift_r(w[j / 4], w[j / 4 + 1], 8 * off));
-            const uint2 sv = lds64(entry_addr(c, j & 3, lane_tab));
-            const uint32_t nl = __funnelshift_l(hh, hl, 1) ^ sv.x, nh = __funnelshift_l(hl, hh, 1) ^ sv.y;
-            hl = nl;
-            hh = nh;
-        }
-        h[t] = ((uint64_t)hh << 32) | hl;
+        bool newline;
+        h[t] = text_window_hash<L>(text, start[t], lane_tab, &newline);  // windows with a '\n' are not queued
         bi[t] = bit_index<1>(g, h[t], 0);
         v[t] = __ldg(main_words + (bi[t] >> 5));
     }
 #pragma unroll
     for (int t = 0; t < PER_LANE; t++) {
         if (!((v[t] >> (bi[t] & 31)) & 1u)) continue;
-        if (!full_check_from(g, main_words, h[t], 1)) continue;
-        set_all<2>(g, J->ff_words, h[t]);
-        const uint32_t slot = atomicAdd(J->counters + CNT_HITS, 1u);
-        if (slot < J->hits_cap) J->hits[slot] = HitRec{start[t], h[t]};
+        if (full_check_from(g, main_words, h[t], 1)) record_hit(J, g, start[t], h[t]);
     }
     __syncwarp();
+}
+
+// What a warp does when its streams are done: their newline summary, and in the CTA of the job's last work item the
+// text's end after its last whole stream (less than one stream), a window per thread, where a launch of its own took 60
+// us for 12 KB. z is the thread's stream, nl_span its first '\n' (low half, 0xffff: none) and its last. One function,
+// so that the byte loop keeps its registers.
+template <int L>
+__device__ __noinline__ void finish_streams(const FastJob* J, uint64_t z, uint32_t nl_span, int threads, uint32_t lane_tab,
+                                            uint32_t* error_flag) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t n = J->n, n_streams = J->n_streams, slen = (uint64_t)J->rows * kRowBytes;
+    const uint64_t pos = z * slen;
+    const bool active = z < n_streams, any = active && (nl_span & 0xffffu) != 0xffffu;
+    long long f = any ? (long long)(pos + (nl_span & 0xffffu)) : LLONG_MAX;
+    long long l = any ? (long long)(pos + (nl_span >> 16)) : -1;
+    // reduce over the lanes whose streams share a tile
+    const uint32_t spt_log2 = J->streams_per_tile_log2;
+    const int G = 1 << spt_log2;
+    for (int o = 1; o < G; o <<= 1) {
+        f = min(f, __shfl_xor_sync(0xffffffffu, f, o));
+        l = max(l, __shfl_xor_sync(0xffffffffu, l, o));
+    }
+    uint64_t tile = z >> spt_log2;
+    bool write = active && (lane & (G - 1)) == 0;
+    const uint64_t covered = n_streams * slen;
+    if (covered < n && z / threads == J->n_supertiles - 1) {
+        const Geom g = J->g;
+        for (uint64_t p = covered + threadIdx.x; p < n; p += threads) {
+            if (p + 1 < L) continue;
+            bool newline;
+            const uint64_t h = text_window_hash<L>(J->text, p + 1 - L, lane_tab, &newline);
+            if (!newline && full_check_from(g, J->main_words, h, 0)) record_hit(J, g, p + 1 - L, h);
+        }
+        __syncwarp();
+        // the last stream's warp adds the newlines of the text's end to the tile it falls in, which may be a new one
+        const uint64_t z0 = z - lane;
+        if (z0 < n_streams && n_streams <= z0 + 32) {
+            long long tf = LLONG_MAX, tl = -1;
+            for (long long c = (long long)covered + 16 * lane; c < (long long)n; c += 512) {
+                const uint4 v = chunk16(J->text, c, (long long)n);
+                const uint32_t w[4] = {nl_bytes(v.x), nl_bytes(v.y), nl_bytes(v.z), nl_bytes(v.w)};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    if (!w[q]) continue;
+                    tf = min(tf, c + 4 * q + (__ffs(w[q]) - 1) / 8);
+                    tl = max(tl, c + 4 * q + (31 - __clz(w[q])) / 8);
+                }
+            }
+            for (int o = 16; o; o >>= 1) {
+                tf = min(tf, __shfl_xor_sync(0xffffffffu, tf, o));
+                tl = max(tl, __shfl_xor_sync(0xffffffffu, tl, o));
+            }
+            const uint64_t end_tile = n_streams >> spt_log2;
+            if (tile == end_tile) {
+                f = min(f, tf);
+                l = max(l, tl);
+            }
+            if (n_streams % G == 0 && lane == 31) {
+                // no stream is in that tile; lane 31 writes no other one (G is at least 8)
+                tile = end_tile;
+                f = tf;
+                l = tl;
+                write = true;
+            }
+        }
+    }
+    if (write) {
+        if (tile < J->n_tiles) {
+            J->tile_first_nl[tile] = f;
+            J->tile_last_nl[tile] = l;
+        } else {
+            atomicOr(error_flag, 0x200u);
+        }
+    }
+}
+
+// The current job as the byte loop reads it, once per part: kept in shared memory, so that it holds no registers.
+struct JobState {
+    int job;
+    uint32_t rows;  // 0: the job's table does not fit or did not arrive, and its parts fail the self-check
+    uint32_t n_supertiles;
+    uint32_t s1_bmask;      // byte offset of the stage-1 table word of bit (h & (T-1)): (h >> 3) & s1_bmask
+    uint32_t s2, s2_bmask;  // the second probe's table: the same, or with S = 1 a word of ones
+    uint32_t a_mask, b_mask;  // dense modes: the regions of the two pipelined probes
+    const uint32_t *a_words, *b_words;
+    uint64_t n_streams;
+    uint32_t tables;  // tables loaded so far: the parity of their barrier
+};
+
+// Makes job `job` current: all threads of the CTA call it at the same stage, where every warp is done with the job
+// before. With `s1` its stage-1 table (T = C >> shift bits) is loaded there.
+__device__ __noinline__ void change_job(const FastJob* jobs, int job, JobState* s, uint32_t s1, uint32_t* s1p,
+                                        uint32_t max_s1_words, uint32_t ones, uint32_t tbar, uint32_t* error_flag) {
+    const FastJob* J = jobs + job;
+    const uint32_t tid = threadIdx.x;
+    __syncthreads();
+    const bool fits = !s1 || J->stage1_nwords <= max_s1_words;
+    const uint32_t nw = s1 && fits ? J->stage1_nwords : 0u;  // a power of two
+    const uint32_t parity = s->tables & 1u;
+    if (tid == 0) {
+        const uint32_t bmask = ((J->g.cache_mask >> J->stage1_shift) >> 3) & ~3u;
+        s->job = job;
+        s->rows = fits ? J->rows : 0u;
+        s->n_supertiles = J->n_supertiles;
+        s->s1_bmask = bmask;
+        s->s2 = J->g.s > 1 ? s1 : ones;
+        s->s2_bmask = J->g.s > 1 ? bmask : 0u;
+        s->a_mask = J->a_mask;
+        s->b_mask = J->b_mask;
+        s->a_words = J->main_words + J->a_add / 32;
+        s->b_words = J->main_words + J->b_add / 32;
+        s->n_streams = J->n_streams;
+        if (nw >= 4) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // after plain stores to a table
+            mbar_expect_tx(tbar, 4 * nw);
+            bulk_load(s1, J->stage1_words, 4 * nw, tbar);
+        }
+    }
+    if (nw >= 4) {
+        if (!mbar_wait_bounded(tbar, parity)) {
+            atomicOr(error_flag, 4u);
+            s->rows = 0;
+        }
+    } else if (tid < nw) {
+        s1p[tid] = J->stage1_words[tid];  // regions of 32 and 64 bits
+    }
+    __syncthreads();
+    if (tid == 0 && nw >= 4) s->tables++;  // read next after the barrier of the next change
 }
 
 template <int N>
@@ -355,13 +515,14 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     auto fbar = [&](uint32_t k) { return bar0 + 8u * (k & 1u); };
     auto ebar = [&](uint32_t k) { return bar0 + 16u + 8u * (k & 1u); };
     int* meta = reinterpret_cast<int*>(smem + 2 * kStageBytes + kTabBytes + 32);  // [stage][4]: job, item, part, valid
-    const uint32_t ones = bar0 + 64u;
+    const uint32_t ones = bar0 + 64u, tbar = bar0 + 72u;  // the table's load completes on tbar
     const uint32_t queues = bar0 + 128u;
     const uint32_t s1 = queues + (THREADS / 32) * 4u * kQueueCap;
     uint32_t* s1p = reinterpret_cast<uint32_t*>(smem + (s1 - base));
     // the load sequencer's state (thread 0 only) and each warp's first text position
     __shared__ int s_abort;
     __shared__ uint32_t s_ni, s_nj;
+    __shared__ JobState s_job;
     __shared__ int s_nr;
     __shared__ uint64_t s_wpos[THREADS / 32];
 
@@ -423,6 +584,8 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     };
     if (tid == 0) {
         s_abort = 0;
+        s_job.job = -1;
+        s_job.tables = 0;
         s_ni = blockIdx.x;
         s_nj = 0;
         s_nr = -1;
@@ -430,6 +593,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
             mbar_init(fbar(b), 1);
             mbar_init(ebar(b), THREADS / 32);
         }
+        mbar_init(tbar, 1);
         *reinterpret_cast<uint32_t*>(smem + (ones - base)) = 0xFFFFFFFFu;  // the S = 1 second-probe word
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // publication gate: a bounded poll, and no load in flight if it gives up
@@ -456,12 +620,12 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     __syncthreads();
 
     const uint32_t lane_tab = tab + (uint32_t)(lane & 15) * 8u;  // entry c of this lane's copy: + c * 128
-    const uint32_t lane_out = kTwoTables ? lane_tab + 128u * 128u : lane_tab;
     // S-box entry of byte i of the 64-byte span (p, c): as it enters the window, and rotated by LEN as it leaves
     auto sbox_in = [&](const uint32_t (&c)[8], int i) { return lds64(entry_addr(c[i >> 2], i & 3, lane_tab)); };
     auto sbox_out = [&](const uint32_t (&p)[8], const uint32_t (&c)[8], int i) {
-        const uint2 o = lds64(i >= L ? entry_addr(c[(i - L) >> 2], (i - L) & 3, lane_out)
-                                     : entry_addr(p[(i - L + 32) >> 2], (i - L + 32) & 3, lane_out));
+        const uint2 o = lds64_at<kTwoTables ? 128 * 128 : 0>(
+            i >= L ? entry_addr(c[(i - L) >> 2], (i - L) & 3, lane_tab)
+                   : entry_addr(p[(i - L + 32) >> 2], (i - L + 32) & 3, lane_tab));
         return kTwoTables ? o : make_uint2(o.y, o.x);
     };
     // Zeroes the block's high bytes where the table does not map them (rare in text: one test per block).
@@ -476,19 +640,13 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     const uint32_t qaddr = queues + (uint32_t)warp * 4u * kQueueCap;
     const unsigned lt_mask = (1u << lane) - 1u;
 
-    // the current job's parameters (reloaded when the job changes)
-    int cur_job = -1;
-    uint32_t R = 0, s1_bmask = 0;
-    uint32_t a_mask = 0, b_mask = 0;  // dense modes: the regions of the two pipelined probes
-    const uint32_t *a_words = nullptr, *b_words = nullptr;
-    uint32_t s2 = s1, s2_bmask = 0;  // sparse mode: the second probe's table (the stage-1 table, or with S = 1 a word of ones)
-    bool s1_fits = true;
-    auto job_desc = [&]() { return jobs + cur_job; };
+    auto job_desc = [&]() { return jobs + s_job.job; };
 
     int qn = 0;  // warp-uniform queue fill
     auto flush = [&]() {
         __syncwarp();
-        flush_queue<L, kQueueCap / 32>(job_desc(), qaddr, qn, s_wpos[warp], (uint64_t)R * kRowBytes, lane, lane_tab);
+        flush_queue<L, kQueueCap / 32>(job_desc(), qaddr, qn, s_wpos[warp], (uint64_t)s_job.rows * kRowBytes, lane,
+                                         lane_tab);
         qn = 0;
     };
     // Queues the windows whose bits are set in each lane's mask; bit i is the window ending at pos + i in the lane's
@@ -519,7 +677,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     uint32_t prev[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     // newline mask of the previous block (bit 31 forced at the text's start, where nothing precedes offset 0)
     uint32_t nl_prev = 0;
-    uint32_t first_nl = ~0u, last_nl = ~0u;  // first and last '\n' of the stream so far
+    uint32_t nl_span = 0xffffu;  // first (low half, 0xffff: none) and last '\n' of the stream so far
 
     for (uint32_t k = 0;; k++) {
         {
@@ -545,41 +703,17 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         const int job = m[0], r = m[2];
         const uint32_t st = (uint32_t)m[1];
         if (tid == 0 && !issue(k + 1)) s_abort = 1;
-        if (job != cur_job) {
-            cur_job = job;
-            const FastJob* J = job_desc();
-            const Geom g = J->g;
-            R = J->rows;
-            s1_fits = !kTable || J->stage1_nwords <= max_s1_words;
-            // stage-1 table of T = C >> shift bits, folded modulo T: the byte offset of bit (h & (T-1))'s
-            // word is (h >> 3) & s1_bmask
-            s1_bmask = (((g.cache_mask >> J->stage1_shift) >> 3) & ~3u);
-            a_mask = J->a_mask;
-            a_words = J->main_words + J->a_add / 32;
-            b_mask = J->b_mask;
-            b_words = J->main_words + J->b_add / 32;
-            s2 = g.s > 1 ? s1 : ones;
-            s2_bmask = g.s > 1 ? s1_bmask : 0u;
-            if constexpr (kTable) {
-                // every warp is done with the previous job's table before it is overwritten (all warps change
-                // job at the same stage)
-                __syncthreads();
-                const uint32_t nw = s1_fits ? J->stage1_nwords : 0u;
-                const uint32_t* src = J->stage1_words;
-                for (uint32_t i = tid; i < nw; i += THREADS) s1p[i] = src[i];
-                __syncthreads();
-            }
-        }
+        if (job != s_job.job) change_job(jobs, job, &s_job, kTable ? s1 : 0u, s1p, max_s1_words, ones, tbar, error_flag);
+        const uint32_t R = s_job.rows;
 
         // self-checks: a bad descriptor or sequencing records a code and skips the work
-        if ((uint32_t)job >= n_jobs || st >= job_desc()->n_supertiles || r < -1 || r >= (int)R * kParts || !s1_fits) {
+        if ((uint32_t)job >= n_jobs || st >= s_job.n_supertiles || r < -1 || r >= (int)R * kParts) {
             if (tid == 0) atomicOr(error_flag, 0x100u);
             __syncwarp();
             if (lane == 0) mbar_arrive(ebar(k));
             continue;
         }
-        const uint64_t z = (uint64_t)st * THREADS + tid;
-        const bool active = z < job_desc()->n_streams;
+        const bool active = (uint64_t)st * THREADS + tid < s_job.n_streams;
         const uint8_t* row = smem + (k & 1) * kStageBytes + tid * kPart;
         const int sw = (tid >> 1) & 3;  // the 64-byte swizzle XORs a 16-byte chunk's index with its address bits 7 and 8
 
@@ -600,11 +734,14 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                 hl = nl;
                 hh = nh;
             }
-            nl_prev = newline_mask32(prev) | (z == 0 ? 0x80000000u : 0u);  // text start: nothing before offset 0
-            first_nl = last_nl = ~0u;
+            nl_prev = newline_mask32(prev) | (st == 0 && tid == 0 ? 0x80000000u : 0u);  // text start: nothing before offset 0
+            nl_span = 0xffffu;
             if (lane == 0) s_wpos[warp] = ((uint64_t)st * THREADS + (uint64_t)warp * 32) * R * kRowBytes;
         } else {
             const uint32_t pos0 = (uint32_t)r * kPart;  // this part's first byte in the stream
+            const uint32_t s1_bmask = s_job.s1_bmask, s2 = s_job.s2, s2_bmask = s_job.s2_bmask;
+            const uint32_t a_mask = s_job.a_mask, b_mask = s_job.b_mask;
+            const uint32_t *const a_words = s_job.a_words, *const b_words = s_job.b_words;
 #pragma unroll 1
             for (int b = 0; b < kPart / 32; b++) {
                 uint32_t cur[8];
@@ -663,8 +800,8 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                 if constexpr (kSparse) enqueue(pass & valid, pos0 + (uint32_t)(32 * b));
                 else enqueue(pass, pos0 + (uint32_t)(32 * b - kLag));
                 if (nlm) {
-                    last_nl = pos0 + (uint32_t)(32 * b + 31 - __clz(nlm));
-                    if (first_nl == ~0u) first_nl = pos0 + (uint32_t)(32 * b + __ffs(nlm) - 1);
+                    const uint32_t at = pos0 + (uint32_t)(32 * b);
+                    nl_span = min(nl_span & 0xffffu, at + (uint32_t)__ffs(nlm) - 1u) | (at + 31u - __clz(nlm)) << 16;
                 }
                 nl_prev = nlm;
 #pragma unroll
@@ -686,26 +823,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                     enqueue(rest, pos0 + (uint32_t)(kPart - kLag));
                 }
                 if (qn) flush();  // the queue keeps its candidates across the stream's parts, not across streams
-                // per-16 KiB-tile newline summary: reduce over the lanes whose streams share the tile
-                const FastJob* J = job_desc();
-                const uint64_t pos = z * R * kRowBytes;
-                long long f = active && first_nl != ~0u ? (long long)(pos + first_nl) : LLONG_MAX;
-                long long l = active && last_nl != ~0u ? (long long)(pos + last_nl) : -1;
-                const uint32_t spt_log2 = J->streams_per_tile_log2;
-                const int G = 1 << spt_log2;
-                for (int o = 1; o < G; o <<= 1) {
-                    f = min(f, __shfl_xor_sync(0xffffffffu, f, o));
-                    l = max(l, __shfl_xor_sync(0xffffffffu, l, o));
-                }
-                if (active && (lane & (G - 1)) == 0) {
-                    const uint64_t tile = z >> spt_log2;
-                    if (tile < J->n_tiles) {
-                        J->tile_first_nl[tile] = f;
-                        J->tile_last_nl[tile] = l;
-                    } else {
-                        atomicOr(error_flag, 0x200u);
-                    }
-                }
+                finish_streams<L>(job_desc(), (uint64_t)st * THREADS + tid, nl_span, THREADS, lane_tab, error_flag);
             }
         }
         // this warp is done reading the stage
@@ -726,8 +844,8 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
     return fn;
 }
 
-// static shared memory of k_scan_fast<., THREADS, .> (sequencer, warp positions)
-constexpr size_t static_smem(int threads) { return 8 * (size_t)(threads / 32) + 64; }
+// static shared memory of k_scan_fast<., THREADS, .> (sequencer, current job, warp positions)
+constexpr size_t static_smem(int threads) { return 8 * (size_t)(threads / 32) + 160; }
 
 constexpr size_t fixed_smem(int threads) {
     return 1024 + 2 * (size_t)threads * kPart + kTabBytes + 128 + (threads / 32) * 4 * (size_t)kQueueCap;
@@ -762,7 +880,7 @@ cudaError_t launch_len(const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_
         FFBF_CASE(256, 0);
         FFBF_CASE(384, 0);
         FFBF_CASE(512, 0);
-        FFBF_CASE(768, 0);
+        FFBF_CASE(640, 0);
         FFBF_CASE(192, 1);
         FFBF_CASE(256, 1);
         FFBF_CASE(384, 1);
@@ -797,9 +915,12 @@ uint32_t stage1_shift_for(const Geom& g, int threads) {
     while (((uint64_t)g.cache_bits >> sh) / 8 > room) sh++;
     return sh;
 }
-// the 512-thread kernel's table also fits the 768-thread one, which large texts use (launch_threads)
+// the 512-thread kernel's table also fits the 640-thread one, which large texts use (launch_config)
 static_assert(kSmemLimit - fixed_smem(512) - static_smem(512) - 64 < 131072, "512 threads: a 2^19-bit table");
-static_assert(kSmemLimit - fixed_smem(768) - static_smem(768) - 64 >= 65536, "768 threads: a 2^19-bit table");
+static_assert(kSmemLimit - fixed_smem(640) - static_smem(640) - 64 >= 65536, "640 threads: a 2^19-bit table");
+
+// mode 3 reads the 512-thread table at every CTA size it takes
+int table_threads(const FastConfig& cfg) { return cfg.mode == 3 ? 512 : config_threads(cfg); }
 
 uint32_t stage1_words_for(const Geom& g, int threads) {
     return (uint32_t)(((uint64_t)g.cache_bits >> stage1_shift_for(g, threads)) / 32);
@@ -842,37 +963,54 @@ ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, doub
 int config_threads(const FastConfig& cfg) {
     if (cfg.mode == 1) return cfg.threads == 256 ? 256 : cfg.threads == 192 && cfg.order < 2 ? 192 : 384;
     if (cfg.mode == 2) return cfg.threads == 192 || cfg.threads == 384 ? cfg.threads : 256;
-    if (cfg.mode == 3) return cfg.threads == 768 ? 768 : 512;
+    if (cfg.mode == 3)  // launch_config fits the size to the text
+        return cfg.threads == 192 || cfg.threads == 256 || cfg.threads == 384 || cfg.threads == 640 ? cfg.threads : 512;
     return cfg.threads == 384 || cfg.threads == 512 ? cfg.threads : 256;
 }
 
 int fast_ctas_per_sm(const FastConfig& cfg) { return cfg.mode == 1 && config_threads(cfg) == 192 ? 2 : 1; }
 
-namespace {
-
-// What the busiest CTA slot of a scan alone on the GPU takes, in quarter rows: waves of equal items, each its rows
-// and its halo, whose up to 32 hashed bytes are a quarter of a row's work (measured: 256 MiB of the plain workload, 2
-// waves of 16 rows against 7 of 4, took 571 against 528 us).
-uint64_t wave_cost(uint64_t n, int threads, uint64_t slots, uint32_t rows) {
-    const uint64_t items = (n / kScanTile * kScanTile / ((uint64_t)rows * kRowBytes) + threads - 1) / threads;
-    return (items + slots - 1) / slots * (4 * rows + 1);
+uint32_t fast_tile_bytes(uint32_t rows) {
+    uint32_t streams = 1;
+    while (streams < 32 && streams * rows * kRowBytes < (uint32_t)kScanTile) streams *= 2;
+    return streams * rows * kRowBytes;
 }
 
-}  // namespace
-
 FastConfig launch_config(const FastConfig& cfg, uint64_t n, int num_sms, bool batch) {
-    // Mode 3 runs 768 threads where 24 warps per SM, which hide more of the hash's and the tables' latency than 16
-    // (plain 4 GiB: 911 -> 931 GB/s; LEN 24, 40k patterns in 2^22 + 2^26 bits: 560 -> 623, so about 1.07), finish
-    // before 16 warps with smaller items would (plain 64 MiB: 144 us with 512 threads, 164 with 768). In a batch
-    // other jobs fill the GPU, so the job only has to have four items of its own.
-    FastConfig c = cfg;
-    if (c.mode != 3) return c;
-    FastConfig wide = cfg;
-    wide.threads = 768;
-    if (batch) return n >= 4ull * 4 * kRowBytes * 768 ? wide : c;
-    const uint64_t cost = wave_cost(n, 512, num_sms, fast_rows(n, c, num_sms, false)) * 512 * 107;
-    const uint64_t wide_cost = wave_cost(n, 768, num_sms, fast_rows(n, wide, num_sms, false)) * 768 * 100;
-    return wide_cost < cost ? wide : c;
+    FastConfig best = cfg;
+    if (batch) {
+        // other jobs fill the GPU: mode 3 runs 640 threads where the job has four such items of its own
+        if (cfg.mode == 3 && n >= 4ull * 4 * kRowBytes * 640) best.threads = 640;
+        best.rows = fast_rows(n, best, num_sms, true);
+        return best;
+    }
+    // Alone, the scan lasts as many waves of equal items as the busiest CTA slot takes. An item's streams are walked a
+    // byte per step of all threads, tau ns each (plain workload; at 4 GiB, where all sizes are full, 640 threads take
+    // 4.83 ms, 512 4.79, 384 5.16, 256 5.99, 192 7.56), and an item costs its rows and about 16 steps more. With powers
+    // of two from 4 rows and 512 or 768 threads only, 64 MiB took 131 us (now 109), 8 MiB 114 (39), 1 MiB 129 (31).
+    struct Size {
+        int threads;
+        double tau;
+    };
+    static const Size sparse[] = {{640, 106.0}, {512, 84.0}, {384, 66.0}, {256, 50.0}, {192, 44.0}};
+    constexpr double kItemBytes = 16.0;
+    double best_cost = 0;
+    const uint32_t min_rows = n < kShortRowsText ? 1 : 4;
+    for (int i = 0; i < (cfg.mode == 3 ? 5 : 1); i++) {
+        FastConfig c = cfg;
+        if (cfg.mode == 3) c.threads = sparse[i].threads;
+        const uint64_t threads = config_threads(c), slots = (uint64_t)num_sms * fast_ctas_per_sm(c);
+        for (uint32_t rows = 16; rows >= min_rows; rows--) {
+            const uint64_t items = (n / (rows * kRowBytes) + threads - 1) / threads;
+            const double cost = (double)((items + slots - 1) / slots) * (rows * kRowBytes + kItemBytes) * sparse[i].tau;
+            if (best_cost == 0 || cost < best_cost) {
+                best_cost = cost;
+                best = c;
+                best.rows = rows;
+            }
+        }
+    }
+    return best;
 }
 
 uint32_t fast_rows(uint64_t n, const FastConfig& cfg, int num_sms, bool batch) {
@@ -884,28 +1022,33 @@ uint32_t fast_rows(uint64_t n, const FastConfig& cfg, int num_sms, bool batch) {
         while (rows > 4 && tiles_bytes < 4ull * rows * kRowBytes * threads) rows >>= 1;
         return rows;
     }
-    // alone: the row count with the least work per CTA slot; ties go to the longer items
+    // alone: waves of equal items over the CTA slots, an item its rows and a quarter row for its halo; the row count
+    // with the least work wins, ties go to the longer items
     const uint64_t slots = (uint64_t)num_sms * (uint64_t)fast_ctas_per_sm(cfg);
     uint32_t best = 16;
-    for (uint32_t rows = 8; rows >= 4; rows >>= 1)
-        if (wave_cost(n, threads, slots, rows) < wave_cost(n, threads, slots, best)) best = rows;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t rows = 16; rows >= 4; rows >>= 1) {
+        const uint64_t items = (tiles_bytes / ((uint64_t)rows * kRowBytes) + threads - 1) / threads;
+        const uint64_t cost = (items + slots - 1) / slots * (4 * rows + 1);  // in quarter rows
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = rows;
+        }
+    }
     return best;
 }
 
-uint64_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, uint32_t rows,
-                       FastJob* job, cudaError_t* err) {
-    *err = cudaSuccess;
+cudaError_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, FastJob* job) {
     const int threads = config_threads(cfg);
-    const uint64_t fast_tiles = a.n / kScanTile;  // whole 16 KiB tiles; the rest goes to the generic kernel
+    const uint32_t rows = cfg.rows;
     const uint64_t slen = (uint64_t)rows * kRowBytes;
-    const uint64_t n_streams = fast_tiles * kScanTile / slen;
+    const uint64_t n_streams = a.n / slen;
+    if (n_streams == 0 || a.tile_bytes != fast_tile_bytes(rows)) return cudaErrorInvalidValue;
     memset(job, 0, sizeof *job);
     job->n_streams = n_streams;
     job->rows = rows;
     job->n_supertiles = (uint32_t)((n_streams + threads - 1) / threads);
-    uint32_t spt = (uint32_t)(kScanTile / slen), lg = 0;
-    while ((1u << lg) < spt) lg++;
-    job->streams_per_tile_log2 = lg;
+    while ((slen << job->streams_per_tile_log2) < a.tile_bytes) job->streams_per_tile_log2++;
     job->g = a.g;
     job->main_words = a.main_words;
     job->ff_words = a.ff_words;
@@ -913,14 +1056,14 @@ uint64_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const Fa
     job->stage1_words = stage1_words;
     // the table the kernel reads: the sparse mode's, or the dense mode's prefilter (order 2)
     const bool reads_table = cfg.mode != 1 || cfg.order >= 2;
-    job->stage1_shift = reads_table ? stage1_shift_for(a.g, threads == 768 ? 512 : threads) : 0;
+    job->stage1_shift = reads_table ? stage1_shift_for(a.g, table_threads(cfg)) : 0;
     job->stage1_nwords = reads_table ? (uint32_t)(((uint64_t)a.g.cache_bits >> job->stage1_shift) / 32) : 0;
     {
         // dense mode: regions of the pipelined probes, index functions f0/f1 (order 0) or f2/f3 (order 1,
         // which only K >= 4 filters set)
         if (cfg.mode < 0 || cfg.mode > 3 ||
             (cfg.mode == 1 && (a.g.k < 2 || ((cfg.order & 1) && a.g.k < 4) || cfg.order < 0 || cfg.order > 3)))
-            *err = cudaErrorInvalidValue;
+            return cudaErrorInvalidValue;
         const uint32_t fa = (cfg.order & 1) ? 2u : 0u, fb = fa + 1;
         job->a_mask = fa < a.g.s ? a.g.cache_mask : a.g.ext_mask;
         job->a_add = fa < a.g.s ? 0u : a.g.cache_bits;
@@ -932,6 +1075,7 @@ uint64_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const Fa
     job->counters = a.counters;
     job->tile_first_nl = a.tile_first_nl;
     job->tile_last_nl = a.tile_last_nl;
+    job->n = a.n;
     job->n_tiles = a.ntiles;
     // FFBF_TEXT_L2=normal keeps the default L2 policy for the text's loads (for comparisons)
     static const bool evict_first = [] {
@@ -939,18 +1083,14 @@ uint64_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const Fa
         return !(v && strcmp(v, "normal") == 0);
     }();
     job->text_evict_first = evict_first ? 1u : 0u;
-    if (n_streams > 0) {
-        const uint32_t box_streams = (uint32_t)box_streams_for(threads);
-        cuuint64_t dims[3] = {(cuuint64_t)kRowBytes, (cuuint64_t)rows, (cuuint64_t)n_streams};
-        cuuint64_t strides[2] = {(cuuint64_t)kRowBytes, (cuuint64_t)slen};
-        cuuint32_t box[3] = {(cuuint32_t)kPart, 1u, box_streams};
-        cuuint32_t estr[3] = {1u, 1u, 1u};
-        CUresult cr = encoder()(&job->tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void*)a.text, dims, strides, box, estr,
-                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (cr != CUDA_SUCCESS) *err = cudaErrorInvalidValue;
-    }
-    return fast_tiles * kScanTile;
+    cuuint64_t dims[3] = {(cuuint64_t)kRowBytes, (cuuint64_t)rows, (cuuint64_t)n_streams};
+    cuuint64_t strides[2] = {(cuuint64_t)kRowBytes, (cuuint64_t)slen};
+    cuuint32_t box[3] = {(cuuint32_t)kPart, 1u, (cuuint32_t)box_streams_for(threads)};
+    cuuint32_t estr[3] = {1u, 1u, 1u};
+    const CUresult cr = encoder()(&job->tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void*)a.text, dims, strides, box, estr,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return cr == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 cudaError_t launch_fast_jobs(uint32_t len, const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_jobs,
@@ -966,33 +1106,13 @@ cudaError_t launch_fast_jobs(uint32_t len, const FastConfig& cfg, const FastJob*
     }
 }
 
-cudaError_t scan_tail(const ScanArgs& a, uint64_t covered, cudaStream_t st) {
-    const uint64_t ntiles = (a.n + kScanTile - 1) / kScanTile;
-    const uint64_t first = covered / kScanTile;
-    if (first >= ntiles) return cudaSuccess;
-    ScanArgs t = a;
-    t.tile_begin = first;
-    t.cache_in_smem = a.g.cache_bits <= kSmemCacheMaxBits;
-    const int grid = scan_generic_grid(a.g, t.cache_in_smem, ntiles - first);
-    if (grid <= 0) return cudaErrorInvalidConfiguration;
-    return scan_generic(t, grid, st);
-}
-
-cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& base, int num_sms,
+cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, int num_sms,
                       FastJob* h_job, FastJob* d_job, cudaStream_t st) {
-    const FastConfig cfg = launch_config(base, a.n, num_sms, false);
-    const uint32_t rows = cfg.rows ? cfg.rows : fast_rows(a.n, cfg, num_sms, false);
-    cudaError_t e;
-    const uint64_t covered = fill_fast_job(a, stage1_words, cfg, rows, h_job, &e);
+    cudaError_t e = fill_fast_job(a, stage1_words, cfg, h_job);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_job, h_job, sizeof(FastJob), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return e;
-    if (h_job->n_supertiles) {
-        e = cudaMemcpyAsync(d_job, h_job, sizeof(FastJob), cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) return e;
-        e = launch_fast_jobs(a.g.len, cfg, d_job, 1, h_job->n_supertiles, h_job->stage1_nwords,
-                             a.counters + CNT_ERROR, num_sms, st);  // ctl = {CNT_ERROR, CNT_QUEUE}
-        if (e != cudaSuccess) return e;
-    }
-    return scan_tail(a, covered, st);
+    return launch_fast_jobs(a.g.len, cfg, d_job, 1, h_job->n_supertiles, h_job->stage1_nwords, a.counters + CNT_ERROR,
+                            num_sms, st);  // ctl = {CNT_ERROR, CNT_QUEUE}
 }
 
 // Stage-1 table of T = C >> sh bits for the sparse mode: bit j = OR of the cache bits i with i mod T == j

@@ -14,7 +14,7 @@ struct alignas(64) FastJob {
     uint32_t rows;           // rows per stream (tile size: a supertile is THREADS * rows * 128 bytes)
     uint32_t n_supertiles;   // ceil(n_streams / THREADS)
     uint32_t item_begin;     // first work item of this job; the next job's item_begin ends it
-    uint32_t streams_per_tile_log2;  // log2(16384 / (rows * 128))
+    uint32_t streams_per_tile_log2;  // streams per newline tile (fast_tile_bytes)
     Geom g;
     const uint32_t* main_words;
     uint32_t* ff_words;
@@ -31,7 +31,8 @@ struct alignas(64) FastJob {
     uint32_t* counters;
     long long* tile_first_nl;
     long long* tile_last_nl;
-    uint64_t n_tiles;  // 16 KiB tiles of the text (bounds the newline summary writes)
+    uint64_t n;        // text bytes; those after the last whole stream are scanned with the last work item
+    uint64_t n_tiles;  // tiles of the newline summaries (bounds their writes)
     // 1: the text's TMA loads carry an L2 evict-first policy (every text byte is read once, so its lines
     // should leave L2 before the filter's do); 0: the default policy
     uint32_t text_evict_first;
@@ -42,7 +43,7 @@ struct alignas(64) FastJob {
 
 // How a job is scanned: CTA size, probe mode, rows per stream (0: chosen from the text size), and in the dense mode
 // the probe order. Modes 0, 2 and 3 are the sparse kernel (shared-memory stage 1) at 256/384/512, 192/256/384 and 512
-// threads, the last grown to 768 for large texts (launch_config); mode 1 is the dense one (pipelined L2 probes). Orders:
+// threads, the last from 192 to 640 as each text's size asks (launch_config); mode 1 is the dense one (pipelined L2 probes). Orders:
 // 0: the pipelined probes are index functions f0 = h1 and f1 = h2; 1: f2 = rot16(h1) and f3 = rot16(h2), the better
 // pair when their region is sparser; 2 and 3: f0 and f1 are tested against the stage-1 table first, and f0 (order 2)
 // or f2 (order 3) is then probed for the windows that pass. The order only changes which bits are tested first: a
@@ -66,9 +67,16 @@ ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, doub
 bool fast_scan_supported(const Geom& g, uint64_t n);
 
 int config_threads(const FastConfig& cfg);
+// The CTA size whose shared memory the configuration's stage-1 table is sized for.
+int table_threads(const FastConfig& cfg);
 
-// The configuration a text of n bytes is launched with, alone on the GPU or in a batch (see mode 3 above).
+// The configuration a text of n bytes is launched with, alone on the GPU or in a batch: rows per stream, and in mode 3
+// the CTA size.
 FastConfig launch_config(const FastConfig& cfg, uint64_t n, int num_sms, bool batch);
+// Bytes per tile of the newline summaries of a scan with that many rows per stream: as many streams as reach 16 KiB, a
+// power of two of at most 32. Texts below kShortRowsText may be scanned with less than four rows.
+uint32_t fast_tile_bytes(uint32_t rows);
+constexpr uint64_t kShortRowsText = 64ull << 20;
 
 // Stage-1 table for a CTA size: a copy of the cache region when it fits in the shared memory the kernel
 // leaves over, otherwise its fold to C >> shift bits.
@@ -79,21 +87,18 @@ cudaError_t build_stage1(const uint32_t* main_words, const Geom& g, int threads,
 // CTAs of the tuned kernel resident per SM for a configuration (two for the 192-thread dense kernel).
 int fast_ctas_per_sm(const FastConfig& cfg);
 
-// Rows per stream for a text of n bytes, alone on the GPU or in a batch.
+// Rows per stream for a text of n bytes: a power of two, from 4 to 16, alone on the GPU or in a batch.
 uint32_t fast_rows(uint64_t n, const FastConfig& cfg, int num_sms, bool batch);
 
-// Fills *job (host memory) for the whole 16 KiB tiles of a.text and returns the bytes it covers; the
-// caller sets item_begin. scan_tail runs the generic kernel over the tiles from `covered` on.
-uint64_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, uint32_t rows,
-                       FastJob* job, cudaError_t* err);
-cudaError_t scan_tail(const ScanArgs& a, uint64_t covered, cudaStream_t st);
+// Fills *job (host memory) for a.text, whose a.tile_bytes is fast_tile_bytes(cfg.rows); the caller sets item_begin.
+cudaError_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, FastJob* job);
 
 // One launch of the tuned kernel over n_jobs device-resident jobs sharing LEN and configuration.
 // d_ctl[0] collects error flags; d_ctl[1] is the work-queue counter and must be zero at launch.
 cudaError_t launch_fast_jobs(uint32_t len, const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_jobs,
                              uint32_t n_items, uint32_t max_s1_words, uint32_t* d_ctl, int num_sms, cudaStream_t st);
 
-// A plain scan: one job (h_job pinned host staging, d_job device copy) plus the generic tail.
+// A plain scan: one job (h_job pinned host staging, d_job device copy).
 cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, int num_sms,
                       FastJob* h_job, FastJob* d_job, cudaStream_t st);
 

@@ -108,6 +108,7 @@ extern "C" ffbf_status ffbf_scan_static(const ffbf_params* p, const uint32_t* d_
     a.counters = counters;
     a.tile_first_nl = tiles;
     a.tile_last_nl = tiles + kMaxTiles;
+    a.tile_bytes = ffbf::kScanTile;
     a.ntiles = ntiles;
     a.tile_begin = 0;
     a.cache_in_smem = p->cache_bits <= ffbf::kSmemCacheMaxBits;
@@ -127,7 +128,7 @@ extern "C" ffbf_status ffbf_scan_static(const ffbf_params* p, const uint32_t* d_
     const uint32_t n = found < kMaxHits ? found : kMaxHits;
     if (n) {
         if (ffbf::resolve_lines(d_text, len, p->len, hits, n, tiles, tiles + kMaxTiles, tiles + 2 * kMaxTiles,
-                                tiles + 3 * kMaxTiles, ntiles, lines, st) != cudaSuccess) {
+                                tiles + 3 * kMaxTiles, ffbf::kScanTile, ntiles, lines, st) != cudaSuccess) {
             cudaGetLastError();
             return FFBF_ECUDA;
         }

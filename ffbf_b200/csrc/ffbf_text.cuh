@@ -60,18 +60,20 @@ __device__ __forceinline__ long long first_nl_fwd(const uint8_t* text, long long
 
 // Start of the line that holds offset w: one past the last '\n' before w in that '\n's tile, 0 at the text's start, or -1
 // when the tile of w - 1 holds none before w.
-__device__ __forceinline__ long long line_start_in_tile(const uint8_t* text, uint64_t n, uint64_t w) {
+__device__ __forceinline__ long long line_start_in_tile(const uint8_t* text, uint64_t n, uint64_t w,
+                                                        uint32_t tile_bytes) {
     if (w == 0) return 0;
     const long long p =
-        last_nl_back(text, (long long)n, (long long)((w - 1) / kScanTile * kScanTile), (long long)w - 1);
+        last_nl_back(text, (long long)n, (long long)((w - 1) / tile_bytes * tile_bytes), (long long)w - 1);
     return p >= 0 ? p + 1 : -1;
 }
 
 // End of the line whose bytes before q hold no '\n' back to the window: the first '\n' at or after q in q's tile, n
 // when q is the text's end, or -1 when that tile holds none.
-__device__ __forceinline__ long long line_end_in_tile(const uint8_t* text, uint64_t n, uint64_t q) {
+__device__ __forceinline__ long long line_end_in_tile(const uint8_t* text, uint64_t n, uint64_t q,
+                                                      uint32_t tile_bytes) {
     if (q >= n) return (long long)n;
-    const uint64_t hi = min(n, (q / kScanTile + 1) * (uint64_t)kScanTile);
+    const uint64_t hi = min(n, (q / tile_bytes + 1) * (uint64_t)tile_bytes);
     return first_nl_fwd(text, (long long)n, (long long)q, (long long)hi);
 }
 
