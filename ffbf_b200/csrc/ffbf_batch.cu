@@ -297,7 +297,7 @@ ffbf_status ffbf_batch_prepare(ffbf_batch* b) {
         for (const auto& j : b->jobs) {
             const uint32_t cap = (uint32_t)std::min<uint64_t>(ffbf::kSmallResults, std::max<uint64_t>(512, j.len / 8192));
             b->result_at.push_back({bytes, cap});
-            bytes += 64 + 3 * 8 * (size_t)cap;
+            bytes += ffbf::result_bytes(cap);
         }
         auto block = std::make_shared<PinnedBlock>();
         if (cudaMallocHost(&block->p, bytes + 16 * b->n_ctl) != cudaSuccess) {

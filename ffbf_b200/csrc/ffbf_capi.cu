@@ -79,21 +79,40 @@ ffbf_status ensure_order(ffbf_ctx* c, size_t bytes) {
     return FFBF_OK;
 }
 
-// The pinned buffer of the single-launch results.
-ffbf_status ensure_results(ffbf_ctx* c) {
-    if (c->h_res) return FFBF_OK;
-    if (cudaMallocHost(&c->h_res, ffbf::kResultBytes) != cudaSuccess) {
+// Pinned room for `cap` single-launch results. The first kFirstResults come with the context's counters (pinning
+// memory costs a call up to a millisecond); a larger result gets the full size once.
+constexpr uint32_t kFirstResults = 2048;
+
+ffbf_status ensure_results(ffbf_ctx* c, uint32_t cap) {
+    if (c->res_cap >= cap) return FFBF_OK;
+    uint8_t* p = nullptr;
+    if (cudaMallocHost(&p, ffbf::result_bytes(ffbf::kSmallResults)) != cudaSuccess) {
         cudaGetLastError();
-        c->h_res = nullptr;
         return fail(c, FFBF_ENOMEM_HOST, "pinned result buffer");
     }
+    if (c->h_res_own) cudaFreeHost(c->h_res_own);
+    c->h_res = c->h_res_own = p;
+    c->res_cap = ffbf::kSmallResults;
     return FFBF_OK;
 }
 
 ffbf::ResultHead* result_head(ffbf_ctx* c) { return reinterpret_cast<ffbf::ResultHead*>(c->h_res); }
 
 uint64_t* result_array(ffbf_ctx* c, int i) {
-    return reinterpret_cast<uint64_t*>(c->h_res + 64) + (size_t)i * ffbf::kSmallResults;
+    return reinterpret_cast<uint64_t*>(c->h_res + 64) + (size_t)i * c->res_cap;
+}
+
+// The context's pinned counters, with room for the first results behind them.
+bool alloc_pinned(ffbf_ctx* c) {
+    if (cudaMallocHost(&c->h_counters, 64 + ffbf::result_bytes(kFirstResults)) != cudaSuccess) {
+        cudaGetLastError();
+        c->h_counters = nullptr;
+        return false;
+    }
+    static_assert(ffbf::CNT_WORDS * sizeof(uint32_t) <= 64, "the results follow the counters");
+    c->h_res = reinterpret_cast<uint8_t*>(c->h_counters) + 64;
+    c->res_cap = kFirstResults;
+    return true;
 }
 
 ffbf_status enter(ffbf_ctx* c) {
@@ -417,11 +436,7 @@ ffbf_status ffbf_create(const ffbf_params* p, int device, ffbf_ctx** out) {
     if (dalloc_t(c, &c->d_main, c->filter_bytes / 4) || dalloc_t(c, &c->d_ff, c->filter_bytes / 4) ||
         dalloc_t(c, &c->d_counters, ffbf::CNT_WORDS))
         return bail(FFBF_ENOMEM_DEVICE);
-    if (cudaMallocHost(&c->h_counters, ffbf::CNT_WORDS * sizeof(uint32_t)) != cudaSuccess) {
-        cudaGetLastError();
-        c->h_counters = nullptr;
-        return bail(FFBF_ENOMEM_HOST);
-    }
+    if (!alloc_pinned(c)) return bail(FFBF_ENOMEM_HOST);
     if (cudaMemsetAsync(c->d_main, 0, c->filter_bytes, c->st) != cudaSuccess ||
         cudaMemsetAsync(c->d_ff, 0, c->filter_bytes, c->st) != cudaSuccess ||
         cudaStreamSynchronize(c->st) != cudaSuccess) {
@@ -463,9 +478,7 @@ ffbf_status create_scan_slot(int device, ffbf_ctx** out) {
         ffbf_destroy(c);
         return FFBF_ENOMEM_DEVICE;
     }
-    if (cudaMallocHost(&c->h_counters, ffbf::CNT_WORDS * sizeof(uint32_t)) != cudaSuccess) {
-        cudaGetLastError();
-        c->h_counters = nullptr;
+    if (!alloc_pinned(c)) {
         ffbf_destroy(c);
         return FFBF_ENOMEM_HOST;
     }
@@ -501,7 +514,7 @@ void ffbf_destroy(ffbf_ctx* c) {
     for (auto& kv : c->allocs) cudaFree(kv.first);
     c->allocs.clear();
     if (c->h_counters) cudaFreeHost(c->h_counters);
-    if (c->h_res) cudaFreeHost(c->h_res);
+    if (c->h_res_own) cudaFreeHost(c->h_res_own);
     if (c->h_job) cudaFreeHost(c->h_job);
     if (c->h_jobs) cudaFreeHost(c->h_jobs);
     for (auto ev : c->pipe_events) cudaEventDestroy(ev);
@@ -723,14 +736,16 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
         // the general path below takes the others
         const uint8_t* res = c->ready;
         uint32_t cap = c->ready_cap;
-        if (!res) {
-            TRY(ensure_results(c));
+        for (int attempt = 0; !c->ready && attempt < 2; attempt++) {
             res = c->h_res;
-            cap = ffbf::kSmallResults;
+            cap = c->res_cap;
             CUDA_TRY(c, ffbf::collect_hits(collect_job(make_scan_args(c), c->d_hitlines, c->h_res, cap,
-                                                          ffbf::kCollectAlone),
-                                              c->st));
+                                                       ffbf::kCollectAlone),
+                                           c->st));
             TRY(sync(c));
+            const uint64_t n = result_head(c)->n;
+            if (n <= cap || n > ffbf::kSmallResults || n > c->hits_cap) break;
+            TRY(ensure_results(c, ffbf::kSmallResults));
         }
         const ffbf::ResultHead* head = reinterpret_cast<const ffbf::ResultHead*>(res);
         if (head->done) {
@@ -1079,7 +1094,6 @@ ffbf_status ffbf_prune(ffbf_ctx* c, ffbf_prune_result* out) {
     const uint64_t n = c->npat;
     uint64_t cnt = 0;
     if (n) {
-        TRY(ensure_results(c));
         TRY(ensure_tmp(c, ffbf::prune_blocks(n)));
         uint32_t* counts = reinterpret_cast<uint32_t*>(c->d_tmp);
         // the bit and id buffers are kept between calls: a cudaFree would wait for the whole device
@@ -1097,18 +1111,19 @@ ffbf_status ffbf_prune(ffbf_ctx* c, ffbf_prune_result* out) {
             c->ids_cap = want;
             return FFBF_OK;
         };
-        if (!c->d_ids && ids_room(std::min<uint64_t>(n, ffbf::kSmallIds)) != FFBF_OK) c->err.clear();
+        if (!c->d_ids && ids_room(std::min<uint64_t>(n, ffbf::kSmallResults)) != FFBF_OK) c->err.clear();
+        const uint64_t host_cap = 3ull * c->res_cap;
         CUDA_TRY(c, ffbf::prune_count(c->d_pstart, c->d_pend, c->d_phash, n, c->g, c->d_ff, c->d_pbits, counts, c->st));
         CUDA_TRY(c, ffbf::prune_emit(c->d_pbits, counts, n, c->d_ids, c->ids_cap, result_head(c), result_array(c, 0),
-                                     c->st));
+                                     host_cap, c->st));
         TRY(sync(c));
         cnt = result_head(c)->n;
         if (c->ids_cap < cnt) {
             TRY(ids_room(cnt));
             CUDA_TRY(c, ffbf::prune_emit(c->d_pbits, counts, n, c->d_ids, c->ids_cap, result_head(c),
-                                         result_array(c, 0), c->st));
+                                         result_array(c, 0), host_cap, c->st));
         }
-        if (cnt <= ffbf::kSmallIds) {
+        if (cnt <= host_cap) {
             c->r_ids.assign(result_array(c, 0), result_array(c, 0) + cnt);
         } else {
             c->r_ids.resize(cnt);
@@ -1177,17 +1192,19 @@ ffbf_status verify_pass(ffbf_ctx* c, uint32_t nh, const uint8_t* d_text, uint64_
         TRY(dalloc_t(c, &c->d_mpid, cap));
         c->match_cap = cap;
     }
-    for (int attempt = 0; attempt < 2; attempt++) {
+    for (int attempt = 0; attempt < 3; attempt++) {
         CUDA_TRY(c, ffbf::verify_collect(ffbf::VerifyJob{c->d_hits, nh, c->match_cap, d_text, text_len, c->d_keys,
                                                          c->d_vals, tsize - 1, c->d_pat, c->d_pstart, c->d_pend,
                                                          c->d_moff, c->d_mpid, c->d_counters, result_head(c),
-                                                         result_array(c, 0), result_array(c, 1)},
+                                                         result_array(c, 0), result_array(c, 1), c->res_cap},
                                          c->st));
         CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * 4, c->st));
         TRY(sync(c));
         if (result_head(c)->error) return fail(c, FFBF_ECUDA, "verification table overflow");
         const uint64_t nm = result_head(c)->n;
-        if (nm <= c->match_cap) break;
+        if (nm <= c->match_cap && (nm <= c->res_cap || nm > ffbf::kSmallResults || c->host_order)) break;
+        if (nm <= ffbf::kSmallResults) TRY(ensure_results(c, ffbf::kSmallResults));
+        if (nm <= c->match_cap) continue;
         uint64_t cap = nm + nm / 4 + 1024;
         if (cap > 0xffffffffull) return fail(c, FFBF_EINVAL, "more than 2^32 matches");
         dfree(c, c->d_moff);
@@ -1253,7 +1270,6 @@ ffbf_status ffbf_verify(ffbf_ctx* c, ffbf_matches* out) {
     CUDA_TRY(c, cudaMemsetAsync(c->d_vals, 0xff, tsize * 4, c->st));
     CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * 4, c->st));
     CUDA_TRY(c, ffbf::table_build(c->d_ids, c->nids, c->d_phash, c->d_keys, c->d_vals, tsize - 1, c->d_counters, c->st));
-    TRY(ensure_results(c));
     std::vector<uint64_t> off;
     std::vector<uint32_t> pid;
     if (!c->segmented) {

@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kPruneBlock) k_prune_count(const uint64_t* sta
 // per thread, in place of a scan launch).
 __global__ void __launch_bounds__(kPruneBlock) k_prune_emit(const uint32_t* bits, const uint32_t* counts,
                                                             uint64_t npat, uint64_t* ids, uint64_t ids_cap,
-                                                            ResultHead* head, uint64_t* host_ids) {
+                                                            ResultHead* head, uint64_t* host_ids, uint64_t host_cap) {
     __shared__ uint32_t s_warp[32];
     uint32_t before = 0;
     for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kPruneBlock) before += counts[b];
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kPruneBlock) k_prune_emit(const uint32_t* bits
     const uint64_t at = base + block_sum(keep, s_warp, &total);
     if (keep) {
         if (at < ids_cap) ids[at] = i;
-        if (at < kSmallIds) host_ids[at] = i;
+        if (at < host_cap) host_ids[at] = i;
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) head->n = (unsigned long long)base + total;
 }
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kThreads) k_verify_collect(VerifyJob a) {
                       a.match_cap, a.counters);
     if (!last_cta(a.counters + CNT_QUEUE, gridDim.x, &s_flag)) return;
     const uint32_t nm = __ldcg(a.counters + CNT_MATCHES);
-    const bool small = nm <= kSmallResults && nm <= a.match_cap;
+    const bool small = nm <= kSmallResults && nm <= a.match_cap && nm <= a.out_cap;
     if (small) {
         auto pid = [&](uint64_t key) { return __ldcg(a.m_pid + ((uint32_t)key & (kSmallResults - 1))); };
         sort_records(
@@ -364,9 +364,9 @@ cudaError_t prune_count(const uint64_t* d_start, const uint64_t* d_end, const ui
 }
 
 cudaError_t prune_emit(const uint32_t* d_bits, const uint32_t* d_counts, uint64_t npat, uint64_t* d_ids,
-                       uint64_t ids_cap, ResultHead* head, uint64_t* host_ids, cudaStream_t st) {
+                       uint64_t ids_cap, ResultHead* head, uint64_t* host_ids, uint64_t host_cap, cudaStream_t st) {
     k_prune_emit<<<(unsigned)prune_blocks(npat), kPruneBlock, 0, st>>>(d_bits, d_counts, npat, d_ids, ids_cap, head,
-                                                                     host_ids);
+                                                                     host_ids, host_cap);
     note_launches(1);
     return cudaGetLastError();
 }

@@ -6,14 +6,13 @@
 namespace ffbf {
 
 constexpr uint32_t kSmallResults = 16384;  // hit windows or matches the single-launch paths order
-constexpr uint32_t kSmallIds = 16384;      // pruned ids the prune writes to host memory itself
 
 // Head of a pinned result buffer. `done` is 1 when the arrays behind it hold the whole result; `error` holds a
 // verification's error flags.
 struct ResultHead {
     unsigned long long n, n_lines, error, done;
 };
-constexpr size_t kResultBytes = 64 + 3 * 8 * (size_t)kSmallResults;  // a head and three arrays
+constexpr size_t result_bytes(uint32_t cap) { return 64 + 3 * 8 * (size_t)cap; }  // a head and three arrays
 
 // What the hit collection of one scan reads and writes.
 struct CollectJob {
@@ -46,16 +45,16 @@ uint32_t collect_ctas(const CollectJob& job);
 cudaError_t collect_hits_multi(const CollectJob* d_jobs, const uint2* d_items, uint32_t n_items, cudaStream_t st);
 
 // Feed-forward prune of npat patterns: a bit per pattern in d_bits, counts per kPruneBlock patterns in d_counts, the
-// ascending ids in d_ids (the first ids_cap) and in host_ids (the first kSmallIds), their number in head->n.
+// ascending ids in d_ids (the first ids_cap) and in host_ids (the first host_cap), their number in head->n.
 constexpr uint32_t kPruneBlock = 1024;
 inline uint64_t prune_blocks(uint64_t npat) { return (npat + kPruneBlock - 1) / kPruneBlock; }
 cudaError_t prune_count(const uint64_t* d_start, const uint64_t* d_end, const uint64_t* d_hash, uint64_t npat,
                         const Geom& g, const uint32_t* d_ff, uint32_t* d_bits, uint32_t* d_counts, cudaStream_t st);
 cudaError_t prune_emit(const uint32_t* d_bits, const uint32_t* d_counts, uint64_t npat, uint64_t* d_ids,
-                       uint64_t ids_cap, ResultHead* head, uint64_t* host_ids, cudaStream_t st);
+                       uint64_t ids_cap, ResultHead* head, uint64_t* host_ids, uint64_t host_cap, cudaStream_t st);
 
 // Exact matches of nhits hit records (verify_window), ordered by (offset, pattern id) and written to host memory
-// when there are at most kSmallResults of them; head->n is their number in any case. d_counters must be zero;
+// when there are at most out_cap and kSmallResults of them; head->n is their number in any case. d_counters must be zero;
 // CNT_QUEUE counts finished CTAs.
 struct VerifyJob {
     const HitRec* hits;
@@ -73,6 +72,7 @@ struct VerifyJob {
     ResultHead* head;
     uint64_t* out_off;
     uint64_t* out_pid;
+    uint32_t out_cap;
 };
 cudaError_t verify_collect(const VerifyJob& job, cudaStream_t st);
 

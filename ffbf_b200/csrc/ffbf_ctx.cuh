@@ -125,8 +125,10 @@ struct ffbf_ctx {
     uint32_t match_cap = 0;
     std::vector<uint64_t> r_moff, r_mpid;
 
-    // pinned results of the single-launch paths: a ResultHead, then up to three arrays of kSmallResults words
-    uint8_t* h_res = nullptr;
+    // pinned results of the single-launch paths: a ResultHead, then three arrays of res_cap words, behind h_counters or
+    // in a block of their own
+    uint8_t *h_res = nullptr, *h_res_own = nullptr;
+    uint32_t res_cap = 0;
     // the pending scan's results where a batch has collected them already (head, then three arrays of ready_cap words)
     std::shared_ptr<PinnedBlock> ready_block;
     const uint8_t* ready = nullptr;

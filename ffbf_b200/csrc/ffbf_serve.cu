@@ -762,7 +762,7 @@ ffbf_status ffbf_server_create(int device, uint64_t arena_bytes, uint32_t slots,
         s->slot_host.emplace_back();
         auto& h = s->slot_host.back();
         if (cudaEventCreateWithFlags(&h.done, cudaEventDisableTiming) != cudaSuccess ||
-            cudaMallocHost(&h.res, ffbf::kResultBytes) != cudaSuccess) {
+            cudaMallocHost(&h.res, ffbf::result_bytes(ffbf::kSmallResults)) != cudaSuccess) {
             cudaGetLastError();
             return bail(FFBF_ENOMEM_HOST);
         }
