@@ -83,7 +83,7 @@ ffbf_status build_plan(const std::vector<PlanJob>& jobs, int num_sms, ScanPlan& 
         if (use_fast(c, c->text_len)) {
             TRY(prepare_fast(c));
             // in a batch other jobs fill the GPU, so CTA size and rows per stream follow this job's size alone
-            const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->text_len, num_sms, true);
+            const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, c->text_len, num_sms, true);
             c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
             const ffbf::ScanArgs a = make_scan_args(c);
             plan.args.push_back(a);
@@ -425,7 +425,7 @@ ffbf_status ffbf_batch_autotune(ffbf_batch* b, size_t sample_bytes, uint32_t* n_
     for (size_t i = 0; i < b->jobs.size(); i++) {
         ffbf_ctx* c = b->jobs[i].c;
         TRY(enter(c));
-        if (!use_fast(c, b->jobs[i].len)) continue;
+        if (!tunable(c, b->jobs[i].len)) continue;
         TRY(prepare_fast(c));  // builds the stage-1 table and measures its fill
         const std::vector<uint64_t> key = {c->g.len, c->g.k, c->g.s, c->g.cache_bits, c->g.nbits,
                                            (uint64_t)(c->stage1_fill * 16.0)};
@@ -467,7 +467,7 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
                           int* mode) {
     TRY(enter(c));
     if (!d_text || ((uintptr_t)d_text & 15)) return fail(c, FFBF_EINVAL, "device text must be 16-byte aligned");
-    if (!use_fast(c, sample_len)) return fail(c, FFBF_EINVAL, "the tuned scan does not cover this geometry or size");
+    if (!tunable(c, sample_len)) return fail(c, FFBF_EINVAL, "the tuned scan does not cover this geometry or size");
     // keep the feed-forward filter: the trial scans set bits in it
     uint32_t* saved = nullptr;
     TRY(dalloc_t(c, &saved, c->filter_bytes / 4));
@@ -501,7 +501,7 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
         if (s != FFBF_OK) break;
         double score = ms;
         if (per_sm) {
-            const ffbf::FastConfig run = ffbf::launch_config(cand, sample_len, c->num_sms, false);
+            const ffbf::FastConfig run = ffbf::launch_config(cand, c->g.len, sample_len, c->num_sms, false);
             const int t = ffbf::config_threads(run);
             const uint64_t streams = sample_len / ((uint64_t)run.rows * 128);
             const uint64_t items = (streams + t - 1) / t;

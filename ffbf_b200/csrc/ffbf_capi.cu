@@ -262,10 +262,16 @@ ffbf_status prepare_fast(ffbf_ctx* c) {
     }
     if (c->force_mode >= 0) c->cfg.mode = c->force_mode;
     if (c->cfg.mode == 3) c->cfg.threads = 512;  // launch_config picks the size for each text
-    // the dense mode probes distinct index functions: with K = 1 only the sparse mode applies
+    // the dense mode probes distinct index functions: with K = 1 only the sparse mode applies; with S = 0 no probe
+    // falls in the cache region, and only the dense mode without its table does
     if (c->g.k < 2 && c->cfg.mode == 1) c->cfg.mode = 0;
+    if (c->g.s < 1 && c->cfg.mode != 1) {
+        c->cfg.mode = 1;
+        c->cfg.threads = 192;
+    }
     // the dense mode's probe order is the filter's, unless the environment fixes it (orders 1 and 3 need f2 and f3)
     c->cfg.order = c->force_order >= 0 ? c->force_order : c->probe_order;
+    if (c->g.s < 1 && c->cfg.order >= 2) c->cfg.order = 1;
     if (c->g.k < 4 && c->cfg.order == 1) c->cfg.order = 0;
     if (c->g.k >= 4 && c->cfg.order == 2) c->cfg.order = 3;
     // the table the configured kernel reads (a dense kernel without prefilter reads none)
@@ -300,6 +306,10 @@ ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* r
                             arrays + 2 * (size_t)cap, cap, per_cta};
 }
 
+bool tunable(const ffbf_ctx* c, uint64_t n) {
+    return use_fast(c, n) && ffbf::compiled_len(c->g.len) && c->g.s >= 1;
+}
+
 bool use_fast(const ffbf_ctx* c, uint64_t n) { return ffbf::fast_scan_supported(c->g, n) && !c->force_generic; }
 
 ffbf_status launch_scan(ffbf_ctx* c) {
@@ -309,7 +319,7 @@ ffbf_status launch_scan(ffbf_ctx* c) {
     if (use_fast(c, n)) {
         c->scan_path = 1;
         TRY(prepare_fast(c));
-        const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, n, c->num_sms, false);
+        const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, n, c->num_sms, false);
         c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
         CUDA_TRY(c, ffbf::scan_fast(make_scan_args(c), c->d_stage1, cfg, c->num_sms, c->h_job, c->d_job, c->st));
     } else {
@@ -874,7 +884,7 @@ ffbf_status scan_host_pipelined(ffbf_ctx* c, const uint8_t* text, size_t len) {
     TRY(prepare_fast(c));
     c->scan_path = 1;
     const uint64_t chunk = pipe_chunk(len);
-    ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, chunk, c->num_sms, false);
+    ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, chunk, c->num_sms, false);
     if (len >= ffbf::kShortRowsText && cfg.rows < 4) cfg.rows = 4;
     c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
     ffbf::FastJob job;
@@ -1333,13 +1343,13 @@ ffbf_status ffbf_test_line(ffbf_ctx* c, const uint8_t* line, size_t len, int* hi
 
 ffbf_status ffbf_debug_scan_unpublished(ffbf_ctx* c, const uint8_t* d_text, size_t len, uint32_t spins) {
     TRY(enter(c));
-    if (!use_fast(c, len)) return fail(c, FFBF_EINVAL, "the tuned scan does not cover this geometry or size");
+    if (!tunable(c, len)) return fail(c, FFBF_EINVAL, "the tuned scan does not cover this geometry or size");
     TRY(setup_scan_state(c, d_text, len));
     if (!c->d_gate) TRY(dalloc_t(c, &c->d_gate, 1));
     CUDA_TRY(c, cudaMemsetAsync(c->d_gate, 0, sizeof(uint32_t), c->st));  // never published
     CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * sizeof(uint32_t), c->st));
     TRY(prepare_fast(c));
-    const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, len, c->num_sms, false);
+    const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, len, c->num_sms, false);
     c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
     CUDA_TRY(c, ffbf::fill_fast_job(make_scan_args(c), c->d_stage1, cfg, c->h_job));
     c->h_job->ready = c->d_gate;

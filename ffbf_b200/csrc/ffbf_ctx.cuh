@@ -204,6 +204,7 @@ ffbf::ScanArgs make_scan_args(ffbf_ctx* c);
 // The single-launch collection of a scan's hits into a pinned buffer of a head and three arrays of cap words.
 ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta);
 bool use_fast(const ffbf_ctx* c, uint64_t n);
+bool tunable(const ffbf_ctx* c, uint64_t n);  // the autotuner takes this geometry and text size
 ffbf_status launch_scan(ffbf_ctx* c);  // counters reset + scan of c->d_text on the context's stream
 // Tile summaries a scan of len bytes may need, and those of the context's current scan.
 uint64_t tiles_for(uint64_t len);

@@ -197,29 +197,52 @@ __device__ __forceinline__ bool full_check_from(const Geom& g, const uint32_t* _
     return true;
 }
 
-// The hash of the window of L bytes at `start`, its bytes read from the text's aligned words that hold them and no
+// LEN as the kernels' template parameter: the common lengths are compiled in; kShort stands for any other one up to 32
+// and kLong for 33 to 63, which the kernel then takes as an argument.
+constexpr int kShort = 0, kLong = -1;
+template <int L>
+__device__ __forceinline__ int len_of(uint32_t len) {
+    return L > 0 ? L : (int)len;
+}
+
+// The hash of the window of LEN bytes at `start`, its bytes read from the text's aligned words that hold them and no
 // others. *newline tells whether one of them is '\n'.
 template <int L>
-__device__ __forceinline__ uint64_t text_window_hash(const uint8_t* __restrict__ text, uint64_t start, uint32_t lane_tab,
-                                                     bool* newline) {
-    constexpr int kWords = (L + 3) / 4;
+__device__ __forceinline__ uint64_t text_window_hash(const uint8_t* __restrict__ text, uint64_t start, uint32_t rt_len,
+                                                     uint32_t lane_tab, bool* newline) {
+    const int len = len_of<L>(rt_len);
     const uint32_t* src = reinterpret_cast<const uint32_t*>(text + (start & ~3ull));
     const uint32_t off = (uint32_t)start & 3u;
+    constexpr int kWords = L > 0 ? (L + 3) / 4 : 1;
     uint32_t w[kWords + 1];
+    if constexpr (L > 0) {  // all loads before the first use
 #pragma unroll
-    for (int q = 0; q <= kWords; q++) w[q] = 4u * q < off + L ? __ldg(src + q) : 0u;
+        for (int q = 0; q <= kWords; q++) w[q] = 4u * q < off + L ? __ldg(src + q) : 0u;
+    } else {
+        w[1] = __ldg(src);
+    }
     uint32_t hl = 0, hh = 0, found = 0;
-#pragma unroll
-    for (int q = 0; q < kWords; q++) {
-        const uint32_t v = __funnelshift_r(w[q], w[q + 1], 8 * off);
+    auto word = [&](int q, uint32_t lo, uint32_t hi) {
+        const uint32_t v = __funnelshift_r(lo, hi, 8 * off);
         const uint32_t c = clear_high_bytes(v);
-        found |= nl_bytes(v) & (4 * q + 4 <= L ? 0xffffffffu : 0xffffffffu >> (8 * (4 * q + 4 - L)));
+        found |= nl_bytes(v) & (4 * q + 4 <= len ? 0xffffffffu : 0xffffffffu >> (8 * (4 * q + 4 - len)));
 #pragma unroll
-        for (int j = 0; j < 4 && 4 * q + j < L; j++) {
+        for (int j = 0; j < 4; j++) {
+            if (4 * q + j >= len) continue;
             const uint2 sv = lds64(entry_addr(c, j, lane_tab));
             const uint32_t nl = __funnelshift_l(hh, hl, 1) ^ sv.x, nh = __funnelshift_l(hl, hh, 1) ^ sv.y;
             hl = nl;
             hh = nh;
+        }
+    };
+    if constexpr (L > 0) {
+#pragma unroll
+        for (int q = 0; q < kWords; q++) word(q, w[q], w[q + 1]);
+    } else {
+        for (int q = 0; 4 * q < len; q++) {
+            w[0] = w[1];
+            w[1] = 4u * (q + 1) < off + len ? __ldg(src + q + 1) : 0u;
+            word(q, w[0], w[1]);
         }
     }
     *newline = found != 0;
@@ -239,6 +262,7 @@ __device__ __forceinline__ void record_hit(const FastJob* J, const Geom& g, uint
 template <int L, int PER_LANE>
 __device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int qn, uint64_t warp_pos0, uint64_t stride,
                                          int lane, uint32_t lane_tab) {
+    const int len = len_of<L>(J->g.len);
     // the job's fields are read here rather than passed: the caller's loop keeps only its hot values live
     const Geom g = J->g;
     const uint32_t* __restrict__ main_words = J->main_words;
@@ -251,9 +275,9 @@ __device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int q
         v[t] = bi[t] = 0;
         if (i >= qn) continue;
         const uint32_t e = lds32_volatile(qaddr + 4u * (uint32_t)i);
-        start[t] = warp_pos0 + (e >> 16) * stride + (e & 0xFFFFu) + 1 - L;
+        start[t] = warp_pos0 + (e >> 16) * stride + (e & 0xFFFFu) + 1 - len;
         bool newline;
-        h[t] = text_window_hash<L>(text, start[t], lane_tab, &newline);  // windows with a '\n' are not queued
+        h[t] = text_window_hash<L>(text, start[t], len, lane_tab, &newline);  // windows with a '\n' are not queued
         bi[t] = bit_index<1>(g, h[t], 0);
         v[t] = __ldg(main_words + (bi[t] >> 5));
     }
@@ -291,10 +315,11 @@ __device__ __noinline__ void finish_streams(const FastJob* J, uint64_t z, uint32
     if (covered < n && z / threads == J->n_supertiles - 1) {
         const Geom g = J->g;
         for (uint64_t p = covered + threadIdx.x; p < n; p += threads) {
-            if (p + 1 < L) continue;
+            const int len = len_of<L>(g.len);
+            if (p + 1 < len) continue;
             bool newline;
-            const uint64_t h = text_window_hash<L>(J->text, p + 1 - L, lane_tab, &newline);
-            if (!newline && full_check_from(g, J->main_words, h, 0)) record_hit(J, g, p + 1 - L, h);
+            const uint64_t h = text_window_hash<L>(J->text, p + 1 - len, len, lane_tab, &newline);
+            if (!newline && full_check_from(g, J->main_words, h, 0)) record_hit(J, g, p + 1 - len, h);
         }
         __syncwarp();
         // the last stream's warp adds the newlines of the text's end to the tile it falls in, which may be a new one
@@ -433,6 +458,52 @@ __device__ __forceinline__ uint32_t window_has_newline(uint32_t prev, uint32_t c
     return rhi;
 }
 
+// The same for a length given at run time, up to 32 or, with the mask `prev2` of the block before `prev`, to 63.
+template <bool LONG>
+__device__ __forceinline__ uint32_t window_has_newline(int len, uint32_t prev2, uint32_t prev, uint32_t cur) {
+    uint32_t m0 = cur, m1 = prev, m2 = prev2;
+    int w = 1;  // m0 covers shifts [0, w)
+    for (; 2 * w <= (LONG ? 32 : len); w *= 2) {
+        m0 |= __funnelshift_l(m1, m0, w);
+        m1 |= LONG ? __funnelshift_l(m2, m1, w) : m1 << w;
+        if (LONG) m2 |= m2 << w;
+    }
+    return len > w ? m0 | __funnelshift_l(m1, m0, len - w) : m0;
+}
+
+// The 32 bytes that leave the window as the block `c` enters it: the bytes LEN before c's, of which p holds the 32
+// before c and pp the 32 before those; K = LEN / 4, and shift 32 - 8 * (LEN % 4) bits.
+template <int K>
+__device__ __forceinline__ void leaving_words(const uint32_t (&pp)[8], const uint32_t (&p)[8], const uint32_t (&c)[8],
+                                              uint32_t shift, uint32_t (&out)[8]) {
+    auto word = [&](int i) { return i >= 0 ? c[i & 7] : i >= -8 ? p[(i + 8) & 7] : pp[(i + 16) & 7]; };
+#pragma unroll
+    for (int q = 0; q < 8; q++) out[q] = __funnelshift_rc(word(q - K - 1), word(q - K), shift);
+}
+
+template <int L>
+__device__ __forceinline__ void leaving_block(const uint32_t (&pp)[8], const uint32_t (&p)[8], const uint32_t (&c)[8],
+                                              int len, uint32_t (&out)[8]) {
+    const uint32_t shift = 32u - 8u * ((uint32_t)len & 3u);
+    switch (len >> 2) {
+#define FFBF_LEAVING(K) \
+    case K: leaving_words<K>(pp, p, c, shift, out); break
+        case 0:
+        default:
+            if constexpr (L == kShort) leaving_words<0>(pp, p, c, shift, out);
+            break;
+        FFBF_LEAVING(8);
+        FFBF_LEAVING(L == kShort ? 1 : 9);
+        FFBF_LEAVING(L == kShort ? 2 : 10);
+        FFBF_LEAVING(L == kShort ? 3 : 11);
+        FFBF_LEAVING(L == kShort ? 4 : 12);
+        FFBF_LEAVING(L == kShort ? 5 : 13);
+        FFBF_LEAVING(L == kShort ? 6 : 14);
+        FFBF_LEAVING(L == kShort ? 7 : 15);
+#undef FFBF_LEAVING
+    }
+}
+
 // Newline mask of a block's 32 bytes: bit i set when byte i is '\n' (exact). Each word's zero-byte mask keeps
 // its high bits (0x80 per '\n'); byte-wise dot products with weights 1, 2, 4, 8 (and 16, 32, 64, 128 for the
 // next word) gather two words' eight bits into bits 7..14 without shifts.
@@ -485,7 +556,7 @@ __host__ __device__ constexpr int box_streams_for(int threads) {
 // consumes load k and records in meta[] which job, item and part each stage holds.
 template <int L, int THREADS, int MODE>
 __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fast(const FastJob* __restrict__ jobs, uint32_t n_jobs,
-                                                          uint32_t n_items, uint32_t max_s1_words,
+                                                          uint32_t n_items, uint32_t max_s1_words, uint32_t rt_len,
                                                           uint32_t* __restrict__ ctl) {
     // ctl[0]: error flags; ctl[1]: the work queue, the count of items handed out past the first wave
     uint32_t* const error_flag = ctl;
@@ -531,7 +602,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         uint64_t* tp = reinterpret_cast<uint64_t*>(smem + 2 * kStageBytes);
         for (int i = tid; i < 256 * 16; i += THREADS) {
             const int c = i >> 4;
-            if constexpr (kTwoTables) tp[i] = c < 128 ? c_sbox[c] : rol64(c_sbox[c - 128], L);
+            if constexpr (kTwoTables) tp[i] = c < 128 ? c_sbox[c] : rol64(c_sbox[c - 128], (uint32_t)len_of<L>(rt_len));
             else tp[i] = c_sbox[(c & 0x80) ? 0 : c];
         }
     }
@@ -622,7 +693,9 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     const uint32_t lane_tab = tab + (uint32_t)(lane & 15) * 8u;  // entry c of this lane's copy: + c * 128
     // S-box entry of byte i of the 64-byte span (p, c): as it enters the window, and rotated by LEN as it leaves
     auto sbox_in = [&](const uint32_t (&c)[8], int i) { return lds64(entry_addr(c[i >> 2], i & 3, lane_tab)); };
+    uint32_t leaving[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // with a run-time LEN, the block of leaving bytes
     auto sbox_out = [&](const uint32_t (&p)[8], const uint32_t (&c)[8], int i) {
+        if constexpr (L <= 0) return lds64_at<128 * 128>(entry_addr(leaving[i >> 2], i & 3, lane_tab));
         const uint2 o = lds64_at<kTwoTables ? 128 * 128 : 0>(
             i >= L ? entry_addr(c[(i - L) >> 2], (i - L) & 3, lane_tab)
                    : entry_addr(p[(i - L + 32) >> 2], (i - L + 32) & 3, lane_tab));
@@ -675,6 +748,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
 
     uint32_t hl = 0, hh = 0;
     uint32_t prev[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    uint32_t prev2[8] = {0, 0, 0, 0, 0, 0, 0, 0}, nl_prev2 = 0;  // the block before prev (kLong)
     // newline mask of the previous block (bit 31 forced at the text's start, where nothing precedes offset 0)
     uint32_t nl_prev = 0;
     uint32_t nl_span = 0xffffu;  // first (low half, 0xffff: none) and last '\n' of the stream so far
@@ -727,13 +801,27 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
             hl = 0;
             hh = 0;
             // the hash of the halo's last LEN bytes, from a zero state: nothing leaves the window
-#pragma unroll
-            for (int j = 32 - L; j < 32; j++) {
-                const uint2 sv = sbox_in(prev, j);
+            const int from = 32 - len_of<L>(rt_len);
+            auto enter = [&](const uint32_t (&w)[8], int j) {
+                const uint2 sv = sbox_in(w, j);
                 const uint32_t nl = __funnelshift_l(hh, hl, 1) ^ sv.x, nh = __funnelshift_l(hl, hh, 1) ^ sv.y;
                 hl = nl;
                 hh = nh;
+            };
+            if constexpr (L == kLong) {
+                const uint4 c4 = *reinterpret_cast<const uint4*>(row + ((0 ^ sw) << 4));
+                const uint4 c5 = *reinterpret_cast<const uint4*>(row + ((1 ^ sw) << 4));
+                prev2[0] = c4.x; prev2[1] = c4.y; prev2[2] = c4.z; prev2[3] = c4.w;
+                prev2[4] = c5.x; prev2[5] = c5.y; prev2[6] = c5.z; prev2[7] = c5.w;
+                map_high_bytes(prev2);
+                nl_prev2 = newline_mask32(prev2);
+#pragma unroll
+                for (int j = 0; j < 32; j++)
+                    if (j - 32 >= from) enter(prev2, j);
             }
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+                if (j >= from) enter(prev, j);
             nl_prev = newline_mask32(prev) | (st == 0 && tid == 0 ? 0x80000000u : 0u);  // text start: nothing before offset 0
             nl_span = 0xffffu;
             if (lane == 0) s_wpos[warp] = ((uint64_t)st * THREADS + (uint64_t)warp * 32) * R * kRowBytes;
@@ -755,7 +843,14 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                 const uint32_t nlm = newline_mask32(cur);
                 // valid windows hold no '\n' (processFile resets the hash there); a stream past the job's end,
                 // which reads zero-filled rows, has none
-                const uint32_t valid = active ? ~window_has_newline<L>(nl_prev, nlm) : 0u;
+                uint32_t crossed;
+                if constexpr (L > 0) {
+                    crossed = window_has_newline<L>(nl_prev, nlm);
+                } else {
+                    crossed = window_has_newline<L == kLong>((int)rt_len, nl_prev2, nl_prev, nlm);
+                    leaving_block<L>(prev2, prev, cur, (int)rt_len, leaving);
+                }
+                const uint32_t valid = active ? ~crossed : 0u;
                 uint32_t pass = 0;
 #pragma unroll
                 for (int j = 0; j < 32; j++) {
@@ -802,6 +897,11 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                 if (nlm) {
                     const uint32_t at = pos0 + (uint32_t)(32 * b);
                     nl_span = min(nl_span & 0xffffu, at + (uint32_t)__ffs(nlm) - 1u) | (at + 31u - __clz(nlm)) << 16;
+                }
+                if constexpr (L == kLong) {
+                    nl_prev2 = nl_prev;
+#pragma unroll
+                    for (int q = 0; q < 8; q++) prev2[q] = prev[q];
                 }
                 nl_prev = nlm;
 #pragma unroll
@@ -852,7 +952,7 @@ constexpr size_t fixed_smem(int threads) {
 }
 
 template <int L, int THREADS, int MODE>
-cudaError_t launch_cfg(const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items, uint32_t max_s1_words,
+cudaError_t launch_cfg(uint32_t len, const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items, uint32_t max_s1_words,
                        uint32_t* d_ctl, int num_sms, cudaStream_t st) {
     const size_t smem =
         fixed_smem(THREADS) + (sparse_mode(MODE) || MODE >= 3 ? 4 * (size_t)max_s1_words : 0);
@@ -862,7 +962,7 @@ cudaError_t launch_cfg(const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items,
     const uint32_t slots = (uint32_t)num_sms * (uint32_t)ctas_per_sm(THREADS, MODE);
     const int grid = (int)(n_items < slots ? n_items : slots);
     if (grid == 0) return cudaSuccess;
-    k_scan_fast<L, THREADS, MODE><<<grid, THREADS, smem, st>>>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl);
+    k_scan_fast<L, THREADS, MODE><<<grid, THREADS, smem, st>>>(d_jobs, n_jobs, n_items, max_s1_words, len, d_ctl);
     note_launches(1);
     return cudaGetLastError();
 }
@@ -870,17 +970,21 @@ cudaError_t launch_cfg(const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items,
 // The kernel of a configuration: its CTA size is config_threads(cfg), the size its descriptors' TMA boxes and work
 // items were made for.
 template <int L>
-cudaError_t launch_len(const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items,
+cudaError_t launch_len(uint32_t len, const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items,
                        uint32_t max_s1_words, uint32_t* d_ctl, int num_sms, cudaStream_t st) {
     const int mode = cfg.mode != 1 ? 0 : 1 + cfg.order;  // kernel mode: 0 sparse, 1..4 dense in probe order 0..3
     switch (16 * config_threads(cfg) + mode) {
 #define FFBF_CASE(T, M) \
-    case 16 * T + M: return launch_cfg<L, T, M>(d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st)
+    case 16 * T + M: return launch_cfg<L, T, M>(len, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st)
         FFBF_CASE(192, 0);
         FFBF_CASE(256, 0);
         FFBF_CASE(384, 0);
         FFBF_CASE(512, 0);
-        FFBF_CASE(640, 0);
+        // (with a run-time LEN the loop does not fit 96 registers)
+        case 16 * 640:
+            if constexpr (L > 0)
+                return launch_cfg<L, 640, 0>(len, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+            return cudaErrorInvalidValue;
         FFBF_CASE(192, 1);
         FFBF_CASE(256, 1);
         FFBF_CASE(384, 1);
@@ -898,14 +1002,11 @@ cudaError_t launch_len(const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_
 
 }  // namespace
 
+bool compiled_len(uint32_t len) { return len == 16 || len == 19 || len == 20 || len == 24 || len == 32; }
+
 bool fast_scan_supported(const Geom& g, uint64_t n) {
-    switch (g.len) {
-        case 16: case 19: case 20: case 24: case 32: break;
-        default: return false;
-    }
-    if (g.s < 1) return false;
-    if (n < (uint64_t)kScanTile) return false;
-    return encoder() != nullptr;
+    if (g.s < 1 && g.k < 2) return false;  // neither a cache-region probe nor two pipelined ones
+    return n >= (uint64_t)kScanTile && encoder() != nullptr;
 }
 
 // Largest power-of-two stage-1 table (in bits, <= C) that fits beside the fixed shared-memory layout.
@@ -951,12 +1052,12 @@ ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, doub
     auto both = [&](double f) { return g.s > 1 ? f * f : f; };
     const double pre_fill = 1.0 - std::pow(1.0 - cache_fill, (double)(1u << stage1_shift_for(g, 384)));
     const double pre = 0.48 + 1.45 * both(pre_fill);
-    if (pre < best_cost) {
+    if (g.s > 0 && pre < best_cost) {
         best.order = g.k >= 4 ? 3 : 2;
         best_cost = pre;
     }
     // Sparse: both table bits; a window that passes costs its lane's queue append and its share of a flush.
-    if (g.k < 2 || 0.345 + 7.35 * both(table_fill) <= best_cost) best.mode = 3;
+    if (g.s > 0 && (g.k < 2 || 0.345 + 7.35 * both(table_fill) <= best_cost)) best.mode = 3;
     return best;
 }
 
@@ -976,11 +1077,11 @@ uint32_t fast_tile_bytes(uint32_t rows) {
     return streams * rows * kRowBytes;
 }
 
-FastConfig launch_config(const FastConfig& cfg, uint64_t n, int num_sms, bool batch) {
+FastConfig launch_config(const FastConfig& cfg, uint32_t len, uint64_t n, int num_sms, bool batch) {
     FastConfig best = cfg;
     if (batch) {
         // other jobs fill the GPU: mode 3 runs 640 threads where the job has four such items of its own
-        if (cfg.mode == 3 && n >= 4ull * 4 * kRowBytes * 640) best.threads = 640;
+        if (cfg.mode == 3 && compiled_len(len) && n >= 4ull * 4 * kRowBytes * 640) best.threads = 640;
         best.rows = fast_rows(n, best, num_sms, true);
         return best;
     }
@@ -999,6 +1100,7 @@ FastConfig launch_config(const FastConfig& cfg, uint64_t n, int num_sms, bool ba
     for (int i = 0; i < (cfg.mode == 3 ? 5 : 1); i++) {
         FastConfig c = cfg;
         if (cfg.mode == 3) c.threads = sparse[i].threads;
+        if (c.threads == 640 && !compiled_len(len)) continue;
         const uint64_t threads = config_threads(c), slots = (uint64_t)num_sms * fast_ctas_per_sm(c);
         for (uint32_t rows = 16; rows >= min_rows; rows--) {
             const uint64_t items = (n / (rows * kRowBytes) + threads - 1) / threads;
@@ -1097,13 +1199,15 @@ cudaError_t launch_fast_jobs(uint32_t len, const FastConfig& cfg, const FastJob*
                              uint32_t n_items, uint32_t max_s1_words, uint32_t* d_ctl, int num_sms,
                              cudaStream_t st) {
     switch (len) {
-        case 16: return launch_len<16>(cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-        case 19: return launch_len<19>(cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-        case 20: return launch_len<20>(cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-        case 24: return launch_len<24>(cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-        case 32: return launch_len<32>(cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-        default: return cudaErrorInvalidValue;
+        case 16: return launch_len<16>(len, cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+        case 19: return launch_len<19>(len, cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+        case 20: return launch_len<20>(len, cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+        case 24: return launch_len<24>(len, cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+        case 32: return launch_len<32>(len, cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
     }
+    if (len < 1 || len > 63) return cudaErrorInvalidValue;
+    if (len < 32) return launch_len<kShort>(len, cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+    return launch_len<kLong>(len, cfg, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
 }
 
 cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, int num_sms,

@@ -65,6 +65,8 @@ ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, doub
 
 // True when the tuned kernel handles this geometry and text size; otherwise the generic scan runs.
 bool fast_scan_supported(const Geom& g, uint64_t n);
+// LENs the tuned kernel is compiled for; it takes the others as an argument.
+bool compiled_len(uint32_t len);
 
 int config_threads(const FastConfig& cfg);
 // The CTA size whose shared memory the configuration's stage-1 table is sized for.
@@ -72,7 +74,7 @@ int table_threads(const FastConfig& cfg);
 
 // The configuration a text of n bytes is launched with, alone on the GPU or in a batch: rows per stream, and in mode 3
 // the CTA size.
-FastConfig launch_config(const FastConfig& cfg, uint64_t n, int num_sms, bool batch);
+FastConfig launch_config(const FastConfig& cfg, uint32_t len, uint64_t n, int num_sms, bool batch);
 // Bytes per tile of the newline summaries of a scan with that many rows per stream: as many streams as reach 16 KiB, a
 // power of two of at most 32. Texts below kShortRowsText may be scanned with less than four rows.
 uint32_t fast_tile_bytes(uint32_t rows);
