@@ -1326,17 +1326,25 @@ ffbf_status ffbf_verify(ffbf_ctx* c, ffbf_matches* out) {
 ffbf_status ffbf_test_line(ffbf_ctx* c, const uint8_t* line, size_t len, int* hit) {
     TRY(enter(c));
     if (!hit || (!line && len)) return fail(c, FFBF_EINVAL, "NULL argument");
-    if (c->small_cap < len + 16) {
-        dfree(c, c->d_small);
-        c->small_cap = 0;
-        TRY(dalloc_t(c, &c->d_small, len + 16));
-        c->small_cap = len + 16;
+    // a short line is read by the kernel from the pinned result room, a longer one is copied to the device
+    unsigned long long* found = &result_head(c)->n;
+    const uint8_t* src = c->h_res + 64;
+    *found = 0;
+    if (len <= 3 * 8 * (size_t)c->res_cap) {
+        if (len) memcpy(c->h_res + 64, line, len);
+    } else {
+        if (c->small_cap < len + 16) {
+            dfree(c, c->d_small);
+            c->small_cap = 0;
+            TRY(dalloc_t(c, &c->d_small, len + 16));
+            c->small_cap = len + 16;
+        }
+        CUDA_TRY(c, cudaMemcpyAsync(c->d_small, line, len, cudaMemcpyHostToDevice, c->st));
+        src = c->d_small;
     }
-    if (len) CUDA_TRY(c, cudaMemcpyAsync(c->d_small, line, len, cudaMemcpyHostToDevice, c->st));
-    CUDA_TRY(c, ffbf::test_line(c->d_small, len, c->g, c->d_main, c->d_counters + 3, c->st));
-    uint32_t r = 0;
-    CUDA_TRY(c, cudaMemcpyAsync(&r, c->d_counters + 3, 4, cudaMemcpyDeviceToHost, c->st));
+    CUDA_TRY(c, ffbf::test_line(src, len, c->g, c->d_main, found, c->st));
     TRY(sync(c));
+    const bool r = *found != 0;
     *hit = r ? 1 : 0;
     return FFBF_OK;
 }

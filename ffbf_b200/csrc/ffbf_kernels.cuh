@@ -98,7 +98,9 @@ cudaError_t filter_encode(const uint32_t* d_main, uint32_t nwords, const uint64_
 cudaError_t filter_deltas(const uint32_t* d_idx, uint64_t n, uint32_t* d_out, cudaStream_t st);
 uint64_t decode_blocks(uint64_t nd);
 
-cudaError_t test_line(const uint8_t* d_line, uint64_t n, const Geom& g, const uint32_t* d_main, uint32_t* d_out,
+// Sets *hit (device or pinned host memory, zero before) when a window of the line hits; the line may be pinned host
+// memory.
+cudaError_t test_line(const uint8_t* line, uint64_t n, const Geom& g, const uint32_t* d_main, unsigned long long* hit,
                       cudaStream_t st);
 
 }  // namespace ffbf
