@@ -102,17 +102,52 @@ uint64_t* result_array(ffbf_ctx* c, int i) {
     return reinterpret_cast<uint64_t*>(c->h_res + 64) + (size_t)i * c->res_cap;
 }
 
-// The context's pinned counters, with room for the first results behind them.
-bool alloc_pinned(ffbf_ctx* c) {
-    if (cudaMallocHost(&c->h_counters, 64 + ffbf::result_bytes(kFirstResults)) != cudaSuccess) {
+// A context's small memory in one allocation each: pinning costs a call one to two milliseconds, a device allocation
+// 0.6, whatever its size. Pinned: counters, the job descriptor's staging, the first results. Device (behind
+// `front_bytes` of the caller's): counters, the fill counts, the job descriptor.
+ffbf_status alloc_small(ffbf_ctx* c, size_t front_bytes, uint8_t** front) {
+    static_assert(ffbf::CNT_WORDS * sizeof(uint32_t) <= 256 && sizeof(ffbf::FastJob) <= 512, "sections of the blocks");
+    uint8_t *h = nullptr, *d = nullptr;
+    TRY(dalloc_t(c, &d, front_bytes + 1024));
+    *front = d;
+    c->d_counters = reinterpret_cast<uint32_t*>(d + front_bytes);
+    c->d_popc = reinterpret_cast<unsigned long long*>(d + front_bytes + 256);
+    c->d_job = reinterpret_cast<ffbf::FastJob*>(d + front_bytes + 512);
+    if (cudaMallocHost(&h, 1024 + ffbf::result_bytes(kFirstResults)) != cudaSuccess) {
         cudaGetLastError();
-        c->h_counters = nullptr;
-        return false;
+        return fail(c, FFBF_ENOMEM_HOST, "pinned context block");
     }
-    static_assert(ffbf::CNT_WORDS * sizeof(uint32_t) <= 64, "the results follow the counters");
-    c->h_res = reinterpret_cast<uint8_t*>(c->h_counters) + 64;
+    c->h_counters = reinterpret_cast<uint32_t*>(h);
+    c->h_job = reinterpret_cast<ffbf::FastJob*>(h + 512);
+    c->h_res = h + 1024;
     c->res_cap = kFirstResults;
-    return true;
+    return FFBF_OK;
+}
+
+// Room for cap hit records and their lines, in one allocation.
+ffbf_status alloc_hits(ffbf_ctx* c, uint64_t cap) {
+    dfree(c, c->d_hits);
+    c->d_hitlines = nullptr;
+    c->hits_cap = 0;
+    uint8_t* d = nullptr;
+    TRY(dalloc_t(c, &d, cap * (sizeof(HitRec) + sizeof(HitLine))));
+    c->d_hits = reinterpret_cast<HitRec*>(d);
+    c->d_hitlines = reinterpret_cast<HitLine*>(d + cap * sizeof(HitRec));
+    c->hits_cap = (uint32_t)cap;
+    return FFBF_OK;
+}
+
+// Room for cap verified matches, in one allocation.
+ffbf_status alloc_matches(ffbf_ctx* c, uint64_t cap) {
+    dfree(c, c->d_moff);
+    c->d_mpid = nullptr;
+    c->match_cap = 0;
+    uint8_t* d = nullptr;
+    TRY(dalloc_t(c, &d, cap * 12));
+    c->d_moff = reinterpret_cast<uint64_t*>(d);
+    c->d_mpid = reinterpret_cast<uint32_t*>(d + cap * 8);
+    c->match_cap = (uint32_t)cap;
+    return FFBF_OK;
 }
 
 ffbf_status enter(ffbf_ctx* c) {
@@ -229,15 +264,6 @@ ffbf_status ensure_stage1(ffbf_ctx* c, int threads, bool force) {
 // unless the autotuner or the environment fixed them, the probe mode and the dense mode's probe order (from the
 // fills of the stage-1 table and of the filter's regions).
 ffbf_status prepare_fast(ffbf_ctx* c) {
-    if (!c->d_popc) TRY(dalloc_t(c, &c->d_popc, 3));
-    if (!c->h_job) {
-        if (cudaMallocHost(&c->h_job, sizeof(ffbf::FastJob)) != cudaSuccess) {
-            cudaGetLastError();
-            c->h_job = nullptr;
-            return fail(c, FFBF_ENOMEM_HOST, "pinned job descriptor");
-        }
-    }
-    if (!c->d_job) TRY(dalloc_t(c, &c->d_job, 1));
     if (c->borrowed) return FFBF_OK;  // the filter's owner built the table and chose the configuration
     if (c->stage1_dirty || !c->d_stage1) {
         TRY(ensure_stage1(c, 512, true));  // measured on the 512-thread table
@@ -351,11 +377,7 @@ ffbf_status setup_scan_state(ffbf_ctx* c, const uint8_t* d_text, size_t len) {
         TRY(dalloc_t(c, &c->d_tiles, 4 * ntiles + 2 * ffbf::tile_agg_words(ntiles)));
         c->tiles_cap = ntiles;
     }
-    if (!c->d_hits) {
-        TRY(dalloc_t(c, &c->d_hits, kInitialHitsCap));
-        TRY(dalloc_t(c, &c->d_hitlines, kInitialHitsCap));
-        c->hits_cap = (uint32_t)kInitialHitsCap;
-    }
+    if (!c->d_hits) TRY(alloc_hits(c, kInitialHitsCap));
     c->d_text = d_text;
     c->text_len = len;
     c->tile_bytes = ffbf::kScanTile;
@@ -443,12 +465,12 @@ ffbf_status ffbf_create(const ffbf_params* p, int device, ffbf_ctx** out) {
         }
         c->device_mem = tot;
     }
-    if (dalloc_t(c, &c->d_main, c->filter_bytes / 4) || dalloc_t(c, &c->d_ff, c->filter_bytes / 4) ||
-        dalloc_t(c, &c->d_counters, ffbf::CNT_WORDS))
-        return bail(FFBF_ENOMEM_DEVICE);
-    if (!alloc_pinned(c)) return bail(FFBF_ENOMEM_HOST);
-    if (cudaMemsetAsync(c->d_main, 0, c->filter_bytes, c->st) != cudaSuccess ||
-        cudaMemsetAsync(c->d_ff, 0, c->filter_bytes, c->st) != cudaSuccess ||
+    const size_t room = (c->filter_bytes + 255) / 256 * 256;
+    uint8_t* filters = nullptr;
+    if ((s = alloc_small(c, 2 * room, &filters)) != FFBF_OK) return bail(s);
+    c->d_main = reinterpret_cast<uint32_t*>(filters);
+    c->d_ff = reinterpret_cast<uint32_t*>(filters + room);
+    if (cudaMemsetAsync(filters, 0, 2 * room, c->st) != cudaSuccess ||
         cudaStreamSynchronize(c->st) != cudaSuccess) {
         cudaGetLastError();
         return bail(FFBF_ECUDA);
@@ -484,13 +506,11 @@ ffbf_status create_scan_slot(int device, ffbf_ctx** out) {
         ffbf_destroy(c);
         return FFBF_ECUDA;
     }
-    if (dalloc_t(c, &c->d_counters, ffbf::CNT_WORDS) != FFBF_OK) {
+    uint8_t* none = nullptr;
+    const ffbf_status st = alloc_small(c, 0, &none);
+    if (st != FFBF_OK) {
         ffbf_destroy(c);
-        return FFBF_ENOMEM_DEVICE;
-    }
-    if (!alloc_pinned(c)) {
-        ffbf_destroy(c);
-        return FFBF_ENOMEM_HOST;
+        return st;
     }
     *out = c;
     return FFBF_OK;
@@ -525,7 +545,6 @@ void ffbf_destroy(ffbf_ctx* c) {
     c->allocs.clear();
     if (c->h_counters) cudaFreeHost(c->h_counters);
     if (c->h_res_own) cudaFreeHost(c->h_res_own);
-    if (c->h_job) cudaFreeHost(c->h_job);
     if (c->h_jobs) cudaFreeHost(c->h_jobs);
     for (auto ev : c->pipe_events) cudaEventDestroy(ev);
     if (c->st_copy) {
@@ -566,21 +585,22 @@ ffbf_status ffbf_set_hbm_budget(ffbf_ctx* c, uint64_t bytes) {
     return FFBF_OK;
 }
 
-ffbf_status ffbf_set_patterns(ffbf_ctx* c, const uint8_t* file, size_t len) {
+}  // extern "C"
+
+namespace {
+
+// Copies a pattern file to the device, finds its lines and hashes their prefixes; with set_bits the hash pass also sets
+// the main filter's bits.
+ffbf_status set_patterns(ffbf_ctx* c, const uint8_t* file, size_t len, int set_bits) {
     TRY(enter(c));
     if (!file && len) return fail(c, FFBF_EINVAL, "pattern buffer is NULL");
     c->have_patterns = false;
     c->have_prune = false;
     dfree(c, c->d_pat);
     dfree(c, c->d_pstart);
-    dfree(c, c->d_pend);
-    dfree(c, c->d_phash);
+    c->d_pend = c->d_phash = nullptr;
     c->npat = 0;
-    try {
-        c->h_pat.assign(file, file + len);
-    } catch (...) {
-        return fail(c, FFBF_ENOMEM_HOST, "host copy of %zu pattern bytes failed", len);
-    }
+    c->pat_len = len;
     TRY(dalloc_t(c, &c->d_pat, len + 16));
     if (len) CUDA_TRY(c, cudaMemcpyAsync(c->d_pat, file, len, cudaMemcpyHostToDevice, c->st));
     const uint64_t nb = ffbf::compact_blocks(len);
@@ -591,31 +611,27 @@ ffbf_status ffbf_set_patterns(ffbf_ctx* c, const uint8_t* file, size_t len) {
     TRY(sync(c));
     const int tail = len > 0 && file[len - 1] != '\n';
     const uint64_t npat = m + (tail ? 1 : 0);
-    uint64_t* d_nl = nullptr;
-    TRY(dalloc_t(c, &d_nl, m + 1));
-    ffbf_status s = FFBF_OK;
-    do {
-        if (ffbf::emit_bytes(c->d_pat, len, '\n', d_nl, c->d_tmp, c->st) != cudaSuccess) {
-            s = fail(c, FFBF_ECUDA, "newline compaction failed");
-            break;
-        }
-        if ((s = dalloc_t(c, &c->d_pstart, npat + 1)) || (s = dalloc_t(c, &c->d_pend, npat + 1)) ||
-            (s = dalloc_t(c, &c->d_phash, npat + 1)))
-            break;
-        if (ffbf::lines_from_newlines(d_nl, m, len, tail, c->d_pstart, c->d_pend, c->st) != cudaSuccess ||
-            ffbf::hash_patterns(c->d_pat, c->d_pstart, c->d_pend, npat, c->g, c->d_phash, c->d_main, 0, c->st) !=
-                cudaSuccess) {
-            s = fail(c, FFBF_ECUDA, "pattern hashing failed: %s", cudaGetErrorString(cudaGetLastError()));
-            break;
-        }
-        s = sync(c);
-    } while (0);
-    dfree(c, d_nl);
-    if (s != FFBF_OK) return s;
+    // one allocation for starts, ends and hashes; the newline positions use the hashes' room until those are written
+    TRY(dalloc_t(c, &c->d_pstart, 3 * (npat + 1)));
+    c->d_pend = c->d_pstart + (npat + 1);
+    c->d_phash = c->d_pend + (npat + 1);
+    if (ffbf::emit_bytes(c->d_pat, len, '\n', c->d_phash, c->d_tmp, c->st) != cudaSuccess ||
+        ffbf::lines_from_newlines(c->d_phash, m, len, tail, c->d_pstart, c->d_pend, c->st) != cudaSuccess ||
+        ffbf::hash_patterns(c->d_pat, c->d_pstart, c->d_pend, npat, c->g, c->d_phash, c->d_main, set_bits, c->st) !=
+            cudaSuccess)
+        return fail(c, FFBF_ECUDA, "pattern hashing failed: %s", cudaGetErrorString(cudaGetLastError()));
+    if (set_bits) c->stage1_dirty = true;
+    TRY(sync(c));
     c->npat = npat;
     c->have_patterns = true;
     return FFBF_OK;
 }
+
+}  // namespace
+
+extern "C" {
+
+ffbf_status ffbf_set_patterns(ffbf_ctx* c, const uint8_t* file, size_t len) { return set_patterns(c, file, len, 0); }
 
 ffbf_status ffbf_build(ffbf_ctx* c) {
     NvtxRange nvtx_("ffbf_build");
@@ -627,8 +643,7 @@ ffbf_status ffbf_build(ffbf_ctx* c) {
 }
 
 ffbf_status ffbf_add_patterns(ffbf_ctx* c, const uint8_t* file, size_t len) {
-    TRY(ffbf_set_patterns(c, file, len));
-    return ffbf_build(c);
+    return set_patterns(c, file, len, 1);
 }
 
 ffbf_status ffbf_load_filter(ffbf_ctx* c, const uint8_t* data, size_t len) {
@@ -779,12 +794,7 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
             // idempotent, so the second pass leaves the same filter.
             uint64_t cap = (uint64_t)nh + nh / 4 + 1024;
             if (cap > 0xffffffffull) return fail(c, FFBF_EINVAL, "more than 2^32 hit windows in one scan");
-            dfree(c, c->d_hits);
-            dfree(c, c->d_hitlines);
-            c->hits_cap = 0;
-            TRY(dalloc_t(c, &c->d_hits, cap));
-            TRY(dalloc_t(c, &c->d_hitlines, cap));
-            c->hits_cap = (uint32_t)cap;
+            TRY(alloc_hits(c, cap));
             TRY(launch_scan(c));
             CUDA_TRY(c, cudaMemcpyAsync(c->h_counters, c->d_counters, ffbf::CNT_WORDS * 4, cudaMemcpyDeviceToHost, c->st));
             TRY(sync(c));
@@ -1152,28 +1162,83 @@ ffbf_status ffbf_prune(ffbf_ctx* c, ffbf_prune_result* out) {
     return FFBF_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// The pruned lines' (start, end) pairs and their bytes, line i at bytes[at[i]]. Gathered on the device; where its memory
+// is short, the whole pattern file and line table come back instead.
+ffbf_status fetch_pruned(ffbf_ctx* c, std::vector<uint64_t>& spans, std::vector<uint8_t>& bytes,
+                         std::vector<uint64_t>& at) {
+    const uint64_t cnt = c->r_ids.size();
+    bool gather = ensure_order(c, 16 * cnt) == FFBF_OK;
+    if (gather) {
+        uint64_t* d_spans = reinterpret_cast<uint64_t*>(c->d_order);
+        CUDA_TRY(c, ffbf::gather_spans(c->d_ids, cnt, c->d_pstart, c->d_pend, d_spans, c->st));
+        CUDA_TRY(c, cudaMemcpyAsync(spans.data(), d_spans, 16 * cnt, cudaMemcpyDeviceToHost, c->st));
+        TRY(sync(c));
+    } else {
+        std::vector<uint64_t> start(c->npat), end(c->npat);
+        CUDA_TRY(c, cudaMemcpyAsync(start.data(), c->d_pstart, 8 * c->npat, cudaMemcpyDeviceToHost, c->st));
+        CUDA_TRY(c, cudaMemcpyAsync(end.data(), c->d_pend, 8 * c->npat, cudaMemcpyDeviceToHost, c->st));
+        TRY(sync(c));
+        for (uint64_t i = 0; i < cnt; i++) {
+            spans[2 * i] = start[c->r_ids[i]];
+            spans[2 * i + 1] = end[c->r_ids[i]];
+        }
+    }
+    for (uint64_t i = 0; i < cnt; i++) at[i + 1] = at[i] + spans[2 * i + 1] - spans[2 * i];
+    // spans, places and bytes share the scratch
+    const size_t total = at[cnt];
+    gather = gather && 2 * total < c->pat_len && ensure_order(c, 24 * cnt + total) == FFBF_OK;
+    c->err.clear();
+    if (gather) {
+        uint64_t* d_spans = reinterpret_cast<uint64_t*>(c->d_order);
+        uint64_t* d_at = d_spans + 2 * cnt;
+        uint8_t* d_bytes = reinterpret_cast<uint8_t*>(d_at + cnt);
+        bytes.resize(total);
+        CUDA_TRY(c, cudaMemcpyAsync(d_spans, spans.data(), 16 * cnt, cudaMemcpyHostToDevice, c->st));
+        CUDA_TRY(c, cudaMemcpyAsync(d_at, at.data(), 8 * cnt, cudaMemcpyHostToDevice, c->st));
+        CUDA_TRY(c, ffbf::gather_lines(c->d_pat, d_spans, d_at, cnt, d_bytes, c->st));
+        CUDA_TRY(c, cudaMemcpyAsync(bytes.data(), d_bytes, total, cudaMemcpyDeviceToHost, c->st));
+    } else {
+        bytes.resize(c->pat_len);
+        CUDA_TRY(c, cudaMemcpyAsync(bytes.data(), c->d_pat, c->pat_len, cudaMemcpyDeviceToHost, c->st));
+        for (uint64_t i = 0; i < cnt; i++) at[i] = spans[2 * i];
+    }
+    return sync(c);
+}
+
+}  // namespace
+
+extern "C" {
+
 ffbf_status ffbf_format_pruned(ffbf_ctx* c, size_t chunk, uint8_t** out, size_t* out_len, uint8_t** index,
                                size_t* index_len) {
     if (!c) return FFBF_EINVAL;
     if (!out || !out_len || !index || !index_len) return fail(c, FFBF_EINVAL, "NULL argument");
     if (!c->have_prune) return fail(c, FFBF_ESTATE, "ffbf_format_pruned needs ffbf_prune first");
     if (chunk == 0) return fail(c, FFBF_EINVAL, "chunk must be > 0");
-    const std::vector<uint8_t>& f = c->h_pat;
-    // line spans of the pattern file, walked in step with the ascending ids
+    TRY(enter(c));
     std::vector<uint8_t> o, ix;
-    uint64_t line = 0, pos = 0;
-    char num[32];
-    for (uint64_t id : c->r_ids) {
-        while (line < id) {
-            const void* nl = memchr(f.data() + pos, '\n', f.size() - pos);
-            pos = nl ? (uint64_t)((const uint8_t*)nl - f.data()) + 1 : f.size();
-            line++;
+    try {
+        // the surviving lines' spans and bytes come back from the device copy of the pattern file
+        const uint64_t cnt = c->r_ids.size();
+        std::vector<uint64_t> spans(2 * cnt);
+        std::vector<uint8_t> bytes;
+        std::vector<uint64_t> at(cnt + 1, 0);
+        if (cnt) TRY(fetch_pruned(c, spans, bytes, at));
+        char num[32];
+        for (uint64_t i = 0; i < cnt; i++) {
+            // format_line addresses the line by its place in the file
+            const uint64_t s = spans[2 * i], e = spans[2 * i + 1];
+            const uint8_t* file = reinterpret_cast<const uint8_t*>((uintptr_t)bytes.data() + at[i] - s);
+            format_line(o, file, c->pat_len, s, e, chunk);
+            const int k = snprintf(num, sizeof num, "%llu\n", (unsigned long long)c->r_ids[i]);
+            ix.insert(ix.end(), num, num + k);
         }
-        const void* nl = memchr(f.data() + pos, '\n', f.size() - pos);
-        uint64_t e = nl ? (uint64_t)((const uint8_t*)nl - f.data()) : f.size();
-        format_line(o, f.data(), f.size(), pos, e, chunk);
-        int k = snprintf(num, sizeof num, "%llu\n", (unsigned long long)id);
-        ix.insert(ix.end(), num, num + k);
+    } catch (...) {
+        return fail(c, FFBF_ENOMEM_HOST, "out of host memory for the pruned patterns");
     }
     TRY(to_host_buffer(c, o, out, out_len));
     ffbf_status s = to_host_buffer(c, ix, index, index_len);
@@ -1193,15 +1258,7 @@ namespace {
 // build's error flags, which come back with the first pass.
 ffbf_status verify_pass(ffbf_ctx* c, uint32_t nh, const uint8_t* d_text, uint64_t text_len, uint64_t tsize,
                         uint64_t base, std::vector<uint64_t>& off_out, std::vector<uint32_t>& pid_out) {
-    if (c->match_cap < std::max<uint32_t>(1024, nh)) {
-        dfree(c, c->d_moff);
-        dfree(c, c->d_mpid);
-        c->match_cap = 0;
-        uint32_t cap = std::max<uint32_t>(1024, nh);
-        TRY(dalloc_t(c, &c->d_moff, cap));
-        TRY(dalloc_t(c, &c->d_mpid, cap));
-        c->match_cap = cap;
-    }
+    if (c->match_cap < std::max<uint32_t>(1024, nh)) TRY(alloc_matches(c, std::max<uint32_t>(1024, nh)));
     for (int attempt = 0; attempt < 3; attempt++) {
         CUDA_TRY(c, ffbf::verify_collect(ffbf::VerifyJob{c->d_hits, nh, c->match_cap, d_text, text_len, c->d_keys,
                                                          c->d_vals, tsize - 1, c->d_pat, c->d_pstart, c->d_pend,
@@ -1217,12 +1274,7 @@ ffbf_status verify_pass(ffbf_ctx* c, uint32_t nh, const uint8_t* d_text, uint64_
         if (nm <= c->match_cap) continue;
         uint64_t cap = nm + nm / 4 + 1024;
         if (cap > 0xffffffffull) return fail(c, FFBF_EINVAL, "more than 2^32 matches");
-        dfree(c, c->d_moff);
-        dfree(c, c->d_mpid);
-        c->match_cap = 0;
-        TRY(dalloc_t(c, &c->d_moff, cap));
-        TRY(dalloc_t(c, &c->d_mpid, cap));
-        c->match_cap = (uint32_t)cap;
+        TRY(alloc_matches(c, cap));
     }
     const uint32_t nm = (uint32_t)result_head(c)->n;
     if (result_head(c)->done && !c->host_order) {
@@ -1271,10 +1323,11 @@ ffbf_status ffbf_verify(ffbf_ctx* c, ffbf_matches* out) {
     while (tsize < 2 * c->nids + 2) tsize <<= 1;
     if (c->table_cap < tsize) {
         dfree(c, c->d_keys);
-        dfree(c, c->d_vals);
         c->table_cap = 0;
-        TRY(dalloc_t(c, &c->d_keys, tsize));
-        TRY(dalloc_t(c, &c->d_vals, tsize));
+        uint8_t* d = nullptr;
+        TRY(dalloc_t(c, &d, tsize * 12));
+        c->d_keys = reinterpret_cast<uint64_t*>(d);
+        c->d_vals = reinterpret_cast<uint32_t*>(d + tsize * 8);
         c->table_cap = tsize;
     }
     CUDA_TRY(c, cudaMemsetAsync(c->d_vals, 0xff, tsize * 4, c->st));
@@ -1289,14 +1342,7 @@ ffbf_status ffbf_verify(ffbf_ctx* c, ffbf_matches* out) {
         for (const auto& sg : c->segs) {
             const uint64_t nh = sg.hr_end - sg.hr_begin;
             if (!nh) continue;
-            if (c->hits_cap < nh) {
-                dfree(c, c->d_hits);
-                dfree(c, c->d_hitlines);
-                c->hits_cap = 0;
-                TRY(dalloc_t(c, &c->d_hits, nh));
-                TRY(dalloc_t(c, &c->d_hitlines, nh));
-                c->hits_cap = (uint32_t)nh;
-            }
+            if (c->hits_cap < nh) TRY(alloc_hits(c, nh));
             if (c->text_cap < sg.len + 64) {
                 dfree(c, c->d_text_own);
                 c->text_cap = 0;

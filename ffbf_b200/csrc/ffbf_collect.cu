@@ -297,6 +297,23 @@ __global__ void __launch_bounds__(kPruneBlock) k_prune_emit(const uint32_t* bits
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) head->n = (unsigned long long)base + total;
 }
 
+__global__ void k_gather_spans(const uint64_t* ids, uint64_t n, const uint64_t* start, const uint64_t* end,
+                               uint64_t* spans) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    spans[2 * i] = start[ids[i]];
+    spans[2 * i + 1] = end[ids[i]];
+}
+
+// A warp per line.
+__global__ void k_gather_lines(const uint8_t* file, const uint64_t* spans, const uint64_t* at, uint64_t n,
+                               uint8_t* out) {
+    const uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
+    if (i >= n) return;
+    const uint64_t s = spans[2 * i], len = spans[2 * i + 1] - s;
+    for (uint64_t b = threadIdx.x & 31; b < len; b += 32) out[at[i] + b] = file[s + b];
+}
+
 // k_verify, and the last CTA orders the matches (offset, then pattern id) when shared memory holds them.
 __global__ void __launch_bounds__(kThreads) k_verify_collect(VerifyJob a) {
     extern __shared__ uint64_t s_key[];
@@ -367,6 +384,22 @@ cudaError_t prune_emit(const uint32_t* d_bits, const uint32_t* d_counts, uint64_
                        uint64_t ids_cap, ResultHead* head, uint64_t* host_ids, uint64_t host_cap, cudaStream_t st) {
     k_prune_emit<<<(unsigned)prune_blocks(npat), kPruneBlock, 0, st>>>(d_bits, d_counts, npat, d_ids, ids_cap, head,
                                                                      host_ids, host_cap);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t gather_spans(const uint64_t* d_ids, uint64_t n, const uint64_t* d_start, const uint64_t* d_end,
+                         uint64_t* d_spans, cudaStream_t st) {
+    if (!n) return cudaSuccess;
+    k_gather_spans<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_ids, n, d_start, d_end, d_spans);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t gather_lines(const uint8_t* d_file, const uint64_t* d_spans, const uint64_t* d_at, uint64_t n,
+                         uint8_t* d_out, cudaStream_t st) {
+    if (!n) return cudaSuccess;
+    k_gather_lines<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(d_file, d_spans, d_at, n, d_out);
     note_launches(1);
     return cudaGetLastError();
 }

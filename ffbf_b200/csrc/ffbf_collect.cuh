@@ -53,6 +53,12 @@ cudaError_t prune_count(const uint64_t* d_start, const uint64_t* d_end, const ui
 cudaError_t prune_emit(const uint32_t* d_bits, const uint32_t* d_counts, uint64_t npat, uint64_t* d_ids,
                        uint64_t ids_cap, ResultHead* head, uint64_t* host_ids, uint64_t host_cap, cudaStream_t st);
 
+// (start, end) of the lines `ids`, and their bytes, line i's to out + at[i].
+cudaError_t gather_spans(const uint64_t* d_ids, uint64_t n, const uint64_t* d_start, const uint64_t* d_end,
+                         uint64_t* d_spans, cudaStream_t st);
+cudaError_t gather_lines(const uint8_t* d_file, const uint64_t* d_spans, const uint64_t* d_at, uint64_t n,
+                         uint8_t* d_out, cudaStream_t st);
+
 // Exact matches of nhits hit records (verify_window), ordered by (offset, pattern id) and written to host memory
 // when there are at most out_cap and kSmallResults of them; head->n is their number in any case. d_counters must be zero;
 // CNT_QUEUE counts finished CTAs.

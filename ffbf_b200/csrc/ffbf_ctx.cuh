@@ -52,7 +52,7 @@ struct ffbf_ctx {
 
     // patterns
     bool have_patterns = false;
-    std::vector<uint8_t> h_pat;
+    uint64_t pat_len = 0;  // bytes of the pattern file, whose only copy is on the device
     uint8_t* d_pat = nullptr;
     uint64_t npat = 0;
     uint64_t* d_pstart = nullptr;
