@@ -215,8 +215,7 @@ ffbf_status to_host_buffer(ffbf_ctx* c, const std::vector<uint8_t>& v, uint8_t**
     return FFBF_OK;
 }
 
-void order_hits(const HitRec* hr, const HitLine* hl, uint32_t nh, std::vector<uint64_t>& hits,
-                std::vector<uint64_t>& ls, std::vector<uint64_t>& le) {
+void order_hits(const HitRec* hr, const HitLine* hl, uint32_t nh, Words& hits, Words& ls, Words& le) {
     std::vector<uint32_t> order(nh);
     for (uint32_t i = 0; i < nh; i++) order[i] = i;
     std::sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return hr[a].off < hr[b].off; });
@@ -832,27 +831,23 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
             uint64_t* d_off = reinterpret_cast<uint64_t*>(c->d_order);
             HitLine* d_lu = reinterpret_cast<HitLine*>(c->d_order + off_bytes);
             uint64_t* d_nl = reinterpret_cast<uint64_t*>(c->d_order + off_bytes + line_bytes);
+            uint64_t *d_ls, *d_le;
             CUDA_TRY(c, ffbf::order_hits(c->d_hits, c->d_hitlines, nh, kb, c->d_order + off_bytes + line_bytes + 256,
-                                         scratch, d_off, d_lu, d_nl, c->st));
+                                         scratch, d_off, d_lu, &d_ls, &d_le, d_nl, c->st));
             uint64_t n_lines = 0;
             c->r_hits.resize(nh);
+            CUDA_TRY(c, cudaMemcpyAsync(&n_lines, d_nl, 8, cudaMemcpyDeviceToHost, c->st));
             if (nh)
                 CUDA_TRY(c, cudaMemcpyAsync(c->r_hits.data(), d_off, nh * 8ull, cudaMemcpyDeviceToHost, c->st));
-            CUDA_TRY(c, cudaMemcpyAsync(&n_lines, d_nl, 8, cudaMemcpyDeviceToHost, c->st));
             TRY(sync(c));
             if (n_lines > nh) return fail(c, FFBF_ECUDA, "line reduction returned %llu lines for %u hits",
                                           (unsigned long long)n_lines, nh);
-            std::vector<HitLine> lines(n_lines);
-            if (n_lines) {
-                CUDA_TRY(c, cudaMemcpyAsync(lines.data(), d_lu, n_lines * sizeof(HitLine), cudaMemcpyDeviceToHost,
-                                            c->st));
-                TRY(sync(c));
-            }
             c->r_ls.resize(n_lines);
             c->r_le.resize(n_lines);
-            for (uint64_t i = 0; i < n_lines; i++) {
-                c->r_ls[i] = lines[i].start;
-                c->r_le[i] = lines[i].end;
+            if (n_lines) {
+                CUDA_TRY(c, cudaMemcpyAsync(c->r_ls.data(), d_ls, n_lines * 8, cudaMemcpyDeviceToHost, c->st));
+                CUDA_TRY(c, cudaMemcpyAsync(c->r_le.data(), d_le, n_lines * 8, cudaMemcpyDeviceToHost, c->st));
+                TRY(sync(c));
             }
         }
         c->scan_pending = false;
@@ -1027,7 +1022,7 @@ ffbf_status ffbf_scan(ffbf_ctx* c, const uint8_t* text, size_t len, ffbf_scan_re
     // the feed-forward filter accumulates over them as over successive scans.
     dfree(c, c->d_text_own);
     c->text_cap = 0;
-    std::vector<uint64_t> hits, ls, le;
+    Words hits, ls, le;
     c->keep_records = true;
     for (uint64_t pos = 0; pos < len;) {
         uint64_t end = std::min<uint64_t>(len, pos + seg);

@@ -133,53 +133,6 @@ __device__ void sort_records(uint32_t n, uint64_t span, uint64_t* s_key, uint16_
     __syncthreads();
 }
 
-// The ends of the line of the window at w, searched by eight lanes of a warp: lanes 0-3 go back from the byte before
-// the window, 64 bytes a step, and return the line's start; lanes 4-7 go forward from the byte behind it and return its
-// end. -1 when the tile of that first byte holds no '\n' on that side. One thread per window took 16-byte steps, each a
-// memory latency, and its warp as long as its longest line.
-__device__ __forceinline__ long long line_end_of_window(const CollectJob& a, uint64_t w, bool active) {
-    const bool back = (threadIdx.x & 4) == 0;
-    const long long n = (long long)a.n;
-    const long long pos = back ? (long long)w - 1 : (long long)(w + a.len);
-    const long long tile = pos / a.tile_bytes * a.tile_bytes;
-    const long long stop = back ? tile : min(n, tile + a.tile_bytes);
-    long long res = -1, c = (pos & ~63LL) + 16 * (threadIdx.x & 3);
-    bool busy = active;
-    if (back ? pos < 0 : pos >= n) {  // the text's first and last byte end a line
-        res = back ? 0 : n;
-        busy = false;
-    }
-    while (__any_sync(0xffffffffu, busy)) {
-        long long at = back ? -1 : LLONG_MAX;
-        if (busy && c < n) {
-            const uint4 v = chunk16(a.text, c, n);
-            const uint32_t m8 = __dp4a(nl_bytes(v.y), 0x80402010u, __dp4a(nl_bytes(v.x), 0x08040201u, 0u)) >> 7;
-            const uint32_t m16 = __dp4a(nl_bytes(v.w), 0x80402010u, __dp4a(nl_bytes(v.z), 0x08040201u, 0u)) << 1;
-            uint32_t m = m8 | m16;
-            // bytes on the searched side of pos, and before `stop` going forward
-            if (back) m &= pos - c >= 15 ? 0xffffu : pos < c ? 0u : (2u << (pos - c)) - 1u;
-            else m &= (pos <= c ? 0xffffu : pos - c >= 16 ? 0u : 0xffffu << (pos - c)) &
-                      (stop - c >= 16 ? 0xffffu : stop <= c ? 0u : (1u << (stop - c)) - 1u);
-            if (m) at = c + (back ? 31 - __clz(m) : __ffs(m) - 1);
-        }
-        for (int d = 1; d < 4; d <<= 1) {
-            const long long o = __shfl_xor_sync(0xffffffffu, at, d);
-            at = back ? max(at, o) : min(at, o);
-        }
-        if (busy) {
-            if (back ? at >= 0 : at != LLONG_MAX) {
-                res = back ? at + 1 : at;
-                busy = false;
-            } else {
-                c += back ? -64 : 64;
-                busy = back ? (c & ~63LL) >= stop : (c & ~63LL) < stop;
-            }
-        }
-    }
-    // a last line without '\n' ends with the text
-    return !back && res < 0 && stop == n ? n : res;
-}
-
 __device__ void collect_one(const CollectJob& a, uint32_t cta) {
     extern __shared__ uint64_t s_key[];
     __shared__ uint32_t s_warp[32], s_flag;
@@ -198,7 +151,7 @@ __device__ void collect_one(const CollectJob& a, uint32_t cta) {
     for (uint32_t i0 = cta * a.per_cta; i0 < end; i0 += kThreads / 8) {
         const uint32_t i = i0 + threadIdx.x / 8;
         const uint64_t w = i < end ? a.hits[i].off : 0u;
-        const long long found = line_end_of_window(a, w, i < end);
+        const long long found = line_end_of_window(a.text, a.n, a.len, a.tile_bytes, w, i < end);
         const long long sp = __shfl_sync(0xffffffffu, found, threadIdx.x & 24);
         const long long ep = __shfl_sync(0xffffffffu, found, (threadIdx.x & 24) + 4);
         if (i < end && (threadIdx.x & 7) == 0) {
@@ -314,16 +267,9 @@ __global__ void k_gather_lines(const uint8_t* file, const uint64_t* spans, const
     for (uint64_t b = threadIdx.x & 31; b < len; b += 32) out[at[i] + b] = file[s + b];
 }
 
-// k_verify, and the last CTA orders the matches (offset, then pattern id) when shared memory holds them.
-__global__ void __launch_bounds__(kThreads) k_verify_collect(VerifyJob a) {
+// Orders the matches (offset, then pattern id) of a.counters when shared memory holds them: one CTA.
+__device__ void order_matches_small(const VerifyJob& a, uint32_t* s_warp) {
     extern __shared__ uint64_t s_key[];
-    __shared__ uint32_t s_warp[32];
-    __shared__ uint32_t s_flag;
-    // neighbouring windows go to different CTAs: a few hundred windows then wait on as many SMs' memory pipes
-    for (uint64_t j = blockIdx.x + (uint64_t)gridDim.x * threadIdx.x; j < a.nhits; j += (uint64_t)gridDim.x * kThreads)
-        verify_window(a.hits[j], a.text, a.n, a.keys, a.vals, a.mask, a.pat, a.pstart, a.pend, a.m_off, a.m_pid,
-                      a.match_cap, a.counters);
-    if (!last_cta(a.counters + CNT_QUEUE, gridDim.x, &s_flag)) return;
     const uint32_t nm = __ldcg(a.counters + CNT_MATCHES);
     const bool small = nm <= kSmallResults && nm <= a.match_cap && nm <= a.out_cap;
     if (small) {
@@ -346,6 +292,28 @@ __global__ void __launch_bounds__(kThreads) k_verify_collect(VerifyJob a) {
         a.head->error = a.counters[CNT_ERROR];
         a.head->done = small;
     }
+}
+
+// Matches of a few windows, ordered by the last CTA to finish.
+__global__ void __launch_bounds__(kThreads) k_verify_collect(VerifyJob a) {
+    __shared__ uint32_t s_warp[32], s_flag;
+    // neighbouring windows go to different CTAs: a few hundred windows then wait on as many SMs' memory pipes
+    for (uint64_t j = blockIdx.x + (uint64_t)gridDim.x * threadIdx.x; j < a.nhits; j += (uint64_t)gridDim.x * kThreads)
+        verify_window(a.hits[j], a.text, a.n, a.keys, a.vals, a.mask, a.pat, a.pstart, a.pend, a.m_off, a.m_pid,
+                      a.match_cap, a.counters);
+    if (last_cta(a.counters + CNT_QUEUE, gridDim.x, &s_flag)) order_matches_small(a, s_warp);
+}
+
+__global__ void __launch_bounds__(256) k_verify(VerifyJob a) {
+    const uint64_t j = blockIdx.x * (uint64_t)256 + threadIdx.x;
+    if (j < a.nhits)
+        verify_window(a.hits[j], a.text, a.n, a.keys, a.vals, a.mask, a.pat, a.pstart, a.pend, a.m_off, a.m_pid,
+                      a.match_cap, a.counters);
+}
+
+__global__ void __launch_bounds__(kThreads) k_order_matches(VerifyJob a) {
+    __shared__ uint32_t s_warp[32];
+    order_matches_small(a, s_warp);
 }
 
 constexpr size_t kSmem = (8 + 2 * (kBuckets / kSmallResults)) * (size_t)kSmallResults;  // keys, 16-bit bucket counts
@@ -407,7 +375,17 @@ cudaError_t gather_lines(const uint8_t* d_file, const uint64_t* d_spans, const u
 cudaError_t verify_collect(const VerifyJob& job, cudaStream_t st) {
     cudaError_t e =
         cudaFuncSetAttribute(k_verify_collect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_order_matches, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return e;
+    if (job.nhits > 2 * kSmallResults) {
+        // many windows: as many threads as the SMs hold, which the fused kernel's shared memory would halve (356k
+        // windows: 299 us against 100), then one CTA orders what is few
+        k_verify<<<(job.nhits + 255) / 256, 256, 0, st>>>(job);
+        k_order_matches<<<1, kThreads, kSmem, st>>>(job);
+        note_launches(2);
+        return cudaGetLastError();
+    }
     const uint32_t ctas = job.nhits / 32 + 1;
     k_verify_collect<<<ctas > 148 ? 148 : ctas, kThreads, kSmem, st>>>(job);
     note_launches(1);

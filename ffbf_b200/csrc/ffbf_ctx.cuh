@@ -8,6 +8,7 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -32,6 +33,24 @@ struct PinnedBlock {
         if (p) cudaFreeHost(p);
     }
 };
+
+// An array of words that a copy from the device fills: growing it does not write it first.
+template <class T>
+struct NoInit : std::allocator<T> {
+    template <class U>
+    struct rebind {
+        using other = NoInit<U>;
+    };
+    template <class U>
+    void construct(U* p) noexcept {
+        ::new (static_cast<void*>(p)) U;
+    }
+    template <class U, class... A>
+    void construct(U* p, A&&... a) {
+        ::new (static_cast<void*>(p)) U(std::forward<A>(a)...);
+    }
+};
+using Words = std::vector<uint64_t, NoInit<uint64_t>>;
 
 struct ffbf_ctx {
     ffbf_params prm{};
@@ -108,13 +127,13 @@ struct ffbf_ctx {
     std::vector<Segment> segs;
     std::vector<ffbf::HitRec> seg_hr;
     ffbf::FastJob* d_job = nullptr;
-    std::vector<uint64_t> r_hits, r_ls, r_le;
+    Words r_hits, r_ls, r_le;
 
     // prune
     bool have_prune = false;
     uint64_t* d_ids = nullptr;
     uint64_t nids = 0;
-    std::vector<uint64_t> r_ids;
+    Words r_ids;
 
     // verify
     uint64_t* d_keys = nullptr;
@@ -196,8 +215,7 @@ ffbf_status enter(ffbf_ctx* c);  // clears the last error and makes the context'
 ffbf_status sync(ffbf_ctx* c);   // waits for the context's stream
 void reset_scan(ffbf_ctx* c);    // forgets the last scan's results
 // Hit windows in text order and their lines, each line once (the hits come in any order).
-void order_hits(const HitRec* hr, const HitLine* hl, uint32_t nh, std::vector<uint64_t>& hits,
-                std::vector<uint64_t>& ls, std::vector<uint64_t>& le);
+void order_hits(const HitRec* hr, const HitLine* hl, uint32_t nh, Words& hits, Words& ls, Words& le);
 // Stage-1 table and probe mode of the tuned scan for the context's filter (no-op for borrowed filters).
 ffbf_status prepare_fast(ffbf_ctx* c);
 ffbf::ScanArgs make_scan_args(ffbf_ctx* c);

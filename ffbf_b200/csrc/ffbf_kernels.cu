@@ -510,14 +510,17 @@ __global__ void __launch_bounds__(1024) k_tile_scan2(const long long* first, con
     }
 }
 
-__global__ void k_resolve(const uint8_t* text, uint64_t n, uint32_t len, const HitRec* hits, uint32_t nhits,
-                          const long long* prev_nl, const long long* next_nl, uint32_t tile_bytes, HitLine* out) {
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nhits) return;
-    const uint64_t w = hits[j].off;
+// Eight lanes per hit window.
+__global__ void __launch_bounds__(256) k_resolve(const uint8_t* text, uint64_t n, uint32_t len, const HitRec* hits,
+                                                 uint32_t nhits, const long long* prev_nl, const long long* next_nl,
+                                                 uint32_t tile_bytes, HitLine* out) {
+    const uint64_t j = (blockIdx.x * (uint64_t)256 + threadIdx.x) / 8;
+    const uint64_t w = j < nhits ? hits[j].off : 0u;
+    const long long found = line_end_of_window(text, n, len, tile_bytes, w, j < nhits);
+    long long p = __shfl_sync(0xffffffffu, found, threadIdx.x & 24);
+    long long e = __shfl_sync(0xffffffffu, found, (threadIdx.x & 24) + 4);
+    if (j >= nhits || (threadIdx.x & 7) != 0) return;
     // the line's ends within the tiles of the window's neighbours, else from the tile summaries
-    long long p = line_start_in_tile(text, n, w, tile_bytes);
-    long long e = line_end_in_tile(text, n, w + len, tile_bytes);
     if (p < 0) p = prev_nl[(w - 1) / tile_bytes] + 1;
     if (e < 0) e = next_nl[(w + len) / tile_bytes] == LLONG_MAX ? (long long)n : next_nl[(w + len) / tile_bytes];
     out[j] = HitLine{(uint64_t)p, (uint64_t)e};
@@ -537,7 +540,7 @@ cudaError_t resolve_lines(const uint8_t* text, uint64_t n, uint32_t len, const H
         note_launches(1);
     }
     if (nhits) {
-        k_resolve<<<(nhits + 255) / 256, 256, 0, st>>>(text, n, len, hits, nhits, prev_nl, next_nl, tile_bytes, out);
+        k_resolve<<<(nhits + 31) / 32, 256, 0, st>>>(text, n, len, hits, nhits, prev_nl, next_nl, tile_bytes, out);
         note_launches(1);
     }
     return cudaGetLastError();

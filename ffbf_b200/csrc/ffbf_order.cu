@@ -41,6 +41,15 @@ __global__ void k_sorted_lines(const HitLine* __restrict__ lines, const uint32_t
     }
 }
 
+__global__ void k_split_lines(const HitLine* __restrict__ lines, const uint64_t* __restrict__ n_lines,
+                              uint64_t* __restrict__ ls, uint64_t* __restrict__ le) {
+    const uint64_t n = *n_lines;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        ls[i] = lines[i].start;
+        le[i] = lines[i].end;
+    }
+}
+
 struct HitsLayout {
     size_t keys, vals_in, vals_out, lines, flags, temp, total;
 };
@@ -92,8 +101,9 @@ int key_bits_for(uint64_t n) {
 size_t order_hits_scratch(uint32_t nh, int key_bits) { return hits_layout(nh, key_bits).total; }
 
 cudaError_t order_hits(const HitRec* d_hits, const HitLine* d_lines, uint32_t nh, int key_bits, void* d_scratch,
-                       size_t scratch_bytes, uint64_t* d_off, HitLine* d_lines_out, uint64_t* d_nlines,
-                       cudaStream_t st) {
+                       size_t scratch_bytes, uint64_t* d_off, HitLine* d_lines_tmp, uint64_t** d_ls, uint64_t** d_le,
+                       uint64_t* d_nlines, cudaStream_t st) {
+    *d_ls = *d_le = nullptr;
     if (nh == 0) return cudaMemsetAsync(d_nlines, 0, sizeof(uint64_t), st);
     const HitsLayout L = hits_layout(nh, key_bits);
     if (scratch_bytes < L.total) return cudaErrorInvalidValue;
@@ -113,7 +123,14 @@ cudaError_t order_hits(const HitRec* d_hits, const HitLine* d_lines, uint32_t nh
     k_sorted_lines<<<grid_for(nh), 256, 0, st>>>(d_lines, vals_out, nh, lines, flags);
     note_launches(1);
     temp_bytes = L.total - L.temp;
-    return cub::DeviceSelect::Flagged(s + L.temp, temp_bytes, lines, flags, d_lines_out, d_nlines, (int64_t)nh, st);
+    e = cub::DeviceSelect::Flagged(s + L.temp, temp_bytes, lines, flags, d_lines_tmp, d_nlines, (int64_t)nh, st);
+    if (e != cudaSuccess) return e;
+    // starts and ends as the two arrays the host keeps, in the room of the selection's input
+    *d_ls = reinterpret_cast<uint64_t*>(lines);
+    *d_le = *d_ls + nh;
+    k_split_lines<<<grid_for(nh), 256, 0, st>>>(d_lines_tmp, d_nlines, *d_ls, *d_le);
+    note_launches(1);
+    return cudaGetLastError();
 }
 
 size_t order_matches_scratch(uint32_t nm, int off_bits) { return match_layout(nm, off_bits).total; }

@@ -21,11 +21,11 @@ int key_bits_for(uint64_t n);
 size_t order_hits_scratch(uint32_t nh, int key_bits);
 
 // Sorts the window starts of nh hit records ascending into d_off (nh words), writes the distinct lines of
-// the sorted windows in text order to d_lines_out (at most nh) and their count to *d_nlines. Window
-// starts must be below 2^key_bits.
+// the sorted windows in text order as two arrays inside d_scratch, *d_ls and *d_le (by way of d_lines_tmp, nh
+// entries), and their count to *d_nlines. Window starts must be below 2^key_bits.
 cudaError_t order_hits(const HitRec* d_hits, const HitLine* d_lines, uint32_t nh, int key_bits, void* d_scratch,
-                       size_t scratch_bytes, uint64_t* d_off, HitLine* d_lines_out, uint64_t* d_nlines,
-                       cudaStream_t st);
+                       size_t scratch_bytes, uint64_t* d_off, HitLine* d_lines_tmp, uint64_t** d_ls, uint64_t** d_le,
+                       uint64_t* d_nlines, cudaStream_t st);
 
 // Device scratch bytes order_matches needs for nm matches.
 size_t order_matches_scratch(uint32_t nm, int off_bits);

@@ -53,7 +53,7 @@ struct Request {
     uint32_t nh = 0;  // hit windows, read back with the batch
     double t_submit = 0, t_admit = 0, t_launch = 0, t_done = 0;
     ffbf_status status = FFBF_OK;
-    std::vector<uint64_t> hits, ls, le;
+    Words hits, ls, le;
 };
 
 constexpr uint64_t kArenaAlign = 256;

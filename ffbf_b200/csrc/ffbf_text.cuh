@@ -1,6 +1,8 @@
 // ffbf_text.cuh -- device helpers on text bytes: the search for a window's line ends and the exact byte compare of a
 // hit window with its candidate patterns.
 #pragma once
+#include <climits>
+
 #include "ffbf_kernels.cuh"
 
 namespace ffbf {
@@ -20,61 +22,52 @@ __device__ __forceinline__ uint4 chunk16(const uint8_t* text, long long c, long 
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Last '\n' in [lo, p] (lo <= p < n), or -1: aligned 16-byte chunks from p down to lo.
-__device__ __forceinline__ long long last_nl_back(const uint8_t* text, long long n, long long lo, long long p) {
-    while (p >= lo) {
-        const long long c = p & ~15LL;
-        const uint4 v = chunk16(text, c, n);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        // bytes of the chunk at offsets max(lo - c, 0) .. p - c
-        const int hi = (int)(p - c), low = (int)max(lo - c, 0LL);
-        for (int q = hi >> 2; q >= (low >> 2); q--) {
-            uint32_t m = nl_bytes(w[q]);
-            // keep byte positions 4q + b with low <= 4q + b <= hi
-            const int b_hi = min(hi - 4 * q, 3), b_lo = max(low - 4 * q, 0);
-            m &= (0xFFFFFFFFu >> (8 * (3 - b_hi))) & (0xFFFFFFFFu << (8 * b_lo));
-            if (m) return c + 4 * q + (31 - __clz(m)) / 8;
-        }
-        p = c - 1;
+// The ends of the line of the window at w, searched by eight lanes of a warp: lanes 0-3 go back from the byte before
+// the window, 64 bytes a step, and return the line's start; lanes 4-7 go forward from the byte behind it and return its
+// end. -1 when the tile of that first byte holds no '\n' on that side. One thread per window took 16-byte steps, each a
+// memory latency, and its warp as long as its longest line.
+__device__ __forceinline__ long long line_end_of_window(const uint8_t* text, uint64_t text_len, uint32_t len,
+                                                        uint32_t tile_bytes, uint64_t w, bool active) {
+    const bool back = (threadIdx.x & 4) == 0;
+    const long long n = (long long)text_len;
+    const long long pos = back ? (long long)w - 1 : (long long)(w + len);
+    const long long tile = pos / tile_bytes * tile_bytes;
+    const long long stop = back ? tile : min(n, tile + tile_bytes);
+    long long res = -1, c = (pos & ~63LL) + 16 * (threadIdx.x & 3);
+    bool busy = active;
+    if (back ? pos < 0 : pos >= n) {  // the text's first and last byte end a line
+        res = back ? 0 : n;
+        busy = false;
     }
-    return -1;
-}
-
-// First '\n' in [q, hi) (q < hi <= n), or -1: aligned 16-byte chunks from q up to hi.
-__device__ __forceinline__ long long first_nl_fwd(const uint8_t* text, long long n, long long q, long long hi) {
-    while (q < hi) {
-        const long long c = q & ~15LL;
-        const uint4 v = chunk16(text, c, n);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        const int low = (int)(q - c), top = (int)min(hi - c, 16LL) - 1;  // offsets low .. top
-        for (int k = low >> 2; k <= (top >> 2); k++) {
-            uint32_t m = nl_bytes(w[k]);
-            const int b_lo = max(low - 4 * k, 0), b_hi = min(top - 4 * k, 3);
-            m &= (0xFFFFFFFFu << (8 * b_lo)) & (0xFFFFFFFFu >> (8 * (3 - b_hi)));
-            if (m) return c + 4 * k + (__ffs(m) - 1) / 8;
+    while (__any_sync(0xffffffffu, busy)) {
+        long long at = back ? -1 : LLONG_MAX;
+        if (busy && c < n) {
+            const uint4 v = chunk16(text, c, n);
+            const uint32_t m8 = __dp4a(nl_bytes(v.y), 0x80402010u, __dp4a(nl_bytes(v.x), 0x08040201u, 0u)) >> 7;
+            const uint32_t m16 = __dp4a(nl_bytes(v.w), 0x80402010u, __dp4a(nl_bytes(v.z), 0x08040201u, 0u)) << 1;
+            uint32_t m = m8 | m16;
+            // bytes on the searched side of pos, and before `stop` going forward
+            if (back) m &= pos - c >= 15 ? 0xffffu : pos < c ? 0u : (2u << (pos - c)) - 1u;
+            else m &= (pos <= c ? 0xffffu : pos - c >= 16 ? 0u : 0xffffu << (pos - c)) &
+                      (stop - c >= 16 ? 0xffffu : stop <= c ? 0u : (1u << (stop - c)) - 1u);
+            if (m) at = c + (back ? 31 - __clz(m) : __ffs(m) - 1);
         }
-        q = c + 16;
+        for (int d = 1; d < 4; d <<= 1) {
+            const long long o = __shfl_xor_sync(0xffffffffu, at, d);
+            at = back ? max(at, o) : min(at, o);
+        }
+        if (busy) {
+            if (back ? at >= 0 : at != LLONG_MAX) {
+                res = back ? at + 1 : at;
+                busy = false;
+            } else {
+                c += back ? -64 : 64;
+                busy = back ? (c & ~63LL) >= stop : (c & ~63LL) < stop;
+            }
+        }
     }
-    return -1;
-}
-
-// Start of the line that holds offset w: one past the last '\n' before w in that '\n's tile, 0 at the text's start, or -1
-// when the tile of w - 1 holds none before w.
-__device__ __forceinline__ long long line_start_in_tile(const uint8_t* text, uint64_t n, uint64_t w,
-                                                        uint32_t tile_bytes) {
-    if (w == 0) return 0;
-    const long long p =
-        last_nl_back(text, (long long)n, (long long)((w - 1) / tile_bytes * tile_bytes), (long long)w - 1);
-    return p >= 0 ? p + 1 : -1;
-}
-
-// End of the line whose bytes before q hold no '\n' back to the window: the first '\n' at or after q in q's tile, n
-// when q is the text's end, or -1 when that tile holds none.
-__device__ __forceinline__ long long line_end_in_tile(const uint8_t* text, uint64_t n, uint64_t q,
-                                                      uint32_t tile_bytes) {
-    if (q >= n) return (long long)n;
-    const uint64_t hi = min(n, (q / tile_bytes + 1) * (uint64_t)tile_bytes);
-    return first_nl_fwd(text, (long long)n, (long long)q, (long long)hi);
+    // a last line without '\n' ends with the text
+    return !back && res < 0 && stop == n ? n : res;
 }
 
 // Slot hash of the verification multimap.
