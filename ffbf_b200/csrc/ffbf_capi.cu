@@ -103,16 +103,16 @@ uint64_t* result_array(ffbf_ctx* c, int i) {
 }
 
 // A context's small memory in one allocation each: pinning costs a call one to two milliseconds, a device allocation
-// 0.6, whatever its size. Pinned: counters, the job descriptor's staging, the first results. Device (behind
-// `front_bytes` of the caller's): counters, the fill counts, the job descriptor.
+// 0.6, whatever its size. Pinned: counters, a job descriptor's staging, the first results. Device (behind
+// `front_bytes` of the caller's): counters, the job descriptor, the fill counts.
 ffbf_status alloc_small(ffbf_ctx* c, size_t front_bytes, uint8_t** front) {
     static_assert(ffbf::CNT_WORDS * sizeof(uint32_t) <= 256 && sizeof(ffbf::FastJob) <= 512, "sections of the blocks");
     uint8_t *h = nullptr, *d = nullptr;
     TRY(dalloc_t(c, &d, front_bytes + 1024));
     *front = d;
     c->d_counters = reinterpret_cast<uint32_t*>(d + front_bytes);
-    c->d_popc = reinterpret_cast<unsigned long long*>(d + front_bytes + 256);
-    c->d_job = reinterpret_cast<ffbf::FastJob*>(d + front_bytes + 512);
+    c->d_job = reinterpret_cast<ffbf::FastJob*>(d + front_bytes + ffbf::kJobOffset);
+    c->d_popc = reinterpret_cast<unsigned long long*>(d + front_bytes + 768);
     if (cudaMallocHost(&h, 1024 + ffbf::result_bytes(kFirstResults)) != cudaSuccess) {
         cudaGetLastError();
         return fail(c, FFBF_ENOMEM_HOST, "pinned context block");
@@ -339,15 +339,15 @@ bool use_fast(const ffbf_ctx* c, uint64_t n) { return ffbf::fast_scan_supported(
 
 ffbf_status launch_scan(ffbf_ctx* c) {
     const uint64_t n = c->text_len;
-    CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * sizeof(uint32_t), c->st));
-    if (n == 0) return FFBF_OK;
-    if (use_fast(c, n)) {
+    if (n && use_fast(c, n)) {
         c->scan_path = 1;
         TRY(prepare_fast(c));
         const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, n, c->num_sms, false);
         c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
-        CUDA_TRY(c, ffbf::scan_fast(make_scan_args(c), c->d_stage1, cfg, c->num_sms, c->h_job, c->d_job, c->st));
+        CUDA_TRY(c, ffbf::scan_fast(make_scan_args(c), c->d_stage1, cfg, c->num_sms, c->st));
     } else {
+        CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * sizeof(uint32_t), c->st));
+        if (n == 0) return FFBF_OK;
         c->scan_path = 0;
         c->tile_bytes = ffbf::kScanTile;
         const ffbf::ScanArgs a = make_scan_args(c);

@@ -49,6 +49,10 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_warp, uint
 
 // True in the last of the launch's (or the job's) `ctas` CTAs to get here, which then sees the others' writes.
 __device__ __forceinline__ bool last_cta(uint32_t* ticket, uint32_t ctas, uint32_t* s_flag) {
+    if (ctas == 1) {  // nobody to wait for
+        __syncthreads();
+        return true;
+    }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) *s_flag = atomicAdd(ticket, 1u) == ctas - 1;

@@ -375,7 +375,18 @@ struct JobState {
     const uint32_t *a_words, *b_words;
     uint64_t n_streams;
     uint32_t tables;  // tables loaded so far: the parity of their barrier
+    int started;      // the job whose table was sent for at the kernel's start
 };
+
+// Sends for a job's stage-1 table (thread 0): its words, or 0 where it does not fit or is too small for a bulk copy.
+__device__ __forceinline__ uint32_t start_table(const FastJob* J, uint32_t s1, uint32_t max_s1_words, uint32_t tbar) {
+    const uint32_t nw = J->stage1_nwords;  // a power of two
+    if (nw > max_s1_words || nw < 4) return 0;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // after plain stores to a table
+    mbar_expect_tx(tbar, 4 * nw);
+    bulk_load(s1, J->stage1_words, 4 * nw, tbar);
+    return nw;
+}
 
 // Makes job `job` current: all threads of the CTA call it at the same stage, where every warp is done with the job
 // before. With `s1` its stage-1 table (T = C >> shift bits) is loaded there.
@@ -385,7 +396,7 @@ __device__ __noinline__ void change_job(const FastJob* jobs, int job, JobState* 
     const uint32_t tid = threadIdx.x;
     __syncthreads();
     const bool fits = !s1 || J->stage1_nwords <= max_s1_words;
-    const uint32_t nw = s1 && fits ? J->stage1_nwords : 0u;  // a power of two
+    const uint32_t nw = s1 && fits ? J->stage1_nwords : 0u;
     const uint32_t parity = s->tables & 1u;
     if (tid == 0) {
         const uint32_t bmask = ((J->g.cache_mask >> J->stage1_shift) >> 3) & ~3u;
@@ -400,11 +411,8 @@ __device__ __noinline__ void change_job(const FastJob* jobs, int job, JobState* 
         s->a_words = J->main_words + J->a_add / 32;
         s->b_words = J->main_words + J->b_add / 32;
         s->n_streams = J->n_streams;
-        if (nw >= 4) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // after plain stores to a table
-            mbar_expect_tx(tbar, 4 * nw);
-            bulk_load(s1, J->stage1_words, 4 * nw, tbar);
-        }
+        if (s1 && s->started != job) start_table(J, s1, max_s1_words, tbar);
+        s->started = -1;
     }
     if (nw >= 4) {
         if (!mbar_wait_bounded(tbar, parity)) {
@@ -598,14 +606,6 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     __shared__ uint64_t s_wpos[THREADS / 32];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    {
-        uint64_t* tp = reinterpret_cast<uint64_t*>(smem + 2 * kStageBytes);
-        for (int i = tid; i < 256 * 16; i += THREADS) {
-            const int c = i >> 4;
-            if constexpr (kTwoTables) tp[i] = c < 128 ? c_sbox[c] : rol64(c_sbox[c - 128], (uint32_t)len_of<L>(rt_len));
-            else tp[i] = c_sbox[(c & 0x80) ? 0 : c];
-        }
-    }
     // Load sequencer, run by thread 0: the next load is part nr (-1: halo) of item ni, which belongs to job nj.
     // Load k waits (bounded) until every warp has released load k - 2's stage; with no item left it completes
     // the stage's full barrier without a load and marks the end in meta. Returns false when the wait gave up.
@@ -657,6 +657,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         s_abort = 0;
         s_job.job = -1;
         s_job.tables = 0;
+        s_job.started = -1;
         s_ni = blockIdx.x;
         s_nj = 0;
         s_nr = -1;
@@ -682,11 +683,26 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
             }
         }
         if (open) {
+            // the first job's table travels while the S-box is laid out
+            if constexpr (kTable) {
+                if (s_ni < n_items) {
+                    while (s_nj + 1 < n_jobs && __ldg(&jobs[s_nj + 1].item_begin) <= s_ni) s_nj++;
+                    if (start_table(jobs + s_nj, s1, max_s1_words, tbar)) s_job.started = (int)s_nj;
+                }
+            }
             issue(0);
         } else {
             meta[3] = 0;
             mbar_arrive(fbar(0));
         }
+    }
+    // a thread per byte value, its 16 copies stored in an order that keeps the lanes on different banks
+    for (int c = tid; c < 256; c += THREADS) {
+        uint64_t* tp = reinterpret_cast<uint64_t*>(smem + 2 * kStageBytes) + 16 * c;
+        const uint64_t v = kTwoTables ? (c < 128 ? c_sbox[c] : rol64(c_sbox[c - 128], (uint32_t)len_of<L>(rt_len)))
+                                      : c_sbox[(c & 0x80) ? 0 : c];
+#pragma unroll
+        for (int q = 0; q < 16; q++) tp[(q + lane) & 15] = v;
     }
     __syncthreads();
 
@@ -765,10 +781,11 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
             }
         }
         if (s_abort) {
-            // Give a load still in flight a bounded chance to land before the shared memory goes away.
+            // Give the loads still in flight a bounded chance to land before the shared memory goes away.
             if (tid == 0 && meta[4 * (k & 1) + 3])
                 for (uint32_t j = 0; j < kWaitLimit && !mbar_try_wait(fbar(k), (k >> 1) & 1u); j++) {
                 }
+            if (tid == 0 && s_job.started >= 0) mbar_wait_bounded(tbar, s_job.tables & 1u);
             break;
         }
         // the stage's meta is written before its full barrier completes, so it is read after the wait
@@ -945,7 +962,7 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
 }
 
 // static shared memory of k_scan_fast<., THREADS, .> (sequencer, current job, warp positions)
-constexpr size_t static_smem(int threads) { return 8 * (size_t)(threads / 32) + 160; }
+constexpr size_t static_smem(int threads) { return 8 * (size_t)(threads / 32) + 168; }
 
 constexpr size_t fixed_smem(int threads) {
     return 1024 + 2 * (size_t)threads * kPart + kTabBytes + 128 + (threads / 32) * 4 * (size_t)kQueueCap;
@@ -1211,11 +1228,20 @@ cudaError_t launch_fast_jobs(uint32_t len, const FastConfig& cfg, const FastJob*
 }
 
 cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, int num_sms,
-                      FastJob* h_job, FastJob* d_job, cudaStream_t st) {
-    cudaError_t e = fill_fast_job(a, stage1_words, cfg, h_job);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_job, h_job, sizeof(FastJob), cudaMemcpyHostToDevice, st);
+                      cudaStream_t st) {
+    // the zeroed counters and the descriptor behind them go over in one copy; from pageable memory, so that the next
+    // scan may be enqueued before this one has started
+    struct {
+        uint8_t counters[kJobOffset];
+        FastJob job;
+    } up;
+    memset(up.counters, 0, sizeof up.counters);
+    static_assert(sizeof up == kJobOffset + sizeof(FastJob), "the device block's layout");
+    cudaError_t e = fill_fast_job(a, stage1_words, cfg, &up.job);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(a.counters, &up, sizeof up, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return e;
-    return launch_fast_jobs(a.g.len, cfg, d_job, 1, h_job->n_supertiles, h_job->stage1_nwords, a.counters + CNT_ERROR,
+    const FastJob* d_job = reinterpret_cast<const FastJob*>(reinterpret_cast<uint8_t*>(a.counters) + kJobOffset);
+    return launch_fast_jobs(a.g.len, cfg, d_job, 1, up.job.n_supertiles, up.job.stage1_nwords, a.counters + CNT_ERROR,
                             num_sms, st);  // ctl = {CNT_ERROR, CNT_QUEUE}
 }
 

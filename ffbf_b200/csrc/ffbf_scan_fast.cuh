@@ -100,9 +100,10 @@ cudaError_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const
 cudaError_t launch_fast_jobs(uint32_t len, const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_jobs,
                              uint32_t n_items, uint32_t max_s1_words, uint32_t* d_ctl, int num_sms, cudaStream_t st);
 
-// A plain scan: one job (h_job pinned host staging, d_job device copy).
+// A plain scan: one job, whose descriptor lies kJobOffset bytes behind the counters, which this zeroes.
+constexpr size_t kJobOffset = 256;
 cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, int num_sms,
-                      FastJob* h_job, FastJob* d_job, cudaStream_t st);
+                      cudaStream_t st);
 
 // Number of set bits in n words, written to *d_out (device).
 cudaError_t popcount_words(const uint32_t* w, uint32_t n, unsigned long long* d_out, cudaStream_t st);
