@@ -118,6 +118,7 @@ ffbf_status alloc_small(ffbf_ctx* c, size_t front_bytes, uint8_t** front) {
         return fail(c, FFBF_ENOMEM_HOST, "pinned context block");
     }
     c->h_counters = reinterpret_cast<uint32_t*>(h);
+    memset(h + 512 - ffbf::kJobOffset, 0, ffbf::kJobOffset);  // stays zero: a scan's first counters (scan_fast)
     c->h_job = reinterpret_cast<ffbf::FastJob*>(h + 512);
     c->h_res = h + 1024;
     c->res_cap = kFirstResults;
@@ -344,7 +345,8 @@ ffbf_status launch_scan(ffbf_ctx* c) {
         TRY(prepare_fast(c));
         const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, n, c->num_sms, false);
         c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
-        CUDA_TRY(c, ffbf::scan_fast(make_scan_args(c), c->d_stage1, cfg, c->num_sms, c->st));
+        CUDA_TRY(c, ffbf::scan_fast(make_scan_args(c), c->d_stage1, cfg, c->num_sms,
+                                   reinterpret_cast<uint8_t*>(c->h_job) - ffbf::kJobOffset, c->st));
     } else {
         CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * sizeof(uint32_t), c->st));
         if (n == 0) return FFBF_OK;

@@ -1228,20 +1228,14 @@ cudaError_t launch_fast_jobs(uint32_t len, const FastConfig& cfg, const FastJob*
 }
 
 cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, int num_sms,
-                      cudaStream_t st) {
-    // the zeroed counters and the descriptor behind them go over in one copy; from pageable memory, so that the next
-    // scan may be enqueued before this one has started
-    struct {
-        uint8_t counters[kJobOffset];
-        FastJob job;
-    } up;
-    memset(up.counters, 0, sizeof up.counters);
-    static_assert(sizeof up == kJobOffset + sizeof(FastJob), "the device block's layout");
-    cudaError_t e = fill_fast_job(a, stage1_words, cfg, &up.job);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(a.counters, &up, sizeof up, cudaMemcpyHostToDevice, st);
+                      uint8_t* h_block, cudaStream_t st) {
+    FastJob* h_job = reinterpret_cast<FastJob*>(h_block + kJobOffset);
+    cudaError_t e = fill_fast_job(a, stage1_words, cfg, h_job);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(a.counters, h_block, kJobOffset + sizeof(FastJob), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return e;
     const FastJob* d_job = reinterpret_cast<const FastJob*>(reinterpret_cast<uint8_t*>(a.counters) + kJobOffset);
-    return launch_fast_jobs(a.g.len, cfg, d_job, 1, up.job.n_supertiles, up.job.stage1_nwords, a.counters + CNT_ERROR,
+    return launch_fast_jobs(a.g.len, cfg, d_job, 1, h_job->n_supertiles, h_job->stage1_nwords, a.counters + CNT_ERROR,
                             num_sms, st);  // ctl = {CNT_ERROR, CNT_QUEUE}
 }
 

@@ -100,10 +100,12 @@ cudaError_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const
 cudaError_t launch_fast_jobs(uint32_t len, const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_jobs,
                              uint32_t n_items, uint32_t max_s1_words, uint32_t* d_ctl, int num_sms, cudaStream_t st);
 
-// A plain scan: one job, whose descriptor lies kJobOffset bytes behind the counters, which this zeroes.
+// A plain scan: one job, whose descriptor lies kJobOffset bytes behind the counters. One copy zeroes the counters and
+// brings the descriptor, from pinned h_block (kJobOffset zero bytes, then room for the descriptor), which stays as it
+// is for as long as the copy may run, a replayed stream capture included.
 constexpr size_t kJobOffset = 256;
 cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, int num_sms,
-                      cudaStream_t st);
+                      uint8_t* h_block, cudaStream_t st);
 
 // Number of set bits in n words, written to *d_out (device).
 cudaError_t popcount_words(const uint32_t* w, uint32_t n, unsigned long long* d_out, cudaStream_t st);
