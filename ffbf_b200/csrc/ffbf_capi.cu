@@ -266,7 +266,7 @@ ffbf_status ensure_stage1(ffbf_ctx* c, int threads, bool force) {
 ffbf_status prepare_fast(ffbf_ctx* c) {
     if (c->borrowed) return FFBF_OK;  // the filter's owner built the table and chose the configuration
     if (c->stage1_dirty || !c->d_stage1) {
-        TRY(ensure_stage1(c, 512, true));  // measured on the 512-thread table
+        TRY(ensure_stage1(c, 384, true));  // the table of mode 3 and of the prefiltered dense kernel
         CUDA_TRY(c, ffbf::popcount_words(c->d_stage1, c->stage1_words, c->d_popc, c->st));
         const uint32_t cw = c->g.cache_bits / 32, ew = (uint32_t)(((uint64_t)c->g.ext_mask + 1) / 32);
         CUDA_TRY(c, ffbf::popcount_words(c->d_main, cw, c->d_popc + 1, c->st));

@@ -11,11 +11,12 @@
 // apart. The swizzle XORs a 16-byte chunk's index with bits of its thread's number, so the 16-byte reads of a
 // quarter-warp hit eight different bank groups.
 //
-// Hash. h <- rol64(h,1) ^ S[in] ^ rol64(S[out], LEN) (hash_rot_sbox_pre_2.h:42-51 with the ring folded into
-// the outgoing byte, still in registers), on two 32-bit halves. S sits in shared memory as 16 interleaved
-// copies of 8-byte entries, so the 16 lanes of each half-warp read disjoint banks whatever their bytes, and a byte's
-// entry address is one byte-wise dot product (dp4a) of the text word, off the ALU pipe that the rest of the hash
-// fills. Bytes with the high bit set hash as byte 0 (ffbf.cpp:127-130).
+// Hash. h <- rol64(h,1) ^ S[in] ^ rol64(S[out], LEN) (hash_rot_sbox_pre_2.h:42-51 without its ring of bytes), on two
+// 32-bit halves. S sits in shared memory as 16 interleaved copies of 8-byte entries, so the 16 lanes of each half-warp
+// read disjoint banks whatever their bytes, and a byte's entry address is one byte-wise dot product (dp4a) of the text
+// word, off the ALU pipe that the rest of the hash fills. The sparse kernel keeps the last LEN entries in registers and
+// rotates the one that leaves; the others look the leaving byte, still in registers, up in a second table of rotated
+// entries. Bytes with the high bit set hash as byte 0 (ffbf.cpp:127-130).
 //
 // Probes. Sparse filters test the first two index functions against a shared-memory table: the cache region itself
 // when it fits, else its fold (bit j = OR of the cache bits i with i mod T == j), which only rejects windows the full
@@ -28,12 +29,14 @@
 // newline mask per 32-byte block. Each stream's first and last '\n' feed the newline summaries, per tile of 16
 // KiB or a little more, that the line resolver reads.
 //
-// What bounds it. Sparse: the shared-memory pipe (9 wavefronts per warp and byte: 4 for the two S-box entries, 3.5
-// for the first table probe's random words, the rest for the predicated second probe and the text) and the ALU pipe,
-// at 16 to 20 warps per SM. Dense: the L1TEX unit, which looks up one random sector per clock and SM (words, 1M patterns: 0.93
-// of that). On one B200, before -> now, GB/s of text: 10k patterns, 4 GiB 662 -> 890, 64 MiB 443 -> 618, 8 MiB 69 -> 215; LEN
-// 24, 8k patterns in 2^20 + 2^24 bits, 2 GiB 487 -> 855 and 40k in 2^22 + 2^26 299 -> 647; 150k in 2^23 + 2^27, 256 MiB
-// 295 -> 511; words, 1M patterns 311 -> 354; 4M 16-byte signatures 245 -> 272.
+// What bounds it. Sparse: the ALU pipe (8.5 of the 9.7 clocks that a warp spends on a byte: two rotations, a table
+// address and its bit per probe) and the shared-memory pipe (7.2 wavefronts: 2 for the S-box entry, 3.5 for the first
+// table probe's random words, the rest for the predicated second probe and the text), at 12 to 16 warps per SM. Dense:
+// the L1TEX unit, which looks up one random sector per clock and SM (words, 1M patterns: 0.93 of that). On one B200,
+// before -> now, GB/s of text: 10k patterns, 4 GiB 662 -> 992, 64 MiB 443 -> 736, 8 MiB 69 -> 248; LEN 24, 8k patterns in
+// 2^20 + 2^24 bits, 2 GiB 487 -> 955 and 40k in 2^22 + 2^26 299 -> 637; LEN 19, 50k in 2^24 + 2^28, 256 MiB 350 -> 688; LEN
+// 24, 150k in 2^23 + 2^27, 256 MiB 295 -> 547; LEN 40, 8k in 2^20 + 2^24, 2 GiB 168 -> 805; words, 1M patterns 311 -> 351;
+// 4M 16-byte signatures 245 -> 275.
 //
 // Every mbarrier wait is bounded; on timeout the CTA records an error flag and stops.
 #include <cuda.h>
@@ -54,6 +57,7 @@ namespace {
 
 constexpr int kRowBytes = 128;
 constexpr int kTabBytes = 256 * 16 * 8;  // 16 copies of the 256-entry S-box
+constexpr int kHalfTabBytes = kTabBytes / 2;
 constexpr int kQueueCap = 64;            // candidates per warp queue
 constexpr uint32_t kWaitLimit = 1u << 24;
 constexpr size_t kSmemLimit = 232448;    // opt-in shared memory per block on sm_100
@@ -543,6 +547,14 @@ __device__ __forceinline__ uint32_t newline_mask32(const uint32_t (&w)[8]) {
 // a warp vote and a queue append per byte this took the sparse scan of a 4 GiB text from 662 to 749 GB/s.
 __host__ __device__ constexpr bool sparse_mode(int mode) { return mode == 0; }
 
+// Whether the byte loop keeps the window's LEN S-box entries in registers and rotates the leaving one there, instead of
+// reading it from the rotated table: the sparse mode at the compiled lengths but 32, whose 64 registers spill beside the
+// loop's at 384 threads (92 bytes). Two shifts per byte take the place of 2 of 9.2 shared-memory wavefronts and of a dp4a,
+// and the table's other half makes room for a 2^20-bit stage-1 table beside 512 threads: 1 GiB, 10k patterns, 822 ->
+// 850 GB/s from the registers alone (512 threads, 2^19 bits), 964 with both; 2 GiB in 2^20 + 2^24 bits 789 -> 955.
+__host__ __device__ constexpr bool keeps_entries(int mode, int len) { return sparse_mode(mode) && len > 0 && len != 32; }
+__host__ __device__ constexpr int tab_bytes(int mode, int len) { return keeps_entries(mode, len) ? kHalfTabBytes : kTabBytes; }
+
 // CTAs per SM: dense modes 1 and 2 at 192 threads run two CTAs per SM (12 warps, as one 384-thread CTA, but two
 // independent pipelines); every other configuration runs one.
 __host__ __device__ constexpr int ctas_per_sm(int threads, int mode) {
@@ -577,10 +589,12 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     constexpr bool kPre = MODE == 3 || MODE == 4;  // dense with the shared-memory prefilter and one pipelined probe
     constexpr int kLag = kPre ? kRing : 2 * kRing;  // bytes from a window's first probe to its verdict
     constexpr bool kTable = kSparse || kPre;  // reads the stage-1 table
-    // S-box layout: 16 bank-private copies of S[0..127] and of rol64(S[0..127], LEN), so the byte that leaves the
-    // window needs no rotation; a block's high bytes are cleared beforehand (they hash as byte 0). With LEN = 32
-    // the rotation only swaps the halves, and the table holds all 256 bytes once.
+    // S-box layout: 16 bank-private copies of S[0..127] and, where the leaving byte is looked up, of rol64(S[0..127],
+    // LEN), so that it needs no rotation; a block's high bytes are cleared beforehand (they hash as byte 0). With LEN =
+    // 32 the rotation only swaps the halves, and the table holds all 256 bytes once.
     constexpr bool kTwoTables = L != 32;
+    constexpr bool kEntries = keeps_entries(MODE, L);
+    constexpr int kTab = tab_bytes(MODE, L);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -588,12 +602,12 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     // layout: [stage 0][stage 1][S tables][mbarriers, meta, a word of ones (128 B)][warp queues][stage-1 table]
     const uint32_t stage0 = base;
     const uint32_t tab = base + 2 * kStageBytes;
-    const uint32_t bar0 = tab + kTabBytes;
+    const uint32_t bar0 = tab + kTab;
     // Stage k & 1's "full" barrier completes when load k lands, its "empty" barrier when every warp is done reading
     // it; load k + 2 reuses the stage only after that, and warps otherwise run apart by up to a stage.
     auto fbar = [&](uint32_t k) { return bar0 + 8u * (k & 1u); };
     auto ebar = [&](uint32_t k) { return bar0 + 16u + 8u * (k & 1u); };
-    int* meta = reinterpret_cast<int*>(smem + 2 * kStageBytes + kTabBytes + 32);  // [stage][4]: job, item, part, valid
+    int* meta = reinterpret_cast<int*>(smem + 2 * kStageBytes + kTab + 32);  // [stage][4]: job, item, part, valid
     const uint32_t ones = bar0 + 64u, tbar = bar0 + 72u;  // the table's load completes on tbar
     const uint32_t queues = bar0 + 128u;
     const uint32_t s1 = queues + (THREADS / 32) * 4u * kQueueCap;
@@ -697,7 +711,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         }
     }
     // a thread per byte value, its 16 copies stored in an order that keeps the lanes on different banks
-    for (int c = tid; c < 256; c += THREADS) {
+    for (int c = tid; c < kTab / 128; c += THREADS) {
         uint64_t* tp = reinterpret_cast<uint64_t*>(smem + 2 * kStageBytes) + 16 * c;
         const uint64_t v = kTwoTables ? (c < 128 ? c_sbox[c] : rol64(c_sbox[c - 128], (uint32_t)len_of<L>(rt_len)))
                                       : c_sbox[(c & 0x80) ? 0 : c];
@@ -763,6 +777,9 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     for (int q = 0; q < kR; q++) ring_v[q] = ring_a[q] = ring_b[q] = ring2_v[q] = ring2_b[q] = 0;
 
     uint32_t hl = 0, hh = 0;
+    uint32_t el[kEntries ? L : 1], eh[kEntries ? L : 1];  // the S-box entries of the LEN bytes before the block
+#pragma unroll
+    for (int q = 0; q < (kEntries ? L : 1); q++) el[q] = eh[q] = 0;
     uint32_t prev[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     uint32_t prev2[8] = {0, 0, 0, 0, 0, 0, 0, 0}, nl_prev2 = 0;  // the block before prev (kLong)
     // newline mask of the previous block (bit 31 forced at the text's start, where nothing precedes offset 0)
@@ -824,6 +841,10 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                 const uint32_t nl = __funnelshift_l(hh, hl, 1) ^ sv.x, nh = __funnelshift_l(hl, hh, 1) ^ sv.y;
                 hl = nl;
                 hh = nh;
+                if constexpr (kEntries) {
+                    el[j >= 32 - L ? j - (32 - L) : 0] = sv.x;
+                    eh[j >= 32 - L ? j - (32 - L) : 0] = sv.y;
+                }
             };
             if constexpr (L == kLong) {
                 const uint4 c4 = *reinterpret_cast<const uint4*>(row + ((0 ^ sw) << 4));
@@ -869,9 +890,20 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                 }
                 const uint32_t valid = active ? ~crossed : 0u;
                 uint32_t pass = 0;
+                uint32_t cl[kEntries ? 32 : 1], ch[kEntries ? 32 : 1];  // the block's S-box entries
 #pragma unroll
                 for (int j = 0; j < 32; j++) {
-                    const uint2 sv = sbox_in(cur, j), o = sbox_out(prev, cur, j);
+                    const uint2 sv = sbox_in(cur, j);
+                    uint2 o;
+                    if constexpr (kEntries) {
+                        const uint32_t pl = j < L ? el[j < L ? j : 0] : cl[j < L ? 0 : j - L];
+                        const uint32_t ph = j < L ? eh[j < L ? j : 0] : ch[j < L ? 0 : j - L];
+                        o = make_uint2(__funnelshift_l(ph, pl, L), __funnelshift_l(pl, ph, L));
+                        cl[j] = sv.x;
+                        ch[j] = sv.y;
+                    } else {
+                        o = sbox_out(prev, cur, j);
+                    }
                     const uint32_t nl = __funnelshift_l(hh, hl, 1), nh = __funnelshift_l(hl, hh, 1);
                     hl = nl ^ sv.x ^ o.x;
                     hh = nh ^ sv.y ^ o.y;
@@ -907,6 +939,13 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                         ring_a[slot] = rot_const<kRot>(hl);
                         ring_b[slot] = rot_const<kRot>(hh);
                         ring_v[slot] = ldg_if(a_words + ((ring_a[slot] & a_mask) >> 5), issue);
+                    }
+                }
+                if constexpr (kEntries) {
+#pragma unroll
+                    for (int q = 0; q < L; q++) {
+                        el[q] = cl[32 - L + q];
+                        eh[q] = ch[32 - L + q];
                     }
                 }
                 if constexpr (kSparse) enqueue(pass & valid, pos0 + (uint32_t)(32 * b));
@@ -964,15 +1003,15 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
 // static shared memory of k_scan_fast<., THREADS, .> (sequencer, current job, warp positions)
 constexpr size_t static_smem(int threads) { return 8 * (size_t)(threads / 32) + 168; }
 
-constexpr size_t fixed_smem(int threads) {
-    return 1024 + 2 * (size_t)threads * kPart + kTabBytes + 128 + (threads / 32) * 4 * (size_t)kQueueCap;
+constexpr size_t fixed_smem(int threads, int table_bytes = kTabBytes) {
+    return 1024 + 2 * (size_t)threads * kPart + table_bytes + 128 + (threads / 32) * 4 * (size_t)kQueueCap;
 }
 
 template <int L, int THREADS, int MODE>
 cudaError_t launch_cfg(uint32_t len, const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items, uint32_t max_s1_words,
                        uint32_t* d_ctl, int num_sms, cudaStream_t st) {
     const size_t smem =
-        fixed_smem(THREADS) + (sparse_mode(MODE) || MODE >= 3 ? 4 * (size_t)max_s1_words : 0);
+        fixed_smem(THREADS, tab_bytes(MODE, L)) + (sparse_mode(MODE) || MODE >= 3 ? 4 * (size_t)max_s1_words : 0);
     cudaError_t e =
         cudaFuncSetAttribute(k_scan_fast<L, THREADS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -997,11 +1036,6 @@ cudaError_t launch_len(uint32_t len, const FastConfig& cfg, const FastJob* d_job
         FFBF_CASE(256, 0);
         FFBF_CASE(384, 0);
         FFBF_CASE(512, 0);
-        // (with a run-time LEN the loop does not fit 96 registers)
-        case 16 * 640:
-            if constexpr (L > 0)
-                return launch_cfg<L, 640, 0>(len, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
-            return cudaErrorInvalidValue;
         FFBF_CASE(192, 1);
         FFBF_CASE(256, 1);
         FFBF_CASE(384, 1);
@@ -1033,12 +1067,12 @@ uint32_t stage1_shift_for(const Geom& g, int threads) {
     while (((uint64_t)g.cache_bits >> sh) / 8 > room) sh++;
     return sh;
 }
-// the 512-thread kernel's table also fits the 640-thread one, which large texts use (launch_config)
-static_assert(kSmemLimit - fixed_smem(512) - static_smem(512) - 64 < 131072, "512 threads: a 2^19-bit table");
-static_assert(kSmemLimit - fixed_smem(640) - static_smem(640) - 64 >= 65536, "640 threads: a 2^19-bit table");
+// mode 3's table fits beside its largest CTAs (launch_config)
+static_assert(kSmemLimit - fixed_smem(384) - static_smem(384) - 64 >= 131072, "384 threads: a 2^20-bit table");
+static_assert(kSmemLimit - fixed_smem(512, kHalfTabBytes) - static_smem(512) - 64 >= 131072, "512: a 2^20-bit table");
 
-// mode 3 reads the 512-thread table at every CTA size it takes
-int table_threads(const FastConfig& cfg) { return cfg.mode == 3 ? 512 : config_threads(cfg); }
+// mode 3 reads the 384-thread table at every CTA size it takes
+int table_threads(const FastConfig& cfg) { return cfg.mode == 3 ? 384 : config_threads(cfg); }
 
 uint32_t stage1_words_for(const Geom& g, int threads) {
     return (uint32_t)(((uint64_t)g.cache_bits >> stage1_shift_for(g, threads)) / 32);
@@ -1047,8 +1081,9 @@ uint32_t stage1_words_for(const Geom& g, int threads) {
 ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, double ext_fill) {
     // Costs per window in units of one L2 probe per window (3.1 ps on the whole GPU: 148 SMs, each looking up one
     // random sector per clock). Measured against the model: words, 1M patterns, order 1: 354 GB/s; 150k printable
-    // patterns in 2^23 + 2^27 bits, order 3: 511 GB/s (order 1: 323); 40k in 2^22 + 2^26, mode 3: 622, order 3: 630;
-    // 8k in 2^20 + 2^24, mode 3: 879, order 3: 638.
+    // patterns in 2^23 + 2^27 bits, order 3: 547 GB/s (order 1: 323, mode 3: 309); 40k in 2^22 + 2^26, mode 3: 625,
+    // order 3: 637; 50k in 2^24 + 2^28 (LEN 19), mode 3: 688, order 3: 601; 8k in 2^20 + 2^24, mode 3: 955, order 3:
+    // 653.
     // Orders 0 and 1: the first probe always, the second when the first passes, and a queued window's full test
     // (about three probes' worth of issue and flush work) when both pass. A probe of a region that the L1 left
     // beside the shared memory can largely hold (about 64 KiB) mostly hits there.
@@ -1073,8 +1108,11 @@ ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, doub
         best.order = g.k >= 4 ? 3 : 2;
         best_cost = pre;
     }
-    // Sparse: both table bits; a window that passes costs its lane's queue append and its share of a flush.
-    if (g.s > 0 && (g.k < 2 || 0.345 + 7.35 * both(table_fill) <= best_cost)) best.mode = 3;
+    // Sparse: both table bits; a window that passes costs its lane's queue append and its share of a flush, much more
+    // of it where its exact first probe passes too (cache_fill / table_fill of them) and others follow.
+    const double base = compiled_len(g.len) && keeps_entries(0, (int)g.len) ? 0.325 : 0.38;
+    if (g.s > 0 && (g.k < 2 || base + both(table_fill) * (13.0 + 70.0 * cache_fill / std::max(table_fill, 1e-9)) <= best_cost))
+        best.mode = 3;
     return best;
 }
 
@@ -1082,7 +1120,7 @@ int config_threads(const FastConfig& cfg) {
     if (cfg.mode == 1) return cfg.threads == 256 ? 256 : cfg.threads == 192 && cfg.order < 2 ? 192 : 384;
     if (cfg.mode == 2) return cfg.threads == 192 || cfg.threads == 384 ? cfg.threads : 256;
     if (cfg.mode == 3)  // launch_config fits the size to the text
-        return cfg.threads == 192 || cfg.threads == 256 || cfg.threads == 384 || cfg.threads == 640 ? cfg.threads : 512;
+        return cfg.threads == 192 || cfg.threads == 256 || cfg.threads == 384 ? cfg.threads : 512;
     return cfg.threads == 384 || cfg.threads == 512 ? cfg.threads : 256;
 }
 
@@ -1095,33 +1133,38 @@ uint32_t fast_tile_bytes(uint32_t rows) {
 }
 
 FastConfig launch_config(const FastConfig& cfg, uint32_t len, uint64_t n, int num_sms, bool batch) {
-    FastConfig best = cfg;
-    if (batch) {
-        // other jobs fill the GPU: mode 3 runs 640 threads where the job has four such items of its own
-        if (cfg.mode == 3 && compiled_len(len) && n >= 4ull * 4 * kRowBytes * 640) best.threads = 640;
-        best.rows = fast_rows(n, best, num_sms, true);
-        return best;
-    }
-    // Alone, the scan lasts as many waves of equal items as the busiest CTA slot takes. An item's streams are walked a
-    // byte per step of all threads, tau ns each (plain workload; at 4 GiB, where all sizes are full, 640 threads take
-    // 4.83 ms, 512 4.79, 384 5.16, 256 5.99, 192 7.56), and an item costs its rows and about 16 steps more. With powers
-    // of two from 4 rows and 512 or 768 threads only, 64 MiB took 131 us (now 109), 8 MiB 114 (39), 1 MiB 129 (31).
+    // Mode 3's CTA sizes, the largest first, and the time of a step in which each of its threads takes a byte (ns; 4
+    // GiB plain text, and 2 GiB at LEN 21 and 32). The kernel that keeps its S-box entries in registers leaves room
+    // for its table beside 512 threads; the others take 384 at most: with half the table 640 threads scanned 2 GiB at
+    // 712 GB/s (LEN 21) and 840 (32), 384 with the whole one at 803 and 887.
     struct Size {
         int threads;
         double tau;
     };
-    static const Size sparse[] = {{640, 106.0}, {512, 84.0}, {384, 66.0}, {256, 50.0}, {192, 44.0}};
+    static const Size kept[] = {{512, 76.3}, {384, 59.1}, {256, 46.3}, {192, 45.1}};
+    static const Size read[] = {{384, 68.0}, {256, 52.0}, {192, 49.0}};
+    const bool keeps = compiled_len(len) && keeps_entries(0, (int)len);
+    const Size* sizes = keeps ? kept : read;
+    FastConfig best = cfg;
+    if (batch) {
+        // other jobs fill the GPU
+        if (cfg.mode == 3) best.threads = sizes[0].threads;
+        best.rows = fast_rows(n, best, num_sms, true);
+        return best;
+    }
+    // Alone, the scan lasts as many waves of equal items as the busiest CTA slot takes; an item costs its rows and
+    // about 16 steps more. With powers of two from 4 rows and 512 or 768 threads only, 64 MiB took 131 us (now 92), 8
+    // MiB 114 (31), 1 MiB 129 (28).
     constexpr double kItemBytes = 16.0;
     double best_cost = 0;
     const uint32_t min_rows = n < kShortRowsText ? 1 : 4;
-    for (int i = 0; i < (cfg.mode == 3 ? 5 : 1); i++) {
+    for (int i = 0; i < (cfg.mode != 3 ? 1 : keeps ? 4 : 3); i++) {
         FastConfig c = cfg;
-        if (cfg.mode == 3) c.threads = sparse[i].threads;
-        if (c.threads == 640 && !compiled_len(len)) continue;
+        if (cfg.mode == 3) c.threads = sizes[i].threads;
         const uint64_t threads = config_threads(c), slots = (uint64_t)num_sms * fast_ctas_per_sm(c);
         for (uint32_t rows = 16; rows >= min_rows; rows--) {
             const uint64_t items = (n / (rows * kRowBytes) + threads - 1) / threads;
-            const double cost = (double)((items + slots - 1) / slots) * (rows * kRowBytes + kItemBytes) * sparse[i].tau;
+            const double cost = (double)((items + slots - 1) / slots) * (rows * kRowBytes + kItemBytes) * sizes[i].tau;
             if (best_cost == 0 || cost < best_cost) {
                 best_cost = cost;
                 best = c;

@@ -43,7 +43,7 @@ struct alignas(64) FastJob {
 
 // How a job is scanned: CTA size, probe mode, rows per stream (0: chosen from the text size), and in the dense mode
 // the probe order. Modes 0, 2 and 3 are the sparse kernel (shared-memory stage 1) at 256/384/512, 192/256/384 and 512
-// threads, the last from 192 to 640 as each text's size asks (launch_config); mode 1 is the dense one (pipelined L2 probes). Orders:
+// threads, the last from 192 to 512 as each text's size asks (launch_config); mode 1 is the dense one (pipelined L2 probes). Orders:
 // 0: the pipelined probes are index functions f0 = h1 and f1 = h2; 1: f2 = rot16(h1) and f3 = rot16(h2), the better
 // pair when their region is sparser; 2 and 3: f0 and f1 are tested against the stage-1 table first, and f0 (order 2)
 // or f2 (order 3) is then probed for the windows that pass. The order only changes which bits are tested first: a
@@ -56,7 +56,7 @@ struct FastConfig {
 };
 
 // Mode (1 or 3) and dense probe order with the least expected time per window, from the fills (fraction of set bits)
-// of the 512-thread kernel's stage-1 table, of the cache region and of the external region. Orders 1 and 3 need f2
+// of the 384-thread kernel's stage-1 table, of the cache region and of the external region. Orders 1 and 3 need f2
 // and f3 among the K index functions (K >= 4).
 struct ScanChoice {
     int mode, order;

@@ -267,7 +267,7 @@ ffbf_status ffbf_debug_scan_unpublished(ffbf_ctx* ctx, const uint8_t* d_text, si
 
 /* The tuned scan's current configuration for this context (CTA threads; mode 1 pipelined L2 probes, modes 0, 2 and 3
  * shared-memory stage 1, which differ in the CTA sizes they take: 256/384/512, 192/256/384 and 512; mode 3 fits
- * the size, 192 to 640, to each text), as the autotuner or the filter's fill chose it. Before the first scan or tuning
+ * the size, 192 to 512, to each text), as the autotuner or the filter's fill chose it. Before the first scan or tuning
  * it reports the defaults. */
 ffbf_status ffbf_get_scan_config(const ffbf_ctx* ctx, int* threads, int* mode);
 
