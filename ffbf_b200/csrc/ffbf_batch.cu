@@ -95,7 +95,7 @@ ffbf_status build_plan(const std::vector<PlanJob>& jobs, int num_sms, ScanPlan& 
             for (auto& g : groups)
                 if (g.len == c->g.len && (g.cfg.mode == 1) == (cfg.mode == 1) &&
                     ffbf::config_threads(g.cfg) == ffbf::config_threads(cfg) &&
-                    (cfg.mode != 1 || g.cfg.order == cfg.order))
+                    (cfg.mode != 1 || g.cfg.order == cfg.order) && g.cfg.halves == cfg.halves)
                     gp = &g;
             if (!gp) {
                 groups.push_back(Group{c->g.len, cfg, {}});

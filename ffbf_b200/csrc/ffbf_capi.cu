@@ -253,7 +253,7 @@ ffbf_status ensure_stage1(ffbf_ctx* c, int threads, bool force) {
     if (!force && c->d_stage1 && c->stage1_threads == threads) return FFBF_OK;
     const uint32_t nw = ffbf::stage1_words_for(c->g, threads);
     if (c->d_stage1 && c->stage1_words != nw) dfree(c, c->d_stage1);
-    if (!c->d_stage1) TRY(dalloc_t(c, &c->d_stage1, nw));
+    if (!c->d_stage1) TRY(dalloc_t(c, &c->d_stage1, ffbf::table_halves(c->g) ? 2 * nw : nw));
     c->stage1_words = nw;
     c->stage1_threads = threads;
     CUDA_TRY(c, ffbf::build_stage1(c->d_main, c->g, threads, c->d_stage1, c->st));
@@ -300,6 +300,7 @@ ffbf_status prepare_fast(ffbf_ctx* c) {
     if (c->g.s < 1 && c->cfg.order >= 2) c->cfg.order = 1;
     if (c->g.k < 4 && c->cfg.order == 1) c->cfg.order = 0;
     if (c->g.k >= 4 && c->cfg.order == 2) c->cfg.order = 3;
+    c->cfg.halves = c->cfg.mode == 3 && ffbf::table_halves(c->g);
     // the table the configured kernel reads (a dense kernel without prefilter reads none)
     if (c->cfg.mode != 1 || c->cfg.order >= 2) TRY(ensure_stage1(c, ffbf::table_threads(c->cfg), false));
     return FFBF_OK;

@@ -29,12 +29,12 @@
 // newline mask per 32-byte block. Each stream's first and last '\n' feed the newline summaries, per tile of 16
 // KiB or a little more, that the line resolver reads.
 //
-// What bounds it. Sparse: the ALU pipe (8.5 of the 9.7 clocks that a warp spends on a byte: two rotations, a table
-// address and its bit per probe) and the shared-memory pipe (7.2 wavefronts: 2 for the S-box entry, 3.5 for the first
-// table probe's random words, the rest for the predicated second probe and the text), at 12 to 16 warps per SM. Dense:
+// What bounds it. Sparse: the shared-memory pipe (7.2 wavefronts of the 9 clocks that a warp spends on a byte: 2 for the
+// S-box entry, 3.5 for the first table probe's random words, the rest for the predicated second probe and the text), the
+// ALU pipe (6.5) and the issue slots (6.2), at 12 to 16 warps per SM. Dense:
 // the L1TEX unit, which looks up one random sector per clock and SM (words, 1M patterns: 0.93 of that). On one B200,
-// before -> now, GB/s of text: 10k patterns, 4 GiB 662 -> 992, 64 MiB 443 -> 736, 8 MiB 69 -> 248; LEN 24, 8k patterns in
-// 2^20 + 2^24 bits, 2 GiB 487 -> 955 and 40k in 2^22 + 2^26 299 -> 637; LEN 19, 50k in 2^24 + 2^28, 256 MiB 350 -> 688; LEN
+// before -> now, GB/s of text: 10k patterns, 4 GiB 662 -> 1067, 64 MiB 443 -> 799, 8 MiB 69 -> 292; LEN 24, 8k patterns in
+// 2^20 + 2^24 bits, 2 GiB 487 -> 1017 and 40k in 2^22 + 2^26 299 -> 645; LEN 19, 50k in 2^24 + 2^28, 256 MiB 350 -> 714; LEN
 // 24, 150k in 2^23 + 2^27, 256 MiB 295 -> 547; LEN 40, 8k in 2^20 + 2^24, 2 GiB 168 -> 805; words, 1M patterns 311 -> 351;
 // 4M 16-byte signatures 245 -> 275.
 //
@@ -163,6 +163,23 @@ __device__ __forceinline__ uint32_t lds32_if(uint32_t addr, bool pred) {
     return v;
 }
 
+// A 16-bit entry, zero-extended, and the same where `pred` holds (0 elsewhere).
+__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
+    uint32_t v;
+    asm("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds16_if(uint32_t addr, bool pred) {
+    uint32_t v;
+    asm("{\n\t.reg .pred q;\n\t.reg .u16 t;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.u16 t, 0;\n\t@q ld.shared.u16 t, [%1];\n\t"
+        "cvt.u32.u16 %0, t;\n\t}"
+        : "=r"(v)
+        : "r"(addr), "r"((uint32_t)pred));
+    return v;
+}
+// base + 2 * the upper half of w in one dot product: the address of a 16-bit entry
+__device__ __forceinline__ uint32_t half_addr(uint32_t w, uint32_t base) { return __dp2a_lo(w, 0x0200u, base); }
+
 // Global load of one filter word when `pred` holds (0 otherwise); read-only path.
 __device__ __forceinline__ uint32_t ldg_if(const uint32_t* p, bool pred) {
     uint32_t v;
@@ -209,9 +226,13 @@ __device__ __forceinline__ int len_of(uint32_t len) {
     return L > 0 ? L : (int)len;
 }
 
+// Mode 5 keeps the hash rotated by this (its S-box entries are), so that the upper half of each word of it is the low
+// 16 bits of one index function and the other word's low bits follow them.
+constexpr uint32_t kHalvesRot = 48;
+
 // The hash of the window of LEN bytes at `start`, its bytes read from the text's aligned words that hold them and no
 // others. *newline tells whether one of them is '\n'.
-template <int L>
+template <int L, bool HALVES>
 __device__ __forceinline__ uint64_t text_window_hash(const uint8_t* __restrict__ text, uint64_t start, uint32_t rt_len,
                                                      uint32_t lane_tab, bool* newline) {
     const int len = len_of<L>(rt_len);
@@ -250,7 +271,8 @@ __device__ __forceinline__ uint64_t text_window_hash(const uint8_t* __restrict__
         }
     }
     *newline = found != 0;
-    return ((uint64_t)hh << 32) | hl;
+    const uint64_t h = ((uint64_t)hh << 32) | hl;
+    return HALVES ? rol64(h, 64 - kHalvesRot) : h;
 }
 
 __device__ __forceinline__ void record_hit(const FastJob* J, const Geom& g, uint64_t start, uint64_t h) {
@@ -263,7 +285,7 @@ __device__ __forceinline__ void record_hit(const FastJob* J, const Geom& g, uint
 // window's end, {position in the stream | lane << 16}. Each lane reads its windows' bytes back from the text (still in
 // L2), hashes them and runs the full K-bit test: few windows get here, so this costs less than carrying every
 // window's hash to its test in the byte loop. All of a lane's first probes are issued before any is used.
-template <int L, int PER_LANE>
+template <int L, bool HALVES, int PER_LANE>
 __device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int qn, uint64_t warp_pos0, uint64_t stride,
                                          int lane, uint32_t lane_tab) {
     const int len = len_of<L>(J->g.len);
@@ -281,7 +303,7 @@ __device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int q
         const uint32_t e = lds32_volatile(qaddr + 4u * (uint32_t)i);
         start[t] = warp_pos0 + (e >> 16) * stride + (e & 0xFFFFu) + 1 - len;
         bool newline;
-        h[t] = text_window_hash<L>(text, start[t], len, lane_tab, &newline);  // windows with a '\n' are not queued
+        h[t] = text_window_hash<L, HALVES>(text, start[t], len, lane_tab, &newline);  // windows with a '\n' are not queued
         bi[t] = bit_index<1>(g, h[t], 0);
         v[t] = __ldg(main_words + (bi[t] >> 5));
     }
@@ -297,7 +319,7 @@ __device__ __noinline__ void flush_queue(const FastJob* J, uint32_t qaddr, int q
 // text's end after its last whole stream (less than one stream), a window per thread, where a launch of its own took 60
 // us for 12 KB. z is the thread's stream, nl_span its first '\n' (low half, 0xffff: none) and its last. One function,
 // so that the byte loop keeps its registers.
-template <int L>
+template <int L, bool HALVES>
 __device__ __noinline__ void finish_streams(const FastJob* J, uint64_t z, uint32_t nl_span, int threads, uint32_t lane_tab,
                                             uint32_t* error_flag) {
     const int lane = threadIdx.x & 31;
@@ -322,7 +344,7 @@ __device__ __noinline__ void finish_streams(const FastJob* J, uint64_t z, uint32
             const int len = len_of<L>(g.len);
             if (p + 1 < len) continue;
             bool newline;
-            const uint64_t h = text_window_hash<L>(J->text, p + 1 - len, len, lane_tab, &newline);
+            const uint64_t h = text_window_hash<L, HALVES>(J->text, p + 1 - len, len, lane_tab, &newline);
             if (!newline && full_check_from(g, J->main_words, h, 0)) record_hit(J, g, p + 1 - len, h);
         }
         __syncwarp();
@@ -375,6 +397,7 @@ struct JobState {
     uint32_t n_supertiles;
     uint32_t s1_bmask;      // byte offset of the stage-1 table word of bit (h & (T-1)): (h >> 3) & s1_bmask
     uint32_t s2, s2_bmask;  // the second probe's table: the same, or with S = 1 a word of ones
+    uint32_t twice;  // 0x10001: repeats a 16-bit entry in both halves, by a multiplication that the ALU pipe is spared
     uint32_t a_mask, b_mask;  // dense modes: the regions of the two pipelined probes
     const uint32_t *a_words, *b_words;
     uint64_t n_streams;
@@ -408,6 +431,7 @@ __device__ __noinline__ void change_job(const FastJob* jobs, int job, JobState* 
         s->rows = fits ? J->rows : 0u;
         s->n_supertiles = J->n_supertiles;
         s->s1_bmask = bmask;
+        s->twice = 0x10001u;
         s->s2 = J->g.s > 1 ? s1 : ones;
         s->s2_bmask = J->g.s > 1 ? bmask : 0u;
         s->a_mask = J->a_mask;
@@ -533,6 +557,11 @@ __device__ __forceinline__ uint32_t newline_mask32(const uint32_t (&w)[8]) {
 // Kernel modes.
 // MODE 0 (sparse filters): both first index functions are tested against a shared-memory table, the cache region
 // itself when it fits, else its fold, which only rejects windows the full test rejects.
+// MODE 5: MODE 0 for a table of exactly 2^20 bits (any cache region from 2^20 bits on), S >= 2 and the lengths that keep
+// their entries. The table is 65536 entries of 16 bits, and the hash is kept rotated by 48 (a rotation of the S-box), so
+// that each word's upper half is the low 16 bits of one index function: an entry's address is one dot product, without
+// the shift, the mask and the sum, and the other word's low bits choose the bit. That takes 4 of 17 instructions per
+// byte off the ALU pipe: 10k patterns, 4 GiB 992 -> 1067 GB/s, 64 MiB 762 -> 799; 8k in 2^20 + 2^24, 2 GiB 957 -> 1017.
 // MODE 1 (dense filters, where a shared-memory table would pass most windows): the exact probes of the first two
 // index functions are global loads, the first issued per valid window, the second for the windows that pass it;
 // both are consumed kRing bytes later from register rings, so L2 latency overlaps the hashing of the next windows.
@@ -545,7 +574,7 @@ __device__ __forceinline__ uint32_t newline_mask32(const uint32_t (&w)[8]) {
 // In every mode the byte loop over a 32-byte block is one branch-free stretch: a window's verdict is shifted into a
 // 32-bit register mask, and only after the block do the lanes with surviving windows queue their positions. Against
 // a warp vote and a queue append per byte this took the sparse scan of a 4 GiB text from 662 to 749 GB/s.
-__host__ __device__ constexpr bool sparse_mode(int mode) { return mode == 0; }
+__host__ __device__ constexpr bool sparse_mode(int mode) { return mode == 0 || mode == 5; }
 
 // Whether the byte loop keeps the window's LEN S-box entries in registers and rotates the leaving one there, instead of
 // reading it from the rotated table: the sparse mode at the compiled lengths but 32, whose 64 registers spill beside the
@@ -593,6 +622,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     // LEN), so that it needs no rotation; a block's high bytes are cleared beforehand (they hash as byte 0). With LEN =
     // 32 the rotation only swaps the halves, and the table holds all 256 bytes once.
     constexpr bool kTwoTables = L != 32;
+    constexpr bool kHalves = MODE == 5;
     constexpr bool kEntries = keeps_entries(MODE, L);
     constexpr int kTab = tab_bytes(MODE, L);
     extern __shared__ uint8_t smem_raw[];
@@ -713,7 +743,8 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     // a thread per byte value, its 16 copies stored in an order that keeps the lanes on different banks
     for (int c = tid; c < kTab / 128; c += THREADS) {
         uint64_t* tp = reinterpret_cast<uint64_t*>(smem + 2 * kStageBytes) + 16 * c;
-        const uint64_t v = kTwoTables ? (c < 128 ? c_sbox[c] : rol64(c_sbox[c - 128], (uint32_t)len_of<L>(rt_len)))
+        const uint64_t v = kHalves ? rol64(c_sbox[c], kHalvesRot)
+                           : kTwoTables ? (c < 128 ? c_sbox[c] : rol64(c_sbox[c - 128], (uint32_t)len_of<L>(rt_len)))
                                       : c_sbox[(c & 0x80) ? 0 : c];
 #pragma unroll
         for (int q = 0; q < 16; q++) tp[(q + lane) & 15] = v;
@@ -748,7 +779,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     int qn = 0;  // warp-uniform queue fill
     auto flush = [&]() {
         __syncwarp();
-        flush_queue<L, kQueueCap / 32>(job_desc(), qaddr, qn, s_wpos[warp], (uint64_t)s_job.rows * kRowBytes, lane,
+        flush_queue<L, kHalves, kQueueCap / 32>(job_desc(), qaddr, qn, s_wpos[warp], (uint64_t)s_job.rows * kRowBytes, lane,
                                          lane_tab);
         qn = 0;
     };
@@ -866,6 +897,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         } else {
             const uint32_t pos0 = (uint32_t)r * kPart;  // this part's first byte in the stream
             const uint32_t s1_bmask = s_job.s1_bmask, s2 = s_job.s2, s2_bmask = s_job.s2_bmask;
+            const uint32_t twice = s_job.twice;
             const uint32_t a_mask = s_job.a_mask, b_mask = s_job.b_mask;
             const uint32_t *const a_words = s_job.a_words, *const b_words = s_job.b_words;
 #pragma unroll 1
@@ -910,9 +942,15 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                     if constexpr (kSparse) {
                         // the second probe is loaded only where the first passes: its random words would cost the
                         // shared-memory pipe, which bounds this loop, another 3.5 wavefronts per warp
-                        const uint32_t w0 = lds32(s1 + ((hl >> 3) & s1_bmask));
-                        const uint32_t w1 =
-                            lds32_if(s2 + ((hh >> 3) & s2_bmask), (__funnelshift_r(w0, w0, hl) & 1u) != 0);
+                        uint32_t w0, w1;
+                        if constexpr (kHalves) {
+                            w0 = lds16(half_addr(hh, s1)) * twice;
+                            w1 = lds16_if(half_addr(hl, s1), (__funnelshift_r(w0, w0, hl) & 1u) != 0) * twice;
+                            pass = __funnelshift_r(pass, __funnelshift_r(w1, w1, hh), 1);
+                            continue;
+                        }
+                        w0 = lds32(s1 + ((hl >> 3) & s1_bmask));
+                        w1 = lds32_if(s2 + ((hh >> 3) & s2_bmask), (__funnelshift_r(w0, w0, hl) & 1u) != 0);
                         pass = __funnelshift_r(pass, __funnelshift_r(w1, w1, hh), 1);  // the bit enters at bit 31
                     } else {
                         const int slot = j % kRing;
@@ -979,7 +1017,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
                     enqueue(rest, pos0 + (uint32_t)(kPart - kLag));
                 }
                 if (qn) flush();  // the queue keeps its candidates across the stream's parts, not across streams
-                finish_streams<L>(job_desc(), (uint64_t)st * THREADS + tid, nl_span, THREADS, lane_tab, error_flag);
+                finish_streams<L, kHalves>(job_desc(), (uint64_t)st * THREADS + tid, nl_span, THREADS, lane_tab, error_flag);
             }
         }
         // this warp is done reading the stage
@@ -1001,7 +1039,7 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
 }
 
 // static shared memory of k_scan_fast<., THREADS, .> (sequencer, current job, warp positions)
-constexpr size_t static_smem(int threads) { return 8 * (size_t)(threads / 32) + 168; }
+constexpr size_t static_smem(int threads) { return 8 * (size_t)(threads / 32) + 176; }
 
 constexpr size_t fixed_smem(int threads, int table_bytes = kTabBytes) {
     return 1024 + 2 * (size_t)threads * kPart + table_bytes + 128 + (threads / 32) * 4 * (size_t)kQueueCap;
@@ -1028,7 +1066,16 @@ cudaError_t launch_cfg(uint32_t len, const FastJob* d_jobs, uint32_t n_jobs, uin
 template <int L>
 cudaError_t launch_len(uint32_t len, const FastConfig& cfg, const FastJob* d_jobs, uint32_t n_jobs, uint32_t n_items,
                        uint32_t max_s1_words, uint32_t* d_ctl, int num_sms, cudaStream_t st) {
-    const int mode = cfg.mode != 1 ? 0 : 1 + cfg.order;  // kernel mode: 0 sparse, 1..4 dense in probe order 0..3
+    // kernel mode: 0 and 5 sparse, 1..4 dense in probe order 0..3
+    const int mode = cfg.mode == 1 ? 1 + cfg.order : cfg.mode == 3 && cfg.halves ? 5 : 0;
+    if constexpr (keeps_entries(5, L)) {
+        if (mode == 5) switch (config_threads(cfg)) {
+            case 192: return launch_cfg<L, 192, 5>(len, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+            case 256: return launch_cfg<L, 256, 5>(len, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+            case 384: return launch_cfg<L, 384, 5>(len, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+            case 512: return launch_cfg<L, 512, 5>(len, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st);
+        }
+    }
     switch (16 * config_threads(cfg) + mode) {
 #define FFBF_CASE(T, M) \
     case 16 * T + M: return launch_cfg<L, T, M>(len, d_jobs, n_jobs, n_items, max_s1_words, d_ctl, num_sms, st)
@@ -1074,6 +1121,11 @@ static_assert(kSmemLimit - fixed_smem(512, kHalfTabBytes) - static_smem(512) - 6
 // mode 3 reads the 384-thread table at every CTA size it takes
 int table_threads(const FastConfig& cfg) { return cfg.mode == 3 ? 384 : config_threads(cfg); }
 
+bool table_halves(const Geom& g) {
+    return g.s >= 2 && compiled_len(g.len) && keeps_entries(0, (int)g.len) &&
+           g.cache_bits >> stage1_shift_for(g, 384) == 1u << 20;
+}
+
 uint32_t stage1_words_for(const Geom& g, int threads) {
     return (uint32_t)(((uint64_t)g.cache_bits >> stage1_shift_for(g, threads)) / 32);
 }
@@ -1083,7 +1135,7 @@ ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, doub
     // random sector per clock). Measured against the model: words, 1M patterns, order 1: 354 GB/s; 150k printable
     // patterns in 2^23 + 2^27 bits, order 3: 547 GB/s (order 1: 323, mode 3: 309); 40k in 2^22 + 2^26, mode 3: 625,
     // order 3: 637; 50k in 2^24 + 2^28 (LEN 19), mode 3: 688, order 3: 601; 8k in 2^20 + 2^24, mode 3: 955, order 3:
-    // 653.
+    // 653 (before mode 3 read 16-bit entries, which gains it 4 to 8 %).
     // Orders 0 and 1: the first probe always, the second when the first passes, and a queued window's full test
     // (about three probes' worth of issue and flush work) when both pass. A probe of a region that the L1 left
     // beside the shared memory can largely hold (about 64 KiB) mostly hits there.
@@ -1134,7 +1186,7 @@ uint32_t fast_tile_bytes(uint32_t rows) {
 
 FastConfig launch_config(const FastConfig& cfg, uint32_t len, uint64_t n, int num_sms, bool batch) {
     // Mode 3's CTA sizes, the largest first, and the time of a step in which each of its threads takes a byte (ns; 4
-    // GiB plain text, and 2 GiB at LEN 21 and 32). The kernel that keeps its S-box entries in registers leaves room
+    // GiB plain text, and 2 GiB at LEN 21 and 32; with 16-bit entries about 7 % less, all sizes alike). The kernel that keeps its S-box entries in registers leaves room
     // for its table beside 512 threads; the others take 384 at most: with half the table 640 threads scanned 2 GiB at
     // 712 GB/s (LEN 21) and 840 (32), 384 with the whole one at 803 and 887.
     struct Size {
@@ -1153,8 +1205,8 @@ FastConfig launch_config(const FastConfig& cfg, uint32_t len, uint64_t n, int nu
         return best;
     }
     // Alone, the scan lasts as many waves of equal items as the busiest CTA slot takes; an item costs its rows and
-    // about 16 steps more. With powers of two from 4 rows and 512 or 768 threads only, 64 MiB took 131 us (now 92), 8
-    // MiB 114 (31), 1 MiB 129 (28).
+    // about 16 steps more. With powers of two from 4 rows and 512 or 768 threads only, 64 MiB took 131 us (now 84), 8
+    // MiB 114 (29).
     constexpr double kItemBytes = 16.0;
     double best_cost = 0;
     const uint32_t min_rows = n < kShortRowsText ? 1 : 4;
@@ -1215,11 +1267,11 @@ cudaError_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const
     job->main_words = a.main_words;
     job->ff_words = a.ff_words;
     job->text = a.text;
-    job->stage1_words = stage1_words;
     // the table the kernel reads: the sparse mode's, or the dense mode's prefilter (order 2)
     const bool reads_table = cfg.mode != 1 || cfg.order >= 2;
     job->stage1_shift = reads_table ? stage1_shift_for(a.g, table_threads(cfg)) : 0;
     job->stage1_nwords = reads_table ? (uint32_t)(((uint64_t)a.g.cache_bits >> job->stage1_shift) / 32) : 0;
+    job->stage1_words = stage1_words + (cfg.mode == 3 && cfg.halves ? job->stage1_nwords : 0u);
     {
         // dense mode: regions of the pipelined probes, index functions f0/f1 (order 0) or f2/f3 (order 1,
         // which only K >= 4 filters set)
@@ -1294,12 +1346,35 @@ __global__ void k_stage1_fold(const uint32_t* main_words, uint32_t sh, uint32_t*
     out[w] = v;
 }
 
+// The same 2^20 bits as 65536 entries of 16: bit i of the table is bit i >> 16 of entry i & 0xFFFF. A warp turns 64
+// entries: lane l reads the words of 32 of them in one sixteenth of the table, and 32 votes collect the entries.
+__global__ void k_stage1_halves(const uint32_t* table, uint32_t* out) {
+    const uint32_t lane = threadIdx.x & 31, k = 2 * (blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32);
+    const uint32_t w = table[(lane & 15) * 2048 + k + (lane >> 4)];
+    uint32_t v = 0;
+#pragma unroll
+    for (uint32_t t = 0; t < 32; t++) {
+        const uint32_t m = __ballot_sync(0xffffffffu, (w >> t) & 1u);
+        const uint32_t e = lane < 16 ? m & 0xffffu : m >> 16;
+        if ((lane & 15) == t / 2) v |= t & 1 ? e << 16 : e;
+    }
+    out[(k + (lane >> 4)) * 16 + (lane & 15)] = v;
+}
+
 cudaError_t build_stage1(const uint32_t* main_words, const Geom& g, int threads, uint32_t* out, cudaStream_t st) {
     const uint32_t sh = stage1_shift_for(g, threads);
     const uint32_t nwords = (uint32_t)(((uint64_t)g.cache_bits >> sh) / 32);
-    if (sh == 0) return cudaMemcpyAsync(out, main_words, 4ull * nwords, cudaMemcpyDeviceToDevice, st);
-    k_stage1_fold<<<(nwords + 255) / 256, 256, 0, st>>>(main_words, sh, out, nwords);
-    note_launches(1);
+    if (sh == 0) {
+        cudaError_t e = cudaMemcpyAsync(out, main_words, 4ull * nwords, cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) return e;
+    } else {
+        k_stage1_fold<<<(nwords + 255) / 256, 256, 0, st>>>(main_words, sh, out, nwords);
+        note_launches(1);
+    }
+    if (threads == 384 && table_halves(g)) {
+        k_stage1_halves<<<128, 256, 0, st>>>(out, out + nwords);  // 1024 warps
+        note_launches(1);
+    }
     return cudaGetLastError();
 }
 

@@ -53,6 +53,7 @@ struct FastConfig {
     int mode;
     uint32_t rows;
     int order;
+    bool halves = false;  // mode 3: the kernel that reads the table's 16-bit entries (table_halves)
 };
 
 // Mode (1 or 3) and dense probe order with the least expected time per window, from the fills (fraction of set bits)
@@ -84,6 +85,8 @@ constexpr uint64_t kShortRowsText = 64ull << 20;
 // leaves over, otherwise its fold to C >> shift bits.
 uint32_t stage1_shift_for(const Geom& g, int threads);
 uint32_t stage1_words_for(const Geom& g, int threads);
+// Whether mode 3 reads the table as 16-bit entries, which lie behind its words on the device.
+bool table_halves(const Geom& g);
 cudaError_t build_stage1(const uint32_t* main_words, const Geom& g, int threads, uint32_t* out, cudaStream_t st);
 
 // CTAs of the tuned kernel resident per SM for a configuration (two for the 192-thread dense kernel).
