@@ -7,7 +7,7 @@
 // sort is a bucket sort over the text's span, about two buckets per record, each then sorted by one thread (records of
 // one bucket are few unless a text is very uneven, which takes a bitonic network instead: for 8000 windows about 120 us
 // against 10). What bounds it is latency: the dependent loads of a line search, then four passes over the records.
-// 500 windows of a 64 MiB text: 132 -> 28 us a call, 8000 of 1 GiB: 276 -> 45.
+// Whole calls, 500 windows of a 64 MiB text: 132 -> 39 us, 8000 of 1 GiB: 276 -> 89.
 #include <climits>
 
 #include "ffbf_collect.cuh"
@@ -384,7 +384,7 @@ cudaError_t verify_collect(const VerifyJob& job, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     if (job.nhits > 2 * kSmallResults) {
         // many windows: as many threads as the SMs hold, which the fused kernel's shared memory would halve (356k
-        // windows: 299 us against 100), then one CTA orders what is few
+        // windows: 299 us against 218), then one CTA orders what is few
         k_verify<<<(job.nhits + 255) / 256, 256, 0, st>>>(job);
         k_order_matches<<<1, kThreads, kSmem, st>>>(job);
         note_launches(2);
