@@ -29,9 +29,9 @@
 // newline mask per 32-byte block. Each stream's first and last '\n' feed the newline summaries, per tile of 16
 // KiB or a little more, that the line resolver reads.
 //
-// What bounds it. Sparse: the shared-memory pipe (7.2 wavefronts of the 9 clocks that a warp spends on a byte: 2 for the
-// S-box entry, 3.5 for the first table probe's random words, the rest for the predicated second probe and the text), the
-// ALU pipe (6.5) and the issue slots (6.2), at 12 to 16 warps per SM. Dense:
+// What bounds it. Sparse: of the 9 clocks that a warp spends on a byte the ALU pipe is busy for 7.3, the shared-memory
+// pipe for 7.1 (wavefronts: 2 for the S-box entry, 3.5 for the first table probe's random words, the rest for the
+// predicated second probe and the text) and the issue slots for 6.4, at 12 to 16 warps per SM. Dense:
 // the L1TEX unit, which looks up one random sector per clock and SM (words, 1M patterns: 0.93 of that). On one B200,
 // before -> now, GB/s of text: 10k patterns, 4 GiB 662 -> 1067, 64 MiB 443 -> 799, 8 MiB 69 -> 292; LEN 24, 8k patterns in
 // 2^20 + 2^24 bits, 2 GiB 487 -> 1017 and 40k in 2^22 + 2^26 299 -> 645; LEN 19, 50k in 2^24 + 2^28, 256 MiB 350 -> 714; LEN
@@ -560,8 +560,8 @@ __device__ __forceinline__ uint32_t newline_mask32(const uint32_t (&w)[8]) {
 // MODE 5: MODE 0 for a table of exactly 2^20 bits (any cache region from 2^20 bits on), S >= 2 and the lengths that keep
 // their entries. The table is 65536 entries of 16 bits, and the hash is kept rotated by 48 (a rotation of the S-box), so
 // that each word's upper half is the low 16 bits of one index function: an entry's address is one dot product, without
-// the shift, the mask and the sum, and the other word's low bits choose the bit. That takes 4 of 17 instructions per
-// byte off the ALU pipe: 10k patterns, 4 GiB 992 -> 1067 GB/s, 64 MiB 762 -> 799; 8k in 2^20 + 2^24, 2 GiB 957 -> 1017.
+// the shift, the mask and the sum, and the other word's low bits choose the bit. That takes 4 instructions per byte
+// off the ALU pipe: 10k patterns, 4 GiB 992 -> 1067 GB/s, 64 MiB 762 -> 799; 8k in 2^20 + 2^24, 2 GiB 957 -> 1017.
 // MODE 1 (dense filters, where a shared-memory table would pass most windows): the exact probes of the first two
 // index functions are global loads, the first issued per valid window, the second for the windows that pass it;
 // both are consumed kRing bytes later from register rings, so L2 latency overlaps the hashing of the next windows.
