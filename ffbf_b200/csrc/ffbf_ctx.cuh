@@ -92,7 +92,7 @@ struct ffbf_ctx {
     uint64_t tiles_cap = 0;
     uint32_t tile_bytes = ffbf::kScanTile;  // bytes per tile of the last scan's summaries
     int scan_path = 0;             // 0 = generic, 1 = fast
-    uint32_t* d_stage1 = nullptr;  // stage-1 table of the tuned scan (cache copy or its fold)
+    uint32_t* d_stage1 = nullptr;  // stage-1 table of the tuned scan (cache copy or its fold), its 16-bit form behind it
     bool stage1_dirty = true;
     int stage1_threads = 0;        // CTA size the table was sized for
     uint32_t stage1_words = 0;

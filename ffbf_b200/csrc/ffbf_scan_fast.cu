@@ -1163,8 +1163,8 @@ ScanChoice choose_scan(const Geom& g, double table_fill, double cache_fill, doub
     // Sparse: both table bits; a window that passes costs its lane's queue append and its share of a flush, much more
     // of it where its exact first probe passes too (cache_fill / table_fill of them) and others follow.
     const double base = compiled_len(g.len) && keeps_entries(0, (int)g.len) ? 0.325 : 0.38;
-    if (g.s > 0 && (g.k < 2 || base + both(table_fill) * (13.0 + 70.0 * cache_fill / std::max(table_fill, 1e-9)) <= best_cost))
-        best.mode = 3;
+    const double per_pass = 13.0 + 70.0 * cache_fill / std::max(table_fill, 1e-9);
+    if (g.s > 0 && (g.k < 2 || base + both(table_fill) * per_pass <= best_cost)) best.mode = 3;
     return best;
 }
 
@@ -1186,9 +1186,10 @@ uint32_t fast_tile_bytes(uint32_t rows) {
 
 FastConfig launch_config(const FastConfig& cfg, uint32_t len, uint64_t n, int num_sms, bool batch) {
     // Mode 3's CTA sizes, the largest first, and the time of a step in which each of its threads takes a byte (ns; 4
-    // GiB plain text, and 2 GiB at LEN 21 and 32; with 16-bit entries about 7 % less, all sizes alike). The kernel that keeps its S-box entries in registers leaves room
-    // for its table beside 512 threads; the others take 384 at most: with half the table 640 threads scanned 2 GiB at
-    // 712 GB/s (LEN 21) and 840 (32), 384 with the whole one at 803 and 887.
+    // GiB plain text, and 2 GiB at LEN 21 and 32; with 16-bit entries about 7 % less, all sizes alike). The kernel that
+    // keeps its S-box entries in registers leaves room for its table beside 512 threads; the others take 384 at most:
+    // with half the table 640 threads scanned 2 GiB at 712 GB/s (LEN 21) and 840 (32), 384 with the whole one at 803 and
+    // 887.
     struct Size {
         int threads;
         double tau;
