@@ -25,6 +25,7 @@ struct ffbf_batch {
         ffbf_ctx* c;
         const uint8_t* text;
         size_t len;
+        uint32_t tile_bytes;  // of the newline summaries that the prepared launch writes
     };
     // The device buffers and configuration each job's descriptors were built from. A context that has
     // since grown its hit buffer, reloaded its filter, added patterns or been retuned makes the batch
@@ -248,7 +249,7 @@ ffbf_status ffbf_batch_add(ffbf_batch* b, ffbf_ctx* c, const uint8_t* d_text, si
     for (auto& j : b->jobs)
         if (j.c == c) return bfail(b, FFBF_EINVAL, "a context may appear only once in a batch");
     if (b->prepared) batch_release(b);
-    b->jobs.push_back({c, d_text, len});
+    b->jobs.push_back({c, d_text, len, 0});
     return FFBF_OK;
 }
 
@@ -264,7 +265,9 @@ ffbf_status ffbf_batch_prepare(ffbf_batch* b) {
     ffbf_status s = build_plan(pj, b->num_sms, plan, &bad);
     if (s != FFBF_OK) return bfail(b, s, "job " + std::to_string(bad) + ": " + b->jobs[bad].c->err);
     std::vector<uint32_t*> counters;
-    for (const auto& j : b->jobs) {
+    for (size_t i = 0; i < b->jobs.size(); i++) {
+        auto& j = b->jobs[i];
+        j.tile_bytes = plan.args[i].tile_bytes;
         b->keys.push_back(batch_key(j.c));
         counters.push_back(j.c->d_counters);
     }
@@ -367,6 +370,7 @@ ffbf_status ffbf_batch_launch(ffbf_batch* b) {
         reset_scan(j.c);
         j.c->d_text = j.text;
         j.c->text_len = j.len;
+        j.c->tile_bytes = j.tile_bytes;  // a scan of the context's own since may have had another
         j.c->scan_pending = true;
     }
     if (cudaGraphLaunch(b->exec, b->st) != cudaSuccess) {

@@ -386,6 +386,13 @@ ffbf_status setup_scan_state(ffbf_ctx* c, const uint8_t* d_text, size_t len) {
     return FFBF_OK;
 }
 
+cudaError_t resolve_scan_lines(ffbf_ctx* c, uint32_t nh) {
+    if (scan_tiles(c) > c->tiles_cap) return cudaErrorInvalidValue;  // the summaries are of another scan
+    return ffbf::resolve_lines(c->d_text, c->text_len, c->g.len, c->d_hits, nh, c->d_tiles, c->d_tiles + c->tiles_cap,
+                               c->d_tiles + 2 * c->tiles_cap, c->d_tiles + 3 * c->tiles_cap, c->tile_bytes,
+                               scan_tiles(c), c->d_hitlines, c->st, c->d_tiles + 4 * c->tiles_cap);
+}
+
 uint64_t tiles_for(uint64_t len) {
     // tiles are 16 KiB or more, but 4 KiB where a small text's scan may use streams of less than four rows
     const uint64_t tile = len < ffbf::kShortRowsText ? 4096 : ffbf::kScanTile;
@@ -803,10 +810,7 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
             nh = c->h_counters[ffbf::CNT_HITS];
         }
         c->nhits = nh;
-        CUDA_TRY(c, ffbf::resolve_lines(c->d_text, c->text_len, c->g.len, c->d_hits, nh, c->d_tiles,
-                                        c->d_tiles + c->tiles_cap, c->d_tiles + 2 * c->tiles_cap,
-                                        c->d_tiles + 3 * c->tiles_cap, c->tile_bytes, scan_tiles(c), c->d_hitlines,
-                                        c->st, c->d_tiles + 4 * c->tiles_cap));
+        CUDA_TRY(c, resolve_scan_lines(c, nh));
         // Text order on the device: sorted window starts, then the distinct lines of the sorted windows. When
         // the device has no room for the sort's scratch (about 60 bytes per hit window), or FFBF_HOST_ORDER is
         // set, the records are ordered on the host instead; the results are the same.

@@ -227,6 +227,8 @@ ffbf_status launch_scan(ffbf_ctx* c);  // counters reset + scan of c->d_text on 
 // Tile summaries a scan of len bytes may need, and those of the context's current scan.
 uint64_t tiles_for(uint64_t len);
 inline uint64_t scan_tiles(const ffbf_ctx* c) { return (c->text_len + c->tile_bytes - 1) / c->tile_bytes; }
+// Line spans of the first nh hits of the context's current scan, from its tile summaries, enqueued on its stream.
+cudaError_t resolve_scan_lines(ffbf_ctx* c, uint32_t nh);
 // Sizes the scan buffers for a device text of len bytes and resets the results, without launching.
 ffbf_status setup_scan_state(ffbf_ctx* c, const uint8_t* d_text, size_t len);
 

@@ -486,10 +486,7 @@ ffbf_status start_resolve(ffbf_server* s, Request* r) {
         }
         h.cap = cap;
     }
-    cudaError_t e = ffbf::resolve_lines(c->d_text, c->text_len, c->g.len, c->d_hits, nh, c->d_tiles,
-                                        c->d_tiles + c->tiles_cap, c->d_tiles + 2 * c->tiles_cap,
-                                        c->d_tiles + 3 * c->tiles_cap, c->tile_bytes, scan_tiles(c), c->d_hitlines, c->st,
-                                        c->d_tiles + 4 * c->tiles_cap);
+    cudaError_t e = resolve_scan_lines(c, nh);
     if (e == cudaSuccess && nh)
         e = cudaMemcpyAsync(h.hr, c->d_hits, nh * sizeof(HitRec), cudaMemcpyDeviceToHost, c->st);
     if (e == cudaSuccess && nh)
