@@ -102,25 +102,62 @@ uint64_t* result_array(ffbf_ctx* c, int i) {
     return reinterpret_cast<uint64_t*>(c->h_res + 64) + (size_t)i * c->res_cap;
 }
 
+constexpr uint32_t kUploads = 8;          // blocks of the upload ring, taken in halves
+constexpr size_t kUploadBytes = 768;      // zero counters, then a descriptor
+
+// The pinned block for the next upload on the context's stream; nothing that was enqueued earlier still reads it.
+ffbf_status upload_block(ffbf_ctx* c, uint8_t** block) {
+    cudaStreamCaptureStatus capture;
+    CUDA_TRY(c, cudaStreamIsCapturing(c->st, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+        // each replay reads the block again, so no other scan may use it while the context lives
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        CUDA_TRY(c, cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaMallocHost(block, kUploadBytes);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return fail(c, FFBF_ENOMEM_HOST, "pinned upload block");
+        }
+        memset(*block, 0, kUploadBytes);
+        c->captured_uploads.push_back(*block);
+        return FFBF_OK;
+    }
+    constexpr uint32_t half = kUploads / 2;
+    if (c->uploads % half == 0 && c->uploads) {
+        // the half just used up is behind this event; the other one, if it was used, is taken again
+        cudaEvent_t* ev = c->upload_done;
+        const uint32_t used = (c->uploads / half - 1) % 2;
+        if (!ev[used]) CUDA_TRY(c, cudaEventCreateWithFlags(&ev[used], cudaEventDisableTiming));
+        CUDA_TRY(c, cudaEventRecord(ev[used], c->st));
+        if (c->uploads >= kUploads) CUDA_TRY(c, cudaEventSynchronize(ev[1 - used]));
+    }
+    *block = c->h_uploads + c->uploads++ % kUploads * kUploadBytes;
+    return FFBF_OK;
+}
+
 // A context's small memory in one allocation each: pinning costs a call one to two milliseconds, a device allocation
-// 0.6, whatever its size. Pinned: counters, a job descriptor's staging, the first results. Device (behind
-// `front_bytes` of the caller's): counters, the job descriptor, the fill counts.
+// 0.6, whatever its size. Pinned: counters, the upload ring, the first results. Device (behind `front_bytes` of the
+// caller's): counters, the job descriptor, the fill counts.
 ffbf_status alloc_small(ffbf_ctx* c, size_t front_bytes, uint8_t** front) {
-    static_assert(ffbf::CNT_WORDS * sizeof(uint32_t) <= 256 && sizeof(ffbf::FastJob) <= 512, "sections of the blocks");
+    static_assert(ffbf::CNT_WORDS * sizeof(uint32_t) <= 256 && sizeof(ffbf::FastJob) <= 512 &&
+                      ffbf::kJobOffset + sizeof(ffbf::FastJob) <= kUploadBytes,
+                  "sections of the blocks");
+    constexpr size_t kBeforeResults = 256 + kUploads * kUploadBytes;
     uint8_t *h = nullptr, *d = nullptr;
     TRY(dalloc_t(c, &d, front_bytes + 1024));
     *front = d;
     c->d_counters = reinterpret_cast<uint32_t*>(d + front_bytes);
     c->d_job = reinterpret_cast<ffbf::FastJob*>(d + front_bytes + ffbf::kJobOffset);
     c->d_popc = reinterpret_cast<unsigned long long*>(d + front_bytes + 768);
-    if (cudaMallocHost(&h, 1024 + ffbf::result_bytes(kFirstResults)) != cudaSuccess) {
+    if (cudaMallocHost(&h, kBeforeResults + ffbf::result_bytes(kFirstResults)) != cudaSuccess) {
         cudaGetLastError();
         return fail(c, FFBF_ENOMEM_HOST, "pinned context block");
     }
     c->h_counters = reinterpret_cast<uint32_t*>(h);
-    memset(h + 512 - ffbf::kJobOffset, 0, ffbf::kJobOffset);  // stays zero: a scan's first counters (scan_fast)
-    c->h_job = reinterpret_cast<ffbf::FastJob*>(h + 512);
-    c->h_res = h + 1024;
+    c->h_uploads = h + 256;
+    memset(c->h_uploads, 0, kUploads * kUploadBytes);  // the counters in each stay zero
+    c->h_res = h + kBeforeResults;
     c->res_cap = kFirstResults;
     return FFBF_OK;
 }
@@ -160,6 +197,7 @@ ffbf_status enter(ffbf_ctx* c) {
 
 ffbf_status sync(ffbf_ctx* c) {
     CUDA_TRY(c, cudaStreamSynchronize(c->st));
+    c->uploads = 0;  // every upload has been read
     return FFBF_OK;
 }
 
@@ -346,8 +384,9 @@ ffbf_status launch_scan(ffbf_ctx* c) {
         TRY(prepare_fast(c));
         const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, n, c->num_sms, false);
         c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
-        CUDA_TRY(c, ffbf::scan_fast(make_scan_args(c), c->d_stage1, cfg, c->num_sms,
-                                   reinterpret_cast<uint8_t*>(c->h_job) - ffbf::kJobOffset, c->st));
+        uint8_t* block;
+        TRY(upload_block(c, &block));
+        CUDA_TRY(c, ffbf::scan_fast(make_scan_args(c), c->d_stage1, cfg, c->num_sms, block, c->st));
     } else {
         CUDA_TRY(c, cudaMemsetAsync(c->d_counters, 0, ffbf::CNT_WORDS * sizeof(uint32_t), c->st));
         if (n == 0) return FFBF_OK;
@@ -553,6 +592,9 @@ void ffbf_destroy(ffbf_ctx* c) {
     for (auto& kv : c->allocs) cudaFree(kv.first);
     c->allocs.clear();
     if (c->h_counters) cudaFreeHost(c->h_counters);
+    for (void* p : c->captured_uploads) cudaFreeHost(p);
+    for (cudaEvent_t ev : c->upload_done)
+        if (ev) cudaEventDestroy(ev);
     if (c->h_res_own) cudaFreeHost(c->h_res_own);
     if (c->h_jobs) cudaFreeHost(c->h_jobs);
     for (auto ev : c->pipe_events) cudaEventDestroy(ev);
@@ -1407,11 +1449,14 @@ ffbf_status ffbf_debug_scan_unpublished(ffbf_ctx* c, const uint8_t* d_text, size
     TRY(prepare_fast(c));
     const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, len, c->num_sms, false);
     c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
-    CUDA_TRY(c, ffbf::fill_fast_job(make_scan_args(c), c->d_stage1, cfg, c->h_job));
-    c->h_job->ready = c->d_gate;
-    c->h_job->ready_spins = spins;
-    CUDA_TRY(c, cudaMemcpyAsync(c->d_job, c->h_job, sizeof(ffbf::FastJob), cudaMemcpyHostToDevice, c->st));
-    CUDA_TRY(c, ffbf::launch_fast_jobs(c->g.len, cfg, c->d_job, 1, c->h_job->n_supertiles, c->h_job->stage1_nwords,
+    uint8_t* block;
+    TRY(upload_block(c, &block));
+    auto* job = reinterpret_cast<ffbf::FastJob*>(block + ffbf::kJobOffset);
+    CUDA_TRY(c, ffbf::fill_fast_job(make_scan_args(c), c->d_stage1, cfg, job));
+    job->ready = c->d_gate;
+    job->ready_spins = spins;
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_job, job, sizeof *job, cudaMemcpyHostToDevice, c->st));
+    CUDA_TRY(c, ffbf::launch_fast_jobs(c->g.len, cfg, c->d_job, 1, job->n_supertiles, job->stage1_nwords,
                                        c->d_counters + ffbf::CNT_ERROR, c->num_sms, c->st));
     CUDA_TRY(c, cudaMemcpyAsync(c->h_counters, c->d_counters, ffbf::CNT_WORDS * 4, cudaMemcpyDeviceToHost, c->st));
     TRY(sync(c));

@@ -114,7 +114,13 @@ struct ffbf_ctx {
     ffbf::FastJob* h_jobs = nullptr;  // pinned
     ffbf::FastJob* d_jobs = nullptr;
     uint32_t jobs_cap = 0;
-    ffbf::FastJob* h_job = nullptr;  // pinned staging of a plain scan's job descriptor
+    // Pinned blocks that the scans' uploads (ffbf::scan_fast) are read from when their turn comes on the stream: a ring
+    // that starts over whenever the stream has been waited for (uploads counts the blocks taken since) and whose halves
+    // are otherwise taken again behind their events; scans recorded into graphs keep blocks of their own.
+    uint8_t* h_uploads = nullptr;
+    uint32_t uploads = 0;
+    cudaEvent_t upload_done[2] = {nullptr, nullptr};
+    std::vector<void*> captured_uploads;
     uint32_t* d_gate = nullptr;      // a publication word that stays zero (ffbf_debug_scan_unpublished)
     // a host text scanned in line-aligned segments (larger than the device holds): the text, the segments
     // and every hit record (absolute offsets, in segment order), which ffbf_verify uses segment by segment

@@ -104,8 +104,8 @@ cudaError_t launch_fast_jobs(uint32_t len, const FastConfig& cfg, const FastJob*
                              uint32_t n_items, uint32_t max_s1_words, uint32_t* d_ctl, int num_sms, cudaStream_t st);
 
 // A plain scan: one job, whose descriptor lies kJobOffset bytes behind the counters. One copy zeroes the counters and
-// brings the descriptor, from pinned h_block (kJobOffset zero bytes, then room for the descriptor), which stays as it
-// is for as long as the copy may run, a replayed stream capture included.
+// brings the descriptor, from pinned h_block (kJobOffset zero bytes, then room for the descriptor). The caller leaves the
+// block as it is until the copy has run, and where the stream is being captured, for as long as the graph may be replayed.
 constexpr size_t kJobOffset = 256;
 cudaError_t scan_fast(const ScanArgs& a, const uint32_t* stage1_words, const FastConfig& cfg, int num_sms,
                       uint8_t* h_block, cudaStream_t st);
