@@ -425,6 +425,13 @@ ffbf_status setup_scan_state(ffbf_ctx* c, const uint8_t* d_text, size_t len) {
     return FFBF_OK;
 }
 
+// A scan whose kernel raised error flags has no results: some of its windows may not have been tested.
+ffbf_status scan_failed(ffbf_ctx* c, uint32_t flags) {
+    reset_scan(c);
+    return fail(c, flags & 4u ? FFBF_ETIMEOUT : FFBF_ECUDA,
+                "scan error flags 0x%x (4: a bounded wait gave up; others: self-checks)", flags);
+}
+
 cudaError_t resolve_scan_lines(ffbf_ctx* c, uint32_t nh) {
     if (scan_tiles(c) > c->tiles_cap) return cudaErrorInvalidValue;  // the summaries are of another scan
     return ffbf::resolve_lines(c->d_text, c->text_len, c->g.len, c->d_hits, nh, c->d_tiles, c->d_tiles + c->tiles_cap,
@@ -824,6 +831,7 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
             TRY(ensure_results(c, ffbf::kSmallResults));
         }
         const ffbf::ResultHead* head = reinterpret_cast<const ffbf::ResultHead*>(res);
+        if (head->error) return scan_failed(c, (uint32_t)head->error);
         if (head->done) {
             const uint64_t* a = reinterpret_cast<const uint64_t*>(res + 64);
             c->nhits = (uint32_t)head->n;
@@ -839,6 +847,7 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
     if (c->scan_pending) {
         CUDA_TRY(c, cudaMemcpyAsync(c->h_counters, c->d_counters, ffbf::CNT_WORDS * 4, cudaMemcpyDeviceToHost, c->st));
         TRY(sync(c));
+        if (c->h_counters[ffbf::CNT_ERROR]) return scan_failed(c, c->h_counters[ffbf::CNT_ERROR]);
         uint32_t nh = c->h_counters[ffbf::CNT_HITS];
         if (nh > c->hits_cap) {
             // Too many hits for the buffer: grow it and scan again. Setting feed-forward bits is
@@ -849,6 +858,7 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
             TRY(launch_scan(c));
             CUDA_TRY(c, cudaMemcpyAsync(c->h_counters, c->d_counters, ffbf::CNT_WORDS * 4, cudaMemcpyDeviceToHost, c->st));
             TRY(sync(c));
+            if (c->h_counters[ffbf::CNT_ERROR]) return scan_failed(c, c->h_counters[ffbf::CNT_ERROR]);
             nh = c->h_counters[ffbf::CNT_HITS];
         }
         c->nhits = nh;

@@ -144,6 +144,7 @@ __device__ void collect_one(const CollectJob& a, uint32_t cta) {
     if (nh > a.cap || nh > a.hits_cap) {  // the general path takes over
         if (cta == 0 && threadIdx.x == 0) {
             a.head->n = nh;
+            a.head->error = a.counters[CNT_ERROR];
             a.head->done = 0;
         }
         return;
@@ -212,6 +213,7 @@ __device__ void collect_one(const CollectJob& a, uint32_t cta) {
     if (threadIdx.x == 0) {
         a.head->n = nh;
         a.head->n_lines = n_lines;
+        a.head->error = a.counters[CNT_ERROR];
         a.head->done = open ? 0 : 1;
     }
 }

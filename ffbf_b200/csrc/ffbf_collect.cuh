@@ -7,8 +7,8 @@ namespace ffbf {
 
 constexpr uint32_t kSmallResults = 16384;  // hit windows or matches the single-launch paths order
 
-// Head of a pinned result buffer. `done` is 1 when the arrays behind it hold the whole result; `error` holds a
-// verification's error flags.
+// Head of a pinned result buffer. `done` is 1 when the arrays behind it hold the whole result; `error` holds the scan's
+// or the verification's error flags.
 struct ResultHead {
     unsigned long long n, n_lines, error, done;
 };

@@ -420,7 +420,7 @@ void launch_ready(ffbf_server* s) {
     for (uint32_t i = 0; i < n; i++) {
         auto& h = s->slot_host[batch[i]->slot];
         h.res_cap = (uint32_t)std::min<uint64_t>(ffbf::kSmallResults, std::max<uint64_t>(512, jobs[i].len / 2048));
-        reinterpret_cast<ffbf::ResultHead*>(h.res)->done = 0;
+        *reinterpret_cast<ffbf::ResultHead*>(h.res) = ffbf::ResultHead{};
         s->h_collect[i] = collect_job(plan.args[i], jobs[i].c->d_hitlines, h.res, h.res_cap, ffbf::kCollectBatch);
         for (uint32_t k = 0; k < ffbf::collect_ctas(s->h_collect[i]); k++) s->h_collect_items[n_items++] = make_uint2(i, k);
     }
@@ -580,6 +580,10 @@ void worker_loop(ffbf_server* s) {
                     }
                     auto& h = s->slot_host[r->slot];
                     const auto* head = reinterpret_cast<const ffbf::ResultHead*>(h.res);
+                    if (head->error) {
+                        finish(s, r, head->error & 4u ? FFBF_ETIMEOUT : FFBF_ECUDA);
+                        continue;
+                    }
                     if (head->done) {
                         const uint64_t* a = reinterpret_cast<const uint64_t*>(h.res + 64);
                         const size_t cap = h.res_cap;

@@ -34,7 +34,7 @@ typedef enum {
     FFBF_EINVAL = 1,          /* bad argument: geometry, NULL pointer, misaligned device pointer, bad file */
     FFBF_ENOMEM_DEVICE = 2,   /* device allocation failed or would exceed the context's HBM budget */
     FFBF_EIO = 3,             /* file open/read/write failed (the *_file entry points) */
-    FFBF_ETIMEOUT = 4,        /* a bounded device-side wait gave up (batched/served forms) */
+    FFBF_ETIMEOUT = 4,        /* a bounded device-side wait gave up */
     FFBF_ECUDA = 5,           /* a CUDA runtime call failed; ffbf_last_error has the CUDA message */
     FFBF_ESTATE = 6,          /* call out of order, e.g. ffbf_build before ffbf_set_patterns */
     FFBF_ENOMEM_HOST = 7      /* host allocation failed */
@@ -121,7 +121,8 @@ typedef struct {
 ffbf_status ffbf_scan(ffbf_ctx* ctx, const uint8_t* text, size_t len, ffbf_scan_result* out);
 
 /* The same scan over a text already in device memory (16-byte aligned), enqueued on the context's
- * stream; ffbf_scan_collect waits for it and fills `out`. */
+ * stream; ffbf_scan_collect waits for it and fills `out`. Collecting a scan whose kernel gave up a bounded
+ * wait gives FFBF_ETIMEOUT, one that failed a self-check FFBF_ECUDA; there is then no scan to collect. */
 ffbf_status ffbf_scan_device(ffbf_ctx* ctx, const uint8_t* d_text, size_t len);
 ffbf_status ffbf_scan_collect(ffbf_ctx* ctx, ffbf_scan_result* out);
 
