@@ -25,7 +25,10 @@ struct ffbf_batch {
         ffbf_ctx* c;
         const uint8_t* text;
         size_t len;
-        uint32_t tile_bytes;  // of the newline summaries that the prepared launch writes
+        uint32_t tile_bytes = 0;  // of the newline summaries that the prepared launch writes
+        std::shared_ptr<uint64_t> scan_no;  // the context's, and its value for the batch's last launch
+        uint64_t launched = 0;
+        bool current() const { return scan_no && *scan_no == launched; }
     };
     // The device buffers and configuration each job's descriptors were built from. A context that has
     // since grown its hit buffer, reloaded its filter, added patterns or been retuned makes the batch
@@ -249,7 +252,7 @@ ffbf_status ffbf_batch_add(ffbf_batch* b, ffbf_ctx* c, const uint8_t* d_text, si
     for (auto& j : b->jobs)
         if (j.c == c) return bfail(b, FFBF_EINVAL, "a context may appear only once in a batch");
     if (b->prepared) batch_release(b);
-    b->jobs.push_back({c, d_text, len, 0});
+    b->jobs.push_back({c, d_text, len});
     return FFBF_OK;
 }
 
@@ -372,6 +375,8 @@ ffbf_status ffbf_batch_launch(ffbf_batch* b) {
         j.c->text_len = j.len;
         j.c->tile_bytes = j.tile_bytes;  // a scan of the context's own since may have had another
         j.c->scan_pending = true;
+        j.scan_no = j.c->scan_no;
+        j.launched = *j.scan_no;
     }
     if (cudaGraphLaunch(b->exec, b->st) != cudaSuccess) {
         cudaGetLastError();
@@ -385,8 +390,10 @@ ffbf_status ffbf_batch_launch(ffbf_batch* b) {
 ffbf_status ffbf_batch_wait(ffbf_batch* b) {
     if (!b) return FFBF_EINVAL;
     cudaError_t e = cudaSetDevice(b->device);
-    // every job's results by one launch, and the control words, behind the graph: one wait for all of them
-    const bool collect = b->results && b->uncollected;
+    // Every job's results by one launch, and the control words, behind the graph: one wait for all of them. Where a
+    // context has been used for another scan since the launch, or is gone, each of the others is collected by itself.
+    const bool collect = b->results && b->uncollected &&
+                         std::all_of(b->jobs.begin(), b->jobs.end(), [](const auto& j) { return j.current(); });
     if (e == cudaSuccess && collect)
         e = ffbf::collect_hits_multi(b->d_collect, b->d_collect_items, b->n_collect_items, b->st);
     if (e == cudaSuccess && b->results)

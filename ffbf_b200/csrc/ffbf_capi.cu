@@ -272,6 +272,7 @@ void order_hits(const HitRec* hr, const HitLine* hl, uint32_t nh, Words& hits, W
 }
 
 void reset_scan(ffbf_ctx* c) {
+    ++*c->scan_no;
     c->have_scan = false;
     c->scan_pending = false;
     c->ready = nullptr;
@@ -596,6 +597,7 @@ void ffbf_destroy(ffbf_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->st) cudaStreamSynchronize(c->st);
+    ++*c->scan_no;
     for (auto& kv : c->allocs) cudaFree(kv.first);
     c->allocs.clear();
     if (c->h_counters) cudaFreeHost(c->h_counters);

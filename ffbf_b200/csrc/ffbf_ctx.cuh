@@ -84,6 +84,9 @@ struct ffbf_ctx {
     const uint8_t* d_text = nullptr;
     uint64_t text_len = 0;
     bool scan_pending = false, have_scan = false;
+    // Number of the context's current scan: every scan takes a new one, and so does the context's end. A batch keeps a
+    // reference, and touches a context after its launch only while the number is the one the launch gave it.
+    std::shared_ptr<uint64_t> scan_no = std::make_shared<uint64_t>(0);
     ffbf::HitRec* d_hits = nullptr;
     ffbf::HitLine* d_hitlines = nullptr;
     uint32_t hits_cap = 0;

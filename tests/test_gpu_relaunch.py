@@ -38,3 +38,34 @@ def test_plain_scans_between_launches(n_hits, nbytes, newline):
             b.launch()
             b.wait()
             assert check(f, PRM, pats, text, f.collect()) >= n_hits
+
+
+def test_wait_after_other_use_of_the_contexts():
+    """A member scanned alone after the launch keeps that scan's results over the batch's wait, and a member that is gone
+    is left alone; the others' results are the batch's."""
+    import torch
+
+    jobs = [planted(30 + n, 400_000 + n, 60 + n) for n in range(3)]
+    other = planted(25, 90_001, 60)[1]  # shorter than the job's text
+    d_other = torch.from_numpy(other).cuda()
+    texts = [torch.from_numpy(t).cuda() for _, t in jobs]
+    filters = [Filter(PRM) for _ in jobs]
+    with Batch() as b:
+        for f, (pats, text), d in zip(filters, jobs, texts):
+            f.add_patterns(pats)
+            b.add(f, d.data_ptr(), text.size)
+        for gone in (False, True):
+            for f in filters:
+                clear(f)
+            b.launch()
+            torch.cuda.synchronize()  # the launch is done, though not waited for through the batch
+            clear(filters[0])
+            filters[0].process_device(d_other.data_ptr(), other.size)
+            if gone:
+                filters[2].close()
+            b.wait()
+            check(filters[0], PRM, jobs[0][0], other, filters[0].collect())
+            for i in (1,) if gone else (1, 2):
+                check(filters[i], PRM, *jobs[i], filters[i].collect())
+    for f in filters:
+        f.close()
