@@ -375,6 +375,9 @@ ffbf_status ffbf_batch_launch(ffbf_batch* b) {
         j.c->text_len = j.len;
         j.c->tile_bytes = j.tile_bytes;  // a scan of the context's own since may have had another
         j.c->scan_pending = true;
+        j.c->segmented = false;  // nor is a host text scanned in segments the current one any more
+        j.c->segs.clear();
+        j.c->seg_hr.clear();
         j.scan_no = j.c->scan_no;
         j.launched = *j.scan_no;
     }

@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from ffbf_b200 import Batch, Filter
+from ffbf_b200 import Batch, Filter, Params
 from test_gpu_collect import PRM, check, planted
 
 pytestmark = pytest.mark.gpu
@@ -69,3 +69,23 @@ def test_wait_after_other_use_of_the_contexts():
                 check(filters[i], PRM, *jobs[i], filters[i].collect())
     for f in filters:
         f.close()
+
+
+def test_launch_after_a_segmented_scan():
+    """A host text scanned in segments on a member is forgotten by the next launch: matches are those of the job's text."""
+    import torch
+
+    prm = Params(20, 5, 2, 1 << 20, 1 << 24)
+    pats, text = planted(200, 300_000, 81)
+    long_text = planted(3000, 40 << 20, 81)[1]
+    d = torch.from_numpy(text).cuda()
+    with Filter(prm) as f, Batch() as b:
+        f.add_patterns(pats)
+        b.add(f, d.data_ptr(), text.size)
+        b.prepare()
+        f.set_hbm_budget(32 << 20)  # segments of about 18 MB
+        check(f, prm, pats, long_text, f.process(long_text))
+        clear(f)
+        b.launch()
+        b.wait()
+        check(f, prm, pats, text, f.collect())
