@@ -1198,6 +1198,7 @@ ffbf_status ffbf_prune(ffbf_ctx* c, ffbf_prune_result* out) {
             TRY(ids_room(cnt));
             CUDA_TRY(c, ffbf::prune_emit(c->d_pbits, counts, n, c->d_ids, c->ids_cap, result_head(c),
                                          result_array(c, 0), host_cap, c->st));
+            TRY(sync(c));  // it writes the pinned room again
         }
         if (cnt <= host_cap) {
             c->r_ids.assign(result_array(c, 0), result_array(c, 0) + cnt);
