@@ -10,13 +10,13 @@ pytestmark = pytest.mark.gpu
 
 
 def test_second_emission_is_waited_for():
-    pats = dg.gen_patterns(5, dg.PRINTABLE, 4_000_000, 16, 16)  # an emission of tens of microseconds
+    pats = dg.gen_patterns(5, dg.PRINTABLE, 32_000_000, 16, 16)  # an emission of some 200 microseconds
     text = pats[:17 * 1000]
     with Filter(Params(16, 5, 2, 1 << 27, 1 << 28)) as f:
         f.add_patterns(pats)
         f.process(text)
         # the smallest budget that suffices leaves less than the 16384 ids that the first buffer would hold
-        for budget in range(1 << 20, 1 << 30, 48 << 10):
+        for budget in range(1 << 30, 1 << 31, 48 << 10):
             f.set_hbm_budget(budget)
             try:
                 ids = f.filter_phrases()

@@ -76,7 +76,7 @@ def test_launch_after_a_segmented_scan():
     import torch
 
     prm = Params(20, 5, 2, 1 << 20, 1 << 24)
-    pats, text = planted(200, 300_000, 81)
+    pats, text = planted(200, 24 << 20, 81)  # longer than a segment: the scan in between replaces no buffer
     long_text = planted(3000, 40 << 20, 81)[1]
     d = torch.from_numpy(text).cuda()
     with Filter(prm) as f, Batch() as b:
