@@ -315,8 +315,8 @@ ffbf_status ffbf_batch_prepare(ffbf_batch* b) {
         b->h_ctl = reinterpret_cast<uint32_t*>(block->p + bytes);
         for (size_t i = 0; i < b->jobs.size(); i++) {
             const auto [at, cap] = b->result_at[i];
-            cj.push_back(collect_job(plan.args[i], b->jobs[i].c->d_hitlines, block->p + at, cap, ffbf::kCollectBatch));
-            for (uint32_t k = 0; k < ffbf::collect_ctas(cj.back()); k++) items.push_back(make_uint2((uint32_t)i, k));
+            cj.push_back(collect_job(plan.args[i], b->jobs[i].c->d_hitlines, block->p + at, cap, ffbf::kCollectBatch, cap));
+            for (uint32_t k = 0; k < cj.back().ctas; k++) items.push_back(make_uint2((uint32_t)i, k));
         }
         b->n_collect_items = (uint32_t)items.size();
         TRY(balloc(b, &b->d_collect, cj.size() + 1));

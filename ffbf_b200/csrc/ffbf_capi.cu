@@ -365,11 +365,13 @@ ffbf::ScanArgs make_scan_args(ffbf_ctx* c) {
     return a;
 }
 
-ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta) {
+ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta,
+                             uint32_t windows) {
     uint64_t* arrays = reinterpret_cast<uint64_t*>(res + 64);
     return ffbf::CollectJob{a.text, a.n, a.g.len, a.hits_cap, a.hits, lines, a.counters, a.tile_first_nl, a.tile_last_nl,
                             a.tile_bytes, a.ntiles, reinterpret_cast<ffbf::ResultHead*>(res), arrays, arrays + cap,
-                            arrays + 2 * (size_t)cap, cap, per_cta};
+                            arrays + 2 * (size_t)cap, cap, per_cta,
+                            std::max(1u, (std::min(cap, windows) + per_cta - 1) / per_cta)};
 }
 
 bool tunable(const ffbf_ctx* c, uint64_t n) {
@@ -825,7 +827,7 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
             res = c->h_res;
             cap = c->res_cap;
             CUDA_TRY(c, ffbf::collect_hits(collect_job(make_scan_args(c), c->d_hitlines, c->h_res, cap,
-                                                       ffbf::kCollectAlone),
+                                                       ffbf::kCollectAlone, cap),
                                            c->st));
             TRY(sync(c));
             const uint64_t n = result_head(c)->n;

@@ -149,11 +149,16 @@ __device__ void collect_one(const CollectJob& a, uint32_t cta) {
         }
         return;
     }
-    const uint32_t ctas = nh ? (nh + a.per_cta - 1) / a.per_cta : 1u;
+    const uint32_t ctas = min(a.ctas, nh ? (nh + a.per_cta - 1) / a.per_cta : 1u);
     if (cta >= ctas) return;
-    const uint32_t end = min(nh, (cta + 1) * a.per_cta);
-    // eight lanes per window; every lane of a warp takes part in every round
-    for (uint32_t i0 = cta * a.per_cta; i0 < end; i0 += kThreads / 8) {
+    // Eight lanes per window; every lane of a warp takes part in every round. A CTA's next windows follow those of all.
+    uint32_t end = min(nh, (cta + 1) * a.per_cta);
+    for (uint32_t i0 = cta * a.per_cta; i0 < nh; i0 += kThreads / 8) {
+        if (i0 >= end) {
+            i0 = end + (ctas - 1) * a.per_cta;
+            end = min(nh, i0 + a.per_cta);
+            if (i0 >= nh) break;
+        }
         const uint32_t i = i0 + threadIdx.x / 8;
         const uint64_t w = i < end ? a.hits[i].off : 0u;
         const long long found = line_end_of_window(a.text, a.n, a.len, a.tile_bytes, w, i < end);
@@ -326,12 +331,10 @@ constexpr size_t kSmem = (8 + 2 * (kBuckets / kSmallResults)) * (size_t)kSmallRe
 
 }  // namespace
 
-uint32_t collect_ctas(const CollectJob& job) { return (job.cap + job.per_cta - 1) / job.per_cta; }
-
 cudaError_t collect_hits(const CollectJob& job, cudaStream_t st) {
     cudaError_t e = cudaFuncSetAttribute(k_collect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return e;
-    k_collect<<<collect_ctas(job), kThreads, kSmem, st>>>(job);
+    k_collect<<<job.ctas, kThreads, kSmem, st>>>(job);
     note_launches(1);
     return cudaGetLastError();
 }

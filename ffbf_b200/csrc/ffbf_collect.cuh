@@ -32,7 +32,8 @@ struct CollectJob {
     uint64_t* line_start;
     uint64_t* line_end;
     uint32_t cap;
-    uint32_t per_cta;  // windows per CTA
+    uint32_t per_cta;  // windows per CTA and round
+    uint32_t ctas;     // CTAs launched for the job; more windows than they take in a round need further ones
 };
 // A scan alone on the GPU spreads its windows over the SMs; among many jobs a CTA takes more of one.
 constexpr uint32_t kCollectAlone = 128, kCollectBatch = 1024;
@@ -40,8 +41,7 @@ constexpr uint32_t kCollectAlone = 128, kCollectBatch = 1024;
 // Lines of a scan's hits, the hits in text order and their distinct lines. Leaves head->done 0 when there are more
 // hits than job.cap, or a line reaches over more than kWalkTiles tiles: resolve_lines and order_hits then do it.
 cudaError_t collect_hits(const CollectJob& job, cudaStream_t st);
-// The same for jobs in device memory: items {job, CTA}, each job's CTAs 0 .. collect_ctas(job) - 1.
-uint32_t collect_ctas(const CollectJob& job);
+// The same for jobs in device memory: items {job, CTA}, each job's CTAs 0 .. ctas - 1.
 cudaError_t collect_hits_multi(const CollectJob* d_jobs, const uint2* d_items, uint32_t n_items, cudaStream_t st);
 
 // Feed-forward prune of npat patterns: a bit per pattern in d_bits, counts per kPruneBlock patterns in d_counts, the

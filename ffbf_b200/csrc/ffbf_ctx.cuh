@@ -228,8 +228,10 @@ void order_hits(const HitRec* hr, const HitLine* hl, uint32_t nh, Words& hits, W
 // Stage-1 table and probe mode of the tuned scan for the context's filter (no-op for borrowed filters).
 ffbf_status prepare_fast(ffbf_ctx* c);
 ffbf::ScanArgs make_scan_args(ffbf_ctx* c);
-// The single-launch collection of a scan's hits into a pinned buffer of a head and three arrays of cap words.
-ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta);
+// The single-launch collection of a scan's hits into a pinned buffer of a head and three arrays of cap words, by CTAs for
+// that many windows a round (the others wait for a second one).
+ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta,
+                             uint32_t windows);
 bool use_fast(const ffbf_ctx* c, uint64_t n);
 bool tunable(const ffbf_ctx* c, uint64_t n);  // the autotuner takes this geometry and text size
 ffbf_status launch_scan(ffbf_ctx* c);  // counters reset + scan of c->d_text on the context's stream

@@ -112,8 +112,7 @@ struct ffbf_server {
     uint2* d_collect_items = nullptr;
     uint2* h_collect_items = nullptr;
     struct SlotHost {
-        uint8_t* res = nullptr;  // pinned: the collected results (a head and three arrays)
-        uint32_t res_cap = 0;    // their capacity in the running batch
+        uint8_t* res = nullptr;  // pinned: the collected results (a head and three arrays of kSmallResults words)
         HitRec* hr = nullptr;    // pinned copies of the slot's hit records and lines, for larger results
         HitLine* hl = nullptr;
         uint32_t cap = 0;
@@ -415,14 +414,17 @@ void launch_ready(ffbf_server* s) {
     up(s->d_args, s->h_args, plan.args.size() * sizeof(ffbf::ScanArgs));
     up(s->d_tail, s->h_tail, plan.tail.size() * sizeof(uint2));
     up(s->d_counters, s->h_counters, (n + n_ctl) * sizeof(uint32_t*));
-    // results: room for one hit window per 2 KiB of text, at least 512
+    // results: CTAs for one hit window per 2 KiB of text, at least 512; a denser request's windows take more rounds (a
+    // CTA that finds nothing to do still costs its launch, and the room is there in any case)
     uint32_t n_items = 0;
     for (uint32_t i = 0; i < n; i++) {
         auto& h = s->slot_host[batch[i]->slot];
-        h.res_cap = (uint32_t)std::min<uint64_t>(ffbf::kSmallResults, std::max<uint64_t>(512, jobs[i].len / 2048));
+        const uint32_t windows =
+            (uint32_t)std::min<uint64_t>(ffbf::kSmallResults, std::max<uint64_t>(512, jobs[i].len / 2048));
         *reinterpret_cast<ffbf::ResultHead*>(h.res) = ffbf::ResultHead{};
-        s->h_collect[i] = collect_job(plan.args[i], jobs[i].c->d_hitlines, h.res, h.res_cap, ffbf::kCollectBatch);
-        for (uint32_t k = 0; k < ffbf::collect_ctas(s->h_collect[i]); k++) s->h_collect_items[n_items++] = make_uint2(i, k);
+        s->h_collect[i] = collect_job(plan.args[i], jobs[i].c->d_hitlines, h.res, ffbf::kSmallResults,
+                                     ffbf::kCollectBatch, windows);
+        for (uint32_t k = 0; k < s->h_collect[i].ctas; k++) s->h_collect_items[n_items++] = make_uint2(i, k);
     }
     up(s->d_collect, s->h_collect, n * sizeof(ffbf::CollectJob));
     up(s->d_collect_items, s->h_collect_items, n_items * sizeof(uint2));
@@ -586,7 +588,7 @@ void worker_loop(ffbf_server* s) {
                     }
                     if (head->done) {
                         const uint64_t* a = reinterpret_cast<const uint64_t*>(h.res + 64);
-                        const size_t cap = h.res_cap;
+                        const size_t cap = ffbf::kSmallResults;
                         r->hits.assign(a, a + head->n);
                         r->ls.assign(a + cap, a + cap + head->n_lines);
                         r->le.assign(a + 2 * cap, a + 2 * cap + head->n_lines);
