@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <map>
 #include <memory>
 #include <new>
@@ -55,9 +56,13 @@ struct ffbf_batch {
     uint64_t graph_kernels = 0;  // kernel nodes of the graph
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    // every job's results, collected by one launch after the graph (ffbf_batch_wait)
+    // Every job's results, collected by one launch after the graph (ffbf_batch_wait): a pinned block of a head per job,
+    // words that the jobs share, and a copy of the control words. d_pool counts the words taken; a launch whose results
+    // need more than there are makes the next one start with a larger block.
     std::shared_ptr<PinnedBlock> results;
-    std::vector<std::pair<size_t, uint32_t>> result_at;  // per job: offset in the block, capacity
+    std::vector<ffbf::CollectJob> collect;
+    uint64_t pool_words = 0, want_words = 0, max_words = 0;
+    unsigned long long* d_pool = nullptr;
     ffbf::CollectJob* d_collect = nullptr;
     uint2* d_collect_items = nullptr;
     uint32_t n_collect_items = 0;
@@ -191,8 +196,8 @@ void batch_release(ffbf_batch* b) {
     for (void* p : b->allocs) cudaFree(p);
     b->allocs.clear();
     b->d_error = nullptr;
-    b->results.reset();
-    b->result_at.clear();
+    b->collect.clear();
+    b->pool_words = b->want_words = 0;  // the block itself stays for the next preparation
     b->n_collect_items = 0;
     b->uncollected = false;
     b->prepared = false;
@@ -209,6 +214,48 @@ ffbf_status balloc(ffbf_batch* b, T** p, size_t count) {
     }
     b->allocs.push_back(v);
     *p = static_cast<T*>(v);
+    return FFBF_OK;
+}
+
+// Pinning costs up to a millisecond per MiB and most jobs have few windows: the jobs share the words, 1 MiB of them at
+// first, at most 32, and the block stays for the batch's next preparation. With room for each job of its own, preparing 48
+// jobs of 64 MiB took 8.7 to 11.9 ms and 256 of 1 MiB 3.3 to 6.9; now 0.56 and 1.1 (with no such room: 0.50 and 0.95).
+constexpr uint64_t kPoolWords = 1 << 17, kMaxPoolWords = 1 << 22;
+
+// Makes the batch's pinned block with room for `words` and points the collection at it. Where they cannot be had, it keeps
+// the block there is, or makes one without words: jobs that find no room are collected one by one.
+ffbf_status make_results(ffbf_batch* b, uint64_t words) {
+    const size_t heads = 64 * b->collect.size(), ctl = 16 * ((size_t)b->n_ctl + 1);
+    auto block = b->results;
+    if (!block || block->bytes < heads + 8 * words + ctl || block.use_count() > 2) {  // 2: no context holds it
+        block = std::make_shared<PinnedBlock>();
+        block->bytes = heads + 8 * words + ctl;
+        if (cudaMallocHost(&block->p, block->bytes) != cudaSuccess) {
+            cudaGetLastError();
+            b->max_words = b->pool_words;
+            if (b->pool_words) return FFBF_OK;
+            words = 0;
+            block->bytes = heads + ctl;
+            if (cudaMallocHost(&block->p, block->bytes) != cudaSuccess) {
+                cudaGetLastError();
+                block->p = nullptr;
+                return bfail(b, FFBF_ENOMEM_HOST, "pinned batch results");
+            }
+        }
+    }
+    for (size_t i = 0; i < b->collect.size(); i++) {
+        b->collect[i].head = reinterpret_cast<ffbf::ResultHead*>(block->p + 64 * i);
+        b->collect[i].words = reinterpret_cast<uint64_t*>(block->p + heads);
+        b->collect[i].n_words = words;
+    }
+    if (!b->collect.empty() && cudaMemcpy(b->d_collect, b->collect.data(), b->collect.size() * sizeof(ffbf::CollectJob),
+                                          cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        return bfail(b, FFBF_ECUDA, "batch table upload failed");
+    }
+    b->h_ctl = reinterpret_cast<uint32_t*>(block->p + heads + 8 * words);
+    b->results = block;
+    b->pool_words = words;
     return FFBF_OK;
 }
 
@@ -278,10 +325,12 @@ ffbf_status ffbf_batch_prepare(ffbf_batch* b) {
     TRY(balloc(b, &d.fast, plan.fast.size() + 1));
     TRY(balloc(b, &d.args, plan.args.size() + 1));
     TRY(balloc(b, &d.tail, plan.tail.size() + 1));
-    TRY(balloc(b, &b->d_error, 4 * (plan.launches.size() + 1)));
+    // a group of control words per launch, and one whose first two count the results' words
+    TRY(balloc(b, &b->d_error, 4 * (plan.launches.size() + 2)));
     b->n_ctl = (uint32_t)plan.launches.size() + 1;
     d.ctl = b->d_error;
-    for (uint32_t i = 0; i < b->n_ctl; i++) counters.push_back(b->d_error + 4 * i);
+    b->d_pool = reinterpret_cast<unsigned long long*>(b->d_error + 4 * b->n_ctl);
+    for (uint32_t i = 0; i <= b->n_ctl; i++) counters.push_back(b->d_error + 4 * i);
     TRY(balloc(b, &d.counters, counters.size() + 1));
     d.n_counters = (uint32_t)counters.size();
     auto up = [](void* dst, const void* src, size_t bytes) {
@@ -291,41 +340,33 @@ ffbf_status ffbf_batch_prepare(ffbf_batch* b) {
         !up(d.args, plan.args.data(), plan.args.size() * sizeof(ffbf::ScanArgs)) ||
         !up(d.tail, plan.tail.data(), plan.tail.size() * sizeof(uint2)) ||
         !up(d.counters, counters.data(), counters.size() * sizeof(uint32_t*)) ||
-        cudaMemset(b->d_error, 0, 16 * b->n_ctl) != cudaSuccess) {
+        cudaMemset(b->d_error, 0, 16 * (b->n_ctl + 1)) != cudaSuccess) {
         cudaGetLastError();
         return bfail(b, FFBF_ECUDA, "batch table upload failed");
     }
-    // the jobs' results: room for one hit window per 8 KiB of text, at least 512; a job with more takes the plain collect
+    // the jobs' results: CTAs for one hit window per 8 KiB of text, at least 512
     {
-        std::vector<ffbf::CollectJob> cj;
         std::vector<uint2> items;
-        size_t bytes = 0;
-        for (const auto& j : b->jobs) {
-            const uint32_t cap = (uint32_t)std::min<uint64_t>(ffbf::kSmallResults, std::max<uint64_t>(512, j.len / 8192));
-            b->result_at.push_back({bytes, cap});
-            bytes += ffbf::result_bytes(cap);
-        }
-        auto block = std::make_shared<PinnedBlock>();
-        if (cudaMallocHost(&block->p, bytes + 16 * b->n_ctl) != cudaSuccess) {
-            cudaGetLastError();
-            block->p = nullptr;
-            return bfail(b, FFBF_ENOMEM_HOST, "pinned batch results");
-        }
-        b->results = block;
-        b->h_ctl = reinterpret_cast<uint32_t*>(block->p + bytes);
+        uint64_t words = 0;
         for (size_t i = 0; i < b->jobs.size(); i++) {
-            const auto [at, cap] = b->result_at[i];
-            cj.push_back(collect_job(plan.args[i], b->jobs[i].c->d_hitlines, block->p + at, cap, ffbf::kCollectBatch, cap));
-            for (uint32_t k = 0; k < cj.back().ctas; k++) items.push_back(make_uint2((uint32_t)i, k));
+            const uint32_t windows =
+                (uint32_t)std::min<uint64_t>(ffbf::kSmallResults, std::max<uint64_t>(512, b->jobs[i].len / 8192));
+            ffbf::CollectJob cj = collect_job(plan.args[i], b->jobs[i].c->d_hitlines, nullptr, ffbf::kSmallResults,
+                                              ffbf::kCollectBatch, windows);
+            cj.used = b->d_pool;
+            for (uint32_t k = 0; k < cj.ctas; k++) items.push_back(make_uint2((uint32_t)i, k));
+            b->collect.push_back(cj);
+            words += 3 * windows;
         }
         b->n_collect_items = (uint32_t)items.size();
-        TRY(balloc(b, &b->d_collect, cj.size() + 1));
+        TRY(balloc(b, &b->d_collect, b->collect.size() + 1));
         TRY(balloc(b, &b->d_collect_items, items.size() + 1));
-        if (!up(b->d_collect, cj.data(), cj.size() * sizeof(ffbf::CollectJob)) ||
-            !up(b->d_collect_items, items.data(), items.size() * sizeof(uint2))) {
+        if (!up(b->d_collect_items, items.data(), items.size() * sizeof(uint2))) {
             cudaGetLastError();
             return bfail(b, FFBF_ECUDA, "batch table upload failed");
         }
+        b->max_words = kMaxPoolWords;
+        TRY(make_results(b, std::min(words, kPoolWords)));
     }
     // one graph: zero the jobs' counters, one tuned launch per group, one generic launch for all tail tiles
     if (cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
@@ -369,6 +410,14 @@ ffbf_status ffbf_batch_launch(ffbf_batch* b) {
                 (use_fast(b->jobs[i].c, b->jobs[i].len) && b->jobs[i].c->stage1_dirty);
     if (stale) TRY(ffbf_batch_prepare(b));
     if (cudaSetDevice(b->device) != cudaSuccess) return bfail(b, FFBF_ECUDA, "cudaSetDevice failed");
+    if (b->want_words > b->pool_words) {
+        if (cudaStreamSynchronize(b->st) != cudaSuccess) {
+            cudaGetLastError();
+            return bfail(b, FFBF_ECUDA, "batch execution failed");
+        }
+        TRY(make_results(b, b->want_words));
+        b->want_words = 0;
+    }
     for (auto& j : b->jobs) {
         reset_scan(j.c);
         j.c->d_text = j.text;
@@ -395,27 +444,32 @@ ffbf_status ffbf_batch_wait(ffbf_batch* b) {
     cudaError_t e = cudaSetDevice(b->device);
     // Every job's results by one launch, and the control words, behind the graph: one wait for all of them. Where a
     // context has been used for another scan since the launch, or is gone, each of the others is collected by itself.
-    const bool collect = b->results && b->uncollected &&
+    const bool collect = b->prepared && b->uncollected &&
                          std::all_of(b->jobs.begin(), b->jobs.end(), [](const auto& j) { return j.current(); });
     if (e == cudaSuccess && collect)
         e = ffbf::collect_hits_multi(b->d_collect, b->d_collect_items, b->n_collect_items, b->st);
-    if (e == cudaSuccess && b->results)
-        e = cudaMemcpyAsync(b->h_ctl, b->d_error, 16 * b->n_ctl, cudaMemcpyDeviceToHost, b->st);
+    if (e == cudaSuccess && b->prepared)
+        e = cudaMemcpyAsync(b->h_ctl, b->d_error, 16 * (b->n_ctl + 1), cudaMemcpyDeviceToHost, b->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return bfail(b, FFBF_ECUDA, std::string("batch execution failed: ") + cudaGetErrorString(e));
     }
     uint32_t flag = 0;
-    if (b->results) {
+    if (b->prepared) {
         for (uint32_t i = 0; i < b->n_ctl; i++) flag |= b->h_ctl[4 * i];
         b->uncollected = false;
         for (size_t i = 0; i < b->jobs.size() && collect && !flag; i++) {
             ffbf_ctx* c = b->jobs[i].c;
             if (!c->scan_pending) continue;  // collected already
             c->ready_block = b->results;
-            c->ready = b->results->p + b->result_at[i].first;
-            c->ready_cap = b->result_at[i].second;
+            c->ready = b->collect[i].head;
+            c->ready_words = b->collect[i].words;
+        }
+        if (collect) {
+            unsigned long long used;
+            memcpy(&used, b->h_ctl + 4 * b->n_ctl, 8);
+            if (used > b->pool_words) b->want_words = std::min<uint64_t>(used + used / 4, b->max_words);
         }
     }
     if (flag) {

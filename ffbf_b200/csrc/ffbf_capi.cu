@@ -367,11 +367,17 @@ ffbf::ScanArgs make_scan_args(ffbf_ctx* c) {
 
 ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta,
                              uint32_t windows) {
-    uint64_t* arrays = reinterpret_cast<uint64_t*>(res + 64);
     return ffbf::CollectJob{a.text, a.n, a.g.len, a.hits_cap, a.hits, lines, a.counters, a.tile_first_nl, a.tile_last_nl,
-                            a.tile_bytes, a.ntiles, reinterpret_cast<ffbf::ResultHead*>(res), arrays, arrays + cap,
-                            arrays + 2 * (size_t)cap, cap, per_cta,
+                            a.tile_bytes, a.ntiles, reinterpret_cast<ffbf::ResultHead*>(res),
+                            reinterpret_cast<uint64_t*>(res + 64), 3ull * cap, nullptr, cap, per_cta,
                             std::max(1u, (std::min(cap, windows) + per_cta - 1) / per_cta)};
+}
+
+void take_results(const ffbf::ResultHead* head, const uint64_t* words, Words& hits, Words& ls, Words& le) {
+    const uint64_t* a = words + head->at;
+    hits.assign(a, a + head->n);
+    ls.assign(a + head->n, a + head->n + head->n_lines);
+    le.assign(a + 2 * head->n, a + 2 * head->n + head->n_lines);
 }
 
 bool tunable(const ffbf_ctx* c, uint64_t n) {
@@ -821,27 +827,24 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
     if (c->scan_pending && !c->host_order && !c->keep_records) {
         // one launch finishes a result of up to kSmallResults windows, unless the scan's batch has done it already;
         // the general path below takes the others
-        const uint8_t* res = c->ready;
-        uint32_t cap = c->ready_cap;
-        for (int attempt = 0; !c->ready && attempt < 2; attempt++) {
-            res = c->h_res;
-            cap = c->res_cap;
+        const ffbf::ResultHead* head = c->ready;
+        const uint64_t* words = c->ready_words;
+        const bool collected = head && (head->done || head->error || head->n > ffbf::kSmallResults);
+        for (int attempt = 0; !collected && attempt < 2; attempt++) {
+            const uint32_t cap = c->res_cap;
+            head = result_head(c);
+            words = result_array(c, 0);
             CUDA_TRY(c, ffbf::collect_hits(collect_job(make_scan_args(c), c->d_hitlines, c->h_res, cap,
                                                        ffbf::kCollectAlone, cap),
                                            c->st));
             TRY(sync(c));
-            const uint64_t n = result_head(c)->n;
-            if (n <= cap || n > ffbf::kSmallResults || n > c->hits_cap) break;
+            if (head->n <= cap || head->n > ffbf::kSmallResults || head->n > c->hits_cap) break;
             TRY(ensure_results(c, ffbf::kSmallResults));
         }
-        const ffbf::ResultHead* head = reinterpret_cast<const ffbf::ResultHead*>(res);
         if (head->error) return scan_failed(c, (uint32_t)head->error);
         if (head->done) {
-            const uint64_t* a = reinterpret_cast<const uint64_t*>(res + 64);
             c->nhits = (uint32_t)head->n;
-            c->r_hits.assign(a, a + head->n);
-            c->r_ls.assign(a + cap, a + cap + head->n_lines);
-            c->r_le.assign(a + 2 * (size_t)cap, a + 2 * (size_t)cap + head->n_lines);
+            take_results(head, words, c->r_hits, c->r_ls, c->r_le);
             c->ready = nullptr;
             c->ready_block.reset();
             c->scan_pending = false;

@@ -140,6 +140,7 @@ __device__ void sort_records(uint32_t n, uint64_t span, uint64_t* s_key, uint16_
 __device__ void collect_one(const CollectJob& a, uint32_t cta) {
     extern __shared__ uint64_t s_key[];
     __shared__ uint32_t s_warp[32], s_flag;
+    __shared__ unsigned long long s_at;
     const uint32_t nh = a.counters[CNT_HITS];
     if (nh > a.cap || nh > a.hits_cap) {  // the general path takes over
         if (cta == 0 && threadIdx.x == 0) {
@@ -191,6 +192,19 @@ __device__ void collect_one(const CollectJob& a, uint32_t cta) {
     for (uint32_t q = threadIdx.x; q < nh; q += kThreads)
         open |= __ldcg(&a.lines[q].start) == ~0ull || __ldcg(&a.lines[q].end) == ~0ull;
     open = (uint32_t)__syncthreads_or((int)open);
+    if (!open) {
+        if (threadIdx.x == 0) s_at = a.used ? atomicAdd(a.used, 3ull * nh) : 0ull;
+        __syncthreads();
+    }
+    if (open || s_at + 3ull * nh > a.n_words) {
+        if (threadIdx.x == 0) {
+            a.head->n = nh;
+            a.head->error = a.counters[CNT_ERROR];
+            a.head->done = 0;
+        }
+        return;
+    }
+    uint64_t *const off = a.words + s_at, *const line_start = off + nh, *const line_end = line_start + nh;
     sort_records(
         nh, a.n, s_key, reinterpret_cast<uint16_t*>(s_key + kSmallResults), s_warp,
         [&](uint32_t q) { return a.hits[q].off; }, [](uint64_t x, uint64_t y) { return x < y; });
@@ -205,13 +219,13 @@ __device__ void collect_one(const CollectJob& a, uint32_t cta) {
             ls = __ldcg(&a.lines[idx].start);
             le = __ldcg(&a.lines[idx].end);
             flag = q == 0 || __ldcg(&a.lines[(uint32_t)s_key[q - 1] & (kSmallResults - 1)].start) != ls;
-            a.off[q] = s_key[q] >> kIndexBits;
+            off[q] = s_key[q] >> kIndexBits;
         }
         uint32_t total;
         const uint32_t at = n_lines + block_sum(flag, s_warp, &total);
         if (flag) {
-            a.line_start[at] = ls;
-            a.line_end[at] = le;
+            line_start[at] = ls;
+            line_end[at] = le;
         }
         n_lines += total;
     }
@@ -219,7 +233,8 @@ __device__ void collect_one(const CollectJob& a, uint32_t cta) {
         a.head->n = nh;
         a.head->n_lines = n_lines;
         a.head->error = a.counters[CNT_ERROR];
-        a.head->done = open ? 0 : 1;
+        a.head->at = s_at;
+        a.head->done = 1;
     }
 }
 

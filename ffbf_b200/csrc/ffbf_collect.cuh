@@ -11,6 +11,7 @@ constexpr uint32_t kSmallResults = 16384;  // hit windows or matches the single-
 // or the verification's error flags.
 struct ResultHead {
     unsigned long long n, n_lines, error, done;
+    unsigned long long at;  // where the arrays start in the job's words: n window starts, n line starts, n line ends
 };
 constexpr size_t result_bytes(uint32_t cap) { return 64 + 3 * 8 * (size_t)cap; }  // a head and three arrays
 
@@ -28,10 +29,10 @@ struct CollectJob {
     uint32_t tile_bytes;
     uint64_t ntiles;
     ResultHead* head;  // pinned
-    uint64_t* off;     // pinned: cap window starts, then line starts, then line ends
-    uint64_t* line_start;
-    uint64_t* line_end;
-    uint32_t cap;
+    uint64_t* words;   // pinned: the arrays (ResultHead::at)
+    uint64_t n_words;  // room there: three per window
+    unsigned long long* used;  // words taken so far where several jobs share them (zero at first); null: all are this job's
+    uint32_t cap;              // most windows
     uint32_t per_cta;  // windows per CTA and round
     uint32_t ctas;     // CTAs launched for the job; more windows than they take in a round need further ones
 };
@@ -39,7 +40,8 @@ struct CollectJob {
 constexpr uint32_t kCollectAlone = 128, kCollectBatch = 1024;
 
 // Lines of a scan's hits, the hits in text order and their distinct lines. Leaves head->done 0 when there are more
-// hits than job.cap, or a line reaches over more than kWalkTiles tiles: resolve_lines and order_hits then do it.
+// hits than job.cap or than shared room is left for, or a line reaches over more than kWalkTiles tiles: resolve_lines and
+// order_hits then do it.
 cudaError_t collect_hits(const CollectJob& job, cudaStream_t st);
 // The same for jobs in device memory: items {job, CTA}, each job's CTAs 0 .. ctas - 1.
 cudaError_t collect_hits_multi(const CollectJob* d_jobs, const uint2* d_items, uint32_t n_items, cudaStream_t st);

@@ -29,6 +29,7 @@ struct NvtxRange {
 // Pinned host memory, shared by a batch and the contexts whose results it holds.
 struct PinnedBlock {
     uint8_t* p = nullptr;
+    size_t bytes = 0;
     ~PinnedBlock() {
         if (p) cudaFreeHost(p);
     }
@@ -157,10 +158,10 @@ struct ffbf_ctx {
     // in a block of their own
     uint8_t *h_res = nullptr, *h_res_own = nullptr;
     uint32_t res_cap = 0;
-    // the pending scan's results where a batch has collected them already (head, then three arrays of ready_cap words)
+    // the pending scan's results where a batch has collected them already: their head, and the words it points into
     std::shared_ptr<PinnedBlock> ready_block;
-    const uint8_t* ready = nullptr;
-    uint32_t ready_cap = 0;
+    const ffbf::ResultHead* ready = nullptr;
+    const uint64_t* ready_words = nullptr;
 
     // scratch for ordered compaction / codec
     uint64_t* d_tmp = nullptr;
@@ -228,8 +229,8 @@ void order_hits(const HitRec* hr, const HitLine* hl, uint32_t nh, Words& hits, W
 // Stage-1 table and probe mode of the tuned scan for the context's filter (no-op for borrowed filters).
 ffbf_status prepare_fast(ffbf_ctx* c);
 ffbf::ScanArgs make_scan_args(ffbf_ctx* c);
-// The single-launch collection of a scan's hits into a pinned buffer of a head and three arrays of cap words, by CTAs for
-// that many windows a round (the others wait for a second one).
+// The single-launch collection of a scan's hits into a pinned buffer of a head and room for cap windows, by CTAs for that
+// many windows a round (the others wait for a second one).
 ffbf::CollectJob collect_job(const ffbf::ScanArgs& a, HitLine* lines, uint8_t* res, uint32_t cap, uint32_t per_cta,
                              uint32_t windows);
 bool use_fast(const ffbf_ctx* c, uint64_t n);
@@ -237,6 +238,8 @@ bool tunable(const ffbf_ctx* c, uint64_t n);  // the autotuner takes this geomet
 ffbf_status launch_scan(ffbf_ctx* c);  // counters reset + scan of c->d_text on the context's stream
 // Tile summaries a scan of len bytes may need, and those of the context's current scan.
 uint64_t tiles_for(uint64_t len);
+// Takes a collected scan's results from a head that says done and its words.
+void take_results(const ffbf::ResultHead* head, const uint64_t* words, Words& hits, Words& ls, Words& le);
 inline uint64_t scan_tiles(const ffbf_ctx* c) { return (c->text_len + c->tile_bytes - 1) / c->tile_bytes; }
 // Line spans of the first nh hits of the context's current scan, from its tile summaries, enqueued on its stream.
 cudaError_t resolve_scan_lines(ffbf_ctx* c, uint32_t nh);

@@ -112,7 +112,7 @@ struct ffbf_server {
     uint2* d_collect_items = nullptr;
     uint2* h_collect_items = nullptr;
     struct SlotHost {
-        uint8_t* res = nullptr;  // pinned: the collected results (a head and three arrays of kSmallResults words)
+        uint8_t* res = nullptr;  // pinned: the collected results (a head and room for kSmallResults windows)
         HitRec* hr = nullptr;    // pinned copies of the slot's hit records and lines, for larger results
         HitLine* hl = nullptr;
         uint32_t cap = 0;
@@ -587,11 +587,7 @@ void worker_loop(ffbf_server* s) {
                         continue;
                     }
                     if (head->done) {
-                        const uint64_t* a = reinterpret_cast<const uint64_t*>(h.res + 64);
-                        const size_t cap = ffbf::kSmallResults;
-                        r->hits.assign(a, a + head->n);
-                        r->ls.assign(a + cap, a + cap + head->n_lines);
-                        r->le.assign(a + 2 * cap, a + 2 * cap + head->n_lines);
+                        take_results(head, reinterpret_cast<const uint64_t*>(h.res + 64), r->hits, r->ls, r->le);
                         finish(s, r, FFBF_OK);
                         continue;
                     }

@@ -89,3 +89,31 @@ def test_launch_after_a_segmented_scan():
         b.launch()
         b.wait()
         check(f, prm, pats, text, f.collect())
+
+
+def test_results_over_the_shared_room():
+    """A batch's jobs share their result room, which follows what a launch needed: jobs that found none are collected by
+    themselves, and the next launch has room for all but those with more than 16384 windows."""
+    import torch
+    from ffbf_b200 import kernel_launches
+
+    jobs = [planted(n, 600_000 + n, 90) for n in (0, 16384, 100, 9000, 511)] + [planted(16390, 600_000, 90)]
+    filters = [Filter(PRM) for _ in jobs]
+    texts = [torch.from_numpy(t).cuda() for _, t in jobs]
+    with Batch() as b:
+        for f, (pats, text), d in zip(filters, jobs, texts):
+            f.add_patterns(pats)
+            b.add(f, d.data_ptr(), text.size)
+        for launch in range(3):
+            for f in filters:
+                clear(f)
+            b.launch()
+            b.wait()
+            before = kernel_launches()
+            results = [f.collect() for f in filters[:-1]]
+            assert (kernel_launches() - before > 0) == (launch == 0)
+            results.append(filters[-1].collect())
+            for f, (pats, text), r in zip(filters, jobs, results):
+                check(f, PRM, pats, text, r)
+    for f in filters:
+        f.close()
