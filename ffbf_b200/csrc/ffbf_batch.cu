@@ -529,8 +529,9 @@ ffbf_status ffbf_batch_autotune(ffbf_batch* b, size_t sample_bytes, uint32_t* n_
 namespace {
 
 // Times the tuned scan's configurations on a sample and keeps the best. per_sm scores by SM-seconds per
-// byte (time x SMs the launch occupies): in a batch many jobs share the GPU, so a configuration whose
-// items fill fewer SMs on a small sample must not win by wall time alone. Otherwise by wall time.
+// byte (time x SMs the launch occupies), each trial with the CTA size and rows that a batch would give such a text: in a
+// batch many jobs share the GPU, so a configuration whose items fill fewer SMs on a small sample must not win by wall time
+// alone. Otherwise by wall time.
 ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len, bool per_sm, int* threads,
                           int* mode) {
     TRY(enter(c));
@@ -540,8 +541,9 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
     uint32_t* saved = nullptr;
     TRY(dalloc_t(c, &saved, c->filter_bytes / 4));
     CUDA_TRY(c, cudaMemcpyAsync(saved, c->d_ff, c->filter_bytes, cudaMemcpyDeviceToDevice, c->st));
-    // shared-memory mode at four CTA sizes (smaller ones have larger tables), dense mode at three (its probe
-    // order follows the filter's fills; 192 runs two CTAs per SM, and probe orders 2 and 3 run 192 as 384)
+    // the sparse kernel in mode 3 (whose CTA size launch_config picks and whose table may have 16-bit entries) and at three
+    // fixed sizes, the dense one at three (its probe order follows the filter's fills; 192 runs two CTAs per SM, and
+    // probe orders 2 and 3 run 192 as 384)
     const ffbf::FastConfig cands[] = {{512, 3, 0, 0}, {384, 0, 0, 0}, {256, 0, 0, 0}, {192, 2, 0, 0},
                                       {384, 1, 0, 0}, {192, 1, 0, 0}, {256, 1, 0, 0}};
     ffbf::FastConfig best = c->cfg;
@@ -551,6 +553,7 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
     cudaEventCreate(&e1);
     const int saved_force = c->force_mode;
     c->force_mode = -1;
+    c->as_batch = per_sm;
     ffbf_status s = FFBF_OK;
     for (const auto& cand : cands) {
         c->cfg = cand;
@@ -569,7 +572,7 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
         if (s != FFBF_OK) break;
         double score = ms;
         if (per_sm) {
-            const ffbf::FastConfig run = ffbf::launch_config(cand, c->g.len, sample_len, c->num_sms, false);
+            const ffbf::FastConfig run = ffbf::launch_config(cand, c->g.len, sample_len, c->num_sms, per_sm);
             const int t = ffbf::config_threads(run);
             const uint64_t streams = sample_len / ((uint64_t)run.rows * 128);
             const uint64_t items = (streams + t - 1) / t;
@@ -581,6 +584,7 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
         }
     }
     c->force_mode = saved_force;
+    c->as_batch = false;
     c->cfg = best;
     c->cfg_tuned = true;
     reset_scan(c);

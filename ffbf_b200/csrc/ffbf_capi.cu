@@ -391,7 +391,7 @@ ffbf_status launch_scan(ffbf_ctx* c) {
     if (n && use_fast(c, n)) {
         c->scan_path = 1;
         TRY(prepare_fast(c));
-        const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, n, c->num_sms, false);
+        const ffbf::FastConfig cfg = ffbf::launch_config(c->cfg, c->g.len, n, c->num_sms, c->as_batch);
         c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
         uint8_t* block;
         TRY(upload_block(c, &block));

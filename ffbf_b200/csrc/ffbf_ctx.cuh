@@ -104,6 +104,7 @@ struct ffbf_ctx {
     double stage1_fill = 0;
     ffbf::FastConfig cfg{512, 0, 0, 0};  // tuned-scan configuration (mode from the stage-1 fill, or the autotuner)
     bool cfg_tuned = false;
+    bool as_batch = false;         // trial scans run as a batch would run them (ffbf_batch_autotune)
     int threads_env = 0;           // FFBF_SCAN_THREADS=256|384|512 in the environment
     int force_mode = -1;           // FFBF_SCAN_MODE=0|1 in the environment
     int force_order = -1;          // FFBF_SCAN_ORDER=0|1|2 in the environment (dense-mode probe order)
