@@ -1257,7 +1257,7 @@ cudaError_t fill_fast_job(const ScanArgs& a, const uint32_t* stage1_words, const
     const int threads = config_threads(cfg);
     const uint32_t rows = cfg.rows;
     const uint64_t slen = (uint64_t)rows * kRowBytes;
-    const uint64_t n_streams = a.n / slen;
+    const uint64_t n_streams = rows ? a.n / slen : 0;
     if (n_streams == 0 || a.tile_bytes != fast_tile_bytes(rows)) return cudaErrorInvalidValue;
     memset(job, 0, sizeof *job);
     job->n_streams = n_streams;

@@ -41,7 +41,7 @@ struct alignas(64) FastJob {
     const uint32_t* ready;
 };
 
-// How a job is scanned: CTA size, probe mode, rows per stream (0: chosen from the text size), and in the dense mode
+// How a job is scanned: CTA size, probe mode, rows per stream (which launch_config sets; 0 before), and in the dense mode
 // the probe order. Modes 0, 2 and 3 are the sparse kernel (shared-memory stage 1) at 256/384/512, 192/256/384 and 512
 // threads, the last from 192 to 512 as each text's size asks (launch_config); mode 1 is the dense one (pipelined L2 probes). Orders:
 // 0: the pipelined probes are index functions f0 = h1 and f1 = h2; 1: f2 = rot16(h1) and f3 = rot16(h2), the better
