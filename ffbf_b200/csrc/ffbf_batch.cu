@@ -38,13 +38,11 @@ struct ffbf_batch {
         const void *main, *ff, *hits, *counters, *tiles, *stage1;
         uint32_t hits_cap;
         uint64_t tiles_cap;
-        int threads, mode;
-        uint32_t rows;
-        int order;
+        int threads, mode, order;
         bool operator==(const Key& o) const {
             return main == o.main && ff == o.ff && hits == o.hits && counters == o.counters && tiles == o.tiles &&
                    stage1 == o.stage1 && hits_cap == o.hits_cap && tiles_cap == o.tiles_cap && threads == o.threads &&
-                   mode == o.mode && rows == o.rows && order == o.order;
+                   mode == o.mode && order == o.order;
         }
     };
     std::vector<Key> keys;
@@ -96,7 +94,6 @@ ffbf_status build_plan(const std::vector<PlanJob>& jobs, int num_sms, ScanPlan& 
             c->tile_bytes = ffbf::fast_tile_bytes(cfg.rows);
             const ffbf::ScanArgs a = make_scan_args(c);
             plan.args.push_back(a);
-            const int threads = ffbf::config_threads(cfg);
             ffbf::FastJob fj;
             if (ffbf::fill_fast_job(a, c->d_stage1, cfg, &fj) != cudaSuccess)
                 return fail(c, FFBF_ECUDA, "tensor map encoding failed");
@@ -176,7 +173,7 @@ ffbf_status autotune_impl(ffbf_ctx* c, const uint8_t* d_text, size_t sample_len,
 ffbf_batch::Key batch_key(const ffbf_ctx* c) {
     return ffbf_batch::Key{c->d_main, c->d_ff,          c->d_hits,      c->d_counters, c->d_tiles,
                            c->d_stage1, c->hits_cap,    c->tiles_cap,   c->cfg.threads, c->cfg.mode,
-                           c->cfg.rows, c->cfg.order};
+                           c->cfg.order};
 }
 
 ffbf_status bfail(ffbf_batch* b, ffbf_status s, const std::string& msg) {

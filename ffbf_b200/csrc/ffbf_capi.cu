@@ -360,7 +360,6 @@ ffbf::ScanArgs make_scan_args(ffbf_ctx* c) {
     a.tile_last_nl = c->d_tiles + c->tiles_cap;
     a.tile_bytes = c->tile_bytes;
     a.ntiles = scan_tiles(c);
-    a.tile_begin = 0;
     a.cache_in_smem = c->g.cache_bits <= ffbf::kSmemCacheMaxBits;
     return a;
 }
@@ -1010,14 +1009,6 @@ ffbf_status scan_host_pipelined(ffbf_ctx* c, const uint8_t* text, size_t len) {
     }
     return FFBF_OK;
 }
-
-}  // namespace
-
-extern "C" {
-
-}  // extern "C"
-
-namespace {
 
 // One host text that fits the device: copied (overlapped with the scan when large) and scanned.
 ffbf_status scan_one(ffbf_ctx* c, const uint8_t* text, size_t len, ffbf_scan_result* out) {

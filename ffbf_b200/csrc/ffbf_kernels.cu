@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_generic(ScanArgs a) {
     if (a.cache_in_smem)
         for (uint32_t w = tid; w < a.g.cache_bits / 32; w += kScanThreads) s_cache[w] = a.main_words[w];
     const uint32_t* cache_words = a.cache_in_smem ? s_cache : a.main_words;
-    for (uint64_t tile = a.tile_begin + blockIdx.x; tile < a.ntiles; tile += gridDim.x)
+    for (uint64_t tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
         generic_tile(a, tile, s_sbox, s_nl, s_text, cache_words);
 }
 
@@ -364,7 +364,7 @@ cudaError_t scan_generic(const ScanArgs& a, int grid, cudaStream_t st) {
     size_t smem = scan_smem_bytes(a.cache_in_smem, a.g);
     cudaError_t e = cudaFuncSetAttribute(k_scan_generic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    if (a.ntiles <= a.tile_begin) return cudaSuccess;
+    if (!a.ntiles) return cudaSuccess;
     k_scan_generic<<<grid, kScanThreads, smem, st>>>(a);
     note_launches(1);
     return cudaGetLastError();

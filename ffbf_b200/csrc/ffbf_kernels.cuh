@@ -52,7 +52,6 @@ struct ScanArgs {
     long long* tile_last_nl;
     uint32_t tile_bytes;  // kScanTile for the generic scan
     uint64_t ntiles;
-    uint64_t tile_begin;  // first tile this launch handles (tiles before it belong to another kernel)
     int cache_in_smem;
 };
 

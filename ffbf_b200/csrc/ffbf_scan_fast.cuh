@@ -92,7 +92,8 @@ cudaError_t build_stage1(const uint32_t* main_words, const Geom& g, int threads,
 // CTAs of the tuned kernel resident per SM for a configuration (two for the 192-thread dense kernel).
 int fast_ctas_per_sm(const FastConfig& cfg);
 
-// Rows per stream for a text of n bytes: a power of two, from 4 to 16, alone on the GPU or in a batch.
+// Rows per stream for a text of n bytes: a power of two, from 4 to 16, in a batch, or alone on the GPU where only those
+// are compared (launch_config takes every row count and CTA size for a lone text).
 uint32_t fast_rows(uint64_t n, const FastConfig& cfg, int num_sms, bool batch);
 
 // Fills *job (host memory) for a.text, whose a.tile_bytes is fast_tile_bytes(cfg.rows); the caller sets item_begin.

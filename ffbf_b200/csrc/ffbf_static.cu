@@ -110,7 +110,6 @@ extern "C" ffbf_status ffbf_scan_static(const ffbf_params* p, const uint32_t* d_
     a.tile_last_nl = tiles + kMaxTiles;
     a.tile_bytes = ffbf::kScanTile;
     a.ntiles = ntiles;
-    a.tile_begin = 0;
     a.cache_in_smem = p->cache_bits <= ffbf::kSmemCacheMaxBits;
     if (ntiles) {
         const int grid = ffbf::scan_generic_grid(a.g, a.cache_in_smem, ntiles);
