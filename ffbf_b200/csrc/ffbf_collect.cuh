@@ -46,9 +46,11 @@ cudaError_t collect_hits(const CollectJob& job, cudaStream_t st);
 // The same for jobs in device memory: items {job, CTA}, each job's CTAs 0 .. ctas - 1.
 cudaError_t collect_hits_multi(const CollectJob* d_jobs, const uint2* d_items, uint32_t n_items, cudaStream_t st);
 
-// Feed-forward prune of npat patterns: a bit per pattern in d_bits, counts per kPruneBlock patterns in d_counts, the
-// ascending ids in d_ids (the first ids_cap) and in host_ids (the first host_cap), their number in head->n.
+// Feed-forward prune of npat patterns: a bit per pattern in d_bits, counts per kPruneBlock patterns in d_counts (beyond
+// kPrefixBlocks of them the sums of the counts before), the ascending ids in d_ids (the first ids_cap) and in host_ids
+// (the first host_cap), their number in head->n.
 constexpr uint32_t kPruneBlock = 1024;
+constexpr uint64_t kPrefixBlocks = 8192;
 inline uint64_t prune_blocks(uint64_t npat) { return (npat + kPruneBlock - 1) / kPruneBlock; }
 cudaError_t prune_count(const uint64_t* d_start, const uint64_t* d_end, const uint64_t* d_hash, uint64_t npat,
                         const Geom& g, const uint32_t* d_ff, uint32_t* d_bits, uint32_t* d_counts, cudaStream_t st);
