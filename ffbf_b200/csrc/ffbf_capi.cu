@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <charconv>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -668,6 +669,7 @@ ffbf_status set_patterns(ffbf_ctx* c, const uint8_t* file, size_t len, int set_b
     c->d_pend = c->d_phash = nullptr;
     c->npat = 0;
     c->pat_len = len;
+    c->h_pat = {};
     TRY(dalloc_t(c, &c->d_pat, len + 16));
     if (len) CUDA_TRY(c, cudaMemcpyAsync(c->d_pat, file, len, cudaMemcpyHostToDevice, c->st));
     const uint64_t nb = ffbf::compact_blocks(len);
@@ -1219,46 +1221,42 @@ ffbf_status ffbf_prune(ffbf_ctx* c, ffbf_prune_result* out) {
 
 namespace {
 
-// The pruned lines' (start, end) pairs and their bytes, line i at bytes[at[i]]. Gathered on the device; where its memory
-// is short, the whole pattern file and line table come back instead.
-ffbf_status fetch_pruned(ffbf_ctx* c, std::vector<uint64_t>& spans, std::vector<uint8_t>& bytes,
-                         std::vector<uint64_t>& at) {
+// The pattern file on the host: brought back by the first call that needs it, kept until the patterns change.
+ffbf_status host_patterns(ffbf_ctx* c) {
+    if (c->h_pat.size() == c->pat_len) return FFBF_OK;
+    c->h_pat.resize(c->pat_len);
+    const cudaError_t e =
+        cudaMemcpyAsync(c->h_pat.data(), c->d_pat, c->pat_len, cudaMemcpyDeviceToHost, c->st);
+    const ffbf_status s = e == cudaSuccess ? sync(c) : fail(c, FFBF_ECUDA, "pattern file read failed: %s", cudaGetErrorString(e));
+    if (s != FFBF_OK) c->h_pat.clear();
+    return s;
+}
+
+// The pruned lines' (start, end) pairs and their bytes, line i at bytes[at[i]], gathered on the device. False where its
+// memory is short or the lines make up half the file.
+ffbf_status gather_pruned(ffbf_ctx* c, std::vector<uint64_t>& spans, std::vector<uint8_t>& bytes,
+                          std::vector<uint64_t>& at, bool* gathered) {
     const uint64_t cnt = c->r_ids.size();
-    bool gather = ensure_order(c, 16 * cnt) == FFBF_OK;
-    if (gather) {
+    *gathered = ensure_order(c, 16 * cnt) == FFBF_OK;
+    if (*gathered) {
         uint64_t* d_spans = reinterpret_cast<uint64_t*>(c->d_order);
         CUDA_TRY(c, ffbf::gather_spans(c->d_ids, cnt, c->d_pstart, c->d_pend, d_spans, c->st));
         CUDA_TRY(c, cudaMemcpyAsync(spans.data(), d_spans, 16 * cnt, cudaMemcpyDeviceToHost, c->st));
         TRY(sync(c));
-    } else {
-        std::vector<uint64_t> start(c->npat), end(c->npat);
-        CUDA_TRY(c, cudaMemcpyAsync(start.data(), c->d_pstart, 8 * c->npat, cudaMemcpyDeviceToHost, c->st));
-        CUDA_TRY(c, cudaMemcpyAsync(end.data(), c->d_pend, 8 * c->npat, cudaMemcpyDeviceToHost, c->st));
-        TRY(sync(c));
-        for (uint64_t i = 0; i < cnt; i++) {
-            spans[2 * i] = start[c->r_ids[i]];
-            spans[2 * i + 1] = end[c->r_ids[i]];
-        }
+        for (uint64_t i = 0; i < cnt; i++) at[i + 1] = at[i] + spans[2 * i + 1] - spans[2 * i];
+        // spans, places and bytes share the scratch
+        *gathered = 2 * at[cnt] < c->pat_len && ensure_order(c, 24 * cnt + at[cnt]) == FFBF_OK;
     }
-    for (uint64_t i = 0; i < cnt; i++) at[i + 1] = at[i] + spans[2 * i + 1] - spans[2 * i];
-    // spans, places and bytes share the scratch
-    const size_t total = at[cnt];
-    gather = gather && 2 * total < c->pat_len && ensure_order(c, 24 * cnt + total) == FFBF_OK;
     c->err.clear();
-    if (gather) {
-        uint64_t* d_spans = reinterpret_cast<uint64_t*>(c->d_order);
-        uint64_t* d_at = d_spans + 2 * cnt;
-        uint8_t* d_bytes = reinterpret_cast<uint8_t*>(d_at + cnt);
-        bytes.resize(total);
-        CUDA_TRY(c, cudaMemcpyAsync(d_spans, spans.data(), 16 * cnt, cudaMemcpyHostToDevice, c->st));
-        CUDA_TRY(c, cudaMemcpyAsync(d_at, at.data(), 8 * cnt, cudaMemcpyHostToDevice, c->st));
-        CUDA_TRY(c, ffbf::gather_lines(c->d_pat, d_spans, d_at, cnt, d_bytes, c->st));
-        CUDA_TRY(c, cudaMemcpyAsync(bytes.data(), d_bytes, total, cudaMemcpyDeviceToHost, c->st));
-    } else {
-        bytes.resize(c->pat_len);
-        CUDA_TRY(c, cudaMemcpyAsync(bytes.data(), c->d_pat, c->pat_len, cudaMemcpyDeviceToHost, c->st));
-        for (uint64_t i = 0; i < cnt; i++) at[i] = spans[2 * i];
-    }
+    if (!*gathered) return FFBF_OK;
+    uint64_t* d_spans = reinterpret_cast<uint64_t*>(c->d_order);
+    uint64_t* d_at = d_spans + 2 * cnt;
+    uint8_t* d_bytes = reinterpret_cast<uint8_t*>(d_at + cnt);
+    bytes.resize(at[cnt]);
+    CUDA_TRY(c, cudaMemcpyAsync(d_spans, spans.data(), 16 * cnt, cudaMemcpyHostToDevice, c->st));
+    CUDA_TRY(c, cudaMemcpyAsync(d_at, at.data(), 8 * cnt, cudaMemcpyHostToDevice, c->st));
+    CUDA_TRY(c, ffbf::gather_lines(c->d_pat, d_spans, d_at, cnt, d_bytes, c->st));
+    CUDA_TRY(c, cudaMemcpyAsync(bytes.data(), d_bytes, bytes.size(), cudaMemcpyDeviceToHost, c->st));
     return sync(c);
 }
 
@@ -1275,20 +1273,42 @@ ffbf_status ffbf_format_pruned(ffbf_ctx* c, size_t chunk, uint8_t** out, size_t*
     TRY(enter(c));
     std::vector<uint8_t> o, ix;
     try {
-        // the surviving lines' spans and bytes come back from the device copy of the pattern file
+        // A few lines of a large file come back by themselves. For a small file, or many lines, the whole file does, once:
+        // 1M lines of 1M took 182 ms with their spans and places, 125 by a walk over the file.
         const uint64_t cnt = c->r_ids.size();
-        std::vector<uint64_t> spans(2 * cnt);
-        std::vector<uint8_t> bytes;
-        std::vector<uint64_t> at(cnt + 1, 0);
-        if (cnt) TRY(fetch_pruned(c, spans, bytes, at));
         char num[32];
-        for (uint64_t i = 0; i < cnt; i++) {
-            // format_line addresses the line by its place in the file
-            const uint64_t s = spans[2 * i], e = spans[2 * i + 1];
-            const uint8_t* file = reinterpret_cast<const uint8_t*>((uintptr_t)bytes.data() + at[i] - s);
+        auto put = [&](const uint8_t* file, uint64_t s, uint64_t e, uint64_t id) {
             format_line(o, file, c->pat_len, s, e, chunk);
-            const int k = snprintf(num, sizeof num, "%llu\n", (unsigned long long)c->r_ids[i]);
-            ix.insert(ix.end(), num, num + k);
+            char* end = std::to_chars(num, num + sizeof num, id).ptr;
+            *end++ = '\n';
+            ix.insert(ix.end(), num, end);
+        };
+        bool gathered = false;
+        if (cnt && c->h_pat.empty() && c->pat_len > (256u << 10) && 4 * cnt < c->npat) {
+            std::vector<uint64_t> spans(2 * cnt), at(cnt + 1, 0);
+            std::vector<uint8_t> bytes;
+            TRY(gather_pruned(c, spans, bytes, at, &gathered));
+            for (uint64_t i = 0; i < cnt && gathered; i++) {
+                // format_line addresses the line by its place in the file
+                const uint8_t* file = reinterpret_cast<const uint8_t*>((uintptr_t)bytes.data() + at[i] - spans[2 * i]);
+                put(file, spans[2 * i], spans[2 * i + 1], c->r_ids[i]);
+            }
+        }
+        if (cnt && !gathered) {
+            TRY(host_patterns(c));
+            const uint8_t* f = c->h_pat.data();
+            uint64_t line = 0, pos = 0;
+            auto line_end = [&] {
+                const void* nl = memchr(f + pos, '\n', c->pat_len - pos);
+                return nl ? (uint64_t)((const uint8_t*)nl - f) : c->pat_len;
+            };
+            for (uint64_t id : c->r_ids) {  // ascending
+                for (; line < id; line++) pos = line_end() + 1;
+                const uint64_t e = line_end();
+                put(f, pos, e, id);
+                pos = e + 1;
+                line++;
+            }
         }
     } catch (...) {
         return fail(c, FFBF_ENOMEM_HOST, "out of host memory for the pruned patterns");

@@ -72,7 +72,8 @@ struct ffbf_ctx {
 
     // patterns
     bool have_patterns = false;
-    uint64_t pat_len = 0;  // bytes of the pattern file, whose only copy is on the device
+    uint64_t pat_len = 0;  // bytes of the pattern file, which is kept on the device
+    std::vector<uint8_t, NoInit<uint8_t>> h_pat;  // and here once a call has needed it whole (host_patterns)
     uint8_t* d_pat = nullptr;
     uint64_t npat = 0;
     uint64_t* d_pstart = nullptr;
