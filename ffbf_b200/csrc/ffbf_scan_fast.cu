@@ -115,6 +115,12 @@ __device__ __forceinline__ void tma_load_3d_hint(uint32_t dst, const CUtensorMap
         : "memory");
 }
 
+// Before a thread's first load through a tensor map that a host copy has written to global memory: the map may still be
+// cached as it was for an earlier launch, with another text or another box.
+__device__ __forceinline__ void acquire_map(const CUtensorMap* map) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
+
 // An untiled copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) completed on an mbarrier.
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -646,7 +652,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
     __shared__ int s_abort;
     __shared__ uint32_t s_ni, s_nj;
     __shared__ JobState s_job;
-    __shared__ int s_nr;
+    __shared__ int s_nr, s_map;  // s_map: the job whose tensor map thread 0 has acquired
     __shared__ uint64_t s_wpos[THREADS / 32];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -668,6 +674,10 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         }
         while (nj + 1 < n_jobs && __ldg(&jobs[nj + 1].item_begin) <= ni) nj++;
         const FastJob* J = jobs + nj;
+        if (s_map != (int)nj) {
+            acquire_map(&J->tmap);
+            s_map = (int)nj;
+        }
         const uint32_t R = __ldg(&J->rows);
         const uint32_t st = ni - __ldg(&J->item_begin);
         const int y = nr < 0 ? (int)R - 1 : nr / kParts;
@@ -705,6 +715,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(THREADS, MODE)) k_scan_fa
         s_ni = blockIdx.x;
         s_nj = 0;
         s_nr = -1;
+        s_map = -1;
         for (uint32_t b = 0; b < 2; b++) {
             mbar_init(fbar(b), 1);
             mbar_init(ebar(b), THREADS / 32);
