@@ -197,6 +197,13 @@ size_t scan_smem_bytes(int cache_in_smem, const Geom& g) {
     return b;
 }
 
+// k_scan_generic's limit for any cache region, as the limit is the function's and threads may launch with different ones.
+static int generic_smem_limit() {
+    Geom g{};
+    g.cache_bits = kSmemCacheMaxBits;
+    return (int)scan_smem_bytes(1, g);
+}
+
 // One 16 KiB tile of the generic scan (window ends [tile*T, tile*T + T)). The caller provides the shared
 // S-box copy, the tile newline accumulator, the padded staging buffer and the cache-region words to probe
 // (shared-memory copy or the global filter).
@@ -350,7 +357,8 @@ cudaError_t gather_counters(uint32_t* const* d_ptrs, uint32_t n, uint32_t* d_out
 
 int scan_generic_grid(const Geom& g, int cache_in_smem, uint64_t ntiles) {
     size_t smem = scan_smem_bytes(cache_in_smem, g);
-    if (cudaFuncSetAttribute(k_scan_generic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_scan_generic, cudaFuncAttributeMaxDynamicSharedMemorySize, generic_smem_limit()) !=
+        cudaSuccess)
         return 0;
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
@@ -362,7 +370,7 @@ int scan_generic_grid(const Geom& g, int cache_in_smem, uint64_t ntiles) {
 
 cudaError_t scan_generic(const ScanArgs& a, int grid, cudaStream_t st) {
     size_t smem = scan_smem_bytes(a.cache_in_smem, a.g);
-    cudaError_t e = cudaFuncSetAttribute(k_scan_generic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_scan_generic, cudaFuncAttributeMaxDynamicSharedMemorySize, generic_smem_limit());
     if (e != cudaSuccess) return e;
     if (!a.ntiles) return cudaSuccess;
     k_scan_generic<<<grid, kScanThreads, smem, st>>>(a);

@@ -1061,8 +1061,9 @@ cudaError_t launch_cfg(uint32_t len, const FastJob* d_jobs, uint32_t n_jobs, uin
                        uint32_t* d_ctl, int num_sms, cudaStream_t st) {
     const size_t smem =
         fixed_smem(THREADS, tab_bytes(MODE, L)) + (sparse_mode(MODE) || MODE >= 3 ? 4 * (size_t)max_s1_words : 0);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_scan_fast<L, THREADS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit is the function's, not the launch's: one value, so that threads launching with different tables agree
+    cudaError_t e = cudaFuncSetAttribute(k_scan_fast<L, THREADS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(kSmemLimit - static_smem(THREADS)));
     if (e != cudaSuccess) return e;
     const uint32_t slots = (uint32_t)num_sms * (uint32_t)ctas_per_sm(THREADS, MODE);
     const int grid = (int)(n_items < slots ? n_items : slots);
