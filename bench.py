@@ -495,8 +495,7 @@ def run_batched(args, local):
         "autotune_classes": n_classes,
         "configs": dict(collections.Counter(
             (f"dense-{f.config()[0]}-order{f.probe_order()}" if f.config()[1] == 1 else
-             f"sparse-deferred-{f.config()[0]}" if f.config()[1] == 2 else
-             f"sparse-staged-{f.config()[0]}" if f.config()[1] == 3 else f"sparse-{f.config()[0]}")
+             f"sparse-fitted-{f.config()[0]}" if f.config()[1] == 3 else f"sparse-{f.config()[0]}")
             for f in filters)),
         "timing": "host clock between device-idle points, median of steps; batched_device = CUDA events",
         "lone_jobs_without_gaps": ideal,
@@ -887,7 +886,7 @@ def run_leg(workload, args):
         cmd.append("--no-cpu-baseline")
     p = subprocess.run(cmd, capture_output=True, text=True, env=dict(os.environ, WORLD_SIZE="1", RANK="0"))
     if p.returncode != 0:
-        return {"error": f"exit {p.returncode}: {p.stderr.strip().splitlines()[-1] if p.stderr.strip() else ''}"}
+        return {"error": f"exit {p.returncode}: " + " | ".join(p.stderr.strip().splitlines()[-8:])[-1500:]}
     d = json.loads(p.stdout.strip().splitlines()[-1])
     if workload in d:
         return dict(d[workload], clocks=d.get("clocks"))
