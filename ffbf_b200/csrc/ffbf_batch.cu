@@ -289,7 +289,7 @@ const char* ffbf_batch_last_error(const ffbf_batch* b) { return b ? b->err.c_str
 
 void* ffbf_batch_stream(ffbf_batch* b) { return b ? (void*)b->st : nullptr; }
 
-ffbf_status ffbf_batch_add(ffbf_batch* b, ffbf_ctx* c, const uint8_t* d_text, size_t len) {
+ffbf_status ffbf_batch_add(ffbf_batch* b, ffbf_ctx* c, const uint8_t* d_text, size_t len) try {
     if (!b || !c) return FFBF_EINVAL;
     if (c->device != b->device) return bfail(b, FFBF_EINVAL, "context and batch are on different devices");
     if (((uintptr_t)d_text & 15) != 0 || (!d_text && len)) return bfail(b, FFBF_EINVAL, "device text must be 16-byte aligned");
@@ -298,9 +298,11 @@ ffbf_status ffbf_batch_add(ffbf_batch* b, ffbf_ctx* c, const uint8_t* d_text, si
     if (b->prepared) batch_release(b);
     b->jobs.push_back({c, d_text, len});
     return FFBF_OK;
+} catch (...) {
+    return FFBF_ENOMEM_HOST;
 }
 
-ffbf_status ffbf_batch_prepare(ffbf_batch* b) {
+ffbf_status ffbf_batch_prepare(ffbf_batch* b) try {
     NvtxRange nvtx_("ffbf_batch_prepare");
     if (!b) return FFBF_EINVAL;
     if (cudaSetDevice(b->device) != cudaSuccess) return bfail(b, FFBF_ECUDA, "cudaSetDevice failed");
@@ -396,9 +398,11 @@ ffbf_status ffbf_batch_prepare(ffbf_batch* b) {
     }
     b->prepared = true;
     return FFBF_OK;
+} catch (...) {
+    return FFBF_ENOMEM_HOST;
 }
 
-ffbf_status ffbf_batch_launch(ffbf_batch* b) {
+ffbf_status ffbf_batch_launch(ffbf_batch* b) try {
     NvtxRange nvtx_("ffbf_batch_launch");
     if (!b) return FFBF_EINVAL;
     bool stale = !b->prepared || b->keys.size() != b->jobs.size();
@@ -434,6 +438,8 @@ ffbf_status ffbf_batch_launch(ffbf_batch* b) {
     ffbf::note_launches(b->graph_kernels);
     b->uncollected = true;
     return FFBF_OK;
+} catch (...) {
+    return FFBF_ENOMEM_HOST;
 }
 
 ffbf_status ffbf_batch_wait(ffbf_batch* b) {
@@ -477,7 +483,7 @@ ffbf_status ffbf_batch_wait(ffbf_batch* b) {
     return FFBF_OK;
 }
 
-ffbf_status ffbf_batch_autotune(ffbf_batch* b, size_t sample_bytes, uint32_t* n_classes) {
+ffbf_status ffbf_batch_autotune(ffbf_batch* b, size_t sample_bytes, uint32_t* n_classes) try {
     NvtxRange nvtx_("ffbf_batch_autotune");
     if (!b) return FFBF_EINVAL;
     if (n_classes) *n_classes = 0;
@@ -519,6 +525,8 @@ ffbf_status ffbf_batch_autotune(ffbf_batch* b, size_t sample_bytes, uint32_t* n_
     if (n_classes) *n_classes = (uint32_t)classes.size();
     batch_release(b);  // the next launch prepares with the tuned configurations
     return FFBF_OK;
+} catch (...) {
+    return FFBF_ENOMEM_HOST;
 }
 
 }  // extern "C"

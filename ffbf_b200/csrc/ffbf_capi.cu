@@ -44,6 +44,9 @@ ffbf_status fail(ffbf_ctx* c, ffbf_status s, const char* fmt, ...) {
 }
 
 
+// What an entry point returns when a host allocation throws; the message fits a string without one.
+ffbf_status no_host_memory(ffbf_ctx* c) { return fail(c, FFBF_ENOMEM_HOST, "no host memory"); }
+
 ffbf_status dalloc(ffbf_ctx* c, void** p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
@@ -779,19 +782,21 @@ ffbf_status ffbf_save_filter(ffbf_ctx* c, uint8_t** data, size_t* len) {
     return FFBF_OK;
 }
 
-ffbf_status ffbf_load_filter_file(ffbf_ctx* c, const char* path) {
+ffbf_status ffbf_load_filter_file(ffbf_ctx* c, const char* path) try {
     if (!c) return FFBF_EINVAL;
     if (!path) return fail(c, FFBF_EINVAL, "path is NULL");
-    FILE* f = fopen(path, "rb");
+    std::unique_ptr<FILE, int (*)(FILE*)> f(fopen(path, "rb"), fclose);
     if (!f) return fail(c, FFBF_EIO, "cannot open %s", path);
     std::vector<uint8_t> buf;
     uint8_t tmp[1 << 16];
     size_t r;
-    while ((r = fread(tmp, 1, sizeof tmp, f)) > 0) buf.insert(buf.end(), tmp, tmp + r);
-    bool bad = ferror(f);
-    fclose(f);
+    while ((r = fread(tmp, 1, sizeof tmp, f.get())) > 0) buf.insert(buf.end(), tmp, tmp + r);
+    const bool bad = ferror(f.get());
+    f.reset();
     if (bad) return fail(c, FFBF_EIO, "error while reading the filter file %s", path);
     return ffbf_load_filter(c, buf.data(), buf.size());
+} catch (...) {
+    return no_host_memory(c);
 }
 
 ffbf_status ffbf_save_filter_file(ffbf_ctx* c, const char* path) {
@@ -812,16 +817,18 @@ ffbf_status ffbf_save_filter_file(ffbf_ctx* c, const char* path) {
     return FFBF_OK;
 }
 
-ffbf_status ffbf_scan_device(ffbf_ctx* c, const uint8_t* d_text, size_t len) {
+ffbf_status ffbf_scan_device(ffbf_ctx* c, const uint8_t* d_text, size_t len) try {
     NvtxRange nvtx_("ffbf_scan_device");
     TRY(enter(c));
     TRY(setup_scan_state(c, d_text, len));
     TRY(launch_scan(c));
     c->scan_pending = true;
     return FFBF_OK;
+} catch (...) {
+    return no_host_memory(c);
 }
 
-ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
+ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) try {
     NvtxRange nvtx_("ffbf_scan_collect");
     TRY(enter(c));
     if (!c->scan_pending && !c->have_scan) return fail(c, FFBF_ESTATE, "no scan to collect");
@@ -929,6 +936,8 @@ ffbf_status ffbf_scan_collect(ffbf_ctx* c, ffbf_scan_result* out) {
         out->line_end = c->r_le.data();
     }
     return FFBF_OK;
+} catch (...) {
+    return no_host_memory(c);
 }
 
 }  // extern "C"
@@ -1065,7 +1074,7 @@ ffbf_status segment_size(ffbf_ctx* c, uint64_t len, uint64_t* seg) {
 
 extern "C" {
 
-ffbf_status ffbf_scan(ffbf_ctx* c, const uint8_t* text, size_t len, ffbf_scan_result* out) {
+ffbf_status ffbf_scan(ffbf_ctx* c, const uint8_t* text, size_t len, ffbf_scan_result* out) try {
     NvtxRange nvtx_("ffbf_scan");
     TRY(enter(c));
     if (!text && len) return fail(c, FFBF_EINVAL, "text is NULL");
@@ -1129,10 +1138,13 @@ ffbf_status ffbf_scan(ffbf_ctx* c, const uint8_t* text, size_t len, ffbf_scan_re
         out->line_end = c->r_le.data();
     }
     return FFBF_OK;
+} catch (...) {
+    c->keep_records = false;
+    return no_host_memory(c);
 }
 
 ffbf_status ffbf_format_lines(ffbf_ctx* c, const uint8_t* text, size_t len, size_t chunk, uint8_t** out,
-                              size_t* out_len) {
+                              size_t* out_len) try {
     if (!c) return FFBF_EINVAL;
     if (!out || !out_len || (!text && len)) return fail(c, FFBF_EINVAL, "NULL argument");
     if (!c->have_scan) return fail(c, FFBF_ESTATE, "ffbf_format_lines needs a collected scan");
@@ -1141,6 +1153,8 @@ ffbf_status ffbf_format_lines(ffbf_ctx* c, const uint8_t* text, size_t len, size
     std::vector<uint8_t> v;
     for (size_t i = 0; i < c->r_ls.size(); i++) format_line(v, text, len, c->r_ls[i], c->r_le[i], chunk);
     return to_host_buffer(c, v, out, out_len);
+} catch (...) {
+    return no_host_memory(c);
 }
 
 ffbf_status ffbf_format_spans(const uint8_t* buf, size_t len, const uint64_t* start, const uint64_t* end, size_t n,
@@ -1160,13 +1174,14 @@ ffbf_status ffbf_format_spans(const uint8_t* buf, size_t len, const uint64_t* st
     return to_host_buffer(nullptr, v, out, out_len);
 }
 
-ffbf_status ffbf_prune(ffbf_ctx* c, ffbf_prune_result* out) {
+ffbf_status ffbf_prune(ffbf_ctx* c, ffbf_prune_result* out) try {
     NvtxRange nvtx_("ffbf_prune");
     TRY(enter(c));
     if (!c->have_patterns) return fail(c, FFBF_ESTATE, "ffbf_prune needs ffbf_set_patterns first");
     if (c->scan_pending) TRY(ffbf_scan_collect(c, nullptr));
     const uint64_t n = c->npat;
     uint64_t cnt = 0;
+    c->have_prune = false;
     if (n) {
         TRY(ensure_tmp(c, ffbf::prune_blocks(n)));
         uint32_t* counts = reinterpret_cast<uint32_t*>(c->d_tmp);
@@ -1215,6 +1230,8 @@ ffbf_status ffbf_prune(ffbf_ctx* c, ffbf_prune_result* out) {
         out->ids = c->r_ids.data();
     }
     return FFBF_OK;
+} catch (...) {
+    return no_host_memory(c);
 }
 
 }  // extern "C"
@@ -1386,7 +1403,7 @@ ffbf_status verify_pass(ffbf_ctx* c, uint32_t nh, const uint8_t* d_text, uint64_
 
 extern "C" {
 
-ffbf_status ffbf_verify(ffbf_ctx* c, ffbf_matches* out) {
+ffbf_status ffbf_verify(ffbf_ctx* c, ffbf_matches* out) try {
     NvtxRange nvtx_("ffbf_verify");
     TRY(enter(c));
     if (c->scan_pending) TRY(ffbf_scan_collect(c, nullptr));
@@ -1440,6 +1457,8 @@ ffbf_status ffbf_verify(ffbf_ctx* c, ffbf_matches* out) {
         out->pattern_ids = c->r_mpid.data();
     }
     return FFBF_OK;
+} catch (...) {
+    return no_host_memory(c);
 }
 
 ffbf_status ffbf_test_line(ffbf_ctx* c, const uint8_t* line, size_t len, int* hit) {

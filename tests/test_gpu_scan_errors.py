@@ -10,13 +10,13 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-def build_cpp(name, tmp_path):
-    """Builds tests/cpp/<name>.cu against libffbf.so and its internal headers; returns the program's path."""
+def build_cpp(name, tmp_path, suffix=".cu"):
+    """Builds tests/cpp/<name><suffix> against libffbf.so and its internal headers; returns the program's path."""
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     exe = str(tmp_path / name)
     lib = os.path.join(ROOT, "ffbf_b200", "_lib")
     subprocess.run([nvcc, "-std=c++17", "-O2", f"-I{os.path.join(ROOT, 'include')}",
-                    f"-I{os.path.join(ROOT, 'ffbf_b200', 'csrc')}", os.path.join(ROOT, "tests", "cpp", name + ".cu"),
+                    f"-I{os.path.join(ROOT, 'ffbf_b200', 'csrc')}", os.path.join(ROOT, "tests", "cpp", name + suffix),
                     "-o", exe, f"-L{lib}", "-lffbf", f"-Xlinker=-rpath,{lib}", "-lcuda"], check=True)
     return exe
 
